@@ -1126,12 +1126,6 @@ int cadmas_create(const cadmas_dims *d, const cadmas_params *p, cadmas_handle **
   h->q.ntx = (d->numi - 2 + TI - 1) / TI;
   h->q.nb = h->q.ntx * ((d->numj - 2 + TJl - 1) / TJl);
   h->q.occ = (p->sweep_occupancy == 1 || p->sweep_occupancy == 2 || p->sweep_occupancy == 4) ? p->sweep_occupancy : 0;
-  h->q.nsm = 148;
-  {
-    int nsm = 0;
-    if (cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, h->device) == cudaSuccess && nsm > 0)
-      h->q.nsm = nsm;
-  }
   if (!sweep_supported(h->q)) {
     g_last_error = "preconditioner block too large for the MILU sweeps; set precond_ti/precond_tj";
     rc = CADMAS_EUNSUPPORTED;
@@ -1999,7 +1993,7 @@ int cadmas_step_ensemble(cadmas_handle **hs, int n, const double *dt, int *statu
 // solve run per grid on the grid's own stream and host thread.
 struct cadmas_batch {
   std::vector<cadmas_handle *> h;
-  int device = 0, nsm = 148, occ = 0;
+  int device = 0;
   cudaStream_t s = nullptr;
   BatchMember *d_m = nullptr, *h_m = nullptr;  // member table (device, pinned host)
   int *d_pre = nullptr;                          // block prefixes (BR_N x (n+1))
@@ -2064,10 +2058,10 @@ static void solve_mixed_batch(cadmas_batch *b, const std::vector<int> &idx, std:
   pre[BR_TILE * (nm + 1) + nm] = (int)ntiles;
   pre[BR_SLAB * (nm + 1) + nm] = (int)nslab;
   pre[BR_ELEM * (nm + 1) + nm] = (int)nelem;
-  const SkewGeo qref = hs[0]->q;
+  SkewGeo qref = hs[0]->q;
+  for (int j = 0; j < nm; ++j) qref.ring |= hs[j]->q.ring;
   const BatchMember *bm = b->d_m;
   const int *dp = b->d_pre;
-  const int nsm = b->nsm, occ = b->occ;
   auto upload = [&]() -> bool {
     return cudaMemcpyAsync(b->d_m, b->h_m, (size_t)nm * sizeof(BatchMember), cudaMemcpyHostToDevice, s) ==
            cudaSuccess;
@@ -2121,8 +2115,8 @@ static void solve_mixed_batch(cadmas_batch *b, const std::vector<int> &idx, std:
     // the inner FP32 solve of every member refining (solve_inner_f)
     launch_b_start_f(s, bm, dp, nm, nslab);
     launch_b_clear(s, bm, nm);
-    bool ok = launch_b_sweep(s, SWEEP_FWD, bm, dp, nm, ntiles, qref, BF_B, -1, -1, false, nsm, occ) &&
-              launch_b_sweep(s, SWEEP_BWD, bm, dp, nm, ntiles, qref, -1, BF_R0, -1, false, nsm, occ);
+    bool ok = launch_b_sweep(s, SWEEP_FWD, bm, dp, nm, ntiles, qref, BF_B, -1, -1, false) &&
+              launch_b_sweep(s, SWEEP_BWD, bm, dp, nm, ntiles, qref, -1, BF_R0, -1, false);
     launch_b_dot_r0f(s, bm, dp, nm, nslab);
     launch_b_fin(s, FIN_BNORM, bm, nm, false);
     launch_b_fin(s, FIN_START, bm, nm, false);
@@ -2132,12 +2126,12 @@ static void solve_mixed_batch(cadmas_batch *b, const std::vector<int> &idx, std:
     int batch = std::max(2, std::min(last, 64));
     for (int guard = 0; guard < 100000 && ok; ++guard) {
       for (int k = 0; k < batch && ok; ++k) {
-        ok = launch_b_sweep(s, SWEEP_FWD_AX, bm, dp, nm, ntiles, qref, BF_PV, -1, -1, false, nsm, occ) &&
-             launch_b_sweep(s, SWEEP_BWD1, bm, dp, nm, ntiles, qref, BF_R0, BF_AP, -1, false, nsm, occ);
+        ok = launch_b_sweep(s, SWEEP_FWD_AX, bm, dp, nm, ntiles, qref, BF_PV, -1, -1, false) &&
+             launch_b_sweep(s, SWEEP_BWD1, bm, dp, nm, ntiles, qref, BF_R0, BF_AP, -1, false);
         launch_b_fin(s, FIN_ALPHA, bm, nm, true);
         launch_b_axpyf(s, bm, dp, nm, nslab);
-        ok = ok && launch_b_sweep(s, SWEEP_FWD_AX, bm, dp, nm, ntiles, qref, BF_RR, -1, -1, false, nsm, occ) &&
-             launch_b_sweep(s, SWEEP_BWD5, bm, dp, nm, ntiles, qref, BF_R0, BF_AE, BF_RR, true, nsm, occ);
+        ok = ok && launch_b_sweep(s, SWEEP_FWD_AX, bm, dp, nm, ntiles, qref, BF_RR, -1, -1, false) &&
+             launch_b_sweep(s, SWEEP_BWD5, bm, dp, nm, ntiles, qref, BF_R0, BF_AE, BF_RR, true);
         launch_b_fin5(s, bm, nm);
         launch_b_upd3f(s, bm, dp, nm, nslab);
         launch_b_commit(s, bm, nm);
@@ -2195,7 +2189,6 @@ static void solve_mixed_batch(cadmas_batch *b, const std::vector<int> &idx, std:
 int cadmas_batch_create(cadmas_handle **hs, int n, cadmas_batch **out) {
   if (!hs || !out || n < 1) return CADMAS_EINVAL;
   *out = nullptr;
-  long long ntiles = 0;
   for (int i = 0; i < n; ++i) {
     cadmas_handle *h = hs[i];
     if (!h) return CADMAS_EINVAL;
@@ -2210,14 +2203,11 @@ int cadmas_batch_create(cadmas_handle **hs, int n, cadmas_batch **out) {
     }
     for (int j = 0; j < i; ++j)
       if (hs[j] == h) { g_last_error = "a handle twice in a batch"; return CADMAS_EINVAL; }
-    ntiles += h->q.nb;
   }
   cadmas_batch *b = new cadmas_batch();
   b->h.assign(hs, hs + n);
   b->device = hs[0]->device;
-  b->nsm = hs[0]->q.nsm;
-  b->occ = hs[0]->q.occ;
-  if (!b_sweeps_supported(hs[0]->q, b->nsm, b->occ, ntiles)) {
+  if (!b_sweeps_supported(hs[0]->q)) {
     delete b;
     g_last_error = "preconditioner block too large for the batched FP32 sweeps";
     return CADMAS_EUNSUPPORTED;
@@ -2352,6 +2342,7 @@ int cadmas_test_stall_sweeps(cadmas_handle *h, int from_step) {
   const int v = from_step >= 0 ? from_step : (1 << 30);
   CK(cudaMemcpyAsync(&h->st->stall_from, &v, sizeof(int), cudaMemcpyHostToDevice, h->s));
   CK(cudaStreamSynchronize(h->s));
+  h->q.ring = from_step >= 0 ? 1 : 0;  // the form whose copies stall
   return CADMAS_OK;
 }
 

@@ -23,6 +23,7 @@
 #include <mutex>
 #include "cadmas_dev.cuh"
 #include "kernels.h"
+#include "sweep_cp.cuh"
 #include <algorithm>
 
 namespace cadmas {
@@ -220,6 +221,15 @@ __device__ __forceinline__ long long sl_index(const SkewGeo &q, int b, int w, in
   return ((long long)b * q.W + w) * q.T + t;
 }
 
+// Store the coefficients AD, ALI, ALJ, ALK, AUI, AUJ, AUK of column t of a
+// slab as chunks, DD = 0.
+__device__ __forceinline__ void sys_put(double *sys, long long slab, int T, int t, const double *v) {
+  const double e[8] = {v[4], v[5], v[6], 0.0, v[1], v[2], v[3], v[0]};
+#pragma unroll
+  for (int c = 0; c < 4; ++c)
+    *reinterpret_cast<double2 *>(sys + sys_chunk<double>(slab, c, T, t)) = make_double2(e[2 * c], e[2 * c + 1]);
+}
+
 // Copy the Poisson system (7 coefficients, interleaved per slab; DD set to
 // 0 for MZDCMP to fill), INDC, BB and X0 into the skewed layout.  Entries
 // outside the tile or the interior get 0 (INDC -1).  warm: keep the
@@ -244,11 +254,8 @@ __device__ __forceinline__ void to_skew_elem(const Geo &g, const SkewGeo &q, con
       bv = A_.bb[c];
       xv = warm ? (ic != -1 ? xsl[e] : 0.0) : X0[c];
     }
-    constexpr int cs[7] = {SYS_AD, SYS_ALI, SYS_ALJ, SYS_ALK, SYS_AUI, SYS_AUJ, SYS_AUK};
-#pragma unroll
-    for (int c = 0; c < 7; ++c) S.sys[sys_at(bw, cs[c], q.T, t)] = v[c];
-    S.sys[sys_at(bw, SYS_DD, q.T, t)] = 0.0;
-    S.sys[sys_at(bw, SYS_T, q.T, t)] = 0.0;
+    sys_put(S.sys, bw, q.T, t, v);
+    S.sys[sys_t(bw, q.T, t)] = 0.0;
     S.indc[e] = ic;
     bsl[e] = bv;
     xsl[e] = xv;
@@ -263,13 +270,14 @@ __global__ void k_to_skew(Geo g, SkewGeo q, SysPtr A_, const int *INDC, SkewSys 
 }
 
 // The same conversion, one block per row tj of a layout tile b: the row's
-// interior cells of all layers, (NK-2) x TI values of one array at a time,
-// are staged in shared memory with coalesced loads and then written slab
-// by slab (TIp consecutive entries of a slab per row).  Same values as
-// to_skew_elem; used when a panel fits in shared memory.
+// interior cells of all layers, (NK-2) x TI values of two arrays at a
+// time, are staged in shared memory with coalesced loads and then written
+// slab by slab (TIp consecutive entries of a slab per row): the two arrays
+// of a chunk of the system together, then BB with X0 (or, warm, BB alone).
+// Same values as to_skew_elem; used when two panels fit in shared memory.
 __global__ void k_to_skew_rows(Geo g, SkewGeo q, SysPtr A_, const int *INDC, SkewSys S, const double *X0,
                                double *bsl, double *xsl, int warm) {
-  extern __shared__ __align__(16) double pan[];  // [(NK-2) * TI]
+  extern __shared__ __align__(16) double pan[];  // [2][(NK-2) * TI]
   pdl_enter();
   const int b = blockIdx.x / q.TJ, tj = blockIdx.x % q.TJ;
   const int TI = q.TI, TIp = q.TIp, T = q.T, W = q.W, nk = g.NK - 2;
@@ -278,7 +286,7 @@ __global__ void k_to_skew_rows(Geo g, SkewGeo q, SysPtr A_, const int *INDC, Ske
   const int npan = nk * TI, nent = W * TIp;
   const long long slab0 = (long long)b * W;
   int *ipan = reinterpret_cast<int *>(pan);
-  // INDC, then DD = T = 0, INDC and the warm guess
+  // INDC, then T = 0, INDC and the warm guess
 #pragma unroll 4
   for (int x = threadIdx.x; x < npan; x += blockDim.x) {
     const int k = 2 + x / TI, ti = x % TI;
@@ -290,36 +298,40 @@ __global__ void k_to_skew_rows(Geo g, SkewGeo q, SysPtr A_, const int *INDC, Ske
     const int ic = (ti < TI && k >= 2 && k <= g.NK - 1) ? ipan[(k - 2) * TI + ti] : -1;
     const long long e = (slab0 + w) * T + t;
     S.indc[e] = ic;
-    S.sys[sys_at(slab0 + w, SYS_DD, T, t)] = 0.0;
-    S.sys[sys_at(slab0 + w, SYS_T, T, t)] = 0.0;
+    S.sys[sys_t(slab0 + w, T, t)] = 0.0;
     if (warm) xsl[e] = ic != -1 ? xsl[e] : 0.0;
   }
-  // AD, ALI, ALJ, ALK, AUI, AUJ, AUK, BB and (not warm) X0
-  const double *src[9] = {A_.ad, A_.ali, A_.alj, A_.alk, A_.aui, A_.auj, A_.auk, A_.bb, X0};
-  constexpr int cs[7] = {SYS_AD, SYS_ALI, SYS_ALJ, SYS_ALK, SYS_AUI, SYS_AUJ, SYS_AUK};
-  const int na = warm ? 8 : 9;
+  // chunks {AUI,AUJ}, {AUK,DD = 0}, {ALI,ALJ}, {ALK,AD}; BB and X0
+  const double *src[10] = {A_.aui, A_.auj, A_.auk, nullptr, A_.ali, A_.alj, A_.alk, A_.ad, A_.bb, warm ? nullptr : X0};
 #pragma unroll 1
-  for (int a = 0; a < na; ++a) {
+  for (int a = 0; a < 5; ++a) {
     __syncthreads();
-    const double *sa = src[a];
+    const double *s0 = src[2 * a], *s1 = src[2 * a + 1];
 #pragma unroll 4
     for (int x = threadIdx.x; x < npan; x += blockDim.x) {
       const int k = 2 + x / TI, ti = x % TI;
-      pan[x] = ti < wi ? sa[cid(g, is + ti, J, k)] : 0.0;
+      const long long c = cid(g, is + ti, J, k);
+      pan[x] = ti < wi ? s0[c] : 0.0;
+      pan[npan + x] = ti < wi && s1 ? s1[c] : 0.0;
     }
     __syncthreads();
     for (int x = threadIdx.x; x < nent; x += blockDim.x) {
       const int w = x / TIp, ti = x % TIp, k = 2 + w - ti - tj, t = ti + TIp * tj;
-      const double v = (ti < TI && k >= 2 && k <= g.NK - 1) ? pan[(k - 2) * TI + ti] : 0.0;
-      if (a < 7) S.sys[sys_at(slab0 + w, cs[a], T, t)] = v;
-      else if (a == 7) bsl[(slab0 + w) * T + t] = v;
-      else xsl[(slab0 + w) * T + t] = v;
+      const bool in = ti < TI && k >= 2 && k <= g.NK - 1;
+      const int p = in ? (k - 2) * TI + ti : 0;
+      const double v0 = in ? pan[p] : 0.0, v1 = in ? pan[npan + p] : 0.0;
+      if (a < 4) {
+        *reinterpret_cast<double2 *>(S.sys + sys_chunk<double>(slab0 + w, a, T, t)) = make_double2(v0, v1);
+      } else {
+        bsl[(slab0 + w) * T + t] = v0;
+        if (!warm) xsl[(slab0 + w) * T + t] = v1;
+      }
     }
   }
 }
-// Shared memory of k_to_skew_rows (0: the panel does not fit, k_to_skew).
+// Shared memory of k_to_skew_rows (0: the panels do not fit, k_to_skew).
 static size_t to_skew_rows_bytes(const Geo &g, const SkewGeo &q) {
-  const size_t b = (size_t)(g.NK - 2) * q.TI * sizeof(double);
+  const size_t b = 2 * (size_t)(g.NK - 2) * q.TI * sizeof(double);
   return b <= 64 * 1024 ? b : 0;
 }
 
@@ -374,11 +386,10 @@ __device__ __forceinline__ void dcmp_body(const Geo &g, const SkewGeo &q, V U, c
     const int k = 2 + s - ti - tj;
     if (valid && k >= 2 && k <= g.NK - 1) {
       const long long slab = slab0 + s, e = slab * Tl + tl;
-      const V *sy = S.sys + sys_at(slab, 0, Tl, tl);
       const int sl = s % R;
       constexpr int cs[7] = {SYS_AD, SYS_ALI, SYS_ALJ, SYS_ALK, SYS_AUI, SYS_AUJ, SYS_AUK};
 #pragma unroll
-      for (int c = 0; c < 7; ++c) cp_async_v(&rg.v(sl, c, tid), sy + (long long)cs[c] * Tl);
+      for (int c = 0; c < 7; ++c) cp_async_v(&rg.v(sl, c, tid), S.sys + sys_at<V>(slab, cs[c], Tl, tl));
       cp_async4(&rg.ind(sl, tid), S.indc + e);
     }
     cp_commit();
@@ -415,7 +426,7 @@ __device__ __forceinline__ void dcmp_body(const Geo &g, const SkewGeo &q, V U, c
                     rg.v(sl, 3, tid) * dk1 * au3);
         if (dd <= z) bad = true;
       }
-      S.sys[sys_at(slab0 + s, SYS_DD, Tl, tl)] = dd;
+      S.sys[sys_at<V>(slab0 + s, SYS_DD, Tl, tl)] = dd;
       rg.xb[cur * T + tid] = dd;
       dk1 = dd;
       au3 = rg.v(sl, 6, tid) + U * (rg.v(sl, 4, tid) + rg.v(sl, 5, tid));
@@ -572,20 +583,12 @@ __device__ __forceinline__ void cluster_barrier() {
 // and their evaluation order are those of the reference loops, so the
 // results do not change.  The step loop is unrolled by the ring length so
 // slot addresses and mbarrier phases are constants.
-// CT, CTIP: the layout tile's T and TIp at compile time (0: from q), so
-// that the slot offsets of a common tile shape are immediates and take no
-// registers.
-template <int D, int MODE, typename V, int CS, int CT = 0, int CTIP = 0>
-__device__ __forceinline__ void sweep_body(const Geo &g, const SkewGeo &q_, const SkewSysT<V> &S, const V *vin,
-                                           V *vout, SolveState *st, const V *vin2, double *rb, int bx, int by) {
+template <int MODE, typename V, int CS>
+__device__ __forceinline__ void sweep_body(const Geo &g, const SkewGeo &q, const SkewSysT<V> &S, const V *vin,
+                                           V *vout, SolveState *st, const V *vin2, double *rb, int bx, int by,
+                                           const int D) {
   constexpr bool BWD = MODE >= SWEEP_BWD;
   constexpr int NDOT = sweep_ndot(MODE);
-  SkewGeo q = q_;
-  if (CT > 0) {
-    q.T = CT;
-    q.TIp = CTIP;
-    q.TJ = CT / (CTIP > 0 ? CTIP : 1);
-  }
   // CS = 2: the thread blocks of a cluster are the two layout tiles of one
   // preconditioner block; every block of a cluster runs through the two
   // cluster barriers below, so none returns early.
@@ -596,18 +599,16 @@ __device__ __forceinline__ void sweep_body(const Geo &g, const SkewGeo &q_, cons
     cluster_barrier();
     return;
   }
-  constexpr int R = D + 2;
+  const int R = D + 2;
   constexpr int AHEAD = (MODE == SWEEP_FWD_AX) ? 2 : 1;  // preparing step s+1 reads the slot of step s+AHEAD
   extern __shared__ __align__(16) double sm[];
   const int T = q.T, TIp = q.TIp;
   const int Tc = (T + 31) & ~31;
   constexpr int ES = (int)sizeof(V);
   const int SS = sweep_slot(q, MODE, ES);
-  // slot offsets of the system arrays
-  constexpr int SF = sweep_sys_first(MODE) - sweep_sys_dst(MODE);
-  const int oDD = (SYS_DD - SF) * T, oAD = (SYS_AD - SF) * T, oALI = (SYS_ALI - SF) * T,
-            oALJ = (SYS_ALJ - SF) * T, oALK = (SYS_ALK - SF) * T, oAUI = (SYS_AUI - SF) * T,
-            oAUJ = (SYS_AUJ - SF) * T, oAUK = (SYS_AUK - SF) * T;
+  // position in a slot of the coefficients' run, and in it of a column's coefficient
+  constexpr int RUN = MODE == SWEEP_FWD_AX ? 0 : 1;  // in units of T (after Y or T)
+  auto co = [&](const V *slot, int c, int tt) { return slot[RUN * T + sys_in_run<V>(c, T, tt)]; };
   unsigned long long *bar = reinterpret_cast<unsigned long long *>(sm);
   V *ring = reinterpret_cast<V *>(sm + ((R + 1) & ~1));
   V *xb = ring + (size_t)R * SS;
@@ -699,7 +700,7 @@ __device__ __forceinline__ void sweep_body(const Geo &g, const SkewGeo &q_, cons
 
   if (producer) {
 #pragma unroll 1
-    for (int u = 0; u < D; ++u) issue(u, u % R);
+    for (int u = 0; u < D; ++u) issue(u, u);
   }
 
   // Column geometry: active steps slo..shi (k inside 2..NK-1).
@@ -707,145 +708,168 @@ __device__ __forceinline__ void sweep_body(const Geo &g, const SkewGeo &q_, cons
   const bool ex0 = (t.ti == 0), ex1 = (t.ti == t.wi - 1), ey0 = (t.tj == 0), ey1 = (t.tj == t.wj - 1);
   const int slo = BWD ? ri + rj : t.ti + t.tj, shi = slo + g.NK - 3;
   const bool col = t.valid && !producer;
-  const int hl = halo_left(q, ES) + TIp * t.tj + halo_lofs(q, ES), hr = halo_right(q, ES) + TIp * t.tj,
-            hd = halo_down(q, ES) + t.ti, hu = halo_up(q, ES) + t.ti;
+  const int hti = col ? t.ti : 0, htj = col ? t.tj : 0;  // in range for threads without a column too
+  const int hl = halo_left(q, ES) + TIp * htj + halo_lofs(q, ES), hr = halo_right(q, ES) + TIp * htj,
+            hd = halo_down(q, ES) + hti, hu = halo_up(q, ES) + hti;
   // forward: T into the system block; backward: X
   V *vp = BWD ? vout + ((long long)b * q.W + nsteps - 1) * T + tid
-                              : S.sys + sys_at((long long)b * q.W, SYS_T, T, tid);
+                              : S.sys + sys_t((long long)b * q.W, T, tid);
   const long long vstep = BWD ? -(long long)T : (long long)SYS_N * T;
+
+  // Neighbouring column's entry of the exchange buffer and of the ring
+  // (the own entry where the tile has none; the value is then replaced).
+  const int tr = min(tid, T - 1);  // threads past the layout's T columns read entry T-1 and store nothing
+  const bool hx = BWD ? ri > 0 : t.ti > 0, hy = BWD ? rj > 0 : t.tj > 0;
+  const int ox = col && hx ? tr + (BWD ? 1 : -1) : tr, oy = col && hy ? tr + (BWD ? TIp : -TIp) : tr;
+  // P neighbours on the far side (inside the tile, else the halo)
+  const int oxp = col && !ex1 ? tr + 1 : tr, oyp = col && !ey1 ? tr + TIp : tr;
+  // first active step; a column that has no cells (or gave up waiting) never becomes active
+  int sfirst = col ? slo : (1 << 29);
+  const unsigned nact = (unsigned)(g.NK - 3);
 
   // Prepared values of the next step.
   bool act = false;             // the column has a cell at this step
   V dd = V(0);              // DD of the cell (0: not computed)
   V y0 = V(0);              // FWD: Y or A*P;  BWD: T
   V c1 = V(0), c2 = V(0), c3 = V(0);  // FWD: ALI*DD(i-1), ALJ*DD(j-1), ALK*DD(k-1); BWD: AUI, AUJ, AUK
-  V dk1 = V(0), pk1 = V(0);  // DD and P of this column at the previous step (FWD)
+  V dk1 = V(0), pk1 = V(0);  // DD and P of this column at the previous step (FWD; 0 below the interior)
+  V pcol = V(0);             // P of this column at the step to prepare (FWD_AX)
   V xk1 = V(0);             // result of this column at the previous step
   V q0 = V(0), q1 = V(0);   // NDOT: R0 and RR of the cell
   double a0 = 0.0, a1 = 0.0, a2 = 0.0, a3 = 0.0, a4 = 0.0;  // NDOT: this column's sums
   // Prepare step s: cs = slot of s, ps = slot of s-1, ns = slot of s+1.
+  // Straight-line: every thread loads and computes whether or not it has a
+  // cell at this step (all addresses lie in the ring), and `act` decides
+  // what is stored.
   auto prepare = [&](int s, const V *cs, const V *ps, const V *ns) {
-    act = col && s >= slo && s <= shi;
-    if (!act) return;
+    act = (unsigned)(s - sfirst) <= nact;
+    dd = co(cs, SYS_DD, tr);
     if (MODE == SWEEP_FWD_AX) {
-      const int k = 2 + s - t.ti - t.tj;
-      const V d = cs[oDD + tid], pc = cs[8 * T + tid];
-      if (d != V(0)) {
-        const V pxm = ex0 ? cs[hl] : ps[8 * T + tid - 1];
-        const V pym = ey0 ? cs[hd] : ps[8 * T + tid - TIp];
-        const V pzm = (k > 2) ? pk1 : V(0);
-        const V pxp = ex1 ? cs[hr] : ns[8 * T + tid + 1];
-        const V pyp = ey1 ? cs[hu] : ns[8 * T + tid + TIp];
-        const V pzp = (k < g.NK - 1) ? ns[8 * T + tid] : V(0);
-        y0 = cs[oAD + tid] * pc + cs[oALI + tid] * pxm + cs[oALJ + tid] * pym + cs[oALK + tid] * pzm +
-             cs[oAUI + tid] * pxp + cs[oAUJ + tid] * pyp + cs[oAUK + tid] * pzp;
-        const V d1 = (t.ti > 0) ? ps[oDD + tid - 1] : V(0);
-        const V d2 = (t.tj > 0) ? ps[oDD + tid - TIp] : (rrow ? din[(size_t)(s + lag) * TIp + t.ti] : V(0));
-        c1 = cs[oALI + tid] * d1;
-        c2 = cs[oALJ + tid] * d2;
-        c3 = cs[oALK + tid] * dk1;
-      }
-      dd = d; dk1 = d; pk1 = pc;
+      const V pc = pcol;
+      const V pn = ns[8 * T + tr];
+      const V pxm = *(ex0 ? cs + hl : ps + 8 * T + ox);
+      const V pym = *(ey0 ? cs + hd : ps + 8 * T + oy);
+      const V pzm = pk1;
+      const V pxp = *(ex1 ? cs + hr : ns + 8 * T + oxp);
+      const V pyp = *(ey1 ? cs + hu : ns + 8 * T + oyp);
+      const V pzp = (s < shi) ? pn : V(0);
+      const V ali = co(cs, SYS_ALI, tr), alj = co(cs, SYS_ALJ, tr), alk = co(cs, SYS_ALK, tr);
+      const V d1 = hx ? co(ps, SYS_DD, ox) : V(0);
+      const V d2 = hy ? co(ps, SYS_DD, oy) : (CS == 2 && rrow && act ? din[(size_t)(s + lag) * TIp + t.ti] : V(0));
+      y0 = co(cs, SYS_AD, tr) * pc + ali * pxm + alj * pym + alk * pzm + co(cs, SYS_AUI, tr) * pxp +
+           co(cs, SYS_AUJ, tr) * pyp + co(cs, SYS_AUK, tr) * pzp;
+      c1 = ali * d1;
+      c2 = alj * d2;
+      c3 = alk * dk1;
+      dk1 = act ? dd : V(0);
+      pk1 = act ? pc : V(0);
+      pcol = pn;
     } else if (MODE == SWEEP_FWD) {
-      const V d = cs[oDD + tid];
-      if (d != V(0)) {
-        const V d1 = (t.ti > 0) ? ps[oDD + tid - 1] : V(0);
-        const V d2 = (t.tj > 0) ? ps[oDD + tid - TIp] : (rrow ? din[(size_t)(s + lag) * TIp + t.ti] : V(0));
-        y0 = cs[tid];
-        c1 = cs[oALI + tid] * d1;
-        c2 = cs[oALJ + tid] * d2;
-        c3 = cs[oALK + tid] * dk1;
-      }
-      dd = d; dk1 = d;
+      const V d1 = hx ? co(ps, SYS_DD, ox) : V(0);
+      const V d2 = hy ? co(ps, SYS_DD, oy) : (CS == 2 && rrow && act ? din[(size_t)(s + lag) * TIp + t.ti] : V(0));
+      y0 = cs[tr];
+      c1 = co(cs, SYS_ALI, tr) * d1;
+      c2 = co(cs, SYS_ALJ, tr) * d2;
+      c3 = co(cs, SYS_ALK, tr) * dk1;
+      dk1 = act ? dd : V(0);
     } else {
-      dd = cs[oDD + tid];
-      if (dd != V(0)) { y0 = cs[tid]; c1 = cs[oAUI + tid]; c2 = cs[oAUJ + tid]; c3 = cs[oAUK + tid]; }
-      if (NDOT > 0) q0 = cs[5 * T + tid];
-      if (NDOT == 5) q1 = cs[6 * T + tid];
+      y0 = cs[tr];
+      c1 = co(cs, SYS_AUI, tr);
+      c2 = co(cs, SYS_AUJ, tr);
+      c3 = co(cs, SYS_AUK, tr);
+      if (NDOT > 0) q0 = cs[5 * T + tr];
+      if (NDOT == 5) q1 = cs[6 * T + tr];
     }
   };
-  auto slot_ptr = [&](int r) -> const V * { return ring + (size_t)r * SS; };
-
   bool ok = true;
+  // slots of steps s, s+1 and s+2 (R >= 4), the exchange buffers of steps
+  // s and s-1, and the slot of step s+1+AHEAD with its phase
+  const V *ps = ring, *cs = ring + SS, *ns = ring + 2 * (size_t)SS;
+  const V *const rend = ring + (size_t)R * SS;
+  V *xc = xb, *xp = xb + T;
+  int ru = AHEAD;
+  unsigned pu = 0;
+  // whether the newest data that preparing step s+1 reads has arrived;
+  // tested a step ahead, so the test's latency is hidden
+  bool ready = true;
   if (!producer) {
-    for (int u = 0; u < AHEAD; ++u) if (ok) ok = wait_data(u, u % R, (unsigned)((u / R) & 1));
+    for (int u = 0; u < AHEAD; ++u) if (ok) ok = wait_data(u, u, 0u);
     if (CS == 2 && ok && rrow && col && 0 >= slo && 0 <= shi) ok = mbar_wait_cluster(smem_u32(xfull + lag), 0u, st);
-    if (ok) prepare(0, slot_ptr(0), slot_ptr(R - 1), slot_ptr(1 % R));
-    else s_abort[0] = 1;
+    if (!ok) { sfirst = 1 << 29; s_abort[0] = 1; }
+    if (MODE == SWEEP_FWD_AX) pcol = ring[8 * T + tr];
+    prepare(0, ring, rend - SS, ring + SS);
+    ready = !ok || ru >= nsteps || mbar_test(bar0 + 8u * ru, 0u);
   }
   bool aborted = false;
   int issued = min(min(D, nsteps), stall_from) - 1;  // last step whose copies were issued (producer)
-  unsigned ph = 0;                  // (s0 / R) & 1, also the ring cycle's s_abort entry
+  int rs = 0, rd = D;               // slots of steps s and s+D
+  unsigned ph = 0;                  // parity of the ring cycle s / R: its s_abort entry
 #pragma unroll 1
-  for (int s0 = 0; s0 < nsteps && !aborted; s0 += R, ph ^= 1u) {
-#pragma unroll
-    for (int r = 0; r < R; ++r) {
-      const int s = s0 + r;
-      if (s >= nsteps) break;
-      if (producer) {
-        issue(s + D, (r + D) % R);
-        if (s + D < nsteps && s + D < stall_from) issued = s + D;
-      } else {
-        // Test the data of the step to prepare next now, so the test's
-        // latency overlaps the recurrence; wait only if it is not there.
-        const int u = s + AHEAD;  // newest data that preparing s+1 reads
-        const unsigned ubar = bar0 + 8u * ((r + AHEAD) % R), upar = ph ^ (unsigned)((r + AHEAD) / R);
-        const bool ready = !ok || u >= nsteps || mbar_test(ubar, upar);
-        // the recurrence of step s
-        V xcur = V(0);
-        if (act && ok) {
-          const int cur = (s & 1) * T, prv = T - cur;
-          V x = V(0);
-          if (dd != V(0)) {
-            const V xr = rrow ? xin[(size_t)(s + lag) * TIp + t.ti] : V(0);  // partner tile's row
-            if (BWD) {
-              const V x1 = (ri > 0) ? xb[prv + tid + 1] : V(0);
-              const V x2 = (rj > 0) ? xb[prv + tid + TIp] : xr;
-              x = (y0 - c1 * x1 - c2 * x2 - c3 * xk1) * dd;
-            } else {
-              const V x1 = (t.ti > 0) ? xb[prv + tid - 1] : V(0);
-              const V x2 = (t.tj > 0) ? xb[prv + tid - TIp] : xr;
-              x = y0 - c1 * x1 - c2 * x2 - c3 * xk1;
-            }
-          }
-          xb[cur + tid] = x;
-          *vp = x;
-          xk1 = x;
-          xcur = x;
-          // products of two single-precision values are exact in double
-          if (NDOT == 1) a0 += (double)q0 * (double)x;
-          if (NDOT == 5) {
-            const double r = (double)q1, e = (double)x, z = (double)q0;
-            a0 += r * e;
-            a1 += e * e;
-            a2 += r * r;
-            a3 += z * r;
-            a4 += z * e;
-          }
-        }
-        vp += vstep;
-        if (CS == 2 && srow) {  // this step's boundary-row values to the partner tile
-          const unsigned off = (unsigned)(((size_t)s * TIp + t.ti) * ES), fb = r_full + 8u * (unsigned)s;
-          st_async(r_xin + off, xcur, fb);
-          if (!BWD) st_async(r_din + off, act ? dd : V(0), fb);
-        }
-        // prepare step s+1
-        if (!ready) {
-          ok = mbar_wait_st(ubar, upar, st);
-          if (!ok) s_abort[ph] = 1;
-        }
-        if (CS == 2 && ok && rrow && col && s + 1 >= slo && s + 1 <= shi) {
-          ok = mbar_wait_cluster(smem_u32(xfull + (s + 1 + lag)), 0u, st);
-          if (!ok) s_abort[ph] = 1;
-        }
-        if (ok && s + 1 < nsteps) prepare(s + 1, slot_ptr((r + 1) % R), slot_ptr(r), slot_ptr((r + 2) % R));
+  for (int s = 0; s < nsteps; ++s) {
+    if (producer) {
+      issue(s + D, rd);
+      if (s + D < nsteps && s + D < stall_from) issued = s + D;
+      if (++rd == R) rd = 0;
+    } else {
+      // newest data that preparing step s+1 reads: step s+AHEAD, slot ru
+      if (!ready) {
+        ok = mbar_wait_st(bar0 + 8u * ru, pu, st);
+        if (!ok) { sfirst = 1 << 29; act = false; s_abort[ph] = 1; }
       }
-      __syncthreads();
+      if (++ru == R) { ru = 0; pu ^= 1u; }
+      // Straight-line from here to the stores: the recurrence of step s
+      // (a chain of dependent operations) and the preparation of step
+      // s+1 (independent of it) are scheduled into one another.
+      const V xl1 = xp[ox], xl2 = xp[oy];
+      const V xr = (CS == 2 && rrow && act) ? xin[(size_t)(s + lag) * TIp + t.ti] : V(0);  // partner tile's row
+      const V x1 = hx ? xl1 : V(0), x2 = hy ? xl2 : xr;
+      const bool a = act;
+      const V d = dd, z0 = q0, z1 = q1;
+      V x = y0 - c1 * x1 - c2 * x2 - c3 * xk1;
+      if (BWD) x = x * d;
+      if (CS == 2 && ok && rrow && col && s + 1 >= slo && s + 1 <= shi) {
+        ok = mbar_wait_cluster(smem_u32(xfull + (s + 1 + lag)), 0u, st);
+        if (!ok) { sfirst = 1 << 29; s_abort[ph] = 1; }
+      }
+      prepare(s + 1, cs, ps, ns);
+      x = (a && d != V(0)) ? x : V(0);
+      if (a) {
+        xc[tid] = x;
+        *vp = x;
+      }
+      xk1 = x;
+      vp += vstep;
+      // products of two single-precision values are exact in double;
+      // outside the column's cells x is 0 and so are the other factors
+      if (NDOT == 1) a0 += (double)(a ? z0 : V(0)) * (double)x;
+      if (NDOT == 5) {
+        const double rv = (double)(a ? z1 : V(0)), e = (double)x, z = (double)(a ? z0 : V(0));
+        a0 += rv * e;
+        a1 += e * e;
+        a2 += rv * rv;
+        a3 += z * rv;
+        a4 += z * e;
+      }
+      if (CS == 2 && srow) {  // this step's boundary-row values to the partner tile
+        const unsigned off = (unsigned)(((size_t)s * TIp + t.ti) * ES), fb = r_full + 8u * (unsigned)s;
+        st_async(r_xin + off, x, fb);
+        if (!BWD) st_async(r_din + off, a ? d : V(0), fb);
+      }
+      ready = !ok || s + 1 + AHEAD >= nsteps || mbar_test(bar0 + 8u * ru, pu);
+      ps = cs; cs = ns; ns += SS;
+      if (ns == rend) ns = ring;
+      V *const xs = xc; xc = xp; xp = xs;
     }
-    // A timed-out wait stops the sweep at the end of this ring cycle; the
-    // threads that gave up skip their remaining waits and work meanwhile.
-    if (s_abort[ph]) aborted = true;
+    __syncthreads();
+    if (++rs == R) {
+      // A timed-out wait stops the sweep at the end of this ring cycle; the
+      // threads that gave up skip their remaining waits and work meanwhile.
+      rs = 0;
+      if (s_abort[ph]) { aborted = true; break; }
+      ph ^= 1u;
+    }
   }
+  if (s_abort[ph]) aborted = true;  // the last, partial cycle
   if (aborted && producer) {
     // Let the copies already issued land (bounded) before the block exits.
     if (lane == 0)
@@ -854,36 +878,16 @@ __device__ __forceinline__ void sweep_body(const Geo &g, const SkewGeo &q_, cons
     if (lane == 0) { st->timeout = 1; st->done = 1; }
   }
   if (NDOT > 0) {
-    // the tile's sums: warps by a butterfly, then the warps' partials by
-    // warp 0, in a fixed order; one partial per tile into rb[c*nb + b]
-    __shared__ double s_red[5][32];
-    double a[5] = {a0, a1, a2, a3, a4};
-#pragma unroll
-    for (int c = 0; c < NDOT; ++c) {
-      double v = a[c];
-#pragma unroll
-      for (int o = 16; o >= 1; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
-      if (lane == 0) s_red[c][tid >> 5] = v;
-    }
-    __syncthreads();
-    if (tid < 32) {
-      const int nw = (int)(blockDim.x >> 5);
-#pragma unroll
-      for (int c = 0; c < NDOT; ++c) {
-        double v = (tid < nw) ? s_red[c][tid] : 0.0;
-#pragma unroll
-        for (int o = 16; o >= 1; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
-        if (tid == 0) rb[(long long)c * q.nb + b] = v;
-      }
-    }
+    const double a[5] = {a0, a1, a2, a3, a4};
+    sweep_sums<NDOT>(a, rb, q.nb, b);
   }
   if (CS == 2) cluster_barrier();  // the partner may still write into this block's shared memory
 }
-template <int D, int MODE, int MAXT, typename V, int CS, int MINB = 1, int CT = 0, int CTIP = 0>
-__global__ void __launch_bounds__(MAXT, MINB)
-    k_sweep(Geo g, SkewGeo q, SkewSysT<V> S, const V *vin, V *vout, SolveState *st, const V *vin2, double *rb) {
+template <int MODE, int MAXT, typename V, int CS>
+__global__ void __launch_bounds__(MAXT, 1)
+    k_sweep(Geo g, SkewGeo q, SkewSysT<V> S, const V *vin, V *vout, SolveState *st, const V *vin2, double *rb, int D) {
   pdl_enter();
-  sweep_body<D, MODE, V, CS, CT, CTIP>(g, q, S, vin, vout, st, vin2, rb, (int)blockIdx.x, (int)blockIdx.y);
+  sweep_body<MODE, V, CS>(g, q, S, vin, vout, st, vin2, rb, (int)blockIdx.x, (int)blockIdx.y, D);
 }
 
 // ------------------------------------------------------------ slab kernels
@@ -937,15 +941,14 @@ __device__ __forceinline__ V skew_ax(const Geo &g, const SkewGeo &q, const SkewS
   const long long bw = e / q.T;
   const int w = (int)(bw % q.W), b = (int)(bw / q.W);
   const int ti = t % q.TIp, tj = t / q.TIp, bx = b % q.ntx, by = b / q.ntx, k = 2 + w - ti - tj;
-  const V *a = S.sys + sys_at(bw, 0, q.T, t);
-  const long long T = q.T;
+  const V *s = S.sys + sys_chunk<V>(bw, 0, q.T, 0);
+  auto a = [&](int c) { return s[sys_in_run<V>(c, q.T, t)]; };
   auto at = [&](int di, int dj, int dk) -> V {
     const long long n = skew_nb(g, q, bx, by, ti + di, tj + dj, k + dk);
     return n < 0 ? V(0) : X[n];
   };
-  return a[SYS_AD * T] * X[e] + a[SYS_ALI * T] * at(-1, 0, 0) + a[SYS_ALJ * T] * at(0, -1, 0) +
-         a[SYS_ALK * T] * at(0, 0, -1) + a[SYS_AUI * T] * at(1, 0, 0) + a[SYS_AUJ * T] * at(0, 1, 0) +
-         a[SYS_AUK * T] * at(0, 0, 1);
+  return a(SYS_AD) * X[e] + a(SYS_ALI) * at(-1, 0, 0) + a(SYS_ALJ) * at(0, -1, 0) + a(SYS_ALK) * at(0, 0, -1) +
+         a(SYS_AUI) * at(1, 0, 0) + a(SYS_AUJ) * at(0, 1, 0) + a(SYS_AUK) * at(0, 0, 1);
 }
 
 // Y = A X on INDC != -1 (VF_MZAX); Y untouched elsewhere.
@@ -1231,9 +1234,18 @@ __global__ void k_commit(SolveState *st) {
 __device__ __forceinline__ void sys_to_f_elem(const SkewGeo &q, const double *sys, float *sysf, long long e) {
   const long long slab = e / q.T;
   const int t = (int)(e - slab * q.T);
-  constexpr int cs[7] = {SYS_AD, SYS_ALI, SYS_ALJ, SYS_ALK, SYS_AUI, SYS_AUJ, SYS_AUK};
+  float v[8];
 #pragma unroll
-  for (int c = 0; c < 7; ++c) sysf[sys_at(slab, cs[c], q.T, t)] = (float)sys[sys_at(slab, cs[c], q.T, t)];
+  for (int c = 0; c < 4; ++c) {
+    const double2 d = *reinterpret_cast<const double2 *>(sys + sys_chunk<double>(slab, c, q.T, t));
+    v[2 * c] = (float)d.x;
+    v[2 * c + 1] = (float)d.y;
+  }
+  v[SYS_DD - SYS_AUI] = 0.0f;  // filled by the FP32 factorisation
+#pragma unroll
+  for (int c = 0; c < 2; ++c)
+    *reinterpret_cast<float4 *>(sysf + sys_chunk<float>(slab, c, q.T, t)) =
+        make_float4(v[4 * c], v[4 * c + 1], v[4 * c + 2], v[4 * c + 3]);
 }
 __global__ void k_sys_to_f(SkewGeo q, const double *sys, float *sysf) {
   pdl_enter();
@@ -1458,14 +1470,12 @@ template <class K> static void set_smem(K kern, size_t bytes) {
   raise_dynamic_smem((const void *)kern, bytes);
 }
 
-static inline dim3 skew_grid(const SkewGeo &q) { return dim3((unsigned)q.ntx, (unsigned)(q.nb / q.ntx)); }
-
 void launch_to_skew(cudaStream_t s, const Geo &g, const SkewGeo &q, const SysPtr &a, const int *indc,
                     const SkewSys &S, const double *x0, double *bsl, double *xsl, int warm) {
   const size_t rb = to_skew_rows_bytes(g, q);
   if (rb > 0) {
     raise_dynamic_smem((const void *)k_to_skew_rows, rb);
-    launch_pdl(k_to_skew_rows, dim3((unsigned)(q.nb * q.TJ)), dim3(128), rb, s, 1, g, q, a, indc, S, x0, bsl, xsl,
+    launch_pdl(k_to_skew_rows, dim3((unsigned)(q.nb * q.TJ)), dim3(256), rb, s, 1, g, q, a, indc, S, x0, bsl, xsl,
                warm);
     return;
   }
@@ -1496,7 +1506,7 @@ void launch_dcmp(cudaStream_t s, const Geo &g, const SkewGeo &q, double U, const
 void launch_dcmp_f(cudaStream_t s, const Geo &g, const SkewGeo &q, double U, const SkewSysF &S, int *pivot_bad) {
   launch_dcmp_t<float>(s, g, q, (float)U, S, pivot_bad);
 }
-// Sweeps: prefetch depth D in {8, 6, 4, 3, 2}, the largest whose ring
+// Bulk-copy ring: prefetch depth D in {8, 6, 4, 3, 2, 1}, the largest whose ring
 // (R = D+2 slots, mbarriers, exchange buffers) fits the 227 KB of shared
 // memory a block may use.
 static size_t sweep_bytes(const SkewGeo &q, int mode, int D, int es) {
@@ -1508,132 +1518,107 @@ static size_t sweep_bytes(const SkewGeo &q, int mode, int D, int es) {
 }
 static int sweep_depth(const SkewGeo &q, int mode, int es) {
   if (sweep_threads(q.T) > (q.split == 2 ? 512 : 1024)) return 0;
-  for (int d : {8, 6, 4, 3, 2}) {
-    if (q.split == 2 && (d == 6 || d == 3)) continue;  // depths built for the cluster form
-    if (sweep_bytes(q, mode, d, es) <= 227 * 1024) return d;
+  // (depth 1 would starve the fused sweep, which reads two steps ahead)
+  for (int d : {8, 6, 4, 3, 2, 1})
+    if (sweep_bytes(q, mode, d, es) <= 227 * 1024 && (d > 1 || mode != SWEEP_FWD_AX)) return d;
+  return 0;
+}
+// ---- dispatch.  The sweeps run in the thread-copy form (k_sweep_cp); the
+// bulk-copy ring (k_sweep) serves clusters (split 2), tiles one column wide
+// and handles with the stall injection on (SkewGeo::ring), whose subject is
+// the ring's waits.
+//
+// Depth of the thread copies: the deepest that the shared memory allows,
+// since a step (0.14 to 0.35 us) is far shorter than the latency of a copy:
+// on 128 tiles of 8x16 columns x 96 layers, FP64, depths 4 and 8 measured
+// 34.8 and 28.8 us (fused forward) and 21.2 and 16.5 us (backward).  More
+// blocks per SM at less depth gain nothing (512 tiles of 16x16 x 128, FP64
+// fused forward: one block at depth 8 240 us, two at depth 4 251 us; FP32:
+// two at depth 8 137 us, four at depth 4 139 us), so only q.occ > 0 limits
+// a block's share.
+static int sweep_cp_threads(int T) { return (T + 31) & ~31; }
+static int sweep_cp_depth(const SkewGeo &q, int mode, int es) {
+  if (q.split != 1 || q.TI < 2 || q.TJ < 2) return 0;
+  const int nt = sweep_cp_threads(q.T);
+  const size_t cap = 227 * 1024, share = (q.occ > 1 ? 226 * 1024 / (size_t)q.occ : cap);
+  int best = 0;
+  for (int d : {16, 8, 4, 2, 1}) {
+    if (d == 16 && nt > 128) continue;
+    if (d == 1 && nt <= 576) continue;
+    const size_t n = sweep_cp_bytes(mode, d, q.T, q.TI, q.TJ, es);
+    if (n <= cap) best = d;   // the shallowest that fits, if none fits the share
+    if (n <= share) return d;
   }
-  return 0;
+  return best;
 }
-// Two thread blocks per SM (q.occ == 2): blocks of at most SWEEP2_THREADS
-// threads, registers capped for two resident blocks, and a ring that
-// leaves room for the second block's (228 KB per SM, 1 KB reserved per
-// block).  Two tiles' wavefronts then interleave on every SM.
-// The register cap (96 for two 288-thread blocks) makes deeper rings
-// spill: depths up to 3 (fused forward sweep, backward sweep with five
-// sums) or 4 (the others) are used.
-constexpr int SWEEP2_THREADS = 288;
-static int sweep_depth2(const SkewGeo &q, int mode, int es) {
-  if (q.split != 1 || sweep_threads(q.T) > SWEEP2_THREADS) return 0;
-  // 16x16 tiles run the instances with the tile's constants compiled in,
-  // which leave room for depth 6 everywhere (8 measured no faster for the
-  // forward sweeps and slower for the backward ones)
-  const bool t256 = q.T == 256 && q.TIp == 16;
-  const int dmax = t256 ? 6 : ((mode == SWEEP_FWD_AX || mode == SWEEP_BWD5) ? 3 : 4);
-  for (int d : {6, 4, 3, 2})
-    if (d <= dmax && sweep_bytes(q, mode, d, es) <= 113 * 1024) return d;
-  return 0;
+template <int D, int MODE, int MAXT, typename V, int MINB>
+static void sweep_cp_go(cudaStream_t s, const Geo &g, const SkewGeo &q, const SkewSysT<V> &S, const V *vin, V *vout,
+                        SolveState *st, const V *vin2, double *rb) {
+  const size_t bytes = sweep_cp_bytes(MODE, D, q.T, q.TI, q.TJ, (int)sizeof(V));
+  const dim3 grid((unsigned)q.ntx, (unsigned)(q.nb / q.ntx)), block((unsigned)sweep_cp_threads(q.T));
+#define SWEEP_GO(CT, CI)                                                                                        \
+  {                                                                                                             \
+    set_smem(k_sweep_cp<D, MODE, MAXT, V, MINB, CT, CI>, bytes);                                                \
+    launch_pdl(k_sweep_cp<D, MODE, MAXT, V, MINB, CT, CI>, grid, block, bytes, s, 1, g, q, S, vin, vout, st, vin2, rb); \
+    return;                                                                                                     \
+  }
+  if constexpr (MAXT == 128) {
+    if (q.T == 128 && q.TIp == 8) SWEEP_GO(128, 8)
+    if (q.T == 128 && q.TIp == 16) SWEEP_GO(128, 16)
+  }
+  if constexpr (MAXT == 256) {
+    if (q.T == 256 && q.TIp == 16) SWEEP_GO(256, 16)
+  }
+  SWEEP_GO(0, 0)
+#undef SWEEP_GO
 }
-// Four thread blocks per SM: the FP32 backward sweeps of 16x16 tiles, ring
-// depth 4 and at most 56 registers, so that up to four tiles per SM run in
-// one wave.  By default where the tiles fill more than two blocks per SM
-// (on 512 tiles: 19.6 against 23.0 ms of backward sweeps per step of the
-// mixed solver), or always with q.occ == 4; the other sweeps follow the
-// default's rule then.
-static bool sweep_four(const SkewGeo &q, int mode) {
-  return (q.occ == 4 || (q.occ == 0 && q.nb > 2 * q.nsm)) && q.split == 1 && mode >= SWEEP_BWD && q.T == 256 &&
-         q.TIp == 16 && sweep_bytes(q, mode, 4, 4) <= 55 * 1024;
+template <int MODE, typename V, int MAXT, int CS>
+static void sweep_ring_go(cudaStream_t s, const Geo &g, const SkewGeo &q, const SkewSysT<V> &S, const V *vin, V *vout,
+                          SolveState *st, const V *vin2, double *rb) {
+  const int d = sweep_depth(q, MODE, (int)sizeof(V));
+  if (d == 0) return;  // rejected by cadmas_create (sweep_supported)
+  const size_t bytes = sweep_bytes(q, MODE, d, (int)sizeof(V));
+  const int nty = q.nb / q.ntx;
+  const dim3 grid((unsigned)q.ntx, (unsigned)(CS == 2 ? (nty + 1) & ~1 : nty)), block((unsigned)sweep_threads(q.T));
+  set_smem(k_sweep<MODE, MAXT, V, CS>, bytes);
+  launch_pdl(k_sweep<MODE, MAXT, V, CS>, grid, block, bytes, s, CS, g, q, S, vin, vout, st, vin2, rb, d);
 }
-// The default's rule for q.occ 0 and 4.
-static int sweep_occ(const SkewGeo &q) { return q.occ == 4 ? 0 : q.occ; }
+// The sweep MODE of a grid.  vin2 and rb: the inner products' second
+// vector and partials (modes 3, 4).
 template <int MODE, typename V>
 static void launch_sweep(cudaStream_t s, const Geo &g, const SkewGeo &q, const SkewSysT<V> &S, const V *vin,
-                         V *vout, SolveState *st) {
-  constexpr int ES = (int)sizeof(V);
-  const V *vnull = nullptr;
-  double *rnull = nullptr;
-  const bool t256 = q.T == 256 && q.TIp == 16;  // 16x16 tiles: the shape's constants compiled in
-  const int d = sweep_depth(q, MODE, ES);
-  const size_t bytes = sweep_bytes(q, MODE, d, ES);
-  const int nty = q.nb / q.ntx;
-  const dim3 block((unsigned)sweep_threads(q.T));
-  // The register budget follows the block size (255, 128 or 64 registers
-  // for blocks of up to 256, 512 or 1024 threads).
-  const int nt = sweep_threads(q.T);
-  const int mt = nt <= 256 ? 256 : (nt <= 512 ? 512 : 1024);
-  if (q.split == 2) {
-    // one cluster of two thread blocks per preconditioner block
-    const dim3 grid((unsigned)q.ntx, (unsigned)((nty + 1) & ~1));
-    switch (d * 4096 + mt) {
-#define SWEEP_CASE2(DD, MT)                                                             \
-  case DD * 4096 + MT:                                                                  \
-    set_smem(k_sweep<DD, MODE, MT, V, 2>, bytes);                                       \
-    launch_pdl(k_sweep<DD, MODE, MT, V, 2>, grid, block, bytes, s, 2, g, q, S, vin, vout, st, vnull, rnull); \
-    break;
-      SWEEP_CASE2(8, 256) SWEEP_CASE2(4, 256) SWEEP_CASE2(2, 256)
-      SWEEP_CASE2(8, 512) SWEEP_CASE2(4, 512) SWEEP_CASE2(2, 512)
-#undef SWEEP_CASE2
-      default: return;  // rejected by cadmas_create (sweep_supported)
-    }
-    return;
+                         V *vout, SolveState *st, const V *vin2 = nullptr, double *rb = nullptr) {
+  const int d = q.ring ? 0 : sweep_cp_depth(q, MODE, (int)sizeof(V)), nt = sweep_cp_threads(q.T);
+#define CP_GO(D, MT, MB)                                                       \
+  {                                                                            \
+    sweep_cp_go<D, MODE, MT, V, MB>(s, g, q, S, vin, vout, st, vin2, rb);      \
+    return;                                                                    \
   }
-  const dim3 grid = skew_grid(q);
-  // Two blocks per SM pay where the tiles fill the SMs twice over: there
-  // the sweeps' per-step latency, not the bandwidth, sets the time and a
-  // second tile's wavefront fills it.  The fused FP64 forward sweep keeps
-  // one block: its ring of 8 arrays needs the depth and registers.
-  if constexpr (ES == 4 && MODE >= SWEEP_BWD) {
-    if (sweep_four(q, MODE)) {
-      const size_t b4 = sweep_bytes(q, MODE, 4, ES);
-      set_smem(k_sweep<4, MODE, SWEEP2_THREADS, V, 1, 4, 256, 16>, b4);
-      launch_pdl(k_sweep<4, MODE, SWEEP2_THREADS, V, 1, 4, 256, 16>, grid, block, b4, s, 1, g, q, S, vin, vout, st,
-                 vnull, rnull);
-      return;
+  if (d > 0) {
+    if (nt <= 128) {
+      if (d == 16) CP_GO(16, 128, 1)
+      if (d == 8) CP_GO(8, 128, 1)
+      if (d == 4) CP_GO(4, 128, 1)
+      CP_GO(2, 128, 1)
+    } else if (nt <= 256) {
+      if (d == 8) CP_GO(8, 256, 1)
+      if (d == 4) CP_GO(4, 256, 1)
+      CP_GO(2, 256, 1)
+    } else if (nt <= 576) {
+      if (d == 8) CP_GO(8, 576, 1)
+      if (d == 4) CP_GO(4, 576, 1)
+      CP_GO(2, 576, 1)
+    } else {
+      if (d == 8) CP_GO(8, 1024, 1)
+      if (d == 4) CP_GO(4, 1024, 1)
+      if (d == 2) CP_GO(2, 1024, 1)
+      CP_GO(1, 1024, 1)
     }
   }
-  const int oc = sweep_occ(q);
-  const bool two = oc == 2 || (oc == 0 && q.nb >= 2 * q.nsm && (ES == 4 || MODE >= SWEEP_BWD));
-  if (two) {
-    const int d2 = sweep_depth2(q, MODE, ES);
-    if (d2 > 0) {
-      const size_t bytes2 = sweep_bytes(q, MODE, d2, ES);
-      switch (d2) {
-#define SWEEP_CASE_OCC2(DD)                                                                            \
-  case DD:                                                                                             \
-    if (t256) {                                                                                        \
-      set_smem(k_sweep<DD, MODE, SWEEP2_THREADS, V, 1, 2, 256, 16>, bytes2);                           \
-      launch_pdl(k_sweep<DD, MODE, SWEEP2_THREADS, V, 1, 2, 256, 16>, grid, block, bytes2, s, 1, g, q, S, vin, vout, \
-                 st, vnull, rnull);                                                                    \
-    } else {                                                                                           \
-      set_smem(k_sweep<DD, MODE, SWEEP2_THREADS, V, 1, 2>, bytes2);                                    \
-      launch_pdl(k_sweep<DD, MODE, SWEEP2_THREADS, V, 1, 2>, grid, block, bytes2, s, 1, g, q, S, vin, vout, st, vnull, \
-                 rnull);                                                                               \
-    }                                                                                                  \
-    return;
-        SWEEP_CASE_OCC2(6) SWEEP_CASE_OCC2(4) SWEEP_CASE_OCC2(3) SWEEP_CASE_OCC2(2)
-#undef SWEEP_CASE_OCC2
-        default: break;
-      }
-    }
-  }
-  switch (d * 4096 + mt) {
-#define SWEEP_CASE(DD, MT)                                                              \
-  case DD * 4096 + MT:                                                                  \
-    if (MT == 512 && t256) {                                                            \
-      constexpr int CT_ = MT == 512 ? 256 : 0, CI_ = MT == 512 ? 16 : 0;                \
-      set_smem(k_sweep<DD, MODE, MT, V, 1, 1, CT_, CI_>, bytes);                        \
-      launch_pdl(k_sweep<DD, MODE, MT, V, 1, 1, CT_, CI_>, grid, block, bytes, s, 1, g, q, S, vin, vout, st, vnull, \
-                 rnull);                                                                \
-    } else {                                                                            \
-      set_smem(k_sweep<DD, MODE, MT, V, 1>, bytes);                                     \
-      launch_pdl(k_sweep<DD, MODE, MT, V, 1>, grid, block, bytes, s, 1, g, q, S, vin, vout, st, vnull, rnull); \
-    }                                                                                   \
-    break;
-    SWEEP_CASE(8, 256) SWEEP_CASE(6, 256) SWEEP_CASE(4, 256) SWEEP_CASE(3, 256) SWEEP_CASE(2, 256)
-    SWEEP_CASE(8, 512) SWEEP_CASE(6, 512) SWEEP_CASE(4, 512) SWEEP_CASE(3, 512) SWEEP_CASE(2, 512)
-    SWEEP_CASE(8, 1024) SWEEP_CASE(6, 1024) SWEEP_CASE(4, 1024) SWEEP_CASE(3, 1024) SWEEP_CASE(2, 1024)
-#undef SWEEP_CASE
-    default: return;  // rejected by cadmas_create (sweep_supported)
-  }
+#undef CP_GO
+  if (q.split == 2) sweep_ring_go<MODE, V, 512, 2>(s, g, q, S, vin, vout, st, vin2, rb);
+  else if (sweep_threads(q.T) <= 512) sweep_ring_go<MODE, V, 512, 1>(s, g, q, S, vin, vout, st, vin2, rb);
+  else sweep_ring_go<MODE, V, 1024, 1>(s, g, q, S, vin, vout, st, vin2, rb);
 }
 bool sweep_supported(const SkewGeo &q) {
   const int tb = q.T * q.split;  // threads of the factorisation kernel
@@ -1648,7 +1633,8 @@ bool sweep_supported_f(const SkewGeo &q) {
 template <typename V>
 static void launch_fwd_t(cudaStream_t s, const Geo &g, const SkewGeo &q, const SkewSysT<V> &S, const V *y,
                          const V *spmv_x, SolveState *st, V *ybuf) {
-  if (spmv_x && sweep_depth(q, SWEEP_FWD_AX, (int)sizeof(V)) == 0) {
+  const int es = (int)sizeof(V);
+  if (spmv_x && (q.ring || sweep_cp_depth(q, SWEEP_FWD_AX, es) == 0) && sweep_depth(q, SWEEP_FWD_AX, es) == 0) {
     // Ring of the fused sweep too large for this tile: SpMV first.
     launch_spmv_t<V>(s, g, q, S, spmv_x, ybuf, st);
     y = ybuf;
@@ -1673,65 +1659,15 @@ void launch_bwd_f(cudaStream_t s, const Geo &g, const SkewGeo &q, const SkewSysF
 }
 // The FP32 backward sweep with the inner products that follow it summed
 // on the way (mode 3: (R0,X); mode 4: the five sums of k_dot5f), one
-// partial per tile into rb (rb + c*nb for sum c).  Ring depths 2..4, one
-// layout tile per preconditioner block, blocks of up to 512 threads;
-// false (nothing launched) where that does not hold.
+// partial per tile into rb (rb + c*nb for sum c).  One layout tile per
+// preconditioner block, blocks of up to 512 threads; false (nothing
+// launched) where that does not hold.
 template <int MODE>
 static bool launch_bwd_dots(cudaStream_t s, const Geo &g, const SkewGeo &q, const SkewSysF &S, const float *r0,
                             const float *rr, float *x, double *rb, SolveState *st) {
-  constexpr int ES = 4;
-  if (q.split != 1) return false;
-  const bool t256 = q.T == 256 && q.TIp == 16;
-  const dim3 grid = skew_grid(q), block((unsigned)sweep_threads(q.T));
-  if (sweep_four(q, MODE)) {
-    const size_t b4 = sweep_bytes(q, MODE, 4, ES);
-    set_smem(k_sweep<4, MODE, SWEEP2_THREADS, float, 1, 4, 256, 16>, b4);
-    launch_pdl(k_sweep<4, MODE, SWEEP2_THREADS, float, 1, 4, 256, 16>, grid, block, b4, s, 1, g, q, S, r0, x, st, rr,
-               rb);
-    return true;
-  }
-  const int oc = sweep_occ(q);
-  const bool two = oc == 2 || (oc == 0 && q.nb >= 2 * q.nsm);
-  if (two) {
-    const int d2 = sweep_depth2(q, MODE, ES);
-    const size_t bytes2 = sweep_bytes(q, MODE, d2, ES);
-    switch (d2) {
-#define DOTS_OCC2(DD)                                                                                              \
-  case DD:                                                                                                         \
-    if (t256) {                                                                                                    \
-      set_smem(k_sweep<DD, MODE, SWEEP2_THREADS, float, 1, 2, 256, 16>, bytes2);                                   \
-      launch_pdl(k_sweep<DD, MODE, SWEEP2_THREADS, float, 1, 2, 256, 16>, grid, block, bytes2, s, 1, g, q, S, r0, x, \
-                 st, rr, rb);                                                                                      \
-    } else {                                                                                                       \
-      set_smem(k_sweep<DD, MODE, SWEEP2_THREADS, float, 1, 2>, bytes2);                                            \
-      launch_pdl(k_sweep<DD, MODE, SWEEP2_THREADS, float, 1, 2>, grid, block, bytes2, s, 1, g, q, S, r0, x, st, rr, rb); \
-    }                                                                                                              \
-    return true;
-      DOTS_OCC2(6) DOTS_OCC2(4) DOTS_OCC2(3) DOTS_OCC2(2)
-#undef DOTS_OCC2
-      default: break;
-    }
-  }
-  const int d = std::min(sweep_depth(q, MODE, ES), 4), nt = sweep_threads(q.T);
-  const int mt = nt <= 256 ? 256 : (nt <= 512 ? 512 : 0);
-  if (mt == 0 || d < 2) return false;
-  const size_t bytes = sweep_bytes(q, MODE, d, ES);
-  switch (d * 4096 + mt) {
-#define DOTS_CASE(DD, MT)                                                                            \
-  case DD * 4096 + MT:                                                                               \
-    if (MT == 512 && t256) {                                                                         \
-      constexpr int CT_ = MT == 512 ? 256 : 0, CI_ = MT == 512 ? 16 : 0;                             \
-      set_smem(k_sweep<DD, MODE, MT, float, 1, 1, CT_, CI_>, bytes);                                 \
-      launch_pdl(k_sweep<DD, MODE, MT, float, 1, 1, CT_, CI_>, grid, block, bytes, s, 1, g, q, S, r0, x, st, rr, rb); \
-    } else {                                                                                         \
-      set_smem(k_sweep<DD, MODE, MT, float, 1>, bytes);                                              \
-      launch_pdl(k_sweep<DD, MODE, MT, float, 1>, grid, block, bytes, s, 1, g, q, S, r0, x, st, rr, rb); \
-    }                                                                                                \
-    return true;
-    DOTS_CASE(4, 256) DOTS_CASE(3, 256) DOTS_CASE(2, 256) DOTS_CASE(4, 512) DOTS_CASE(3, 512) DOTS_CASE(2, 512)
-#undef DOTS_CASE
-    default: return false;
-  }
+  if (q.split != 1 || sweep_threads(q.T) > 512 || sweep_depth(q, MODE, 4) < 2) return false;
+  launch_sweep<MODE, float>(s, g, q, S, r0, x, st, rr, rb);
+  return true;
 }
 bool launch_bwd_f_dot1(cudaStream_t s, const Geo &g, const SkewGeo &q, const SkewSysF &S, const float *r0, float *x,
                        double *rb, SolveState *st) {
@@ -1889,14 +1825,24 @@ __global__ void kb_dcmp_f(const BatchMember *bm, const int *pre, int nm) {
   if (!M.active) return;
   dcmp_body<D, float>(M.g, M.q, (float)M.U, M.Sf, M.pivot_bad, (int)(lb_ % M.q.ntx), (int)(lb_ / M.q.ntx));
 }
-template <int D, int MODE, int MAXT, int MINB, int CT = 0, int CTIP = 0>
+template <int D, int MODE, int MAXT, int MINB, int CT, int CTIP>
 __global__ void __launch_bounds__(MAXT, MINB) kb_sweep(const BatchMember *bm, const int *pre, int nm, int vin,
                                                        int vout, int vin2, int rb5) {
   pdl_enter();
   BATCH_BLOCK(BR_TILE)
-  sweep_body<D, MODE, float, 1, CT, CTIP>(M.g, M.q, M.Sf, vin >= 0 ? M.vf[vin] : nullptr, vout >= 0 ? M.vf[vout] : nullptr,
-                                M.st, vin2 >= 0 ? M.vf[vin2] : nullptr, rb5 ? M.rb5 : M.rb0,
-                                (int)(lb_ % M.q.ntx), (int)(lb_ / M.q.ntx));
+  sweep_cp_body<D, MODE, float, CT, CTIP>(M.g, M.q, M.Sf, vin >= 0 ? M.vf[vin] : nullptr,
+                                          vout >= 0 ? M.vf[vout] : nullptr, M.st, vin2 >= 0 ? M.vf[vin2] : nullptr,
+                                          rb5 ? M.rb5 : M.rb0, (int)(lb_ % M.q.ntx), (int)(lb_ / M.q.ntx));
+}
+// the bulk-copy ring: tiles one column wide, or a member with the stall on
+template <int MODE>
+__global__ void __launch_bounds__(512, 1) kb_sweep_ring(const BatchMember *bm, const int *pre, int nm, int vin,
+                                                        int vout, int vin2, int rb5, int D) {
+  pdl_enter();
+  BATCH_BLOCK(BR_TILE)
+  sweep_body<MODE, float, 1>(M.g, M.q, M.Sf, vin >= 0 ? M.vf[vin] : nullptr, vout >= 0 ? M.vf[vout] : nullptr, M.st,
+                             vin2 >= 0 ? M.vf[vin2] : nullptr, rb5 ? M.rb5 : M.rb0, (int)(lb_ % M.q.ntx),
+                             (int)(lb_ / M.q.ntx), D);
 }
 // the solve state of every member cleared up to the wait limit; members
 // outside the pass marked done, so every solver kernel skips them
@@ -2015,58 +1961,67 @@ bool launch_b_dcmp_f(cudaStream_t s, const BatchMember *bm, const int *pre, int 
     default: return false;
   }
 }
-// The batched FP32 sweeps: two blocks per SM (the rule of launch_sweep,
-// counted over all the members' tiles) or one, ring depths 2..4.
-static int b_sweep_depth(const SkewGeo &q, int mode, bool two) {
-  return two ? sweep_depth2(q, mode, 4) : std::min(sweep_depth(q, mode, 4), 4);
-}
-static bool b_two(const SkewGeo &q, int nsm, int occ, long long ntiles) {
-  return occ == 2 || ((occ == 0 || occ == 4) && ntiles >= 2LL * nsm);
-}
-bool b_sweeps_supported(const SkewGeo &q, int nsm, int occ, long long ntiles) {
+// The batched FP32 sweeps: the form and depth of launch_sweep, by the tile
+// shape that the members share (qref; qref.ring for the bulk-copy ring).
+bool b_sweeps_supported(const SkewGeo &q) {
   if (q.split != 1 || sweep_threads(q.T) > 512) return false;
-  const bool two = b_two(q, nsm, occ, ntiles) && sweep_threads(q.T) <= SWEEP2_THREADS;
   for (int mode : {(int)SWEEP_FWD, (int)SWEEP_FWD_AX, (int)SWEEP_BWD, (int)SWEEP_BWD1, (int)SWEEP_BWD5})
-    if (b_sweep_depth(q, mode, two) < 2) return false;
+    if (sweep_depth(q, mode, 4) < 2) return false;
   return true;
 }
 template <int MODE>
 static bool launch_b_sweep_t(cudaStream_t s, const BatchMember *bm, const int *pre, int nm, long long ntiles,
-                             const SkewGeo &q, int vin, int vout, int vin2, int rb5, int nsm, int occ) {
-  const bool two = b_two(q, nsm, occ, ntiles) && sweep_threads(q.T) <= SWEEP2_THREADS;
-  const int d = b_sweep_depth(q, MODE, two);
-  if (d < 2) return false;
-  const bool t256 = q.T == 256 && q.TIp == 16;
-  const size_t bytes = sweep_bytes(q, MODE, d, 4);
-  const dim3 block((unsigned)sweep_threads(q.T));
-  switch (d * 2 + (two ? 1 : 0)) {
-#define BSWEEP(DD, TWO, MT, MB)                                                                        \
-  case DD * 2 + TWO:                                                                                   \
-    if (t256) {                                                                                        \
-      set_smem(kb_sweep<DD, MODE, MT, MB, 256, 16>, bytes);                                            \
-      launch_pdl(kb_sweep<DD, MODE, MT, MB, 256, 16>, bgrid(ntiles), block, bytes, s, 1, bm, pre, nm, vin, vout, \
-                 vin2, rb5);                                                                           \
-    } else {                                                                                           \
-      set_smem(kb_sweep<DD, MODE, MT, MB>, bytes);                                                     \
-      launch_pdl(kb_sweep<DD, MODE, MT, MB>, bgrid(ntiles), block, bytes, s, 1, bm, pre, nm, vin, vout, vin2, rb5); \
-    }                                                                                                  \
+                             const SkewGeo &q, int vin, int vout, int vin2, int rb5) {
+  const int d = q.ring ? 0 : sweep_cp_depth(q, MODE, 4), nt = sweep_cp_threads(q.T);
+  if (d == 0) {
+    const int dr = sweep_depth(q, MODE, 4);
+    if (dr < 2) return false;
+    const size_t bytes = sweep_bytes(q, MODE, dr, 4);
+    set_smem(kb_sweep_ring<MODE>, bytes);
+    launch_pdl(kb_sweep_ring<MODE>, bgrid(ntiles), dim3((unsigned)sweep_threads(q.T)), bytes, s, 1, bm, pre, nm, vin,
+               vout, vin2, rb5, dr);
     return true;
-    BSWEEP(2, 1, SWEEP2_THREADS, 2) BSWEEP(3, 1, SWEEP2_THREADS, 2) BSWEEP(4, 1, SWEEP2_THREADS, 2)
-    BSWEEP(6, 1, SWEEP2_THREADS, 2)
-    BSWEEP(2, 0, 512, 1) BSWEEP(3, 0, 512, 1) BSWEEP(4, 0, 512, 1)
-#undef BSWEEP
-    default: return false;
   }
+  const size_t bytes = sweep_cp_bytes(MODE, d, q.T, q.TI, q.TJ, 4);
+  const dim3 block((unsigned)nt);
+#define BSWEEP(D, MT, MB, CT, CI)                                                                             \
+  {                                                                                                           \
+    set_smem(kb_sweep<D, MODE, MT, MB, CT, CI>, bytes);                                                       \
+    launch_pdl(kb_sweep<D, MODE, MT, MB, CT, CI>, bgrid(ntiles), block, bytes, s, 1, bm, pre, nm, vin, vout, vin2, rb5); \
+    return true;                                                                                              \
+  }
+#define BSWEEP_D(D)                                              \
+  {                                                              \
+    if (nt <= 128) {                                             \
+      if (q.T == 128 && q.TIp == 8) BSWEEP(D, 128, 1, 128, 8)    \
+      if (q.T == 128 && q.TIp == 16) BSWEEP(D, 128, 1, 128, 16)  \
+      BSWEEP(D, 128, 1, 0, 0)                                    \
+    }                                                            \
+    if (nt <= 256) {                                             \
+      if (q.T == 256 && q.TIp == 16) BSWEEP(D, 256, 1, 256, 16)  \
+      BSWEEP(D, 256, 1, 0, 0)                                    \
+    }                                                            \
+    BSWEEP(D, 576, 1, 0, 0)                                      \
+  }
+  if (d == 16) {
+    if (q.T == 128 && q.TIp == 8) BSWEEP(16, 128, 1, 128, 8)
+    if (q.T == 128 && q.TIp == 16) BSWEEP(16, 128, 1, 128, 16)
+    BSWEEP(16, 128, 1, 0, 0)
+  }
+  if (d == 8) BSWEEP_D(8)
+  if (d == 4) BSWEEP_D(4)
+  BSWEEP_D(2)
+#undef BSWEEP_D
+#undef BSWEEP
 }
 bool launch_b_sweep(cudaStream_t s, int mode, const BatchMember *bm, const int *pre, int nm, long long ntiles,
-                    const SkewGeo &q, int vin, int vout, int vin2, bool rb5, int nsm, int occ) {
+                    const SkewGeo &q, int vin, int vout, int vin2, bool rb5) {
   switch (mode) {
-    case SWEEP_FWD: return launch_b_sweep_t<SWEEP_FWD>(s, bm, pre, nm, ntiles, q, vin, vout, vin2, rb5, nsm, occ);
-    case SWEEP_FWD_AX:
-      return launch_b_sweep_t<SWEEP_FWD_AX>(s, bm, pre, nm, ntiles, q, vin, vout, vin2, rb5, nsm, occ);
-    case SWEEP_BWD: return launch_b_sweep_t<SWEEP_BWD>(s, bm, pre, nm, ntiles, q, vin, vout, vin2, rb5, nsm, occ);
-    case SWEEP_BWD1: return launch_b_sweep_t<SWEEP_BWD1>(s, bm, pre, nm, ntiles, q, vin, vout, vin2, rb5, nsm, occ);
-    case SWEEP_BWD5: return launch_b_sweep_t<SWEEP_BWD5>(s, bm, pre, nm, ntiles, q, vin, vout, vin2, rb5, nsm, occ);
+    case SWEEP_FWD: return launch_b_sweep_t<SWEEP_FWD>(s, bm, pre, nm, ntiles, q, vin, vout, vin2, rb5);
+    case SWEEP_FWD_AX: return launch_b_sweep_t<SWEEP_FWD_AX>(s, bm, pre, nm, ntiles, q, vin, vout, vin2, rb5);
+    case SWEEP_BWD: return launch_b_sweep_t<SWEEP_BWD>(s, bm, pre, nm, ntiles, q, vin, vout, vin2, rb5);
+    case SWEEP_BWD1: return launch_b_sweep_t<SWEEP_BWD1>(s, bm, pre, nm, ntiles, q, vin, vout, vin2, rb5);
+    case SWEEP_BWD5: return launch_b_sweep_t<SWEEP_BWD5>(s, bm, pre, nm, ntiles, q, vin, vout, vin2, rb5);
     default: return false;
   }
 }

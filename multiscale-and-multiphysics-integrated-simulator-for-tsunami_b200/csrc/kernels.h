@@ -25,14 +25,17 @@ struct SysPtr {
 };
 
 // The constant part of a solve in the tile-skewed layout of the MILU
-// kernels (k_poisson.cu).  Nine arrays are interleaved slab by slab,
-// sys[(slab*SYS_N + c)*T + t], so the values one wavefront step of a sweep
-// needs are one contiguous run: the backward sweep's {T, AUI, AUJ, AUK,
-// DD}, the fused forward sweep's {AUI .. ALK} and the plain forward
-// sweep's {DD, AD, ALI, ALJ, ALK}.  SYS_T is the forward sweep's result
-// T = MINV_L*Y, written by the forward sweep for the backward sweep that
-// follows it.  INDC is a plain skewed array.
-enum SysArray { SYS_T = 0, SYS_AUI, SYS_AUJ, SYS_AUK, SYS_DD, SYS_AD, SYS_ALI, SYS_ALJ, SYS_ALK, SYS_N };
+// kernels (k_poisson.cu).  Nine arrays are interleaved slab by slab, 9 T
+// values a slab: first SYS_T, the forward sweep's result T = MINV_L*Y,
+// written by the forward sweep for the backward sweep that follows it;
+// then the eight coefficients AUI, AUJ, AUK, DD, ALI, ALJ, ALK, AD in
+// 16-byte chunks of G = 2 (FP64) or 4 (FP32) of them per column, chunk by
+// chunk: coefficient e of column t at T + ((e/G)*T + t)*G + e%G.  So one
+// 16-byte copy moves a chunk of a column, T consecutive chunks are one
+// contiguous run, and the values that a wavefront step of a sweep needs
+// are one too: the backward sweep's {T, AUI .. DD} and the forward
+// sweeps' {AUI .. AD}.  INDC is a plain skewed array.
+enum SysArray { SYS_T = 0, SYS_AUI, SYS_AUJ, SYS_AUK, SYS_DD, SYS_ALI, SYS_ALJ, SYS_ALK, SYS_AD, SYS_N };
 template <typename V> struct SkewSysT {
   V *sys;
   int *indc;
@@ -43,25 +46,34 @@ struct SkewGeo {
   int TI, TJ, TIp, T, W;  // layout tile TI x TJ columns (T = TIp*TJ slots), W slabs per tile
   int ntx, nb;            // layout tiles along x, tiles in total
   int split;  // layout tiles per preconditioner block along y (1 or 2)
-  // Thread blocks of the sweeps per SM (k_poisson.cu): 1, 2, or 0 = by
-  // the rule of launch_sweep (two for the backward sweeps and the FP32
-  // sweeps when there are at least two tiles per SM); nsm = the SMs.
-  int occ, nsm;
+  int occ;    // thread blocks of the sweeps per SM to leave shared memory for (0: one, at full depth)
+  int ring;   // 1: the sweeps' bulk-copy form (the stall injection's subject), 0: by the rule of launch_sweep
 };
 
-__host__ __device__ inline long long sys_at(long long slab, int c, int T, int t) {
-  return (slab * SYS_N + c) * T + t;
+// SYS_T of column t
+__host__ __device__ inline long long sys_t(long long slab, int T, int t) { return slab * SYS_N * T + t; }
+// chunk c of column t
+template <typename V> __host__ __device__ inline long long sys_chunk(long long slab, int c, int T, int t) {
+  return slab * SYS_N * T + T + ((long long)c * T + t) * (16 / (int)sizeof(V));
+}
+// coefficient c (SYS_AUI ..) of column t, in a run of chunks and in the system
+template <typename V> __host__ __device__ inline int sys_in_run(int c, int T, int t) {
+  constexpr int G = 16 / (int)sizeof(V);
+  return (((c - SYS_AUI) / G) * T + t) * G + (c - SYS_AUI) % G;
+}
+template <typename V> __host__ __device__ inline long long sys_at(long long slab, int c, int T, int t) {
+  return slab * SYS_N * T + T + sys_in_run<V>(c, T, t);
 }
 
 // Bulk copies of one wavefront step of the MILU sweeps (k_sweep).  A ring
 // slot holds NV slabs of T values (slab c at c*T):
-// MODE 0: forward sweep of a given vector: {Y, DD, AD, ALI, ALJ, ALK}
-//         (AD unused), copies: Y, system arrays DD..ALK;
-// MODE 1: forward sweep fused with Y = A*P: {AUI, AUJ, AUK, DD, AD, ALI,
-//         ALJ, ALK, P} plus the P values of the four neighbouring tiles at
+// MODE 0: forward sweep of a given vector: {Y, the eight coefficients},
+//         copies: Y, the coefficients;
+// MODE 1: forward sweep fused with Y = A*P: {the eight coefficients, P}
+//         plus the P values of the four neighbouring tiles at
 //         the step's cells (down/up: one row of TIp; left/right: the span
 //         of the neighbour's slab from its last/first column of row 0 to
-//         that of row TJ-1), copies: system arrays AUI..ALK, P, down, up,
+//         that of row TJ-1), copies: the coefficients, P, down, up,
 //         left, right;
 // MODE 2: backward sweep: {T, AUI, AUJ, AUK, DD}, copy: system arrays
 //         T..DD;
@@ -83,14 +95,14 @@ struct SweepCopy {
   int dst, bytes, arr;
 };
 __host__ __device__ inline int sweep_nv(int mode) {
-  return mode == SWEEP_FWD_AX ? 9 : (mode == SWEEP_FWD ? 6 : 5 + (mode - SWEEP_BWD));
+  return mode <= SWEEP_FWD_AX ? 9 : 5 + (mode - SWEEP_BWD);
 }
 __host__ __device__ inline int sweep_ncopy(const SkewGeo &, int mode) {
   return mode == SWEEP_FWD_AX ? 6 : (mode == SWEEP_FWD ? 2 : 1 + (mode - SWEEP_BWD));
 }
 // First system array of a mode's slot and its position there.
 __host__ __device__ constexpr int sweep_sys_first(int mode) {
-  return mode == SWEEP_FWD_AX ? SYS_AUI : (mode == SWEEP_FWD ? SYS_DD : SYS_T);
+  return mode <= SWEEP_FWD_AX ? SYS_AUI : SYS_T;
 }
 __host__ __device__ constexpr int sweep_sys_dst(int mode) { return mode == SWEEP_FWD ? 1 : 0; }
 // Elements per 16 bytes.
@@ -127,10 +139,10 @@ __host__ __device__ inline bool sweep_lane(const SkewGeo &q, int mode, int b, in
   l.dlo = 0; l.dhi = q.W - 1;
   const int sys_c = (mode == SWEEP_FWD) ? 1 : 0;  // copy index of the system block
   if (c == sys_c) {
-    l.base = sys_at(slab0, sweep_sys_first(mode), q.T, 0);
+    l.base = sys_t(slab0, q.T, 0) + sweep_sys_first(mode) * q.T;
     l.wstride = SYS_N * q.T;
     l.dst = sweep_sys_dst(mode) * q.T;
-    l.bytes = (mode == SWEEP_FWD_AX ? 8 : 5) * q.T * es;
+    l.bytes = (mode <= SWEEP_FWD_AX ? 8 : 5) * q.T * es;
     l.arr = 0;
     return true;
   }
@@ -298,8 +310,8 @@ bool launch_b_dcmp_f(cudaStream_t s, const BatchMember *bm, const int *pre, int 
 // FP32 sweep of MODE over the members' tiles: vin, vout, vin2 select
 // float vectors (-1: none), rb5 selects rb5 for the sums (else rb0)
 bool launch_b_sweep(cudaStream_t s, int mode, const BatchMember *bm, const int *pre, int nm, long long ntiles,
-                    const SkewGeo &qref, int vin, int vout, int vin2, bool rb5, int nsm, int occ);
-bool b_sweeps_supported(const SkewGeo &qref, int nsm, int occ, long long ntiles);
+                    const SkewGeo &qref, int vin, int vout, int vin2, bool rb5);
+bool b_sweeps_supported(const SkewGeo &qref);
 void launch_b_clear(cudaStream_t s, const BatchMember *bm, int nm);
 void launch_b_gather(cudaStream_t s, const BatchMember *bm, int nm, double *out);
 void launch_b_residual(cudaStream_t s, const BatchMember *bm, const int *pre, int nm, long long nslab);
