@@ -4,26 +4,33 @@
 //
 // The 3x3x3 convolutions are implicit GEMMs on the tcgen05 tensor cores:
 //   k_conv   D[voxel, cout] = sum over 27 taps and cin of X[voxel+tap, cin]
-//            * W[cout, tap, cin].  A CTA of 128 threads owns 128 voxels
-//            (M = 128) and all Cout (N); per tap every thread gathers its
-//            voxel's neighbour row (Cin BF16 values, zero outside the
-//            volume) into a shared-memory stage while the MMAs of the
-//            previous tap run; one thread issues Cin/16 MMAs (K = 16) per
-//            tap into a TMEM accumulator and commits them to the stage's
-//            mbarrier.  The epilogue reads TMEM (tcgen05.ld), adds the
-//            bias, applies ReLU or a ReLU-backward mask and stores BF16 or
-//            FP32.  The input-gradient of a convolution is the same kernel
-//            with the weights flipped and transposed.
+//            * W[cout, tap, cin].  A CTA owns a tile of bx x by voxels of
+//            one z layer and all Cout (N).  For each of the three layers
+//            z-1, z, z+1 it stages the tile with its halo once in shared
+//            memory, as 16-byte rows of 8 channels per voxel in the linear
+//            order of the padded tile; the nine taps of the layer then read
+//            it through descriptors that start 16 bytes x (the tap's
+//            offset) further on.  A row block of the MMA (M = 128) is 128
+//            consecutive voxels of the padded tile; what falls on the
+//            padding is computed and dropped.  The epilogue reads TMEM
+//            (tcgen05.ld), adds the bias, applies ReLU or a ReLU-backward
+//            mask and stores BF16 or FP32.  The input-gradient of a
+//            convolution is the same kernel with the weights flipped and
+//            transposed.
 //   k_wgrad  dW[(tap,cin), cout] = sum over voxels of X[voxel+tap, cin] *
 //            dY[voxel, cout]: M = 27*Cin rows in tiles of 128, N = Cout,
-//            K = a slice of voxels in chunks of 64; each CTA writes its
-//            slice's partial sums, which k_wgrad_reduce adds in slice order.
+//            K = a slice of voxels in chunks of 64, both operands MN-major
+//            (8 channels of a voxel are 16 consecutive bytes in memory and
+//            in the tile); each CTA writes its slice's partial sums, which
+//            k_wgrad_reduce adds in a fixed order.
 // The rest are elementwise or gather kernels on CUDA cores.
 //
 // Layouts: activations channels-last, voxel v = x + X*(y + Y*(z + Z*b)),
-// value [v*C + c]; weights [cout][tap][cin] with tap = (dz+1)*9 + (dy+1)*3
-// + (dx+1).  Every wait on an mbarrier is bounded: on a timeout the CTA
+// value [v*C + c]; FP32 weights [cout][tap][cin] with tap = (dz+1)*9 +
+// (dy+1)*3 + (dx+1), their BF16 copies [tap][cin/8][cout][cin%8], the order
+// of k_conv's tiles.  Every wait on an mbarrier is bounded: on a timeout the CTA
 // records an error, waits once more for its MMAs, frees its TMEM and ends.
+#include <algorithm>
 #include <cuda_bf16.h>
 #include "cadmas_dev.cuh"
 #include "kernels.h"
@@ -63,117 +70,156 @@ __device__ __forceinline__ bool cta_wait(uint64_t *bar, uint32_t parity) {
 }
 
 // ------------------------------------------------------------- k_conv
-// dynamic shared memory: A stages 2 x 128*KC, B stages 2 x N*KC (BF16),
-// then 2 mbarriers and the TMEM address.
 constexpr int CONV_M = 128;
-
+// Tiling of one convolution: tiles of bx x by voxels, nxt x nyt of them per
+// layer; P = bx + 2 voxels per padded row; MT row blocks of 128; PL rows
+// of a staged layer (the last row block reads 2 P + 2 rows past its own);
+// NST stages (3: all layers resident, 2: the third reuses the first's).
+struct ConvPlan {
+  int bx, by, nxt, nyt, P, PL, MT, NST;
+  uint32_t a_bytes, b_bytes;  // of one stage
+  size_t smem;
+};
 __global__ void __launch_bounds__(128) k_conv(Vol g, const bf16 *__restrict__ X, int Cin,
                                               const bf16 *__restrict__ W, const float *__restrict__ bias,
                                               int Cout, int mode, const bf16 *__restrict__ mask, void *Y,
-                                              int *err) {
+                                              int *err, ConvPlan p) {
   extern __shared__ __align__(1024) unsigned char smem[];
-  const int KC = Cin, N = Cout;
-  const uint32_t a_bytes = CONV_M * KC * 2, b_bytes = N * KC * 2;
-  unsigned char *As[2] = {smem, smem + a_bytes};
-  unsigned char *Bs[2] = {smem + 2 * a_bytes, smem + 2 * a_bytes + b_bytes};
-  uint64_t *bar = reinterpret_cast<uint64_t *>(smem + 2 * a_bytes + 2 * b_bytes);
+  const int N = Cout, C8 = Cin >> 3, P = p.P, PL = p.PL;
+  const uint32_t st_bytes = p.a_bytes + p.b_bytes;
+  uint64_t *bar = reinterpret_cast<uint64_t *>(smem + (size_t)p.NST * st_bytes);
   uint32_t *tslot = reinterpret_cast<uint32_t *>(bar + 2);
   const int tid = threadIdx.x, warp = tid >> 5;
-  const uint32_t ncols = umma::tmem_cols(N);
+  const uint32_t ncols = umma::tmem_cols(p.MT * N);
   if (warp == 0) umma::tmem_alloc(tslot, ncols);
   if (tid == 0) {
     umma::mbar_init(&bar[0], 1);
     umma::mbar_init(&bar[1], 1);
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
   }
+  const uint32_t sm0 = umma::smem_u32(smem);
+  unsigned t = blockIdx.x;
+  const int xt = (int)(t % p.nxt);
+  t /= p.nxt;
+  const int yt = (int)(t % p.nyt);
+  t /= p.nyt;
+  const int z = (int)(t % g.Z), b = (int)(t / g.Z);
+  const int x0 = xt * p.bx, y0 = yt * p.by;
+  // layer z + gi - 1 of the padded tile and its nine taps' weights into a
+  // stage; thread tid takes the 16-byte chunks tid, tid + 128, ... of every
+  // row (chunk q of a row: voxel q / C8, channels 8 (q % C8) ..)
+  const int nrow = p.by + 2;
+  auto load = [&](int gi, int st) {
+    const uint32_t As = sm0 + st * st_bytes, Bs = As + p.a_bytes;
+    const int zz = z + gi - 1;
+    const bool zok = zz >= 0 && zz < g.Z;
+    const bf16 *plane = X + (long long)g.X * g.Y * ((long long)g.Z * b + (zok ? zz : z)) * Cin;
+    for (int q = tid; q < P * C8; q += 128) {
+      const int xx = q / C8, c8 = q - xx * C8, gx = x0 + xx - 1;
+      const bool xok = zok && gx >= 0 && gx < g.X;
+      const bf16 *src = plane + ((long long)(xok ? gx : 0) * Cin + c8 * 8);
+      uint32_t dst = As + (uint32_t)(c8 * PL + xx) * 16u;
+      for (int yy = 0; yy < nrow; ++yy, dst += (uint32_t)P * 16u) {
+        const int gy = y0 + yy - 1;
+        const bool ok = xok && gy >= 0 && gy < g.Y;
+        umma::cp16z(dst, src + (long long)(ok ? gy : 0) * g.X * Cin, ok);
+      }
+    }
+    const int nb = 9 * N * C8;
+    const bf16 *wsrc = W + (long long)gi * nb * 8;
+    for (int q = tid; q < nb; q += 128) umma::cp16z(Bs + (uint32_t)q * 16u, wsrc + q * 8, true);
+    umma::cp_commit();
+  };
+  const bool three = p.NST == 3;
+  load(0, 0);
+  load(1, 1);
+  if (three) load(2, 2);
   umma::fence_before_sync();
   __syncthreads();
   umma::fence_after_sync();
   const uint32_t tmem = *tslot;
   const uint32_t idesc = umma::idesc_bf16_f32(CONV_M, N);
-
-  const long long V = g.n();
-  const long long v = (long long)blockIdx.x * CONV_M + tid;
-  int x = 0, y = 0, z = 0, b = 0;
-  const bool live = v < V;
-  if (live) decomp(g, v, x, y, z, b);
-  bool ok = true;
-  int committed = 0;  // commits issued
-  for (int t = 0; t < 27 && ok; ++t) {
-    const int s = t & 1;
-    if (t >= 2) {
-      // the MMAs of tap t-2 have read stage s
-      if (!cta_wait(&bar[s], ((t - 2) >> 1) & 1)) { ok = false; break; }
-    }
-    // A: this thread's row
-    const int dz = t / 9 - 1, dy = (t / 3) % 3 - 1, dx = t % 3 - 1;
-    const long long nv = live ? nbr(g, x, y, z, b, dx, dy, dz) : -1;
-    const uint4 zero = make_uint4(0, 0, 0, 0);
-    for (int c8 = 0; c8 < KC / 8; ++c8) {
-      uint4 q = zero;
-      if (nv >= 0) q = *reinterpret_cast<const uint4 *>(X + nv * Cin + c8 * 8);
-      *reinterpret_cast<uint4 *>(As[s] + umma::kmajor_offset(CONV_M, tid, c8 * 8)) = q;
-    }
-    // B: the tap's N x KC weights; consecutive threads take consecutive
-    // rows n, whose 16-byte chunks are adjacent in the core matrices
-    const int nq = N * (KC / 8);
-    for (int q = tid; q < nq; q += 128) {
-      const int n = q % N, c8 = q / N;
-      const uint4 w = *reinterpret_cast<const uint4 *>(W + ((long long)n * 27 + t) * Cin + c8 * 8);
-      *reinterpret_cast<uint4 *>(Bs[s] + umma::kmajor_offset(N, n, c8 * 8)) = w;
-    }
-    umma::fence_async_smem();
-    __syncthreads();
-    if (tid == 0) {
-      umma::fence_after_sync();
-      const uint32_t a0 = umma::smem_u32(As[s]), b0 = umma::smem_u32(Bs[s]);
-      for (int kk = 0; kk < KC / 16; ++kk) {
-        const uint64_t ad = umma::smem_desc(a0 + kk * 2 * CONV_M * 16, CONV_M * 16, 128);
-        const uint64_t bd = umma::smem_desc(b0 + kk * 2 * N * 16, N * 16, 128);
-        umma::mma_bf16(tmem, ad, bd, idesc, (t | kk) != 0);
+  // the nine taps of layer gi: per accumulator tap by tap, channels in order
+  auto mmas = [&](int gi, int st) {
+    umma::fence_after_sync();
+    const uint32_t a0 = sm0 + st * st_bytes, b0 = a0 + p.a_bytes;
+    const uint64_t ad0 = umma::smem_desc(a0, (uint32_t)PL * 16u, 128), bd0 = umma::smem_desc(b0, (uint32_t)N * 16u, 128);
+    for (int t9 = 0; t9 < 9; ++t9) {
+      const int off = (t9 / 3) * P + t9 % 3;  // rows from the tap's first voxel
+      for (int kk = 0; kk < C8 / 2; ++kk) {
+        const uint64_t bd = bd0 + (uint64_t)((t9 * C8 + 2 * kk) * N);
+        for (int mt = 0; mt < p.MT; ++mt)
+          umma::mma_bf16(tmem + mt * N, ad0 + (uint64_t)(2 * kk * PL + mt * CONV_M + off), bd, idesc,
+                         (gi | t9 | kk) != 0);
       }
-      umma::mma_commit(&bar[s]);
     }
-    ++committed;
+  };
+  bool ok = true;
+  // layer 0, 1, 2 in turn; with two stages the third layer's copies wait
+  // for the first layer's MMAs
+  if (three) umma::cp_wait<2>(); else umma::cp_wait<1>();
+  umma::fence_async_smem();
+  __syncthreads();
+  if (tid == 0) {
+    mmas(0, 0);
+    umma::mma_commit(&bar[0]);
   }
-  // the last commit covers every MMA issued before it
-  if (committed > 0) {
-    // on an earlier timeout this is the one more bounded wait for the MMAs
-    // in flight before the TMEM is freed
-    const int tl = committed - 1;
-    if (!cta_wait(&bar[tl & 1], (tl >> 1) & 1)) ok = false;
+  if (three) umma::cp_wait<1>(); else umma::cp_wait<0>();
+  umma::fence_async_smem();
+  __syncthreads();
+  if (tid == 0) mmas(1, 1);
+  if (three) {
+    umma::cp_wait<0>();
+  } else {
+    ok = cta_wait(&bar[0], 0);
+    if (ok) load(2, 0);
+    umma::cp_wait<0>();
   }
+  umma::fence_async_smem();
+  __syncthreads();
+  if (tid == 0) {
+    if (ok) mmas(2, three ? 2 : 0);
+    umma::mma_commit(&bar[1]);
+  }
+  // the last commit covers every MMA issued before it (after a timeout
+  // this is the one more bounded wait before the TMEM is freed)
+  if (!cta_wait(&bar[1], 0)) ok = false;
   if (!ok) {
     if (tid == 0) atomicOr(err, 1);
   } else {
     umma::fence_after_sync();
-    const uint32_t lane_base = tmem + ((uint32_t)(warp * 32) << 16);
-    for (int c0 = 0; c0 < N; c0 += 8) {
-      float a[8];
-      umma::tmem_ld8(lane_base + c0, a);
-      if (!live) continue;
-      if (bias)
+    for (int mt = 0; mt < p.MT; ++mt) {
+      const int pos = mt * CONV_M + tid, yy = pos / P, xx = pos - yy * P, gx = x0 + xx, gy = y0 + yy;
+      const bool live = xx < p.bx && yy < p.by && gx < g.X && gy < g.Y;
+      const long long v = (long long)gx + (long long)g.X * (gy + (long long)g.Y * (z + (long long)g.Z * b));
+      const uint32_t lane_base = tmem + ((uint32_t)(warp * 32) << 16) + mt * N;
+      for (int c0 = 0; c0 < N; c0 += 8) {
+        float a[8];
+        umma::tmem_ld8(lane_base + c0, a);
+        if (!live) continue;
+        if (bias)
 #pragma unroll
-        for (int i = 0; i < 8; ++i) a[i] += bias[c0 + i];
-      if (mode == CONV_RELU_BF16) {
+          for (int i = 0; i < 8; ++i) a[i] += bias[c0 + i];
+        if (mode == CONV_RELU_BF16) {
 #pragma unroll
-        for (int i = 0; i < 8; ++i) a[i] = fmaxf(a[i], 0.0f);
-      } else if (mode == CONV_MASK_BF16) {
-        // input gradient times the ReLU derivative of the layer below
-        const uint4 mq = *reinterpret_cast<const uint4 *>(mask + v * Cout + c0);
-        const bf16 *m = reinterpret_cast<const bf16 *>(&mq);
+          for (int i = 0; i < 8; ++i) a[i] = fmaxf(a[i], 0.0f);
+        } else if (mode == CONV_MASK_BF16) {
+          // input gradient times the ReLU derivative of the layer below
+          const uint4 mq = *reinterpret_cast<const uint4 *>(mask + v * Cout + c0);
+          const bf16 *m = reinterpret_cast<const bf16 *>(&mq);
 #pragma unroll
-        for (int i = 0; i < 8; ++i) a[i] = (__bfloat162float(m[i]) > 0.0f) ? a[i] : 0.0f;
-      }
-      if (mode == CONV_F32) {
-        float *o = reinterpret_cast<float *>(Y) + v * Cout + c0;
+          for (int i = 0; i < 8; ++i) a[i] = (__bfloat162float(m[i]) > 0.0f) ? a[i] : 0.0f;
+        }
+        if (mode == CONV_F32) {
+          float *o = reinterpret_cast<float *>(Y) + v * Cout + c0;
 #pragma unroll
-        for (int i = 0; i < 8; ++i) o[i] = a[i];
-      } else {
-        __align__(16) bf16 o[8];
+          for (int i = 0; i < 8; ++i) o[i] = a[i];
+        } else {
+          __align__(16) bf16 o[8];
 #pragma unroll
-        for (int i = 0; i < 8; ++i) o[i] = __float2bfloat16(a[i]);
-        *reinterpret_cast<uint4 *>(reinterpret_cast<bf16 *>(Y) + v * Cout + c0) = *reinterpret_cast<uint4 *>(o);
+          for (int i = 0; i < 8; ++i) o[i] = __float2bfloat16(a[i]);
+          *reinterpret_cast<uint4 *>(reinterpret_cast<bf16 *>(Y) + v * Cout + c0) = *reinterpret_cast<uint4 *>(o);
+        }
       }
     }
   }
@@ -184,86 +230,94 @@ __global__ void __launch_bounds__(128) k_conv(Vol g, const bf16 *__restrict__ X,
 
 // ------------------------------------------------------------ k_wgrad
 // rows m = tap*Cin + cin (27*Cin of them, tiles of 128), N = Cout, K = the
-// voxels of this CTA's slice in chunks of 64.
-constexpr int WG_K = 64;
+// voxels of this CTA's slice in chunks of 64, WG_ST stages.  Tiles in
+// shared memory: [8-channel block][voxel] of 16 bytes, so a thread copies
+// 16 bytes of its voxel (or of its tap's neighbour) at a time.
+constexpr int WG_K = 64, WG_ST = 3;
 
 __global__ void __launch_bounds__(128) k_wgrad(Vol g, const bf16 *__restrict__ X, int Cin,
                                                const bf16 *__restrict__ DY, int Cout, long long slice,
                                                float *__restrict__ part, int *err) {
   extern __shared__ __align__(1024) unsigned char smem[];
-  const int N = Cout;
-  const uint32_t a_bytes = 128 * WG_K * 2, b_bytes = N * WG_K * 2;
-  unsigned char *As[2] = {smem, smem + a_bytes};
-  unsigned char *Bs[2] = {smem + 2 * a_bytes, smem + 2 * a_bytes + b_bytes};
-  uint64_t *bar = reinterpret_cast<uint64_t *>(smem + 2 * a_bytes + 2 * b_bytes);
-  uint32_t *tslot = reinterpret_cast<uint32_t *>(bar + 2);
+  const int N = Cout, C8 = Cin >> 3, N8 = N >> 3;
+  const uint32_t a_bytes = 128 * WG_K * 2, b_bytes = N * WG_K * 2, st_bytes = a_bytes + b_bytes;
+  uint64_t *bar = reinterpret_cast<uint64_t *>(smem + WG_ST * st_bytes);
+  uint32_t *tslot = reinterpret_cast<uint32_t *>(bar + WG_ST);
   const int tid = threadIdx.x, warp = tid >> 5;
   const uint32_t ncols = umma::tmem_cols(N);
   if (warp == 0) umma::tmem_alloc(tslot, ncols);
   if (tid == 0) {
-    umma::mbar_init(&bar[0], 1);
-    umma::mbar_init(&bar[1], 1);
+    for (int i = 0; i < WG_ST; ++i) umma::mbar_init(&bar[i], 1);
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
   }
   umma::fence_before_sync();
   __syncthreads();
   umma::fence_after_sync();
-  const uint32_t tmem = *tslot;
-  const uint32_t idesc = umma::idesc_bf16_f32(128, N);
+  const uint32_t tmem = *tslot, sm0 = umma::smem_u32(smem);
+  const uint32_t idesc = umma::idesc_bf16_f32_mn(128, N);
   const int M = 27 * Cin;
   const int m0 = blockIdx.x * 128;
   const long long V = g.n();
   const long long v0 = (long long)blockIdx.y * slice;
   const long long v1 = min(V, v0 + slice);
-  const int nchunk = (int)((v1 - v0 + WG_K - 1) / WG_K);
-  // thread: voxel k = tid % 64 of each chunk, row half h = tid / 64
+  const int nchunk = v1 > v0 ? (int)((v1 - v0 + WG_K - 1) / WG_K) : 0;
+  // thread: voxel kq of each chunk; of the tile's 16 row blocks (8 channels
+  // of one tap each) h, h+2, ..., of the N8 blocks of dY h, h+2, ...
   const int kq = tid & (WG_K - 1), h = tid >> 6;
-  bool ok = true;
-  int committed = 0;
-  for (int ch = 0; ch < nchunk && ok; ++ch) {
-    const int s = ch & 1;
-    if (ch >= 2 && !cta_wait(&bar[s], ((ch - 2) >> 1) & 1)) { ok = false; break; }
+  int dx[8], dy[8], dz[8], dc[8];  // tap offset and first channel; dc < 0: past the last row
+#pragma unroll
+  for (int i = 0; i < 8; ++i) {
+    const int gb = m0 / 8 + 2 * i + h, t = gb / C8;
+    dx[i] = t % 3 - 1; dy[i] = (t / 3) % 3 - 1; dz[i] = t / 9 - 1;
+    dc[i] = t < 27 ? (gb - t * C8) * 8 : -1;
+  }
+  auto load = [&](int ch) {
+    const uint32_t As = sm0 + (ch % WG_ST) * st_bytes, Bs = As + a_bytes;
     const long long v = v0 + (long long)ch * WG_K + kq;
     const bool live = v < v1;
     int x = 0, y = 0, z = 0, b = 0;
     if (live) decomp(g, v, x, y, z, b);
-    // A: rows m0 + 64h .. m0 + 64h + 63 of column kq
-    for (int r = 64 * h; r < 64 * h + 64; ++r) {
-      const int m = m0 + r;
-      bf16 val = __float2bfloat16(0.0f);
-      if (live && m < M) {
-        const int t = m / Cin, ci = m % Cin;
-        const long long nv = nbr(g, x, y, z, b, t % 3 - 1, (t / 3) % 3 - 1, t / 9 - 1);
-        if (nv >= 0) val = X[nv * Cin + ci];
-      }
-      *reinterpret_cast<bf16 *>(As[s] + umma::kmajor_offset(128, r, kq)) = val;
+#pragma unroll
+    for (int i = 0; i < 8; ++i) {
+      const long long nv = live && dc[i] >= 0 ? nbr(g, x, y, z, b, dx[i], dy[i], dz[i]) : -1;
+      umma::cp16z(As + (uint32_t)((2 * i + h) * WG_K + kq) * 16u, nv >= 0 ? X + nv * Cin + dc[i] : X, nv >= 0);
     }
-    // B: rows n of column kq (half the threads)
-    if (h == 0) {
-      for (int n = 0; n < N; ++n) {
-        const bf16 val = live ? DY[v * Cout + n] : __float2bfloat16(0.0f);
-        *reinterpret_cast<bf16 *>(Bs[s] + umma::kmajor_offset(N, n, kq)) = val;
-      }
-    }
+    for (int n = h; n < N8; n += 2)
+      umma::cp16z(Bs + (uint32_t)(n * WG_K + kq) * 16u, live ? DY + v * Cout + n * 8 : DY, live);
+  };
+  bool ok = true;
+  int committed = 0;
+  for (int c = 0; c < WG_ST - 1; ++c) {
+    if (c < nchunk) load(c);
+    umma::cp_commit();
+  }
+  for (int ch = 0; ch < nchunk; ++ch) {
+    const int s = ch % WG_ST, nx = ch + WG_ST - 1;
+    // chunk nx goes where chunk ch-1 lies: its MMAs must have read it
+    if (ch >= 1 && !cta_wait(&bar[(ch - 1) % WG_ST], ((ch - 1) / WG_ST) & 1)) { ok = false; break; }
+    if (nx < nchunk) load(nx);
+    umma::cp_commit();
+    umma::cp_wait<WG_ST - 1>();
     umma::fence_async_smem();
     __syncthreads();
     if (tid == 0) {
       umma::fence_after_sync();
-      const uint32_t a0 = umma::smem_u32(As[s]), b0 = umma::smem_u32(Bs[s]);
+      const uint32_t a0 = sm0 + s * st_bytes, b0 = a0 + a_bytes;
       for (int kk = 0; kk < WG_K / 16; ++kk) {
-        const uint64_t ad = umma::smem_desc(a0 + kk * 2 * 128 * 16, 128 * 16, 128);
-        const uint64_t bd = umma::smem_desc(b0 + kk * 2 * N * 16, N * 16, 128);
+        const uint64_t ad = umma::smem_desc(a0 + kk * 256, 128, WG_K * 16);
+        const uint64_t bd = umma::smem_desc(b0 + kk * 256, 128, WG_K * 16);
         umma::mma_bf16(tmem, ad, bd, idesc, (ch | kk) != 0);
       }
       umma::mma_commit(&bar[s]);
     }
     ++committed;
   }
+  umma::cp_wait<0>();
   if (committed > 0) {
     // on an earlier timeout this is the one more bounded wait for the MMAs
     // in flight before the TMEM is freed
     const int tl = committed - 1;
-    if (!cta_wait(&bar[tl & 1], (tl >> 1) & 1)) ok = false;
+    if (!cta_wait(&bar[tl % WG_ST], (tl / WG_ST) & 1)) ok = false;
   }
   if (!ok) {
     if (tid == 0) atomicOr(err, 1);
@@ -289,115 +343,177 @@ __global__ void __launch_bounds__(128) k_wgrad(Vol g, const bf16 *__restrict__ X
 }
 
 // dW[cout][tap][cin] = sum over slices (in order) of part[s][tap*Cin+cin][cout]
-__global__ void k_wgrad_reduce(const float *part, int nslices, int Cin, int Cout, float *dW) {
+__global__ void __launch_bounds__(64) k_wgrad_reduce(const float *part, int nslices, int Cin, int Cout, float *dW) {
   const int M = 27 * Cin;
-  const int i = blockIdx.x * blockDim.x + threadIdx.x;
+  const int i = blockIdx.x * 64 + threadIdx.x;
   if (i >= M * Cout) return;
-  const int m = i / Cout, n = i % Cout;
   float s = 0.0f;
-  for (int q = 0; q < nslices; ++q) s += part[((long long)q * M + m) * Cout + n];
-  const int t = m / Cin, ci = m % Cin;
+  for (int q0 = 0; q0 < nslices; q0 += 16) {  // 16 loads in flight, added in order
+    float r[16];
+#pragma unroll
+    for (int j = 0; j < 16; ++j) r[j] = q0 + j < nslices ? part[(long long)(q0 + j) * M * Cout + i] : 0.0f;
+#pragma unroll
+    for (int j = 0; j < 16; ++j)
+      if (q0 + j < nslices) s += r[j];
+  }
+  const int m = i / Cout, n = i % Cout, t = m / Cin, ci = m % Cin;
   dW[((long long)n * 27 + t) * Cin + ci] = s;
 }
 
-// bias gradient: db[c] = sum over voxels of dY[v][c] (FP32 partials per block
-// of 1024 voxels, then the same in order)
-__global__ void k_bias_part(const bf16 *DY, long long V, int C, float *part) {
-  const int c = threadIdx.x;
-  if (c >= C) return;
+// Column sums of a block's rows, in the order of the rows: the rows pass
+// through shared memory (coalesced loads by all threads), one thread per
+// column adds.  The order is the reference's sequential one; what bounds the
+// kernels is that chain (4 cycles per row), not the loads.
+constexpr int SUM_ROWS = 64;
+// bias gradient: db[c] = sum over voxels of dY[v][c] (FP32 partials per
+// block of 1024 voxels, then the same in order); C <= 64
+__global__ void __launch_bounds__(256) k_bias_part(const bf16 *DY, long long V, int C, float *part) {
+  __shared__ float row[2][SUM_ROWS * 64];
   const long long v0 = (long long)blockIdx.x * 1024, v1 = min(V, v0 + 1024);
+  const int C8 = C >> 3;
   float s = 0.0f;
-  for (long long v = v0; v < v1; ++v) s += __bfloat162float(DY[v * C + c]);
-  part[(long long)blockIdx.x * C + c] = s;
+  auto fill = [&](long long v, float *to) {
+    for (int q = threadIdx.x; q < SUM_ROWS * C8; q += 256) {
+      const int r = q / C8, c = (q - r * C8) * 8;
+      if (v + r >= v1) break;
+      const uint4 w = *reinterpret_cast<const uint4 *>(DY + (v + r) * C + c);
+      const bf16 *e = reinterpret_cast<const bf16 *>(&w);
+#pragma unroll
+      for (int i = 0; i < 8; ++i) to[r * C + c + i] = __bfloat162float(e[i]);
+    }
+  };
+  fill(v0, row[0]);
+  int k = 0;
+  for (long long v = v0; v < v1; v += SUM_ROWS, k ^= 1) {
+    __syncthreads();
+    if (v + SUM_ROWS < v1) fill(v + SUM_ROWS, row[k ^ 1]);
+    if (threadIdx.x < C) {
+      const int n = (int)min((long long)SUM_ROWS, v1 - v);
+#pragma unroll 8
+      for (int r = 0; r < n; ++r) s += row[k][r * C + threadIdx.x];
+    }
+  }
+  if (threadIdx.x < C) part[(long long)blockIdx.x * C + threadIdx.x] = s;
 }
-__global__ void k_bias_reduce(const float *part, int nb, int C, float *db) {
-  const int c = threadIdx.x;
-  if (c >= C) return;
+// db[c] = sum of nb block partials in order; C <= 64
+__global__ void __launch_bounds__(256) k_bias_reduce(const float *part, int nb, int C, float *db) {
+  __shared__ float row[2][SUM_ROWS * 64];
   float s = 0.0f;
-  for (int q = 0; q < nb; ++q) s += part[(long long)q * C + c];
-  db[c] = s;
+  auto fill = [&](int q0, float *to) {
+    const int n = min(SUM_ROWS, nb - q0) * C;
+    for (int i = threadIdx.x; i < n; i += 256) to[i] = part[(long long)q0 * C + i];
+  };
+  fill(0, row[0]);
+  int k = 0;
+  for (int q = 0; q < nb; q += SUM_ROWS, k ^= 1) {
+    __syncthreads();
+    if (q + SUM_ROWS < nb) fill(q + SUM_ROWS, row[k ^ 1]);
+    if (threadIdx.x < C) {
+      const int n = min(SUM_ROWS, nb - q);
+#pragma unroll 8
+      for (int r = 0; r < n; ++r) s += row[k][r * C + threadIdx.x];
+    }
+  }
+  if (threadIdx.x < C) db[threadIdx.x] = s;
 }
 
 // ------------------------------------------------ pooling and upsampling
+// All of them move 8 channels (16 bytes) per thread: element i of the
+// launch is channel block i % (C/8) of voxel i / (C/8).  They are bound by
+// memory; one channel per thread took up to five times as long (upsampling
+// and concatenation to 48 channels of 1.3 M voxels: 416 us).
+struct alignas(16) B8 { bf16 v[8]; };
+__device__ __forceinline__ B8 ld8(const bf16 *p) { return *reinterpret_cast<const B8 *>(p); }
+__device__ __forceinline__ void st8(bf16 *p, const B8 &q) { *reinterpret_cast<B8 *>(p) = q; }
+__device__ __forceinline__ bool split8(long long i, long long n, int C, long long &v, int &c) {
+  const int C8 = C >> 3;
+  if (i >= n * C8) return false;
+  v = i / C8;
+  c = (int)(i - v * C8) * 8;
+  return true;
+}
+__device__ __forceinline__ long long coarse_of(const Vol &gc, int x, int y, int z, int b) {
+  return (long long)(x >> 1) + (long long)gc.X * ((long long)(y >> 1) + (long long)gc.Y *
+                                                    ((long long)(z >> 1) + (long long)gc.Z * b));
+}
+// sum of the 8 children of coarse voxel (x,y,z,b), channels c..c+7 of C
+__device__ __forceinline__ void children8(const Vol &gf, int x, int y, int z, int b, const bf16 *F, int C, int c,
+                                          float *s) {
+#pragma unroll
+  for (int i = 0; i < 8; ++i) s[i] = 0.0f;
+#pragma unroll
+  for (int q = 0; q < 8; ++q) {
+    const B8 f = ld8(F + nbr(gf, 2 * x, 2 * y, 2 * z, b, q & 1, (q >> 1) & 1, q >> 2) * C + c);
+#pragma unroll
+    for (int i = 0; i < 8; ++i) s[i] += __bfloat162float(f.v[i]);
+  }
+}
 // 2x2x2 average: coarse (X/2, Y/2, Z/2) from fine
 __global__ void k_pool(Vol gc, const bf16 *F, int C, bf16 *Cc) {
-  const long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= gc.n() * C) return;
-  const long long vc = i / C;
-  const int c = (int)(i % C);
-  int x, y, z, b;
+  long long vc;
+  int c, x, y, z, b;
+  if (!split8(blockIdx.x * (long long)blockDim.x + threadIdx.x, gc.n(), C, vc, c)) return;
   decomp(gc, vc, x, y, z, b);
   const Vol gf{2 * gc.X, 2 * gc.Y, 2 * gc.Z, gc.B};
-  float s = 0.0f;
-  for (int q = 0; q < 8; ++q) {
-    const long long vf = nbr(gf, 2 * x, 2 * y, 2 * z, b, q & 1, (q >> 1) & 1, q >> 2);
-    s += __bfloat162float(F[vf * C + c]);
-  }
-  Cc[i] = __float2bfloat16(0.125f * s);
+  float s[8];
+  children8(gf, x, y, z, b, F, C, c, s);
+  B8 o;
+#pragma unroll
+  for (int i = 0; i < 8; ++i) o.v[i] = __float2bfloat16(0.125f * s[i]);
+  st8(Cc + vc * C + c, o);
 }
-// its backward, added to dF (fine) where acc != 0, else stored
-__global__ void k_pool_bwd(Vol gc, const bf16 *dC, int C, bf16 *dF, int acc) {
+// its backward, added to dF (fine), then masked by the ReLU of the fine
+// activation: dF = bf16(dC/8 + dF) where act > 0, else 0
+__global__ void k_pool_bwd(Vol gc, const bf16 *dC, int C, bf16 *dF, const bf16 *act) {
   const Vol gf{2 * gc.X, 2 * gc.Y, 2 * gc.Z, gc.B};
-  const long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= gf.n() * C) return;
-  const long long vf = i / C;
-  const int c = (int)(i % C);
-  int x, y, z, b;
+  long long vf;
+  int c, x, y, z, b;
+  if (!split8(blockIdx.x * (long long)blockDim.x + threadIdx.x, gf.n(), C, vf, c)) return;
   decomp(gf, vf, x, y, z, b);
-  const long long vc = (long long)(x >> 1) + (long long)gc.X * ((long long)(y >> 1) + (long long)gc.Y *
-                                                                 ((long long)(z >> 1) + (long long)gc.Z * b));
-  float d = 0.125f * __bfloat162float(dC[vc * C + c]);
-  if (acc) d += __bfloat162float(dF[i]);
-  dF[i] = __float2bfloat16(d);
+  const B8 q = ld8(dC + coarse_of(gc, x, y, z, b) * C + c), a = ld8(act + vf * C + c);
+  B8 o = ld8(dF + vf * C + c);
+#pragma unroll
+  for (int i = 0; i < 8; ++i) {
+    float e = 0.125f * __bfloat162float(q.v[i]);
+    e += __bfloat162float(o.v[i]);
+    o.v[i] = __bfloat162float(a.v[i]) > 0.0f ? __float2bfloat16(e) : __float2bfloat16(0.0f);
+  }
+  st8(dF + vf * C + c, o);
 }
 // out[vf] = (coarse[vf/2] (C1 channels), skip[vf] (C2 channels))
 __global__ void k_upcat(Vol gf, const bf16 *Cc, int C1, const bf16 *S, int C2, bf16 *O) {
   const int C = C1 + C2;
-  const long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= gf.n() * C) return;
-  const long long vf = i / C;
-  const int c = (int)(i % C);
-  if (c >= C1) { O[i] = S[vf * C2 + (c - C1)]; return; }
-  int x, y, z, b;
-  decomp(gf, vf, x, y, z, b);
-  const Vol gc{gf.X / 2, gf.Y / 2, gf.Z / 2, gf.B};
-  const long long vc = (long long)(x >> 1) + (long long)gc.X * ((long long)(y >> 1) + (long long)gc.Y *
-                                                                 ((long long)(z >> 1) + (long long)gc.Z * b));
-  O[i] = Cc[vc * C1 + c];
+  long long vf;
+  int c, x, y, z, b;
+  if (!split8(blockIdx.x * (long long)blockDim.x + threadIdx.x, gf.n(), C, vf, c)) return;
+  const bf16 *src = S + vf * C2 + (c - C1);
+  if (c < C1) {
+    decomp(gf, vf, x, y, z, b);
+    const Vol gc{gf.X / 2, gf.Y / 2, gf.Z / 2, gf.B};
+    src = Cc + coarse_of(gc, x, y, z, b) * C1 + c;
+  }
+  st8(O + vf * C + c, ld8(src));
 }
-// backward: dCoarse = sum of the 8 children's first C1 channels; dSkip
-// (+)= the last C2 channels
+// backward: dCoarse = sum of the 8 children's first C1 channels; dSkip =
+// the last C2 channels
 __global__ void k_upcat_bwd_coarse(Vol gc, const bf16 *dO, int C1, int C2, bf16 *dC) {
-  const int C = C1 + C2;
-  const long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= gc.n() * C1) return;
-  const long long vc = i / C1;
-  const int c = (int)(i % C1);
-  int x, y, z, b;
+  long long vc;
+  int c, x, y, z, b;
+  if (!split8(blockIdx.x * (long long)blockDim.x + threadIdx.x, gc.n(), C1, vc, c)) return;
   decomp(gc, vc, x, y, z, b);
   const Vol gf{2 * gc.X, 2 * gc.Y, 2 * gc.Z, gc.B};
-  float s = 0.0f;
-  for (int q = 0; q < 8; ++q) {
-    const long long vf = nbr(gf, 2 * x, 2 * y, 2 * z, b, q & 1, (q >> 1) & 1, q >> 2);
-    s += __bfloat162float(dO[vf * C + c]);
-  }
-  dC[i] = __float2bfloat16(s);
+  float s[8];
+  children8(gf, x, y, z, b, dO, C1 + C2, c, s);
+  B8 o;
+#pragma unroll
+  for (int i = 0; i < 8; ++i) o.v[i] = __float2bfloat16(s[i]);
+  st8(dC + vc * C1 + c, o);
 }
-__global__ void k_upcat_bwd_skip(long long Vf, const bf16 *dO, int C1, int C2, bf16 *dS, int acc) {
-  const int C = C1 + C2;
-  const long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= Vf * C2) return;
-  const long long vf = i / C2;
-  const int c = (int)(i % C2);
-  float d = __bfloat162float(dO[vf * C + C1 + c]);
-  if (acc) d += __bfloat162float(dS[i]);
-  dS[i] = __float2bfloat16(d);
-}
-// dX *= (act > 0) (ReLU backward in place)
-__global__ void k_relu_mask(long long n, const bf16 *act, bf16 *d) {
-  const long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= n) return;
-  if (!(__bfloat162float(act[i]) > 0.0f)) d[i] = __float2bfloat16(0.0f);
+__global__ void k_upcat_bwd_skip(long long Vf, const bf16 *dO, int C1, int C2, bf16 *dS) {
+  long long vf;
+  int c;
+  if (!split8(blockIdx.x * (long long)blockDim.x + threadIdx.x, Vf, C2, vf, c)) return;
+  st8(dS + vf * C2 + c, ld8(dO + vf * (C1 + C2) + C1 + c));
 }
 
 // ------------------------------------------------------------- head
@@ -406,7 +522,11 @@ __global__ void k_head(long long V, const bf16 *A, int C, const float *wh, const
   const long long v = (long long)blockIdx.x * blockDim.x + threadIdx.x;
   if (v >= V) return;
   float s = bh[0];
-  for (int c = 0; c < C; ++c) s += wh[c] * __bfloat162float(A[v * C + c]);
+  for (int c = 0; c < C; c += 8) {
+    const B8 a = ld8(A + v * C + c);
+#pragma unroll
+    for (int i = 0; i < 8; ++i) s += wh[c + i] * __bfloat162float(a.v[i]);
+  }
   Yo[v] = s;
 }
 // masked MSE: dy = 2 (y - t) m / sum(m); per-block partial loss sums
@@ -430,22 +550,43 @@ __global__ void k_mse(long long V, const float *Yo, const float *T, const float 
 }
 // head backward: dA[v][c] = dy[v] wh[c] (BF16), masked by the ReLU of A
 __global__ void k_head_bwd_act(long long V, const float *dy, const bf16 *A, int C, const float *wh, bf16 *dA) {
-  const long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= V * C) return;
-  const long long v = i / C;
-  const int c = (int)(i % C);
-  const float d = (__bfloat162float(A[i]) > 0.0f) ? dy[v] * wh[c] : 0.0f;
-  dA[i] = __float2bfloat16(d);
+  long long v;
+  int c;
+  if (!split8(blockIdx.x * (long long)blockDim.x + threadIdx.x, V, C, v, c)) return;
+  const B8 a = ld8(A + v * C + c);
+  const float d = dy[v];
+  B8 o;
+#pragma unroll
+  for (int i = 0; i < 8; ++i) o.v[i] = __float2bfloat16(__bfloat162float(a.v[i]) > 0.0f ? d * wh[c + i] : 0.0f);
+  st8(dA + v * C + c, o);
 }
 // head parameter gradients: partials over blocks of 1024 voxels of
-// (dy a[c], dy) in FP32
-__global__ void k_head_bwd_par(long long V, const float *dy, const bf16 *A, int C, float *part) {
-  const int c = threadIdx.x;
-  if (c > C) return;
+// (dy a[c], dy) in FP32, C = 16, added in the order of the voxels
+__global__ void __launch_bounds__(256) k_head_bwd_par(long long V, const float *dy, const bf16 *A, int C, float *part) {
+  __shared__ float row[2][SUM_ROWS * 17];
   const long long v0 = (long long)blockIdx.x * 1024, v1 = min(V, v0 + 1024);
   float s = 0.0f;
-  for (long long v = v0; v < v1; ++v) s += dy[v] * (c < C ? __bfloat162float(A[v * C + c]) : 1.0f);
-  part[(long long)blockIdx.x * (C + 1) + c] = s;
+  auto fill = [&](long long v, float *to) {
+    const int r = threadIdx.x >> 1, c = (threadIdx.x & 1) * 8;
+    if (r >= SUM_ROWS || v + r >= v1) return;
+    const float d = dy[v + r];
+    const B8 a = ld8(A + (v + r) * C + c);
+#pragma unroll
+    for (int i = 0; i < 8; ++i) to[r * 17 + c + i] = d * __bfloat162float(a.v[i]);
+    if (c == 0) to[r * 17 + 16] = d * 1.0f;
+  };
+  fill(v0, row[0]);
+  int k = 0;
+  for (long long v = v0; v < v1; v += SUM_ROWS, k ^= 1) {
+    __syncthreads();
+    if (v + SUM_ROWS < v1) fill(v + SUM_ROWS, row[k ^ 1]);
+    if (threadIdx.x <= C) {
+      const int n = (int)min((long long)SUM_ROWS, v1 - v);
+#pragma unroll 8
+      for (int r = 0; r < n; ++r) s += row[k][r * 17 + threadIdx.x];
+    }
+  }
+  if (threadIdx.x <= C) part[(long long)blockIdx.x * (C + 1) + threadIdx.x] = s;
 }
 
 // ---------------------------------------------------- residual loss
@@ -514,23 +655,29 @@ __global__ void k_adam(long long n, float *p, const float *g, float *m, float *v
   v[i] = vi;
   p[i] -= lr * (mi / c1) / (sqrtf(vi / c2) + eps);
 }
-// weights [cout][27][cin] FP32 -> BF16 forward copy and the input-gradient
-// copy Wt[cin][26 - tap][cout]
+// weights [cout][27][cin] FP32 -> BF16 forward copy [tap][cin/8][cout][cin%8]
+// and the input-gradient copy, cin and cout swapped and tap 26 - tap
 __global__ void k_wcast(const float *w, int Cin, int Cout, bf16 *wf, bf16 *wt) {
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= Cout * 27 * Cin) return;
   const int ci = i % Cin, t = (i / Cin) % 27, co = i / (27 * Cin);
   const bf16 q = __float2bfloat16(w[i]);
-  wf[i] = q;
-  if (wt) wt[((long long)ci * 27 + (26 - t)) * Cout + co] = q;
+  wf[((t * (Cin >> 3) + (ci >> 3)) * Cout + co) * 8 + (ci & 7)] = q;
+  if (wt) wt[(((26 - t) * (Cout >> 3) + (co >> 3)) * Cin + ci) * 8 + (co & 7)] = q;
 }
 // network input: 4 FP32 channels per voxel -> 16 BF16 channels (12 zero)
 __global__ void k_pack_in(long long V, const float *x4, bf16 *x16) {
   const long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= V * 16) return;
-  const long long v = i >> 4;
-  const int c = (int)(i & 15);
-  x16[i] = __float2bfloat16(c < 4 ? x4[v * 4 + c] : 0.0f);
+  if (i >= V * 2) return;
+  B8 o;
+#pragma unroll
+  for (int c = 0; c < 8; ++c) o.v[c] = __float2bfloat16(0.0f);
+  if ((i & 1) == 0) {
+    const float4 f = *reinterpret_cast<const float4 *>(x4 + (i >> 1) * 4);
+    o.v[0] = __float2bfloat16(f.x); o.v[1] = __float2bfloat16(f.y);
+    o.v[2] = __float2bfloat16(f.z); o.v[3] = __float2bfloat16(f.w);
+  }
+  st8(x16 + i * 8, o);
 }
 __global__ void k_f32_to_bf16(long long n, const float *a, bf16 *b) {
   const long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
@@ -544,19 +691,53 @@ __global__ void k_fill_bf16(long long n, bf16 *a) {
 // ------------------------------------------------------------ launchers
 static inline unsigned nb(long long n, int t) { return (unsigned)((n + t - 1) / t); }
 
-// At least 56 KB of dynamic shared memory per CTA, so that at most four
-// CTAs share an SM and their TMEM (at most 128 columns each) fits in the
-// SM's 512 columns without an allocation having to wait.
-static size_t smem_floor(size_t b) { return b < 56 * 1024 ? 56 * 1024 : b; }
-size_t conv_smem_bytes(int Cin, int Cout) {
-  return smem_floor((size_t)2 * CONV_M * Cin * 2 + (size_t)2 * Cout * Cin * 2 + 32);
+// The CTAs that share an SM must find their TMEM columns free (512 per
+// SM): a CTA with more columns asks for more shared memory.
+static size_t smem_floor(size_t b, uint32_t cols) {
+  const size_t f = cols <= 128 ? 56 * 1024 : (cols <= 256 ? 80 * 1024 : 120 * 1024);
+  return b < f ? f : b;
 }
-size_t wgrad_smem_bytes(int Cout) { return smem_floor((size_t)2 * 128 * WG_K * 2 + (size_t)2 * Cout * WG_K * 2 + 32); }
+// Tile of a convolution: rows of at most 126 voxels; as many rows as make
+// the least work per voxel, counting the MMAs' rows (128 per row block) and
+// half as much for each staged voxel, within the shared memory of two CTAs
+// per SM where that can be (else of one) and 256 TMEM columns (one row block
+// may use more).  Three stages where they fit.
+static ConvPlan conv_plan(const Vol &g, int Cin, int Cout) {
+  ConvPlan best{};
+  double cost = 0.0;
+  const int nxt0 = (g.X + 125) / 126;
+  for (size_t cap : {(size_t)112 * 1024, (size_t)225 * 1024}) {
+    for (int nxt = nxt0; nxt <= nxt0 + 3; ++nxt)
+      for (int nst = 3; nst >= 2; --nst) {
+        const int bx = (g.X + nxt - 1) / nxt, P = bx + 2;
+        for (int by = 1; by <= g.Y && by <= 128; ++by) {
+          ConvPlan p{};
+          p.bx = bx; p.by = by; p.nxt = nxt; p.nyt = (g.Y + by - 1) / by; p.P = P; p.NST = nst;
+          p.MT = (by * P + CONV_M - 1) / CONV_M;
+          if (p.MT > 1 && p.MT * Cout > 256) break;
+          p.PL = (p.MT * CONV_M + 2 * P + 2 + 7) & ~7;
+          p.PL += 4;  // the two 8-channel rows of a voxel in different banks
+          p.a_bytes = (uint32_t)(Cin / 8 * p.PL * 16);
+          p.b_bytes = (uint32_t)(9 * Cin * Cout * 2);
+          const size_t need = (size_t)nst * (p.a_bytes + p.b_bytes) + 64;
+          if (need > cap) break;
+          p.smem = smem_floor(need, umma::tmem_cols(p.MT * Cout));
+          const double c = (double)nxt * p.nyt * (p.MT * 128.0 + 0.5 * (by + 2) * P + 128.0) * (nst == 2 ? 1.15 : 1.0);
+          if (best.MT == 0 || c < cost) { best = p; cost = c; }
+        }
+      }
+    if (best.MT > 0) break;
+  }
+  return best;
+}
+static size_t wgrad_smem_bytes(int Cout) {
+  return smem_floor((size_t)WG_ST * (128 + Cout) * WG_K * 2 + 64, umma::tmem_cols(Cout));
+}
 
 bool unet_kernels_configure() {
   static int done = 0;
   if (done) return done > 0;
-  const int mx = 200 * 1024;
+  const int mx = 227 * 1024;
   bool ok = cudaFuncSetAttribute(k_conv, cudaFuncAttributeMaxDynamicSharedMemorySize, mx) == cudaSuccess &&
             cudaFuncSetAttribute(k_wgrad, cudaFuncAttributeMaxDynamicSharedMemorySize, mx) == cudaSuccess;
   done = ok ? 1 : -1;
@@ -566,52 +747,53 @@ bool unet_kernels_configure() {
 void launch_conv(cudaStream_t s, int X, int Y, int Z, int B, const void *x, int Cin, const void *w, const float *bias,
                  int Cout, int mode, const void *mask, void *y, int *err) {
   const Vol g{X, Y, Z, B};
-  k_conv<<<nb(g.n(), CONV_M), 128, conv_smem_bytes(Cin, Cout), s>>>(
-      g, (const bf16 *)x, Cin, (const bf16 *)w, bias, Cout, mode, (const bf16 *)mask, y, err);
+  const ConvPlan p = conv_plan(g, Cin, Cout);
+  k_conv<<<(unsigned)((long long)p.nxt * p.nyt * Z * B), 128, p.smem, s>>>(
+      g, (const bf16 *)x, Cin, (const bf16 *)w, bias, Cout, mode, (const bf16 *)mask, y, err, p);
   count_launch();
 }
+// Voxels per slice of a weight gradient.  The slices fix the order in which
+// the tensor cores add (their FP32 accumulation depends on it at 1e-4 of a
+// gradient), so they are the same at every size.
+constexpr long long WGRAD_SLICE = 8192;
+long long wgrad_slices(long long V) { return (V + WGRAD_SLICE - 1) / WGRAD_SLICE; }
 void launch_wgrad(cudaStream_t s, int X, int Y, int Z, int B, const void *x, int Cin, const void *dy, int Cout,
-                  long long slice, float *part, float *dw, int *err) {
+                  float *part, float *dw, int *err) {
   const Vol g{X, Y, Z, B};
-  const int ns = (int)((g.n() + slice - 1) / slice);
+  const int ns = (int)wgrad_slices(g.n());
   dim3 grid((27 * Cin + 127) / 128, ns);
-  k_wgrad<<<grid, 128, wgrad_smem_bytes(Cout), s>>>(g, (const bf16 *)x, Cin, (const bf16 *)dy, Cout, slice, part,
+  k_wgrad<<<grid, 128, wgrad_smem_bytes(Cout), s>>>(g, (const bf16 *)x, Cin, (const bf16 *)dy, Cout, WGRAD_SLICE, part,
                                                       err);
-  k_wgrad_reduce<<<nb(27LL * Cin * Cout, 256), 256, 0, s>>>(part, ns, Cin, Cout, dw);
+  k_wgrad_reduce<<<nb(27LL * Cin * Cout, 64), 64, 0, s>>>(part, ns, Cin, Cout, dw);
   count_launch(2);
 }
 void launch_bias_grad(cudaStream_t s, long long V, const void *dy, int C, float *part, float *db) {
   const int n = (int)nb(V, 1024);
-  k_bias_part<<<n, 128, 0, s>>>((const bf16 *)dy, V, C, part);
-  k_bias_reduce<<<1, 128, 0, s>>>(part, n, C, db);
+  k_bias_part<<<n, 256, 0, s>>>((const bf16 *)dy, V, C, part);
+  k_bias_reduce<<<1, 256, 0, s>>>(part, n, C, db);
   count_launch(2);
 }
 void launch_pool(cudaStream_t s, int Xc, int Yc, int Zc, int B, const void *f, int C, void *c) {
   const Vol gc{Xc, Yc, Zc, B};
-  k_pool<<<nb(gc.n() * C, 256), 256, 0, s>>>(gc, (const bf16 *)f, C, (bf16 *)c);
+  k_pool<<<nb(gc.n() * (C / 8), 256), 256, 0, s>>>(gc, (const bf16 *)f, C, (bf16 *)c);
   count_launch();
 }
-void launch_pool_bwd(cudaStream_t s, int Xc, int Yc, int Zc, int B, const void *dc, int C, void *df, int acc) {
+void launch_pool_bwd(cudaStream_t s, int Xc, int Yc, int Zc, int B, const void *dc, int C, void *df, const void *act) {
   const Vol gc{Xc, Yc, Zc, B};
-  k_pool_bwd<<<nb(gc.n() * 8 * C, 256), 256, 0, s>>>(gc, (const bf16 *)dc, C, (bf16 *)df, acc);
+  k_pool_bwd<<<nb(gc.n() * C, 256), 256, 0, s>>>(gc, (const bf16 *)dc, C, (bf16 *)df, (const bf16 *)act);
   count_launch();
 }
 void launch_upcat(cudaStream_t s, int X, int Y, int Z, int B, const void *c, int C1, const void *sk, int C2, void *o) {
   const Vol gf{X, Y, Z, B};
-  k_upcat<<<nb(gf.n() * (C1 + C2), 256), 256, 0, s>>>(gf, (const bf16 *)c, C1, (const bf16 *)sk, C2, (bf16 *)o);
+  k_upcat<<<nb(gf.n() * ((C1 + C2) / 8), 256), 256, 0, s>>>(gf, (const bf16 *)c, C1, (const bf16 *)sk, C2, (bf16 *)o);
   count_launch();
 }
-void launch_upcat_bwd(cudaStream_t s, int X, int Y, int Z, int B, const void *d, int C1, int C2, void *dc, void *dsk,
-                      int acc) {
+void launch_upcat_bwd(cudaStream_t s, int X, int Y, int Z, int B, const void *d, int C1, int C2, void *dc, void *dsk) {
   const Vol gf{X, Y, Z, B};
   const Vol gc{X / 2, Y / 2, Z / 2, B};
-  k_upcat_bwd_coarse<<<nb(gc.n() * C1, 256), 256, 0, s>>>(gc, (const bf16 *)d, C1, C2, (bf16 *)dc);
-  k_upcat_bwd_skip<<<nb(gf.n() * C2, 256), 256, 0, s>>>(gf.n(), (const bf16 *)d, C1, C2, (bf16 *)dsk, acc);
+  k_upcat_bwd_coarse<<<nb(gc.n() * (C1 / 8), 256), 256, 0, s>>>(gc, (const bf16 *)d, C1, C2, (bf16 *)dc);
+  k_upcat_bwd_skip<<<nb(gf.n() * (C2 / 8), 256), 256, 0, s>>>(gf.n(), (const bf16 *)d, C1, C2, (bf16 *)dsk);
   count_launch(2);
-}
-void launch_relu_mask(cudaStream_t s, long long n, const void *act, void *d) {
-  k_relu_mask<<<nb(n, 256), 256, 0, s>>>(n, (const bf16 *)act, (bf16 *)d);
-  count_launch();
 }
 void launch_head(cudaStream_t s, long long V, const void *a, int C, const float *wh, const float *bh, float *y) {
   k_head<<<nb(V, 256), 256, 0, s>>>(V, (const bf16 *)a, C, wh, bh, y);
@@ -624,8 +806,8 @@ void launch_mse(cudaStream_t s, long long V, const float *y, const float *t, con
 }
 void launch_head_bwd(cudaStream_t s, long long V, const float *dy, const void *a, int C, const float *wh, void *da,
                      float *part) {
-  k_head_bwd_act<<<nb(V * C, 256), 256, 0, s>>>(V, dy, (const bf16 *)a, C, wh, (bf16 *)da);
-  k_head_bwd_par<<<nb(V, 1024), 32, 0, s>>>(V, dy, (const bf16 *)a, C, part);
+  k_head_bwd_act<<<nb(V * (C / 8), 256), 256, 0, s>>>(V, dy, (const bf16 *)a, C, wh, (bf16 *)da);
+  k_head_bwd_par<<<nb(V, 1024), 256, 0, s>>>(V, dy, (const bf16 *)a, C, part);
   count_launch(2);
 }
 void launch_res_fwd(cudaStream_t s, int X, int Y, int Z, int B, const float *y, const float *a7, const float *x4,
@@ -650,11 +832,11 @@ void launch_wcast(cudaStream_t s, const float *w, int Cin, int Cout, void *wf, v
   count_launch();
 }
 void launch_pack_in(cudaStream_t s, long long V, const float *x4, void *x16) {
-  k_pack_in<<<nb(V * 16, 256), 256, 0, s>>>(V, x4, (bf16 *)x16);
+  k_pack_in<<<nb(V * 2, 256), 256, 0, s>>>(V, x4, (bf16 *)x16);
   count_launch();
 }
 void launch_bias_reduce(cudaStream_t s, const float *part, int n, int C, float *out) {
-  k_bias_reduce<<<1, 128, 0, s>>>(part, n, C, out);
+  k_bias_reduce<<<1, 256, 0, s>>>(part, n, C, out);
   count_launch();
 }
 void launch_f32_to_bf16(cudaStream_t s, long long n, const float *a, void *b) {

@@ -407,19 +407,16 @@ void launch_fconv(cudaStream_t s, const Geo &g, const Fld &f, const Prm &p, doub
 // weight gradient, and the U-Net's elementwise kernels
 enum { CONV_BF16 = 0, CONV_RELU_BF16 = 1, CONV_MASK_BF16 = 2, CONV_F32 = 3 };
 bool unet_kernels_configure();
-size_t conv_smem_bytes(int Cin, int Cout);
-size_t wgrad_smem_bytes(int Cout);
+long long wgrad_slices(long long V);
 void launch_conv(cudaStream_t s, int X, int Y, int Z, int B, const void *x, int Cin, const void *w, const float *bias,
                  int Cout, int mode, const void *mask, void *y, int *err);
 void launch_wgrad(cudaStream_t s, int X, int Y, int Z, int B, const void *x, int Cin, const void *dy, int Cout,
-                  long long slice, float *part, float *dw, int *err);
+                  float *part, float *dw, int *err);
 void launch_bias_grad(cudaStream_t s, long long V, const void *dy, int C, float *part, float *db);
 void launch_pool(cudaStream_t s, int Xc, int Yc, int Zc, int B, const void *f, int C, void *c);
-void launch_pool_bwd(cudaStream_t s, int Xc, int Yc, int Zc, int B, const void *dc, int C, void *df, int acc);
+void launch_pool_bwd(cudaStream_t s, int Xc, int Yc, int Zc, int B, const void *dc, int C, void *df, const void *act);
 void launch_upcat(cudaStream_t s, int X, int Y, int Z, int B, const void *c, int C1, const void *sk, int C2, void *o);
-void launch_upcat_bwd(cudaStream_t s, int X, int Y, int Z, int B, const void *d, int C1, int C2, void *dc, void *dsk,
-                      int acc);
-void launch_relu_mask(cudaStream_t s, long long n, const void *act, void *d);
+void launch_upcat_bwd(cudaStream_t s, int X, int Y, int Z, int B, const void *d, int C1, int C2, void *dc, void *dsk);
 void launch_head(cudaStream_t s, long long V, const void *a, int C, const float *wh, const float *bh, float *y);
 void launch_mse(cudaStream_t s, long long V, const float *y, const float *t, const float *m, float inv_n, float *dy,
                 float *lpart);

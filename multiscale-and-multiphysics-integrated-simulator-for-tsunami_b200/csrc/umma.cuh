@@ -40,6 +40,14 @@ __host__ __device__ constexpr uint32_t idesc_bf16_f32(uint32_t M, uint32_t N) {
   return (1u << 4) | (1u << 7) | (1u << 10) | ((N >> 3) << 17) | ((M >> 4) << 24);
 }
 
+// The same with both operands MN-major (bits 15, 16): a tile of R rows
+// (M or N) x K without swizzle in core matrices of 8 K values x 8 rows,
+// 16 bytes (8 rows) per K value; element (r, k) sits at byte
+//   (r / 8) * SBO + (k / 8) * LBO + (k % 8) * 16 + (r % 8) * 2.
+__host__ __device__ constexpr uint32_t idesc_bf16_f32_mn(uint32_t M, uint32_t N) {
+  return idesc_bf16_f32(M, N) | (1u << 15) | (1u << 16);
+}
+
 // TMEM columns to allocate for N FP32 accumulator columns: a power of two
 // of at least 32.
 __host__ __device__ constexpr uint32_t tmem_cols(uint32_t N) {
@@ -85,6 +93,14 @@ __device__ __forceinline__ void fence_after_sync() { asm volatile("tcgen05.fence
 __device__ __forceinline__ void fence_before_sync() { asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory"); }
 // generic-proxy shared-memory writes made visible to the tensor core
 __device__ __forceinline__ void fence_async_smem() { asm volatile("fence.proxy.async.shared::cta;" ::: "memory"); }
+
+// 16 bytes from global to shared memory, zeros where !ok (src must be a
+// valid address all the same)
+__device__ __forceinline__ void cp16z(uint32_t dst, const void *src, bool ok) {
+  asm volatile("cp.async.ca.shared.global [%0], [%1], 16, %2;" ::"r"(dst), "l"(src), "r"(ok ? 16 : 0) : "memory");
+}
+__device__ __forceinline__ void cp_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
+template <int N> __device__ __forceinline__ void cp_wait() { asm volatile("cp.async.wait_group %0;" ::"n"(N) : "memory"); }
 
 __device__ __forceinline__ void mbar_init(uint64_t *bar, uint32_t count) {
   asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(smem_u32(bar)), "r"(count) : "memory");

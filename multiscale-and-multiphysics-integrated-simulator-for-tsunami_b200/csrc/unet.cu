@@ -69,7 +69,6 @@ struct cadmas_unet {
   float *part = nullptr, *bpart = nullptr, *lpart = nullptr;
   float *a7 = nullptr, *r = nullptr;  // pressure systems and residual (residual loss)
   size_t part_n = 0;
-  long long slice = 8192;
   int *err = nullptr;
   std::vector<float> hl;
 };
@@ -128,7 +127,7 @@ void layer_grads(cadmas_unet *n, int l, const void *x, const void *dyl) {
   const Layer &L = TAB.L[l];
   int X, Y, Z;
   dims(n, L.res, X, Y, Z);
-  launch_wgrad(n->s, X, Y, Z, n->B, x, L.cin, dyl, L.cout, n->slice, n->part, n->g + L.w, n->err);
+  launch_wgrad(n->s, X, Y, Z, n->B, x, L.cin, dyl, L.cout, n->part, n->g + L.w, n->err);
   launch_bias_grad(n->s, n->V[L.res], dyl, L.cout, n->bpart, n->g + L.b);
 }
 
@@ -143,28 +142,26 @@ void backward(cadmas_unet *n) {
   layer_grads(n, 8, n->u1, n->d[8]);
   conv(n, 0, n->d[8], 16, n->wt[8], nullptr, 48, CONV_MASK_BF16, n->u1, n->du1);
   // split: d of c42's output (coarse, 32) and of skip1 (16)
-  launch_upcat_bwd(n->s, n->X, n->Y, n->Z, n->B, n->du1, 32, 16, n->d[7], n->d[1], 0);
+  launch_upcat_bwd(n->s, n->X, n->Y, n->Z, n->B, n->du1, 32, 16, n->d[7], n->d[1]);
   // c42, c41
   layer_grads(n, 7, n->a[6], n->d[7]);
   conv(n, 1, n->d[7], 32, n->wt[7], nullptr, 32, CONV_MASK_BF16, n->a[6], n->d[6]);
   layer_grads(n, 6, n->u2, n->d[6]);
   conv(n, 1, n->d[6], 32, n->wt[6], nullptr, 96, CONV_MASK_BF16, n->u2, n->du2);
-  launch_upcat_bwd(n->s, n->X / 2, n->Y / 2, n->Z / 2, n->B, n->du2, 64, 32, n->d[5], n->d[3], 0);
+  launch_upcat_bwd(n->s, n->X / 2, n->Y / 2, n->Z / 2, n->B, n->du2, 64, 32, n->d[5], n->d[3]);
   // c32, c31
   layer_grads(n, 5, n->a[4], n->d[5]);
   conv(n, 2, n->d[5], 64, n->wt[5], nullptr, 64, CONV_MASK_BF16, n->a[4], n->d[4]);
   layer_grads(n, 4, n->p2, n->d[4]);
   conv(n, 2, n->d[4], 64, n->wt[4], nullptr, 32, CONV_BF16, nullptr, n->dp2);
   // skip2 gets the pooled path too, then the ReLU of c22
-  launch_pool_bwd(n->s, n->X / 4, n->Y / 4, n->Z / 4, n->B, n->dp2, 32, n->d[3], 1);
-  launch_relu_mask(n->s, n->V[1] * 32, n->a[3], n->d[3]);
+  launch_pool_bwd(n->s, n->X / 4, n->Y / 4, n->Z / 4, n->B, n->dp2, 32, n->d[3], n->a[3]);
   // c22, c21
   layer_grads(n, 3, n->a[2], n->d[3]);
   conv(n, 1, n->d[3], 32, n->wt[3], nullptr, 32, CONV_MASK_BF16, n->a[2], n->d[2]);
   layer_grads(n, 2, n->p1, n->d[2]);
   conv(n, 1, n->d[2], 32, n->wt[2], nullptr, 16, CONV_BF16, nullptr, n->dp1);
-  launch_pool_bwd(n->s, n->X / 2, n->Y / 2, n->Z / 2, n->B, n->dp1, 16, n->d[1], 1);
-  launch_relu_mask(n->s, n->V[0] * 16, n->a[1], n->d[1]);
+  launch_pool_bwd(n->s, n->X / 2, n->Y / 2, n->Z / 2, n->B, n->dp1, 16, n->d[1], n->a[1]);
   // c12, c11
   layer_grads(n, 1, n->a[0], n->d[1]);
   conv(n, 0, n->d[1], 16, n->wt[1], nullptr, 16, CONV_MASK_BF16, n->a[0], n->d[0]);
@@ -267,7 +264,7 @@ int unet_new(int nx, int ny, int nz, int batch, cudaStream_t stream, cadmas_unet
   AL(n->mk, (size_t)n->V[0]); AL(n->dy, (size_t)n->V[0]);
   // wgrad partial sums: the largest (slices x 27 Cin x Cout) of any layer
   for (int l = 0; l < NL; ++l) {
-    const long long ns = (n->V[TAB.L[l].res] + n->slice - 1) / n->slice;
+    const long long ns = wgrad_slices(n->V[TAB.L[l].res]);
     n->part_n = std::max(n->part_n, (size_t)ns * 27 * TAB.L[l].cin * TAB.L[l].cout);
   }
   AL(n->part, n->part_n);
