@@ -80,7 +80,8 @@ struct ConvPlan {
   uint32_t a_bytes, b_bytes;  // of one stage
   size_t smem;
 };
-__global__ void __launch_bounds__(128) k_conv(Vol g, const bf16 *__restrict__ X, int Cin,
+constexpr int CONV_T = 256;  // threads: eight warps share the copies and the epilogue's row blocks
+__global__ void __launch_bounds__(CONV_T) k_conv(Vol g, const bf16 *__restrict__ X, int Cin,
                                               const bf16 *__restrict__ W, const float *__restrict__ bias,
                                               int Cout, int mode, const bf16 *__restrict__ mask, void *Y,
                                               int *err, ConvPlan p) {
@@ -106,20 +107,21 @@ __global__ void __launch_bounds__(128) k_conv(Vol g, const bf16 *__restrict__ X,
   const int z = (int)(t % g.Z), b = (int)(t / g.Z);
   const int x0 = xt * p.bx, y0 = yt * p.by;
   // layer z + gi - 1 of the padded tile and its nine taps' weights into a
-  // stage; thread tid takes the 16-byte chunks tid, tid + 128, ... of every
+  // stage; thread tid takes the 16-byte chunks tid, tid + CONV_T, ... of every
   // row (chunk q of a row: voxel q / C8, channels 8 (q % C8) ..)
-  const int nrow = p.by + 2;
+  const int nrow = p.by + 2, rsplit = max(1, min(nrow, CONV_T / (P * C8)));
   auto load = [&](int gi, int st) {
     const uint32_t As = sm0 + st * st_bytes, Bs = As + p.a_bytes;
     const int zz = z + gi - 1;
     const bool zok = zz >= 0 && zz < g.Z;
     const bf16 *plane = X + (long long)g.X * g.Y * ((long long)g.Z * b + (zok ? zz : z)) * Cin;
-    for (int q = tid; q < P * C8; q += 128) {
-      const int xx = q / C8, c8 = q - xx * C8, gx = x0 + xx - 1;
+    for (int q = tid; q < P * C8 * rsplit; q += CONV_T) {
+      const int qr = q / (P * C8), qc = q - qr * (P * C8);  // rows qr, qr + rsplit, ...
+      const int xx = qc / C8, c8 = qc - xx * C8, gx = x0 + xx - 1;
       const bool xok = zok && gx >= 0 && gx < g.X;
       const bf16 *src = plane + ((long long)(xok ? gx : 0) * Cin + c8 * 8);
-      uint32_t dst = As + (uint32_t)(c8 * PL + xx) * 16u;
-      for (int yy = 0; yy < nrow; ++yy, dst += (uint32_t)P * 16u) {
+      uint32_t dst = As + (uint32_t)(c8 * PL + xx + qr * P) * 16u;
+      for (int yy = qr; yy < nrow; yy += rsplit, dst += (uint32_t)(P * rsplit) * 16u) {
         const int gy = y0 + yy - 1;
         const bool ok = xok && gy >= 0 && gy < g.Y;
         umma::cp16z(dst, src + (long long)(ok ? gy : 0) * g.X * Cin, ok);
@@ -127,7 +129,7 @@ __global__ void __launch_bounds__(128) k_conv(Vol g, const bf16 *__restrict__ X,
     }
     const int nb = 9 * N * C8;
     const bf16 *wsrc = W + (long long)gi * nb * 8;
-    for (int q = tid; q < nb; q += 128) umma::cp16z(Bs + (uint32_t)q * 16u, wsrc + q * 8, true);
+    for (int q = tid; q < nb; q += CONV_T) umma::cp16z(Bs + (uint32_t)q * 16u, wsrc + q * 8, true);
     umma::cp_commit();
   };
   const bool three = p.NST == 3;
@@ -188,11 +190,11 @@ __global__ void __launch_bounds__(128) k_conv(Vol g, const bf16 *__restrict__ X,
     if (tid == 0) atomicOr(err, 1);
   } else {
     umma::fence_after_sync();
-    for (int mt = 0; mt < p.MT; ++mt) {
-      const int pos = mt * CONV_M + tid, yy = pos / P, xx = pos - yy * P, gx = x0 + xx, gy = y0 + yy;
+    for (int mt = warp >> 2; mt < p.MT; mt += 2) {
+      const int pos = mt * CONV_M + (tid & 127), yy = pos / P, xx = pos - yy * P, gx = x0 + xx, gy = y0 + yy;
       const bool live = xx < p.bx && yy < p.by && gx < g.X && gy < g.Y;
       const long long v = (long long)gx + (long long)g.X * (gy + (long long)g.Y * (z + (long long)g.Z * b));
-      const uint32_t lane_base = tmem + ((uint32_t)(warp * 32) << 16) + mt * N;
+      const uint32_t lane_base = tmem + ((uint32_t)((warp & 3) * 32) << 16) + mt * N;
       for (int c0 = 0; c0 < N; c0 += 8) {
         float a[8];
         umma::tmem_ld8(lane_base + c0, a);
@@ -233,8 +235,9 @@ __global__ void __launch_bounds__(128) k_conv(Vol g, const bf16 *__restrict__ X,
 // voxels of this CTA's slice in chunks of 64, WG_ST stages.  Tiles in
 // shared memory: [8-channel block][voxel] of 16 bytes, so a thread copies
 // 16 bytes of its voxel (or of its tap's neighbour) at a time.
-constexpr int WG_K = 64, WG_ST = 3;
+constexpr int WG_K = 64;
 
+template <int WG_ST>
 __global__ void __launch_bounds__(128) k_wgrad(Vol g, const bf16 *__restrict__ X, int Cin,
                                                const bf16 *__restrict__ DY, int Cout, long long slice,
                                                float *__restrict__ part, int *err) {
@@ -264,26 +267,38 @@ __global__ void __launch_bounds__(128) k_wgrad(Vol g, const bf16 *__restrict__ X
   // thread: voxel kq of each chunk; of the tile's 16 row blocks (8 channels
   // of one tap each) h, h+2, ..., of the N8 blocks of dY h, h+2, ...
   const int kq = tid & (WG_K - 1), h = tid >> 6;
-  int dx[8], dy[8], dz[8], dc[8];  // tap offset and first channel; dc < 0: past the last row
+  int off[8], tap[8];  // the neighbour's first value from the voxel's; tap (27: past the last row)
 #pragma unroll
   for (int i = 0; i < 8; ++i) {
-    const int gb = m0 / 8 + 2 * i + h, t = gb / C8;
-    dx[i] = t % 3 - 1; dy[i] = (t / 3) % 3 - 1; dz[i] = t / 9 - 1;
-    dc[i] = t < 27 ? (gb - t * C8) * 8 : -1;
+    const int gb = m0 / 8 + 2 * i + h, t = min(gb / C8, 27);
+    off[i] = (((t / 9 - 1) * g.Y + (t / 3) % 3 - 1) * g.X + t % 3 - 1) * Cin + (gb - t * C8) * 8;
+    tap[i] = t;
   }
-  auto load = [&](int ch) {
-    const uint32_t As = sm0 + (ch % WG_ST) * st_bytes, Bs = As + a_bytes;
-    const long long v = v0 + (long long)ch * WG_K + kq;
+  // position of the voxel to load next (chunks are loaded in order)
+  long long v = v0 + kq;
+  int x, y, z, b;
+  decomp(g, min(v, V - 1), x, y, z, b);
+  auto load = [&](int st) {
+    const uint32_t As = sm0 + st * st_bytes, Bs = As + a_bytes;
     const bool live = v < v1;
-    int x = 0, y = 0, z = 0, b = 0;
-    if (live) decomp(g, v, x, y, z, b);
+    // taps inside the volume: a bit per (dz, dy, dx)
+    const unsigned mx = 2u | (x > 0 ? 1u : 0u) | (x < g.X - 1 ? 4u : 0u);
+    const unsigned m3 = (y > 0 ? mx : 0u) | mx << 3 | (y < g.Y - 1 ? mx << 6 : 0u);
+    const unsigned in = live ? (z > 0 ? m3 : 0u) | m3 << 9 | (z < g.Z - 1 ? m3 << 18 : 0u) : 0u;
+    const bf16 *xv = X + v * Cin;
 #pragma unroll
     for (int i = 0; i < 8; ++i) {
-      const long long nv = live && dc[i] >= 0 ? nbr(g, x, y, z, b, dx[i], dy[i], dz[i]) : -1;
-      umma::cp16z(As + (uint32_t)((2 * i + h) * WG_K + kq) * 16u, nv >= 0 ? X + nv * Cin + dc[i] : X, nv >= 0);
+      const bool ok = in >> tap[i] & 1u;
+      umma::cp16z(As + (uint32_t)((2 * i + h) * WG_K + kq) * 16u, ok ? xv + off[i] : X, ok);
     }
     for (int n = h; n < N8; n += 2)
       umma::cp16z(Bs + (uint32_t)(n * WG_K + kq) * 16u, live ? DY + v * Cout + n * 8 : DY, live);
+    v += WG_K;
+    x += WG_K;
+    while (x >= g.X) {
+      x -= g.X;
+      if (++y == g.Y) { y = 0; if (++z == g.Z) { z = 0; ++b; } }
+    }
   };
   bool ok = true;
   int committed = 0;
@@ -292,10 +307,10 @@ __global__ void __launch_bounds__(128) k_wgrad(Vol g, const bf16 *__restrict__ X
     umma::cp_commit();
   }
   for (int ch = 0; ch < nchunk; ++ch) {
-    const int s = ch % WG_ST, nx = ch + WG_ST - 1;
+    const int s = ch % WG_ST, nx = ch + WG_ST - 1;  // (WG_ST is a constant)
     // chunk nx goes where chunk ch-1 lies: its MMAs must have read it
     if (ch >= 1 && !cta_wait(&bar[(ch - 1) % WG_ST], ((ch - 1) / WG_ST) & 1)) { ok = false; break; }
-    if (nx < nchunk) load(nx);
+    if (nx < nchunk) load(nx % WG_ST);
     umma::cp_commit();
     umma::cp_wait<WG_ST - 1>();
     umma::fence_async_smem();
@@ -360,59 +375,64 @@ __global__ void __launch_bounds__(64) k_wgrad_reduce(const float *part, int nsli
   dW[((long long)n * 27 + t) * Cin + ci] = s;
 }
 
-// Column sums of a block's rows, in the order of the rows: the rows pass
-// through shared memory (coalesced loads by all threads), one thread per
-// column adds.  The order is the reference's sequential one; what bounds the
-// kernels is that chain (4 cycles per row), not the loads.
-constexpr int SUM_ROWS = 64;
+// Column sums in the order of the rows.  The rows come to shared memory by
+// 16-byte asynchronous copies of all threads, then one thread per column
+// adds them: the sequential order bounds the kernels (4 cycles per row), so
+// the loads must not stand in its way.
 // bias gradient: db[c] = sum over voxels of dY[v][c] (FP32 partials per
 // block of 1024 voxels, then the same in order); C <= 64
 __global__ void __launch_bounds__(256) k_bias_part(const bf16 *DY, long long V, int C, float *part) {
-  __shared__ float row[2][SUM_ROWS * 64];
-  const long long v0 = (long long)blockIdx.x * 1024, v1 = min(V, v0 + 1024);
-  const int C8 = C >> 3;
+  extern __shared__ __align__(1024) unsigned char smem[];
+  const long long v0 = (long long)blockIdx.x * 1024;
+  const int n = (int)min(1024LL, V - v0), nq = n * (C >> 3);
+  const uint32_t sm0 = umma::smem_u32(smem);
+  for (int q = threadIdx.x; q < nq; q += 256) umma::cp16z(sm0 + q * 16, DY + v0 * C + q * 8, true);
+  umma::cp_commit();
+  umma::cp_wait<0>();
+  __syncthreads();
+  if (threadIdx.x >= C) return;
+  const bf16 *e = reinterpret_cast<const bf16 *>(smem) + threadIdx.x;
   float s = 0.0f;
-  auto fill = [&](long long v, float *to) {
-    for (int q = threadIdx.x; q < SUM_ROWS * C8; q += 256) {
-      const int r = q / C8, c = (q - r * C8) * 8;
-      if (v + r >= v1) break;
-      const uint4 w = *reinterpret_cast<const uint4 *>(DY + (v + r) * C + c);
-      const bf16 *e = reinterpret_cast<const bf16 *>(&w);
+  int r = 0;
+  for (; r + 16 <= n; r += 16) {
+    float f[16];
 #pragma unroll
-      for (int i = 0; i < 8; ++i) to[r * C + c + i] = __bfloat162float(e[i]);
-    }
-  };
-  fill(v0, row[0]);
-  int k = 0;
-  for (long long v = v0; v < v1; v += SUM_ROWS, k ^= 1) {
-    __syncthreads();
-    if (v + SUM_ROWS < v1) fill(v + SUM_ROWS, row[k ^ 1]);
-    if (threadIdx.x < C) {
-      const int n = (int)min((long long)SUM_ROWS, v1 - v);
-#pragma unroll 8
-      for (int r = 0; r < n; ++r) s += row[k][r * C + threadIdx.x];
-    }
+    for (int j = 0; j < 16; ++j) f[j] = __bfloat162float(e[(r + j) * C]);
+#pragma unroll
+    for (int j = 0; j < 16; ++j) s += f[j];
   }
-  if (threadIdx.x < C) part[(long long)blockIdx.x * C + threadIdx.x] = s;
+  for (; r < n; ++r) s += __bfloat162float(e[r * C]);
+  part[(long long)blockIdx.x * C + threadIdx.x] = s;
 }
 // db[c] = sum of nb block partials in order; C <= 64
+constexpr int SUM_ROWS = 64;
 __global__ void __launch_bounds__(256) k_bias_reduce(const float *part, int nb, int C, float *db) {
   __shared__ float row[2][SUM_ROWS * 64];
-  float s = 0.0f;
-  auto fill = [&](int q0, float *to) {
+  float s = 0.0f, reg[16];
+  // rows q0 .. of the next stretch in registers while the last one is added
+  auto fetch = [&](int q0) {
     const int n = min(SUM_ROWS, nb - q0) * C;
-    for (int i = threadIdx.x; i < n; i += 256) to[i] = part[(long long)q0 * C + i];
+#pragma unroll
+    for (int j = 0; j < 16; ++j) reg[j] = threadIdx.x + 256 * j < n ? part[(long long)q0 * C + threadIdx.x + 256 * j] : 0.0f;
   };
-  fill(0, row[0]);
+  auto put = [&](float *to) {
+#pragma unroll
+    for (int j = 0; j < 16; ++j)
+      if (threadIdx.x + 256 * j < SUM_ROWS * C) to[threadIdx.x + 256 * j] = reg[j];
+  };
+  fetch(0);
+  put(row[0]);
   int k = 0;
   for (int q = 0; q < nb; q += SUM_ROWS, k ^= 1) {
     __syncthreads();
-    if (q + SUM_ROWS < nb) fill(q + SUM_ROWS, row[k ^ 1]);
+    const bool more = q + SUM_ROWS < nb;
+    if (more) fetch(q + SUM_ROWS);
     if (threadIdx.x < C) {
       const int n = min(SUM_ROWS, nb - q);
-#pragma unroll 8
+#pragma unroll 16
       for (int r = 0; r < n; ++r) s += row[k][r * C + threadIdx.x];
     }
+    if (more) put(row[k ^ 1]);
   }
   if (threadIdx.x < C) db[threadIdx.x] = s;
 }
@@ -730,7 +750,7 @@ static ConvPlan conv_plan(const Vol &g, int Cin, int Cout) {
   }
   return best;
 }
-static size_t wgrad_smem_bytes(int Cout) {
+static size_t wgrad_smem_bytes(int Cout, int WG_ST) {
   return smem_floor((size_t)WG_ST * (128 + Cout) * WG_K * 2 + 64, umma::tmem_cols(Cout));
 }
 
@@ -739,7 +759,9 @@ bool unet_kernels_configure() {
   if (done) return done > 0;
   const int mx = 227 * 1024;
   bool ok = cudaFuncSetAttribute(k_conv, cudaFuncAttributeMaxDynamicSharedMemorySize, mx) == cudaSuccess &&
-            cudaFuncSetAttribute(k_wgrad, cudaFuncAttributeMaxDynamicSharedMemorySize, mx) == cudaSuccess;
+            cudaFuncSetAttribute(k_wgrad<3>, cudaFuncAttributeMaxDynamicSharedMemorySize, mx) == cudaSuccess &&
+            cudaFuncSetAttribute(k_wgrad<8>, cudaFuncAttributeMaxDynamicSharedMemorySize, mx) == cudaSuccess &&
+            cudaFuncSetAttribute(k_bias_part, cudaFuncAttributeMaxDynamicSharedMemorySize, mx) == cudaSuccess;
   done = ok ? 1 : -1;
   return ok;
 }
@@ -748,7 +770,7 @@ void launch_conv(cudaStream_t s, int X, int Y, int Z, int B, const void *x, int 
                  int Cout, int mode, const void *mask, void *y, int *err) {
   const Vol g{X, Y, Z, B};
   const ConvPlan p = conv_plan(g, Cin, Cout);
-  k_conv<<<(unsigned)((long long)p.nxt * p.nyt * Z * B), 128, p.smem, s>>>(
+  k_conv<<<(unsigned)((long long)p.nxt * p.nyt * Z * B), CONV_T, p.smem, s>>>(
       g, (const bf16 *)x, Cin, (const bf16 *)w, bias, Cout, mode, (const bf16 *)mask, y, err, p);
   count_launch();
 }
@@ -762,14 +784,20 @@ void launch_wgrad(cudaStream_t s, int X, int Y, int Z, int B, const void *x, int
   const Vol g{X, Y, Z, B};
   const int ns = (int)wgrad_slices(g.n());
   dim3 grid((27 * Cin + 127) / 128, ns);
-  k_wgrad<<<grid, 128, wgrad_smem_bytes(Cout), s>>>(g, (const bf16 *)x, Cin, (const bf16 *)dy, Cout, WGRAD_SLICE, part,
-                                                      err);
+  // Where the CTAs leave the SMs half empty, eight stages (one CTA per SM)
+  // hide the copies' latency; else three stages and up to four CTAs do.
+  if ((long long)grid.x * grid.y <= 2 * 148)
+    k_wgrad<8><<<grid, 128, wgrad_smem_bytes(Cout, 8), s>>>(g, (const bf16 *)x, Cin, (const bf16 *)dy, Cout, WGRAD_SLICE,
+                                                            part, err);
+  else
+    k_wgrad<3><<<grid, 128, wgrad_smem_bytes(Cout, 3), s>>>(g, (const bf16 *)x, Cin, (const bf16 *)dy, Cout, WGRAD_SLICE,
+                                                            part, err);
   k_wgrad_reduce<<<nb(27LL * Cin * Cout, 64), 64, 0, s>>>(part, ns, Cin, Cout, dw);
   count_launch(2);
 }
 void launch_bias_grad(cudaStream_t s, long long V, const void *dy, int C, float *part, float *db) {
   const int n = (int)nb(V, 1024);
-  k_bias_part<<<n, 256, 0, s>>>((const bf16 *)dy, V, C, part);
+  k_bias_part<<<n, 256, (size_t)1024 * C * 2, s>>>((const bf16 *)dy, V, C, part);
   k_bias_reduce<<<1, 256, 0, s>>>(part, n, C, db);
   count_launch(2);
 }
