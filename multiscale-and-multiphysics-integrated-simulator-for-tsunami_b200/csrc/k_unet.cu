@@ -92,10 +92,15 @@ __global__ void __launch_bounds__(CONV_T) k_conv(Vol g, const bf16 *__restrict__
   uint32_t *tslot = reinterpret_cast<uint32_t *>(bar + 2);
   const int tid = threadIdx.x, warp = tid >> 5;
   const uint32_t ncols = umma::tmem_cols(p.MT * N);
+  // Issuing one MMA takes one thread longer than its 128 x 16 x 16 product
+  // takes the tensor core: lane 0 of warp w issues those of row blocks w,
+  // w + NI, ... (each accumulator's MMAs stay in one thread, in order).
+  const int NI = min(CONV_T / 32, p.MT);
+  const bool issuer = (tid & 31) == 0 && warp < NI;
   if (warp == 0) umma::tmem_alloc(tslot, ncols);
   if (tid == 0) {
-    umma::mbar_init(&bar[0], 1);
-    umma::mbar_init(&bar[1], 1);
+    umma::mbar_init(&bar[0], NI);
+    umma::mbar_init(&bar[1], NI);
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
   }
   const uint32_t sm0 = umma::smem_u32(smem);
@@ -145,14 +150,18 @@ __global__ void __launch_bounds__(CONV_T) k_conv(Vol g, const bf16 *__restrict__
   auto mmas = [&](int gi, int st) {
     umma::fence_after_sync();
     const uint32_t a0 = sm0 + st * st_bytes, b0 = a0 + p.a_bytes;
-    const uint64_t ad0 = umma::smem_desc(a0, (uint32_t)PL * 16u, 128), bd0 = umma::smem_desc(b0, (uint32_t)N * 16u, 128);
-    for (int t9 = 0; t9 < 9; ++t9) {
-      const int off = (t9 / 3) * P + t9 % 3;  // rows from the tap's first voxel
-      for (int kk = 0; kk < C8 / 2; ++kk) {
-        const uint64_t bd = bd0 + (uint64_t)((t9 * C8 + 2 * kk) * N);
-        for (int mt = 0; mt < p.MT; ++mt)
-          umma::mma_bf16(tmem + mt * N, ad0 + (uint64_t)(2 * kk * PL + mt * CONV_M + off), bd, idesc,
-                         (gi | t9 | kk) != 0);
+    for (int mt = warp; mt < p.MT; mt += NI) {
+      const uint64_t ad0 = umma::smem_desc(a0, (uint32_t)PL * 16u, 128) + (uint64_t)(mt * CONV_M);
+      uint64_t bd = umma::smem_desc(b0, (uint32_t)N * 16u, 128);
+      const uint32_t d = tmem + mt * N;
+#pragma unroll
+      for (int t9 = 0; t9 < 9; ++t9) {
+        uint64_t ad = ad0 + (uint64_t)((t9 / 3) * P + t9 % 3);  // rows from the tap's first voxel
+        for (int kk = 0; kk < C8 / 2; ++kk) {
+          umma::mma_bf16(d, ad, bd, idesc, (gi | t9 | kk) != 0);
+          ad += (uint64_t)(2 * PL);
+          bd += (uint64_t)(2 * N);
+        }
       }
     }
   };
@@ -162,14 +171,16 @@ __global__ void __launch_bounds__(CONV_T) k_conv(Vol g, const bf16 *__restrict__
   if (three) umma::cp_wait<2>(); else umma::cp_wait<1>();
   umma::fence_async_smem();
   __syncthreads();
-  if (tid == 0) {
+  if (issuer) {
     mmas(0, 0);
     umma::mma_commit(&bar[0]);
   }
+  __syncwarp();
   if (three) umma::cp_wait<1>(); else umma::cp_wait<0>();
   umma::fence_async_smem();
   __syncthreads();
-  if (tid == 0) mmas(1, 1);
+  if (issuer) mmas(1, 1);
+  __syncwarp();
   if (three) {
     umma::cp_wait<0>();
   } else {
@@ -179,10 +190,11 @@ __global__ void __launch_bounds__(CONV_T) k_conv(Vol g, const bf16 *__restrict__
   }
   umma::fence_async_smem();
   __syncthreads();
-  if (tid == 0) {
+  if (issuer) {
     if (ok) mmas(2, three ? 2 : 0);
     umma::mma_commit(&bar[1]);
   }
+  __syncwarp();
   // the last commit covers every MMA issued before it (after a timeout
   // this is the one more bounded wait before the TMEM is freed)
   if (!cta_wait(&bar[1], 0)) ok = false;
