@@ -580,6 +580,24 @@ __global__ void k_mse(long long V, const float *Yo, const float *T, const float 
   }
   if (threadIdx.x == 0) lpart[blockIdx.x] = red[0];
 }
+// out[0] = sum of a (FP64; block partials in out[1..], added in order)
+__global__ void __launch_bounds__(256) k_sum_part(long long n, const float *a, double *out) {
+  __shared__ double red[8];
+  double s = 0.0;
+  for (long long i = blockIdx.x * 256LL + threadIdx.x; i < n; i += 256LL * SUM_BLOCKS) s += (double)a[i];
+  s = warp_tree(s);
+  if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = s;
+  __syncthreads();
+  if (threadIdx.x != 0) return;
+  for (int i = 1; i < 8; ++i) s += red[i];
+  out[1 + blockIdx.x] = s;
+}
+__global__ void k_sum_fin(double *out) {
+  double s = 0.0;
+  for (int i = threadIdx.x; i < SUM_BLOCKS; i += 32) s += out[1 + i];
+  s = warp_tree(s);
+  if (threadIdx.x == 0) out[0] = s;
+}
 // head backward: dA[v][c] = dy[v] wh[c] (BF16), masked by the ReLU of A
 __global__ void k_head_bwd_act(long long V, const float *dy, const bf16 *A, int C, const float *wh, bf16 *dA) {
   long long v;
@@ -843,6 +861,11 @@ void launch_mse(cudaStream_t s, long long V, const float *y, const float *t, con
                 float *lpart) {
   k_mse<<<nb(V, 256), 256, 0, s>>>(V, y, t, m, inv_n, dy, lpart);
   count_launch();
+}
+void launch_sum(cudaStream_t s, long long n, const float *a, double *out) {
+  k_sum_part<<<SUM_BLOCKS, 256, 0, s>>>(n, a, out);
+  k_sum_fin<<<1, 32, 0, s>>>(out);
+  count_launch(2);
 }
 void launch_head_bwd(cudaStream_t s, long long V, const float *dy, const void *a, int C, const float *wh, void *da,
                      float *part) {

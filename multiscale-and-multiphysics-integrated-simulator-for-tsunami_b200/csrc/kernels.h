@@ -420,6 +420,9 @@ void launch_upcat_bwd(cudaStream_t s, int X, int Y, int Z, int B, const void *d,
 void launch_head(cudaStream_t s, long long V, const void *a, int C, const float *wh, const float *bh, float *y);
 void launch_mse(cudaStream_t s, long long V, const float *y, const float *t, const float *m, float inv_n, float *dy,
                 float *lpart);
+// FP64 sum of a float array into out[0]; out has 1 + SUM_BLOCKS entries
+constexpr int SUM_BLOCKS = 256;
+void launch_sum(cudaStream_t s, long long n, const float *a, double *out);
 void launch_head_bwd(cudaStream_t s, long long V, const float *dy, const void *a, int C, const float *wh, void *da,
                      float *part);
 void launch_adam(cudaStream_t s, long long n, float *p, const float *g, float *m, float *v, float lr, float b1,
