@@ -457,7 +457,6 @@ static int solve(cadmas_handle *h, const SysPtr &a, double *x0, const int *indc,
                  double &bnorm, double &xnorm) {
   cudaStream_t s = h->s;
   const Geo &g = h->g;
-  const size_t vbytes = h->nsl * sizeof(double);
   const double epsa2 = h->P.cgepsa * h->P.cgepsa, epsr2 = h->P.cgepsr * h->P.cgepsr,
                div2 = h->P.cgdiv * h->P.cgdiv;
   const int icgmax = h->P.icgmax;
@@ -465,10 +464,9 @@ static int solve(cadmas_handle *h, const SysPtr &a, double *x0, const int *indc,
   SolveState *st = h->st;
   const SkewGeo &q = h->q;
   const SkewSys &S = h->S;
-  const int *ic = S.indc;  // INDC in the skewed layout (-1 on padding)
-  // vf_m1bcgs.f:79-95: XW = X0, work vectors zero
-  double *zero_list[] = {h->y2, h->r0, h->rr, h->pv, h->ap, h->ae};
-  for (double *z : zero_list) CK(cudaMemsetAsync(z, 0, vbytes, s));
+  const int *ic = S.indc;  // INDC in the skewed layout (-1 where there is no cell)
+  // vf_m1bcgs.f:79-95: XW = X0.  Every work vector is written in full,
+  // zeros where INDC = -1, before it is read.
   CK(cudaMemsetAsync(st, 0, SOLVE_CLEAR_BYTES, s));
   const double U = (h->P.icgtyp != 0) ? h->P.cgpara : 0.0;
   TB(CADMAS_STAGE_DCMP);
@@ -480,21 +478,20 @@ static int solve(cadmas_handle *h, const SysPtr &a, double *x0, const int *indc,
   TB(CADMAS_STAGE_FWD); launch_fwd(s, g, q, S, h->bb_sl, nullptr, st, h->y2); TE();
   TB(CADMAS_STAGE_BWD); launch_bwd(s, g, q, S, h->y2, st); TE();
   TB(CADMAS_STAGE_DOT);
-  launch_dot(s, q, ic, h->y2, h->y2, nullptr, nullptr, h->rb0, nullptr, st);
+  launch_dot_t<double>(s, g, q, h->y2, h->y2, nullptr, nullptr, h->rb0, nullptr, st);
   launch_fin(s, FIN_BNORM, h->rb0, nullptr, nr, st, nullptr, epsa2, epsr2, div2, icgmax);
   TE();
   // YY = A*XW; YY = BB - YY; R0 = MINV*YY; S = (R0,R0)
   TB(CADMAS_STAGE_VEC);
-  launch_spmv(s, g, q, S, h->xw, h->y2, st);
-  launch_bmy(s, q, ic, h->bb_sl, h->y2, st);
+  launch_resid(s, g, q, S, h->bb_sl, h->xw, h->y2, nullptr, nullptr, st);
   TE();
   TB(CADMAS_STAGE_FWD); launch_fwd(s, g, q, S, h->y2, nullptr, st, h->y2); TE();
   TB(CADMAS_STAGE_BWD); launch_bwd(s, g, q, S, h->r0, st); TE();
   TB(CADMAS_STAGE_DOT);
-  launch_dot(s, q, ic, h->r0, h->r0, nullptr, nullptr, h->rb0, nullptr, st);
+  launch_dot_t<double>(s, g, q, h->r0, h->r0, nullptr, nullptr, h->rb0, nullptr, st);
   launch_fin(s, FIN_START, h->rb0, nullptr, nr, st, nullptr, epsa2, epsr2, div2, icgmax);
   TE();
-  TB(CADMAS_STAGE_VEC); launch_copy2(s, q, ic, h->r0, h->rr, h->pv, st); TE();
+  TB(CADMAS_STAGE_VEC); launch_copy2_t<double>(s, q, h->r0, h->rr, h->pv, st); TE();
   // First batch as long as the previous solve; after that batches of 4.
   int batch = std::max(2, std::min(h->last_iter, 64));
   for (int guard = 0; guard < 100000; ++guard) {
@@ -503,22 +500,22 @@ static int solve(cadmas_handle *h, const SysPtr &a, double *x0, const int *indc,
       TB(CADMAS_STAGE_FWD); launch_fwd(s, g, q, S, nullptr, h->pv, st, h->y2); TE();
       TB(CADMAS_STAGE_BWD); launch_bwd(s, g, q, S, h->ap, st); TE();
       TB(CADMAS_STAGE_DOT);
-      launch_dot(s, q, ic, h->r0, h->ap, nullptr, nullptr, h->rb0, nullptr, st);
+      launch_dot_t<double>(s, g, q, h->r0, h->ap, nullptr, nullptr, h->rb0, nullptr, st);
       launch_fin(s, FIN_ALPHA, h->rb0, nullptr, nr, st, nullptr, epsa2, epsr2, div2, icgmax);
       TE();
-      TB(CADMAS_STAGE_VEC); launch_axpy_rr(s, q, ic, h->ap, h->rr, st); TE();
+      TB(CADMAS_STAGE_VEC); launch_axpy_rr(s, q, h->ap, h->rr, st); TE();
       // AE = MINV*(A*RR); OMEGA = (RR,AE)/(AE,AE)
       TB(CADMAS_STAGE_FWD); launch_fwd(s, g, q, S, nullptr, h->rr, st, h->y2); TE();
       TB(CADMAS_STAGE_BWD); launch_bwd(s, g, q, S, h->ae, st); TE();
       TB(CADMAS_STAGE_DOT);
-      launch_dot(s, q, ic, h->rr, h->ae, h->ae, h->ae, h->rb0, h->rb1, st);
+      launch_dot_t<double>(s, g, q, h->rr, h->ae, h->ae, h->ae, h->rb0, h->rb1, st);
       launch_fin(s, FIN_OMEGA, h->rb0, h->rb1, nr, st, nullptr, epsa2, epsr2, div2, icgmax);
       TE();
       // XW += ALPHA*PP + OMEGA*RR; RR -= OMEGA*AE; convergence; BETA
       TB(CADMAS_STAGE_VEC);
-      launch_upd_xr(s, q, ic, h->pv, h->ae, h->r0, h->xw, h->rr, h->rb0, h->rb1, st);
+      launch_upd_xr(s, g, q, h->pv, h->ae, h->r0, h->xw, h->rr, h->rb0, h->rb1, st);
       launch_fin(s, FIN_CONV, h->rb0, h->rb1, nr, st, nullptr, epsa2, epsr2, div2, icgmax);
-      launch_upd_p(s, q, ic, h->rr, h->ap, h->pv, st);
+      launch_upd_p(s, q, h->rr, h->ap, h->pv, st);
       TE();
     }
     CK(cudaGetLastError());
@@ -552,25 +549,23 @@ static int solve_inner_f(cadmas_handle *h, double eps, int &iter) {
   const Geo &g = h->g;
   const SkewGeo &q = h->q;
   const SkewSysF &S = h->Sf;
-  const int *ic = S.indc;
   const long long nr = h->nrb;
   SolveState *st = h->st;
   const double epsa2 = h->P.cgepsa * h->P.cgepsa, epsr2 = eps * eps, div2 = h->P.cgdiv * h->P.cgdiv;
   const int icgmax = h->P.icgmax;
   const size_t vb = h->nsl * sizeof(float);
   const bool fused_dots = h->P.dot_passes == 0;
-  float *zl[] = {h->xf, h->r0f, h->rrf, h->pvf, h->apf, h->aef};
-  for (float *z : zl) CK(cudaMemsetAsync(z, 0, vb, s));
+  CK(cudaMemsetAsync(h->xf, 0, vb, s));  // d = 0; the other vectors are written in full before they are read
   CK(cudaMemsetAsync(st, 0, SOLVE_CLEAR_BYTES, s));
   // YY = MINV*BB, BNORM = (YY,YY); with XW = 0, R0 = YY and S = BNORM
   TB(CADMAS_STAGE_FWD); launch_fwd_f(s, g, q, S, h->bf, nullptr, st, h->y2f); TE();
   TB(CADMAS_STAGE_BWD); launch_bwd_f(s, g, q, S, h->r0f, st); TE();
   TB(CADMAS_STAGE_DOT);
-  launch_dot_t<float>(s, q, ic, h->r0f, h->r0f, nullptr, nullptr, h->rb0, nullptr, st);
+  launch_dot_t<float>(s, g, q, h->r0f, h->r0f, nullptr, nullptr, h->rb0, nullptr, st);
   launch_fin(s, FIN_BNORM, h->rb0, nullptr, nr, st, nullptr, epsa2, epsr2, div2, icgmax);
   launch_fin(s, FIN_START, h->rb0, nullptr, nr, st, nullptr, epsa2, epsr2, div2, icgmax);
   TE();
-  TB(CADMAS_STAGE_VEC); launch_copy2_t<float>(s, q, ic, h->r0f, h->rrf, h->pvf, st); TE();
+  TB(CADMAS_STAGE_VEC); launch_copy2_t<float>(s, q, h->r0f, h->rrf, h->pvf, st); TE();
   int batch = std::max(2, std::min(h->last_iter, 64));
   for (int guard = 0; guard < 100000; ++guard) {
     for (int b = 0; b < batch; ++b) {
@@ -583,7 +578,7 @@ static int solve_inner_f(cadmas_handle *h, double eps, int &iter) {
       if (!d1) launch_bwd_f(s, g, q, S, h->apf, st);
       TE();
       TB(CADMAS_STAGE_DOT);
-      if (!d1) launch_dot2f(s, q, h->r0f, h->apf, h->rb0, st);
+      if (!d1) launch_dot2f(s, g, q, h->r0f, h->apf, h->rb0, st);
       launch_fin(s, FIN_ALPHA, h->rb0, nullptr, d1 ? (long long)q.nb : nr, st, nullptr, epsa2, epsr2, div2, icgmax);
       TE();
       TB(CADMAS_STAGE_VEC); launch_axpyf(s, q, h->apf, h->rrf, st); TE();
@@ -595,7 +590,7 @@ static int solve_inner_f(cadmas_handle *h, double eps, int &iter) {
       if (!d5) launch_bwd_f(s, g, q, S, h->aef, st);
       TE();
       TB(CADMAS_STAGE_DOT);
-      if (!d5) launch_dot5f(s, q, h->r0f, h->rrf, h->aef, h->rb5, st);
+      if (!d5) launch_dot5f(s, g, q, h->r0f, h->rrf, h->aef, h->rb5, st);
       launch_fin5(s, h->rb5, d5 ? (long long)q.nb : nr, st, epsa2, epsr2, div2, icgmax);
       TE();
       TB(CADMAS_STAGE_VEC);
@@ -656,11 +651,9 @@ static int solve_mixed(cadmas_handle *h, const SysPtr &a, double *x0, const int 
     // r = b - A x and the two norms in FP64
     CK(cudaMemsetAsync(st, 0, SOLVE_CLEAR_BYTES, s));
     TB(CADMAS_STAGE_VEC);
-    launch_spmv(s, g, q, h->S, h->xw, h->y2, st);
-    launch_bmy(s, q, ic, h->bb_sl, h->y2, st);
+    launch_resid(s, g, q, h->S, h->bb_sl, h->xw, h->y2, h->rb0, h->rb1, st);
     TE();
     TB(CADMAS_STAGE_DOT);
-    launch_dot(s, q, ic, h->bb_sl, h->bb_sl, h->y2, h->y2, h->rb0, h->rb1, st);
     launch_fin(s, FIN_STORE, h->rb0, h->rb1, nr, st, h->dres + 6, 0, 0, 0, 0);
     TE();
     CK(cudaMemcpyAsync(h->h_res + 6, h->dres + 6, 2 * sizeof(double), cudaMemcpyDeviceToHost, s));
@@ -670,7 +663,7 @@ static int solve_mixed(cadmas_handle *h, const SysPtr &a, double *x0, const int 
     h->mixed_outer++;
     if (r2 <= tol2 * b2) { converged = true; break; }
     const double rn = std::sqrt(r2);
-    launch_scale_to_f(s, q, ic, h->y2, 1.0 / rn, h->bf);
+    launch_scale_to_f(s, q, h->y2, 1.0 / rn, h->bf);
     // Each pass reduces the residual by about its inner tolerance: ask
     // for half the reduction still needed, no less than the FP32 floor,
     // so the last pass stops near CGEPSR instead of far below it.
@@ -682,7 +675,7 @@ static int solve_mixed(cadmas_handle *h, const SysPtr &a, double *x0, const int 
     if (rc) return rc;
     if (it < 0 || it > h->P.icgmax) return fallback();  // factor, divergence or cap
     total += it;
-    launch_add_f(s, q, ic, h->xf, rn, h->xw);
+    launch_add_f(s, q, h->xf, rn, h->xw);
   }
   if (!converged) return fallback();
   // X0 = XW on INDC != -1 (k_x0 requires ITER >= 0: the state is clear)
@@ -1130,7 +1123,9 @@ int cadmas_create(const cadmas_dims *d, const cadmas_params *p, cadmas_handle **
     g_last_error = "preconditioner block too large for the MILU sweeps; set precond_ti/precond_tj";
     rc = CADMAS_EUNSUPPORTED;
   }
-  h->nsl = (size_t)h->q.nb * h->q.W * h->q.T;
+  // tiles overlap by their ramps unless those are longer than the columns
+  h->q.WS = (TI - 1) + (TJl - 1) <= d->numk - 2 ? d->numk - 2 : h->q.W;
+  h->nsl = (size_t)skew_entries(h->q);
   h->nslab = (long long)h->q.nb * h->q.W;
   h->nrb = (h->nslab + ROWS_PER_BLOCK - 1) / ROWS_PER_BLOCK;
   {
@@ -1180,6 +1175,7 @@ int cadmas_create(const cadmas_dims *d, const cadmas_params *p, cadmas_handle **
   // NF starts as all obstacle until set_state; INDC as non-computed.
   cudaMemset(h->nf, 0xff, h->N * sizeof(int));
   cudaMemset(h->indc, 0xff, h->N * sizeof(int));
+  cudaMemset(h->S.indc, 0xff, h->nsl * sizeof(int));  // entries without a cell are never written
   launch_drop_reset(h->s, (long long)h->N, h->drop);
   h->tbub.assign(d->numk, 0.0);
   h->h_active.assign(d->numk + 1, 0);
@@ -2043,7 +2039,7 @@ static void solve_mixed_batch(cadmas_batch *b, const std::vector<int> &idx, std:
   auto fail = [&](int code) { for (int j = 0; j < nm; ++j) if (!rc[j]) rc[j] = code; };
   // member table and block prefixes
   std::vector<int> pre((size_t)BR_N * (nm + 1), 0);
-  long long ntiles = 0, nslab = 0, nelem = 0;
+  long long ntiles = 0, nslab = 0, nelem = 0, nflat = 0;
   for (int j = 0; j < nm; ++j) {
     b->h_m[j] = batch_member_of(hs[j]);
     const SkewGeo &q = hs[j]->q;
@@ -2051,6 +2047,8 @@ static void solve_mixed_batch(cadmas_batch *b, const std::vector<int> &idx, std:
     pre[BR_TILE * (nm + 1) + j] = (int)ntiles;
     pre[BR_SLAB * (nm + 1) + j] = (int)nslab;
     pre[BR_ELEM * (nm + 1) + j] = (int)nelem;
+    pre[BR_FLAT * (nm + 1) + j] = (int)nflat;
+    nflat += (skew_entries(q) + FLAT_BLOCK - 1) / FLAT_BLOCK;
     ntiles += q.nb;
     nslab += hs[j]->nrb;
     nelem += (n + BATCH_ELEM - 1) / BATCH_ELEM;
@@ -2058,6 +2056,7 @@ static void solve_mixed_batch(cadmas_batch *b, const std::vector<int> &idx, std:
   pre[BR_TILE * (nm + 1) + nm] = (int)ntiles;
   pre[BR_SLAB * (nm + 1) + nm] = (int)nslab;
   pre[BR_ELEM * (nm + 1) + nm] = (int)nelem;
+  pre[BR_FLAT * (nm + 1) + nm] = (int)nflat;
   SkewGeo qref = hs[0]->q;
   for (int j = 0; j < nm; ++j) qref.ring |= hs[j]->q.ring;
   const BatchMember *bm = b->d_m;
@@ -2113,14 +2112,14 @@ static void solve_mixed_batch(cadmas_batch *b, const std::vector<int> &idx, std:
     if (nact == 0) break;
     if (!upload()) { error = true; break; }
     // the inner FP32 solve of every member refining (solve_inner_f)
-    launch_b_start_f(s, bm, dp, nm, nslab);
+    launch_b_start_f(s, bm, dp, nm, nflat);
     launch_b_clear(s, bm, nm);
     bool ok = launch_b_sweep(s, SWEEP_FWD, bm, dp, nm, ntiles, qref, BF_B, -1, -1, false) &&
               launch_b_sweep(s, SWEEP_BWD, bm, dp, nm, ntiles, qref, -1, BF_R0, -1, false);
     launch_b_dot_r0f(s, bm, dp, nm, nslab);
     launch_b_fin(s, FIN_BNORM, bm, nm, false);
     launch_b_fin(s, FIN_START, bm, nm, false);
-    launch_b_copy2_f(s, bm, dp, nm, nslab);
+    launch_b_copy2_f(s, bm, dp, nm, nflat);
     int last = 8;
     for (int j = 0; j < nm; ++j) last = std::max(last, hs[j]->last_iter);
     int batch = std::max(2, std::min(last, 64));
@@ -2129,11 +2128,11 @@ static void solve_mixed_batch(cadmas_batch *b, const std::vector<int> &idx, std:
         ok = launch_b_sweep(s, SWEEP_FWD_AX, bm, dp, nm, ntiles, qref, BF_PV, -1, -1, false) &&
              launch_b_sweep(s, SWEEP_BWD1, bm, dp, nm, ntiles, qref, BF_R0, BF_AP, -1, false);
         launch_b_fin(s, FIN_ALPHA, bm, nm, true);
-        launch_b_axpyf(s, bm, dp, nm, nslab);
+        launch_b_axpyf(s, bm, dp, nm, nflat);
         ok = ok && launch_b_sweep(s, SWEEP_FWD_AX, bm, dp, nm, ntiles, qref, BF_RR, -1, -1, false) &&
              launch_b_sweep(s, SWEEP_BWD5, bm, dp, nm, ntiles, qref, BF_R0, BF_AE, BF_RR, true);
         launch_b_fin5(s, bm, nm);
-        launch_b_upd3f(s, bm, dp, nm, nslab);
+        launch_b_upd3f(s, bm, dp, nm, nflat);
         launch_b_commit(s, bm, nm);
       }
       if (!ok || !gather()) { ok = false; break; }
@@ -2158,7 +2157,7 @@ static void solve_mixed_batch(cadmas_batch *b, const std::vector<int> &idx, std:
       if (it < 0 || it > M.icgmax) { fallback[j] = 1; M.active = 0; continue; }  // FP64 takes over
       total[j] += it;
     }
-    launch_b_add_f(s, bm, dp, nm, nslab);  // XW += |r| D where the inner solve ended in ICGMAX
+    launch_b_add_f(s, bm, dp, nm, nflat);  // XW += |r| D where the inner solve ended in ICGMAX
   }
   if (error) { set_cuda_error("batched solve", cudaGetLastError()); fail(CADMAS_ECUDA); return; }
   for (int j = 0; j < nm; ++j)

@@ -214,11 +214,12 @@ inline size_t ring_bytes(int NV, int T, int R, size_t es = sizeof(double)) {
 // k = 2+s-ti-tj) with thread t = ti + TIp*tj.  The arrays that stay constant
 // through a solve (7 coefficients, DD, INDC), the right-hand side and the
 // BiCGSTAB vectors are stored tile by tile in that visiting order,
-//     sl(b, w, t) = (b*W + w)*T + t,   w = (k-2) + ti + tj,
-// b = tile index, W = (NK-2) + (TI-1) + (TJ-1), so the T values a block
-// needs at one step are contiguous and every load of the sweep coalesces.
+//     sl(b, w, t) = (b*WS + w)*T + t,   w = (k-2) + ti + tj,
+// b = tile index, w = 0 .. W-1 (SkewGeo says how tiles overlap), so the T
+// values a block needs at one step are contiguous and every load of the
+// sweep coalesces.
 __device__ __forceinline__ long long sl_index(const SkewGeo &q, int b, int w, int t) {
-  return ((long long)b * q.W + w) * q.T + t;
+  return ((long long)b * skew_stride(q) + w) * q.T + t;
 }
 
 // Store the coefficients AD, ALI, ALJ, ALK, AUI, AUJ, AUK of column t of a
@@ -231,8 +232,9 @@ __device__ __forceinline__ void sys_put(double *sys, long long slab, int T, int 
 }
 
 // Copy the Poisson system (7 coefficients, interleaved per slab; DD set to
-// 0 for MZDCMP to fill), INDC, BB and X0 into the skewed layout.  Entries
-// outside the tile or the interior get 0 (INDC -1).  warm: keep the
+// 0 for MZDCMP to fill), INDC, BB and X0 into the skewed layout (e counts
+// the nb*W*T wavefront entries).  Columns of a tile past the grid get 0
+// (INDC -1).  warm: keep the
 // previous solution already in xsl as the initial guess (0 where INDC is
 // now -1) instead of X0.
 __device__ __forceinline__ void to_skew_elem(const Geo &g, const SkewGeo &q, const SysPtr &A_, const int *INDC,
@@ -244,21 +246,23 @@ __device__ __forceinline__ void to_skew_elem(const Geo &g, const SkewGeo &q, con
     const int w = (int)(bw % q.W), b = (int)(bw / q.W);
     const int ti = t % q.TIp, tj = t / q.TIp;
     const int I = 2 + (b % q.ntx) * q.TI + ti, J = 2 + (b / q.ntx) * q.TJ + tj, k = 2 + w - ti - tj;
+    if (ti >= q.TI || k < 2 || k > g.NK - 1) return;  // the entry is not this tile's
+    const long long slab = (long long)b * skew_stride(q) + w, x = slab * q.T + t;
     double v[7] = {0, 0, 0, 0, 0, 0, 0}, bv = 0.0, xv = 0.0;
     int ic = -1;
-    if (ti < q.TI && I <= g.NI - 1 && J <= g.NJ - 1 && k >= 2 && k <= g.NK - 1) {
+    if (I <= g.NI - 1 && J <= g.NJ - 1) {
       const long long c = cid(g, I, J, k);
       v[0] = A_.ad[c]; v[1] = A_.ali[c]; v[2] = A_.alj[c]; v[3] = A_.alk[c];
       v[4] = A_.aui[c]; v[5] = A_.auj[c]; v[6] = A_.auk[c];
       ic = INDC[c];
       bv = A_.bb[c];
-      xv = warm ? (ic != -1 ? xsl[e] : 0.0) : X0[c];
+      xv = warm ? (ic != -1 ? xsl[x] : 0.0) : X0[c];
     }
-    sys_put(S.sys, bw, q.T, t, v);
-    S.sys[sys_t(bw, q.T, t)] = 0.0;
-    S.indc[e] = ic;
-    bsl[e] = bv;
-    xsl[e] = xv;
+    sys_put(S.sys, slab, q.T, t, v);
+    S.sys[sys_t(slab, q.T, t)] = 0.0;
+    S.indc[x] = ic;
+    bsl[x] = bv;
+    xsl[x] = xv;
   }
 }
 __global__ void k_to_skew(Geo g, SkewGeo q, SysPtr A_, const int *INDC, SkewSys S, const double *X0,
@@ -280,11 +284,11 @@ __global__ void k_to_skew_rows(Geo g, SkewGeo q, SysPtr A_, const int *INDC, Ske
   extern __shared__ __align__(16) double pan[];  // [2][(NK-2) * TI]
   pdl_enter();
   const int b = blockIdx.x / q.TJ, tj = blockIdx.x % q.TJ;
-  const int TI = q.TI, TIp = q.TIp, T = q.T, W = q.W, nk = g.NK - 2;
+  const int TI = q.TI, TIp = q.TIp, T = q.T, nk = g.NK - 2;
   const int is = 2 + (b % q.ntx) * TI, J = 2 + (b / q.ntx) * q.TJ + tj;
   const int wi = (J <= g.NJ - 1) ? min(TI, g.NI - is) : 0;  // columns of the row inside the interior
-  const int npan = nk * TI, nent = W * TIp;
-  const long long slab0 = (long long)b * W;
+  const int npan = nk * TI, nent = (nk + TI - 1) * TIp;  // the row's slabs tj .. tj+nk+TI-2
+  const long long slab0 = (long long)b * skew_stride(q) + tj;
   int *ipan = reinterpret_cast<int *>(pan);
   // INDC, then T = 0, INDC and the warm guess
 #pragma unroll 4
@@ -294,8 +298,9 @@ __global__ void k_to_skew_rows(Geo g, SkewGeo q, SysPtr A_, const int *INDC, Ske
   }
   __syncthreads();
   for (int x = threadIdx.x; x < nent; x += blockDim.x) {
-    const int w = x / TIp, ti = x % TIp, k = 2 + w - ti - tj, t = ti + TIp * tj;
-    const int ic = (ti < TI && k >= 2 && k <= g.NK - 1) ? ipan[(k - 2) * TI + ti] : -1;
+    const int w = x / TIp, ti = x % TIp, t = ti + TIp * tj;
+    if (ti >= TI || (unsigned)(w - ti) >= (unsigned)nk) continue;  // the entry is not this tile's
+    const int ic = ipan[(w - ti) * TI + ti];
     const long long e = (slab0 + w) * T + t;
     S.indc[e] = ic;
     S.sys[sys_t(slab0 + w, T, t)] = 0.0;
@@ -316,10 +321,10 @@ __global__ void k_to_skew_rows(Geo g, SkewGeo q, SysPtr A_, const int *INDC, Ske
     }
     __syncthreads();
     for (int x = threadIdx.x; x < nent; x += blockDim.x) {
-      const int w = x / TIp, ti = x % TIp, k = 2 + w - ti - tj, t = ti + TIp * tj;
-      const bool in = ti < TI && k >= 2 && k <= g.NK - 1;
-      const int p = in ? (k - 2) * TI + ti : 0;
-      const double v0 = in ? pan[p] : 0.0, v1 = in ? pan[npan + p] : 0.0;
+      const int w = x / TIp, ti = x % TIp, t = ti + TIp * tj;
+      if (ti >= TI || (unsigned)(w - ti) >= (unsigned)nk) continue;
+      const int p = (w - ti) * TI + ti;
+      const double v0 = pan[p], v1 = pan[npan + p];
       if (a < 4) {
         *reinterpret_cast<double2 *>(S.sys + sys_chunk<double>(slab0 + w, a, T, t)) = make_double2(v0, v1);
       } else {
@@ -379,7 +384,7 @@ __device__ __forceinline__ void dcmp_body(const Geo &g, const SkewGeo &q, V U, c
   const int r = tj / TJl, tjl = tj % TJl;
   const long long bl = bx + (long long)q.ntx * (by * q.split + r);  // layout tile
   // slab of step s: w = (k-2) + ti + tjl = s - r*TJl
-  const long long slab0 = bl * q.W - (long long)r * TJl;
+  const long long slab0 = bl * skew_stride(q) - (long long)r * TJl;
   const int tl = ti + TIp * tjl;
   const int nsteps = (g.NK - 2) + (wi - 1) + (wj - 1);
   auto prefetch = [&](int s) {
@@ -712,8 +717,8 @@ __device__ __forceinline__ void sweep_body(const Geo &g, const SkewGeo &q, const
   const int hl = halo_left(q, ES) + TIp * htj + halo_lofs(q, ES), hr = halo_right(q, ES) + TIp * htj,
             hd = halo_down(q, ES) + hti, hu = halo_up(q, ES) + hti;
   // forward: T into the system block; backward: X
-  V *vp = BWD ? vout + ((long long)b * q.W + nsteps - 1) * T + tid
-                              : S.sys + sys_t((long long)b * q.W, T, tid);
+  V *vp = BWD ? vout + ((long long)b * skew_stride(q) + nsteps - 1) * T + tid
+                              : S.sys + sys_t((long long)b * skew_stride(q), T, tid);
   const long long vstep = BWD ? -(long long)T : (long long)SYS_N * T;
 
   // Neighbouring column's entry of the exchange buffer and of the ring
@@ -890,25 +895,61 @@ __global__ void __launch_bounds__(MAXT, 1)
   sweep_body<MODE, V, CS>(g, q, S, vin, vout, st, vin2, rb, (int)blockIdx.x, (int)blockIdx.y, D);
 }
 
-// ------------------------------------------------------------ slab kernels
-// The BiCGSTAB vectors live in the skewed layout; a vector kernel maps one
-// warp to one slab (b,w) of T entries and lets lane l visit t = l, l+32, ...
-// The dot products (VF_MZIP) sum in that order: lane partials, warp tree
-// per slab, then the 1024-thread tree over the slab partials (block_final).
-// Padding entries carry INDC = -1 and are skipped like non-computed cells.
-// The hot kernels load every operand of an entry before testing its INDC
-// (all entries of the layout are allocated), so the unrolled loop keeps
-// several entries' loads in flight.
-#define SLAB_LOOP_BEGIN(q)                                                          \
+// ---------------------------------------------- slab and flat kernels
+// The BiCGSTAB vectors live in the skewed layout.  A kernel that forms
+// sums (or needs a cell's place) maps one warp to one wavefront slab (b,w)
+// of T entries and lets lane l visit t = l, l+32, ..., skipping the entries
+// that are not the tile's (they hold cells of another tile).  The dot
+// products (VF_MZIP) sum in that order: lane partials, warp tree per slab,
+// then the 1024-thread tree over the slab partials (block_final).
+// Every vector is zero wherever INDC = -1 and where an entry holds no cell
+// (the sweeps write 0 for non-computed cells), so sums need no INDC, and
+// the kernels without sums pass over the whole arrays (FLAT_LOOP): an update
+// leaves a zero entry zero.
+// What is not the tile's: k = 2 + w - ti - tj outside 2 .. NK-1.
+// The loops stand in two parts, all loads of several entries, then their
+// arithmetic and stores: the compiler may not move a load above the stores of
+// an earlier entry by itself, and one entry's loads in flight per thread
+// left the passes at half the memory's rate.
+#define SLAB_BEGIN(g, q)                                                            \
   const int lane_ = threadIdx.x & 31;                                               \
   const long long slab_ = (long long)BX_ * ROWS_PER_BLOCK + (threadIdx.x >> 5);      \
   if (slab_ < (long long)(q).nb * (q).W) {                                          \
-    _Pragma("unroll 4")                                                             \
-    for (int t_ = lane_; t_ < (q).T; t_ += 32) {                                    \
-      const long long e = slab_ * (q).T + t_;
+    const int b_ = (int)(slab_ / (q).W), w_ = (int)(slab_ - (long long)b_ * (q).W);   \
+    const long long e0_ = ((long long)b_ * skew_stride(q) + w_) * (q).T;             \
+    const unsigned nk_ = (unsigned)((g).NK - 2);
+#define SLAB_END }
+// the U entries t = t0, t0+32, ... of a lane: in[u] whether the tile has it
+#define SLAB_ENTRIES(q, U)                                                          \
+  bool in[U];                                                                       \
+  _Pragma("unroll")                                                                 \
+  for (int u = 0; u < U; ++u) {                                                     \
+    const int t = t0 + 32 * u, tj = t / (q).TIp;                                     \
+    in[u] = t < (q).T && (unsigned)(w_ - (t - tj * (q).TIp) - tj) < nk_;             \
+  }                                                                                 \
+  const long long e = e0_ + t0;
+#define SLAB_LOOP_BEGIN(g, q)                                                       \
+  SLAB_BEGIN(g, q)                                                                  \
+  _Pragma("unroll 4")                                                               \
+  for (int t_ = lane_; t_ < (q).T; t_ += 32) {                                      \
+    const int tj_ = t_ / (q).TIp, ti_ = t_ - tj_ * (q).TIp;                          \
+    const bool in_ = (unsigned)(w_ - ti_ - tj_) < nk_;                               \
+    const long long e = e0_ + t_;
 #define SLAB_LOOP_END \
-    }                 \
-  }
+  }                   \
+  SLAB_END
+// FLAT_BLOCK entries per block of 256 threads, `per` entries (16 bytes) at a
+// time, U of them loaded together; the arrays' lengths are multiples of 4
+#define FLAT_LOOP_BEGIN(q, per, U)                                                  \
+  const long long n_ = skew_entries(q) / (per), i0_ = (long long)BX_ * (FLAT_BLOCK / (per)) + threadIdx.x; \
+  for (int j_ = 0; j_ < FLAT_BLOCK / (per) / 256; j_ += U) {                        \
+    long long e[U];                                                                 \
+    bool in[U];                                                                     \
+    _Pragma("unroll")                                                               \
+    for (int u = 0; u < U; ++u) { e[u] = i0_ + (j_ + u) * 256; in[u] = e[u] < n_; }
+#define FLAT_LOOP_END }
+#define EACH(U) _Pragma("unroll") for (int u = 0; u < U; ++u) if (in[u])
+
 // Partial of one block of a slab sum: each warp's slab sum (warp tree),
 // then the block's ROWS_PER_BLOCK slabs added in slab order by thread 0,
 // into rb[bx] (bx the block's index).  The finaliser then reduces one
@@ -933,15 +974,15 @@ __device__ __forceinline__ bool interior(const Geo &g, int I, int J, int K) {
   return I >= 2 && I <= g.NI - 1 && J >= 2 && J <= g.NJ - 1 && K >= 2 && K <= g.NK - 1;
 }
 
-// A*X at skewed entry e (VF_MZAX expression, vf_mzax.f:46-53).
+// A*X at entry e, column (ti,tj) of tile b, layer k (VF_MZAX expression,
+// vf_mzax.f:46-53).
 template <typename V>
-__device__ __forceinline__ V skew_ax(const Geo &g, const SkewGeo &q, const SkewSysT<V> &S, const V *X,
-                                     long long e) {
-  const int t = (int)(e % q.T);
-  const long long bw = e / q.T;
-  const int w = (int)(bw % q.W), b = (int)(bw / q.W);
-  const int ti = t % q.TIp, tj = t / q.TIp, bx = b % q.ntx, by = b / q.ntx, k = 2 + w - ti - tj;
-  const V *s = S.sys + sys_chunk<V>(bw, 0, q.T, 0);
+__device__ __forceinline__ V skew_ax(const Geo &g, const SkewGeo &q, const SkewSysT<V> &S, const V *X, long long e,
+                                     int b, int ti, int tj, int k) {
+  const long long slab = e / q.T;
+  const int t = (int)(e - slab * q.T);
+  const int bx = b % q.ntx, by = b / q.ntx;
+  const V *s = S.sys + sys_chunk<V>(slab, 0, q.T, 0);
   auto a = [&](int c) { return s[sys_in_run<V>(c, q.T, t)]; };
   auto at = [&](int di, int dj, int dk) -> V {
     const long long n = skew_nb(g, q, bx, by, ti + di, tj + dj, k + dk);
@@ -951,30 +992,46 @@ __device__ __forceinline__ V skew_ax(const Geo &g, const SkewGeo &q, const SkewS
          a(SYS_AUI) * at(1, 0, 0) + a(SYS_AUJ) * at(0, 1, 0) + a(SYS_AUK) * at(0, 0, 1);
 }
 
-// Y = A X on INDC != -1 (VF_MZAX); Y untouched elsewhere.
-template <typename V>
-__device__ __forceinline__ void spmv_body(Geo g, SkewGeo q, SkewSysT<V> S, const V *X, V *Y, const SolveState *st, unsigned BX_) {
-  if (st && st->done) return;
-  SLAB_LOOP_BEGIN(q)
-  if (S.indc[e] != -1) Y[e] = skew_ax(g, q, S, X, e);
-  SLAB_LOOP_END
-}
+// Y = A X on INDC != -1 (VF_MZAX), 0 elsewhere.
 template <typename V>
 __global__ void k_spmv(Geo g, SkewGeo q, SkewSysT<V> S, const V *X, V *Y, const SolveState *st) {
   pdl_enter();
-  spmv_body<V>(g, q, S, X, Y, st, blockIdx.x);
-}
-
-// Y = B - Y on INDC != -1 (vf_m1bcgs.f:124-132)
-__device__ __forceinline__ void bmy_body(SkewGeo q, const int *INDC, const double *B, double *Y, const SolveState *st, unsigned BX_) {
+  const unsigned BX_ = blockIdx.x;
   if (st && st->done) return;
-  SLAB_LOOP_BEGIN(q)
-  if (INDC[e] != -1) Y[e] = B[e] - Y[e];
+  SLAB_LOOP_BEGIN(g, q)
+  if (in_) Y[e] = S.indc[e] != -1 ? skew_ax(g, q, S, X, e, b_, ti_, tj_, 2 + w_ - ti_ - tj_) : V(0);
   SLAB_LOOP_END
 }
-__global__ void k_bmy(SkewGeo q, const int *INDC, const double *B, double *Y, const SolveState *st) {
+
+// Y = B - A X on INDC != -1 (vf_m1bcgs.f:117-132), 0 elsewhere; with rb0
+// also the slab partials of (B,B) and (Y,Y) over INDC != -1.
+__device__ __forceinline__ void resid_body(const Geo &g, const SkewGeo &q, const SkewSys &S, const double *B,
+                                           const double *X, double *Y, double *rb0, double *rb1,
+                                           const SolveState *st, unsigned BX_) {
+  if (st && st->done) return;
+  double s0 = 0.0, s1 = 0.0;
+  const long long nslab = (long long)q.nb * q.W;
+  SLAB_LOOP_BEGIN(g, q)
+  if (in_) {
+    double y = 0.0;
+    if (S.indc[e] != -1) {
+      const double bv = B[e];
+      y = bv - skew_ax(g, q, S, X, e, b_, ti_, tj_, 2 + w_ - ti_ - tj_);
+      s0 = s0 + bv * bv;
+      s1 = s1 + y * y;
+    }
+    Y[e] = y;
+  }
+  SLAB_LOOP_END
+  if (rb0) {
+    slab_store(s0, rb0, nslab, BX_);
+    slab_store(s1, rb1, nslab, BX_);
+  }
+}
+__global__ void k_resid(Geo g, SkewGeo q, SkewSys S, const double *B, const double *X, double *Y, double *rb0,
+                        double *rb1, const SolveState *st) {
   pdl_enter();
-  bmy_body(q, INDC, B, Y, st, blockIdx.x);
+  resid_body(g, q, S, B, X, Y, rb0, rb1, st, blockIdx.x);
 }
 
 // The BiCGSTAB vector kernels below serve the FP64 solve (V = double) and
@@ -984,62 +1041,77 @@ __global__ void k_bmy(SkewGeo q, const int *INDC, const double *B, double *Y, co
 
 // Slab partials of up to two dot products (VF_MZIP).
 template <typename V>
-__device__ __forceinline__ void dot_body(SkewGeo q, const int *INDC, const V *x0, const V *y0, const V *x1, const V *y1,
+__device__ __forceinline__ void dot_body(const Geo &g, const SkewGeo &q, const V *x0, const V *y0, const V *x1, const V *y1,
                       double *rb0, double *rb1, const SolveState *st, unsigned BX_) {
   if (st && st->done) return;
   double s0 = 0.0, s1 = 0.0;
   const long long nslab = (long long)q.nb * q.W;
-  SLAB_LOOP_BEGIN(q)
-  const int ic = INDC[e];
-  const double a0 = (double)x0[e] * (double)y0[e];
-  const double a1 = x1 ? (double)x1[e] * (double)y1[e] : 0.0;
-  if (ic != -1) {
-    s0 = s0 + a0;
-    if (x1) s1 = s1 + a1;
+  SLAB_BEGIN(g, q)
+  for (int t0 = lane_; t0 < q.T; t0 += 128) {
+    SLAB_ENTRIES(q, 4)
+    V a[4], c[4], a1[4], c1[4];
+#pragma unroll
+    for (int u = 0; u < 4; ++u) a[u] = c[u] = a1[u] = c1[u] = V(0);
+    EACH(4) { a[u] = x0[e + 32 * u]; c[u] = y0[e + 32 * u]; }
+    if (x1) EACH(4) { a1[u] = x1[e + 32 * u]; c1[u] = y1[e + 32 * u]; }
+#pragma unroll
+    for (int u = 0; u < 4; ++u) {
+      s0 = s0 + (double)a[u] * (double)c[u];
+      s1 = s1 + (double)a1[u] * (double)c1[u];
+    }
   }
-  SLAB_LOOP_END
+  SLAB_END
   slab_store(s0, rb0, nslab, BX_);
   if (x1) slab_store(s1, rb1, nslab, BX_);
 }
 template <typename V>
-__global__ void k_dot(SkewGeo q, const int *INDC, const V *x0, const V *y0, const V *x1, const V *y1,
+__global__ void k_dot(Geo g, SkewGeo q, const V *x0, const V *y0, const V *x1, const V *y1,
                       double *rb0, double *rb1, const SolveState *st) {
   pdl_enter();
-  dot_body<V>(q, INDC, x0, y0, x1, y1, rb0, rb1, st, blockIdx.x);
+  dot_body<V>(g, q, x0, y0, x1, y1, rb0, rb1, st, blockIdx.x);
 }
 
 // RR = R0, PP = R0
 template <typename V>
-__device__ __forceinline__ void copy2_body(SkewGeo q, const int *INDC, const V *R0, V *RR, V *PP, const SolveState *st, unsigned BX_) {
+__device__ __forceinline__ void copy2_body(const SkewGeo &q, const V *R0, V *RR, V *PP, const SolveState *st, unsigned BX_) {
   if (st->done) return;
-  SLAB_LOOP_BEGIN(q)
-  if (INDC[e] != -1) { RR[e] = R0[e]; PP[e] = R0[e]; }
-  SLAB_LOOP_END
+  constexpr int G = 16 / (int)sizeof(V);
+  const uint4 *r0 = reinterpret_cast<const uint4 *>(R0);
+  uint4 *rr = reinterpret_cast<uint4 *>(RR), *pp = reinterpret_cast<uint4 *>(PP);
+  FLAT_LOOP_BEGIN(q, G, 4)
+  uint4 r[4];
+  EACH(4) r[u] = r0[e[u]];
+  EACH(4) { rr[e[u]] = r[u]; pp[e[u]] = r[u]; }
+  FLAT_LOOP_END
 }
 template <typename V>
-__global__ void k_copy2(SkewGeo q, const int *INDC, const V *R0, V *RR, V *PP, const SolveState *st) {
+__global__ void __launch_bounds__(256) k_copy2(SkewGeo q, const V *R0, V *RR, V *PP, const SolveState *st) {
   pdl_enter();
-  copy2_body<V>(q, INDC, R0, RR, PP, st, blockIdx.x);
+  copy2_body<V>(q, R0, RR, PP, st, blockIdx.x);
 }
 
 // RR = RR - ALPHA*AP (vf_m1bcgs.f:181-189)
-template <typename V>
-__global__ void k_axpy_rr(SkewGeo q, const int *INDC, const V *AP, V *RR, const SolveState *st) {
+__global__ void __launch_bounds__(256) k_axpy_rr(SkewGeo q, const double *AP, double *RR, const SolveState *st) {
   pdl_enter();
   const unsigned BX_ = blockIdx.x;
   if (st->done) return;
   const double alpha = st->alpha;
-  SLAB_LOOP_BEGIN(q)
-  const int ic = INDC[e];
-  const V r = RR[e], a = AP[e];
-  if (ic != -1) RR[e] = (V)(r - alpha * a);
-  SLAB_LOOP_END
+  const double2 *ap = reinterpret_cast<const double2 *>(AP);
+  double2 *rr = reinterpret_cast<double2 *>(RR);
+  FLAT_LOOP_BEGIN(q, 2, 4)
+  double2 r[4], a[4];
+  EACH(4) { r[u] = rr[e[u]]; a[u] = ap[e[u]]; }
+  EACH(4) {
+    r[u].x = r[u].x - alpha * a[u].x;
+    r[u].y = r[u].y - alpha * a[u].y;
+    rr[e[u]] = r[u];
+  }
+  FLAT_LOOP_END
 }
 
 // XW = XW + (ALPHA*PP + OMEGA*RR); RR = RR - OMEGA*AE; slab partials of
 // (RR,RR) and (R0,RR) on the updated RR (vf_m1bcgs.f:206-225).
-template <typename V>
-__global__ void k_upd_xr(SkewGeo q, const int *INDC, const V *PP, const V *AE, const V *R0, V *XW, V *RR,
+__global__ void k_upd_xr(Geo g, SkewGeo q, const double *PP, const double *AE, const double *R0, double *XW, double *RR,
                          double *rb0, double *rb1, const SolveState *st) {
   pdl_enter();
   const unsigned BX_ = blockIdx.x;
@@ -1047,33 +1119,45 @@ __global__ void k_upd_xr(SkewGeo q, const int *INDC, const V *PP, const V *AE, c
   const double alpha = st->alpha, omega = st->omega;
   double s0 = 0.0, s1 = 0.0;
   const long long nslab = (long long)q.nb * q.W;
-  SLAB_LOOP_BEGIN(q)
-  const int ic = INDC[e];
-  const V xw = XW[e], pp = PP[e], rr = RR[e], ae = AE[e], r0 = R0[e];
-  if (ic != -1) {
-    XW[e] = (V)(xw + (alpha * pp + omega * rr));
-    const V r = (V)(rr - omega * ae);
-    RR[e] = r;
-    s0 = s0 + (double)r * (double)r;
-    s1 = s1 + (double)r0 * (double)r;
+  SLAB_BEGIN(g, q)
+  for (int t0 = lane_; t0 < q.T; t0 += 128) {
+    SLAB_ENTRIES(q, 4)
+    double xw[4], pp[4], rr[4], ae[4], r0[4];
+#pragma unroll
+    for (int u = 0; u < 4; ++u) xw[u] = pp[u] = rr[u] = ae[u] = r0[u] = 0.0;
+    EACH(4) { xw[u] = XW[e + 32 * u]; pp[u] = PP[e + 32 * u]; rr[u] = RR[e + 32 * u]; ae[u] = AE[e + 32 * u]; r0[u] = R0[e + 32 * u]; }
+    EACH(4) XW[e + 32 * u] = xw[u] + (alpha * pp[u] + omega * rr[u]);
+#pragma unroll
+    for (int u = 0; u < 4; ++u) {
+      const double r = in[u] ? rr[u] - omega * ae[u] : 0.0;
+      if (in[u]) RR[e + 32 * u] = r;
+      s0 = s0 + r * r;
+      s1 = s1 + r0[u] * r;
+    }
   }
-  SLAB_LOOP_END
+  SLAB_END
   slab_store(s0, rb0, nslab, BX_);
   slab_store(s1, rb1, nslab, BX_);
 }
 
 // PP = RR + BETA*(PP - OMEGA*AP) (vf_m1bcgs.f:229-238)
-template <typename V>
-__global__ void k_upd_p(SkewGeo q, const int *INDC, const V *RR, const V *AP, V *PP, const SolveState *st) {
+__global__ void __launch_bounds__(256) k_upd_p(SkewGeo q, const double *RR, const double *AP, double *PP,
+                                               const SolveState *st) {
   pdl_enter();
   const unsigned BX_ = blockIdx.x;
   if (st->done) return;
   const double beta = st->beta, omega = st->omega;
-  SLAB_LOOP_BEGIN(q)
-  const int ic = INDC[e];
-  const V rr = RR[e], pp = PP[e], ap = AP[e];
-  if (ic != -1) PP[e] = (V)(rr + beta * (pp - omega * ap));
-  SLAB_LOOP_END
+  const double2 *rr = reinterpret_cast<const double2 *>(RR), *ap = reinterpret_cast<const double2 *>(AP);
+  double2 *pp = reinterpret_cast<double2 *>(PP);
+  FLAT_LOOP_BEGIN(q, 2, 4)
+  double2 r[4], a[4], p[4];
+  EACH(4) { r[u] = rr[e[u]]; a[u] = ap[e[u]]; p[u] = pp[e[u]]; }
+  EACH(4) {
+    p[u].x = r[u].x + beta * (p[u].x - omega * a[u].x);
+    p[u].y = r[u].y + beta * (p[u].y - omega * a[u].y);
+    pp[e[u]] = p[u];
+  }
+  FLAT_LOOP_END
 }
 
 // --------------------------------- FP32 inner solves of the mixed solver
@@ -1081,12 +1165,6 @@ __global__ void k_upd_p(SkewGeo q, const int *INDC, const V *RR, const V *AP, V 
 // iteration with fewer passes over the vectors; it is the same method and
 // ends on the same criterion, but its sums are not those of VF_M1BCGS,
 // whose FP64 form (above) keeps the reference's order.
-//   * Every vector is zero wherever INDC = -1 and on the layout's padding
-//     (zeroed at the start of a solve and never written there: the
-//     sweeps write 0 for non-computed cells), so these kernels read no
-//     INDC: an update leaves a zero entry zero and adds nothing to a sum.
-//   * One lane moves 4 consecutive entries (16-byte loads; T is a multiple
-//     of 4 and every slab starts on a 16-byte boundary).
 //   * After the second sweep pair one pass forms the five sums (RR,AE),
 //     (AE,AE), (RR,RR), (R0,RR), (R0,AE); OMEGA, the new |RR|^2 =
 //     (RR,RR) - 2 OMEGA (RR,AE) + OMEGA^2 (AE,AE), the new (R0,RR) =
@@ -1094,55 +1172,66 @@ __global__ void k_upd_p(SkewGeo q, const int *INDC, const V *RR, const V *AP, V 
 //     them (k_fin5), and one pass updates XW, RR and PP together (k_upd3f).
 //     Per iteration a sum drops by about 25 times, so the expansion loses
 //     nothing to cancellation at the tolerances used (FP64 sums).
-#define SLAB4_LOOP_BEGIN(q)                                                         \
+// Four consecutive entries per lane of a slab, as 16-byte loads; keep4
+// clears those that are not the tile's.
+#define SLAB4_LOOP_BEGIN(g, q)                                                      \
   const int lane_ = threadIdx.x & 31;                                               \
   const long long slab_ = (long long)BX_ * ROWS_PER_BLOCK + (threadIdx.x >> 5);      \
   if (slab_ < (long long)(q).nb * (q).W) {                                          \
+    const int b_ = (int)(slab_ / (q).W), w_ = (int)(slab_ - (long long)b_ * (q).W);   \
     const int T4_ = (q).T >> 2;                                                     \
+    const unsigned nk_ = (unsigned)((g).NK - 2);                                     \
     _Pragma("unroll 2")                                                             \
     for (int t_ = lane_; t_ < T4_; t_ += 32) {                                      \
-      const long long e4 = slab_ * T4_ + t_;
+      const int tj_ = 4 * t_ / (q).TIp, s_ = w_ - (4 * t_ - tj_ * (q).TIp) - tj_;     \
+      const long long e4 = ((long long)b_ * skew_stride(q) + w_) * T4_ + t_;
 #define SLAB4_LOOP_END \
     }                  \
   }
+__device__ __forceinline__ float4 keep4(const float4 &a, int s, unsigned nk) {
+  return make_float4((unsigned)s < nk ? a.x : 0.0f, (unsigned)(s - 1) < nk ? a.y : 0.0f,
+                     (unsigned)(s - 2) < nk ? a.z : 0.0f, (unsigned)(s - 3) < nk ? a.w : 0.0f);
+}
 __device__ __forceinline__ double dot4(const float4 &a, const float4 &b) {
   return (double)a.x * (double)b.x + (double)a.y * (double)b.y + (double)a.z * (double)b.z +
          (double)a.w * (double)b.w;
 }
 // slab partials of (R0,AP)
-__global__ void k_dot2f(SkewGeo q, const float *R0, const float *AP, double *rb, const SolveState *st) {
+__global__ void k_dot2f(Geo g, SkewGeo q, const float *R0, const float *AP, double *rb, const SolveState *st) {
   pdl_enter();
   const unsigned BX_ = blockIdx.x;
   if (st->done) return;
   const float4 *r0 = reinterpret_cast<const float4 *>(R0), *ap = reinterpret_cast<const float4 *>(AP);
   double s0 = 0.0;
   const long long nslab = (long long)q.nb * q.W;
-  SLAB4_LOOP_BEGIN(q)
-  s0 += dot4(r0[e4], ap[e4]);
+  SLAB4_LOOP_BEGIN(g, q)
+  s0 += dot4(keep4(r0[e4], s_, nk_), keep4(ap[e4], s_, nk_));
   SLAB4_LOOP_END
   slab_store(s0, rb, nslab, BX_);
 }
 // RR = RR - ALPHA*AP
-__device__ __forceinline__ void axpyf_body(SkewGeo q, const float *AP, float *RR, const SolveState *st, unsigned BX_) {
+__device__ __forceinline__ void axpyf_body(const SkewGeo &q, const float *AP, float *RR, const SolveState *st, unsigned BX_) {
   if (st->done) return;
   const double alpha = st->alpha;
   const float4 *ap = reinterpret_cast<const float4 *>(AP);
   float4 *rr = reinterpret_cast<float4 *>(RR);
-  SLAB4_LOOP_BEGIN(q)
-  const float4 a = ap[e4];
-  float4 r = rr[e4];
-  r.x = (float)(r.x - alpha * a.x); r.y = (float)(r.y - alpha * a.y);
-  r.z = (float)(r.z - alpha * a.z); r.w = (float)(r.w - alpha * a.w);
-  rr[e4] = r;
-  SLAB4_LOOP_END
+  FLAT_LOOP_BEGIN(q, 4, 4)
+  float4 r[4], a[4];
+  EACH(4) { r[u] = rr[e[u]]; a[u] = ap[e[u]]; }
+  EACH(4) {
+    r[u].x = (float)(r[u].x - alpha * a[u].x); r[u].y = (float)(r[u].y - alpha * a[u].y);
+    r[u].z = (float)(r[u].z - alpha * a[u].z); r[u].w = (float)(r[u].w - alpha * a[u].w);
+    rr[e[u]] = r[u];
+  }
+  FLAT_LOOP_END
 }
-__global__ void k_axpyf(SkewGeo q, const float *AP, float *RR, const SolveState *st) {
+__global__ void __launch_bounds__(256) k_axpyf(SkewGeo q, const float *AP, float *RR, const SolveState *st) {
   pdl_enter();
   axpyf_body(q, AP, RR, st, blockIdx.x);
 }
 // block partials of (RR,AE), (AE,AE), (RR,RR), (R0,RR), (R0,AE) into
 // rb + c*nrb, c = 0..4 (nrb = blocks of the launch)
-__global__ void k_dot5f(SkewGeo q, const float *R0, const float *RR, const float *AE, double *rb,
+__global__ void k_dot5f(Geo g, SkewGeo q, const float *R0, const float *RR, const float *AE, double *rb,
                         const SolveState *st) {
   pdl_enter();
   const unsigned BX_ = blockIdx.x;
@@ -1151,8 +1240,8 @@ __global__ void k_dot5f(SkewGeo q, const float *R0, const float *RR, const float
                *ae = reinterpret_cast<const float4 *>(AE);
   double s0 = 0.0, s1 = 0.0, s2 = 0.0, s3 = 0.0, s4 = 0.0;
   const long long nslab = (long long)q.nb * q.W;
-  SLAB4_LOOP_BEGIN(q)
-  const float4 a = r0[e4], r = rr[e4], e = ae[e4];
+  SLAB4_LOOP_BEGIN(g, q)
+  const float4 a = keep4(r0[e4], s_, nk_), r = keep4(rr[e4], s_, nk_), e = keep4(ae[e4], s_, nk_);
   s0 += dot4(r, e);
   s1 += dot4(e, e);
   s2 += dot4(r, r);
@@ -1168,29 +1257,32 @@ __global__ void k_dot5f(SkewGeo q, const float *R0, const float *RR, const float
 }
 // XW = XW + (ALPHA*PP + OMEGA*RR); RR' = RR - OMEGA*AE;
 // PP = RR' + BETA*(PP - OMEGA*AP); RR = RR'
-__device__ __forceinline__ void upd3f_body(SkewGeo q, const float *AE, const float *AP, float *XW, float *RR, float *PP,
+__device__ __forceinline__ void upd3f_body(const SkewGeo &q, const float *AE, const float *AP, float *XW, float *RR, float *PP,
                         const SolveState *st, unsigned BX_) {
   if (st->done) return;
   const double alpha = st->alpha, omega = st->omega, beta = st->beta;
   const float4 *ae = reinterpret_cast<const float4 *>(AE), *ap = reinterpret_cast<const float4 *>(AP);
   float4 *xw = reinterpret_cast<float4 *>(XW), *rr = reinterpret_cast<float4 *>(RR),
          *pp = reinterpret_cast<float4 *>(PP);
-  SLAB4_LOOP_BEGIN(q)
-  const float4 e = ae[e4], a = ap[e4], r = rr[e4], p = pp[e4];
-  float4 x = xw[e4], rn, pn;
-#define UPD3_(c)                                                   \
-  x.c = (float)(x.c + (alpha * p.c + omega * r.c));                \
-  rn.c = (float)(r.c - omega * e.c);                               \
-  pn.c = (float)(rn.c + beta * (p.c - omega * a.c));
-  UPD3_(x) UPD3_(y) UPD3_(z) UPD3_(w)
+  FLAT_LOOP_BEGIN(q, 4, 2)
+  float4 d[2], a[2], r[2], p[2], x[2];
+  EACH(2) { d[u] = ae[e[u]]; a[u] = ap[e[u]]; r[u] = rr[e[u]]; p[u] = pp[e[u]]; x[u] = xw[e[u]]; }
+  EACH(2) {
+    float4 rn, pn;
+#define UPD3_(c)                                                              \
+    x[u].c = (float)(x[u].c + (alpha * p[u].c + omega * r[u].c));             \
+    rn.c = (float)(r[u].c - omega * d[u].c);                                  \
+    pn.c = (float)(rn.c + beta * (p[u].c - omega * a[u].c));
+    UPD3_(x) UPD3_(y) UPD3_(z) UPD3_(w)
 #undef UPD3_
-  xw[e4] = x;
-  rr[e4] = rn;
-  pp[e4] = pn;
-  SLAB4_LOOP_END
+    xw[e[u]] = x[u];
+    rr[e[u]] = rn;
+    pp[e[u]] = pn;
+  }
+  FLAT_LOOP_END
 }
-__global__ void k_upd3f(SkewGeo q, const float *AE, const float *AP, float *XW, float *RR, float *PP,
-                        const SolveState *st) {
+__global__ void __launch_bounds__(256) k_upd3f(SkewGeo q, const float *AE, const float *AP, float *XW, float *RR,
+                                               float *PP, const SolveState *st) {
   pdl_enter();
   upd3f_body(q, AE, AP, XW, RR, PP, st, blockIdx.x);
 }
@@ -1249,41 +1341,53 @@ __device__ __forceinline__ void sys_to_f_elem(const SkewGeo &q, const double *sy
 }
 __global__ void k_sys_to_f(SkewGeo q, const double *sys, float *sysf) {
   pdl_enter();
-  const long long n = (long long)q.nb * q.W * q.T;
+  const long long n = skew_entries(q);
   for (long long e = blockIdx.x * (long long)blockDim.x + threadIdx.x; e < n; e += (long long)gridDim.x * blockDim.x)
     sys_to_f_elem(q, sys, sysf, e);
 }
-// RF = R * scale on INDC != -1 (the right-hand side of an inner solve)
-__device__ __forceinline__ void scale_to_f_body(SkewGeo q, const int *INDC, const double *R, double scale, float *RF, unsigned BX_) {
-  SLAB_LOOP_BEGIN(q)
-  if (INDC[e] != -1) RF[e] = (float)(R[e] * scale);
-  SLAB_LOOP_END
+// RF = R * scale (the right-hand side of an inner solve)
+__device__ __forceinline__ void scale_to_f_body(const SkewGeo &q, const double *R, double scale, float *RF, unsigned BX_) {
+  const double2 *r2 = reinterpret_cast<const double2 *>(R);
+  float4 *rf = reinterpret_cast<float4 *>(RF);
+  FLAT_LOOP_BEGIN(q, 4, 4)
+  double2 a[4], b[4];
+  EACH(4) { a[u] = r2[2 * e[u]]; b[u] = r2[2 * e[u] + 1]; }
+  EACH(4) rf[e[u]] = make_float4((float)(a[u].x * scale), (float)(a[u].y * scale), (float)(b[u].x * scale), (float)(b[u].y * scale));
+  FLAT_LOOP_END
 }
-__global__ void k_scale_to_f(SkewGeo q, const int *INDC, const double *R, double scale, float *RF) {
+__global__ void __launch_bounds__(256) k_scale_to_f(SkewGeo q, const double *R, double scale, float *RF) {
   pdl_enter();
-  scale_to_f_body(q, INDC, R, scale, RF, blockIdx.x);
+  scale_to_f_body(q, R, scale, RF, blockIdx.x);
 }
-// X = X + D * inv_scale on INDC != -1 (the correction of an inner solve)
-__device__ __forceinline__ void add_f_body(SkewGeo q, const int *INDC, const float *D, double inv_scale, double *X, unsigned BX_) {
-  SLAB_LOOP_BEGIN(q)
-  if (INDC[e] != -1) X[e] = X[e] + (double)D[e] * inv_scale;
-  SLAB_LOOP_END
+// X = X + D * inv_scale (the correction of an inner solve)
+__device__ __forceinline__ void add_f_body(const SkewGeo &q, const float *D, double inv_scale, double *X, unsigned BX_) {
+  const float4 *d4 = reinterpret_cast<const float4 *>(D);
+  double2 *x2 = reinterpret_cast<double2 *>(X);
+  FLAT_LOOP_BEGIN(q, 4, 2)
+  float4 d[2];
+  double2 a[2], b[2];
+  EACH(2) { d[u] = d4[e[u]]; a[u] = x2[2 * e[u]]; b[u] = x2[2 * e[u] + 1]; }
+  EACH(2) {
+    a[u].x = a[u].x + (double)d[u].x * inv_scale; a[u].y = a[u].y + (double)d[u].y * inv_scale;
+    b[u].x = b[u].x + (double)d[u].z * inv_scale; b[u].y = b[u].y + (double)d[u].w * inv_scale;
+    x2[2 * e[u]] = a[u];
+    x2[2 * e[u] + 1] = b[u];
+  }
+  FLAT_LOOP_END
 }
-__global__ void k_add_f(SkewGeo q, const int *INDC, const float *D, double inv_scale, double *X) {
+__global__ void __launch_bounds__(256) k_add_f(SkewGeo q, const float *D, double inv_scale, double *X) {
   pdl_enter();
-  add_f_body(q, INDC, D, inv_scale, X, blockIdx.x);
+  add_f_body(q, D, inv_scale, X, blockIdx.x);
 }
 
 // X0 = XW on INDC != -1 when ITER >= 0 (vf_m1bcgs.f:251-261), back to the
 // standard layout.
 __device__ __forceinline__ void x0_body(Geo g, SkewGeo q, const int *INDC, const double *XW, double *X0, const SolveState *st, unsigned BX_) {
   if (st->iter < 0) return;
-  SLAB_LOOP_BEGIN(q)
-  if (INDC[e] != -1) {
-    const int ti = t_ % q.TIp, tj = t_ / q.TIp;
-    const int w = (int)(slab_ % q.W), b = (int)(slab_ / q.W);
-    const int I = 2 + (b % q.ntx) * q.TI + ti, J = 2 + (b / q.ntx) * q.TJ + tj, k = 2 + w - ti - tj;
-    X0[cid(g, I, J, k)] = XW[e];
+  SLAB_LOOP_BEGIN(g, q)
+  if (in_ && INDC[e] != -1) {
+    const int I = 2 + (b_ % q.ntx) * q.TI + ti_, J = 2 + (b_ / q.ntx) * q.TJ + tj_;
+    X0[cid(g, I, J, 2 + w_ - ti_ - tj_)] = XW[e];
   }
   SLAB_LOOP_END
 }
@@ -1299,9 +1403,9 @@ __global__ void k_relres(Geo g, SkewGeo q, SkewSys S, const double *B, const dou
   const unsigned BX_ = blockIdx.x;
   double s0 = 0.0, s1 = 0.0;
   const long long nslab = (long long)q.nb * q.W;
-  SLAB_LOOP_BEGIN(q)
-  if (S.indc[e] != -1) {
-    double r = B[e] - skew_ax(g, q, S, X, e);
+  SLAB_LOOP_BEGIN(g, q)
+  if (in_ && S.indc[e] != -1) {
+    double r = B[e] - skew_ax(g, q, S, X, e, b_, ti_, tj_, 2 + w_ - ti_ - tj_);
     s0 = s0 + r * r;
     s1 = s1 + B[e] * B[e];
   }
@@ -1681,97 +1785,73 @@ static inline unsigned slab_blocks(const SkewGeo &q) {
   return (unsigned)(((long long)q.nb * q.W + ROWS_PER_BLOCK - 1) / ROWS_PER_BLOCK);
 }
 #define SL(kern, ...) launch_pdl(kern, dim3(slab_blocks(q)), dim3(ROW_THREADS), 0, s, 1, __VA_ARGS__)
+static inline unsigned flat_blocks(const SkewGeo &q) { return (unsigned)((skew_entries(q) + FLAT_BLOCK - 1) / FLAT_BLOCK); }
+#define FL(kern, ...) launch_pdl(kern, dim3(flat_blocks(q)), dim3(256), 0, s, 1, __VA_ARGS__)
 template <typename V>
 void launch_spmv_t(cudaStream_t s, const Geo &g, const SkewGeo &q, const SkewSysT<V> &S, const V *x, V *y,
                    const SolveState *st) { SL(k_spmv<V>, g, q, S, x, y, st); }
-void launch_spmv(cudaStream_t s, const Geo &g, const SkewGeo &q, const SkewSys &S, const double *x, double *y,
-                 const SolveState *st) { launch_spmv_t<double>(s, g, q, S, x, y, st); }
-void launch_bmy(cudaStream_t s, const SkewGeo &q, const int *indc, const double *b, double *y,
-                const SolveState *st) { SL(k_bmy, q, indc, b, y, st); }
+void launch_resid(cudaStream_t s, const Geo &g, const SkewGeo &q, const SkewSys &S, const double *b, const double *x,
+                  double *y, double *rb0, double *rb1, const SolveState *st) {
+  SL(k_resid, g, q, S, b, x, y, rb0, rb1, st);
+}
 template <typename V>
-void launch_dot_t(cudaStream_t s, const SkewGeo &q, const int *indc, const V *x0, const V *y0, const V *x1,
+void launch_dot_t(cudaStream_t s, const Geo &g, const SkewGeo &q, const V *x0, const V *y0, const V *x1,
                   const V *y1, double *rb0, double *rb1, const SolveState *st) {
-  SL(k_dot<V>, q, indc, x0, y0, x1, y1, rb0, rb1, st);
+  SL(k_dot<V>, g, q, x0, y0, x1, y1, rb0, rb1, st);
 }
 template <typename V>
-void launch_copy2_t(cudaStream_t s, const SkewGeo &q, const int *indc, const V *r0, V *rr, V *pp,
-                    const SolveState *st) { SL(k_copy2<V>, q, indc, r0, rr, pp, st); }
-template <typename V>
-void launch_axpy_rr_t(cudaStream_t s, const SkewGeo &q, const int *indc, const V *ap, V *rr,
-                      const SolveState *st) { SL(k_axpy_rr<V>, q, indc, ap, rr, st); }
-template <typename V>
-void launch_upd_xr_t(cudaStream_t s, const SkewGeo &q, const int *indc, const V *pp, const V *ae, const V *r0,
-                     V *xw, V *rr, double *rb0, double *rb1, const SolveState *st) {
-  SL(k_upd_xr<V>, q, indc, pp, ae, r0, xw, rr, rb0, rb1, st);
-}
-template <typename V>
-void launch_upd_p_t(cudaStream_t s, const SkewGeo &q, const int *indc, const V *rr, const V *ap, V *pp,
-                    const SolveState *st) { SL(k_upd_p<V>, q, indc, rr, ap, pp, st); }
+void launch_copy2_t(cudaStream_t s, const SkewGeo &q, const V *r0, V *rr, V *pp,
+                    const SolveState *st) { FL(k_copy2<V>, q, r0, rr, pp, st); }
 template void launch_spmv_t<double>(cudaStream_t, const Geo &, const SkewGeo &, const SkewSysT<double> &,
                                     const double *, double *, const SolveState *);
 template void launch_spmv_t<float>(cudaStream_t, const Geo &, const SkewGeo &, const SkewSysT<float> &,
                                    const float *, float *, const SolveState *);
-template void launch_dot_t<double>(cudaStream_t, const SkewGeo &, const int *, const double *, const double *,
+template void launch_dot_t<double>(cudaStream_t, const Geo &, const SkewGeo &, const double *, const double *,
                                    const double *, const double *, double *, double *, const SolveState *);
-template void launch_dot_t<float>(cudaStream_t, const SkewGeo &, const int *, const float *, const float *,
+template void launch_dot_t<float>(cudaStream_t, const Geo &, const SkewGeo &, const float *, const float *,
                                   const float *, const float *, double *, double *, const SolveState *);
-template void launch_copy2_t<double>(cudaStream_t, const SkewGeo &, const int *, const double *, double *,
-                                     double *, const SolveState *);
-template void launch_copy2_t<float>(cudaStream_t, const SkewGeo &, const int *, const float *, float *, float *,
+template void launch_copy2_t<double>(cudaStream_t, const SkewGeo &, const double *, double *, double *,
+                                     const SolveState *);
+template void launch_copy2_t<float>(cudaStream_t, const SkewGeo &, const float *, float *, float *,
                                     const SolveState *);
-template void launch_axpy_rr_t<double>(cudaStream_t, const SkewGeo &, const int *, const double *, double *,
-                                       const SolveState *);
-template void launch_axpy_rr_t<float>(cudaStream_t, const SkewGeo &, const int *, const float *, float *,
-                                      const SolveState *);
-template void launch_upd_xr_t<double>(cudaStream_t, const SkewGeo &, const int *, const double *, const double *,
-                                      const double *, double *, double *, double *, double *, const SolveState *);
-template void launch_upd_xr_t<float>(cudaStream_t, const SkewGeo &, const int *, const float *, const float *,
-                                     const float *, float *, float *, double *, double *, const SolveState *);
-template void launch_upd_p_t<double>(cudaStream_t, const SkewGeo &, const int *, const double *, const double *,
-                                     double *, const SolveState *);
-template void launch_upd_p_t<float>(cudaStream_t, const SkewGeo &, const int *, const float *, const float *,
-                                    float *, const SolveState *);
-void launch_dot(cudaStream_t s, const SkewGeo &q, const int *indc, const double *x0, const double *y0,
-                const double *x1, const double *y1, double *rb0, double *rb1, const SolveState *st) {
-  launch_dot_t<double>(s, q, indc, x0, y0, x1, y1, rb0, rb1, st);
-}
-void launch_copy2(cudaStream_t s, const SkewGeo &q, const int *indc, const double *r0, double *rr, double *pp,
-                  const SolveState *st) { launch_copy2_t<double>(s, q, indc, r0, rr, pp, st); }
-void launch_axpy_rr(cudaStream_t s, const SkewGeo &q, const int *indc, const double *ap, double *rr,
-                    const SolveState *st) { launch_axpy_rr_t<double>(s, q, indc, ap, rr, st); }
-void launch_upd_xr(cudaStream_t s, const SkewGeo &q, const int *indc, const double *pp, const double *ae,
+void launch_axpy_rr(cudaStream_t s, const SkewGeo &q, const double *ap, double *rr,
+                    const SolveState *st) { FL(k_axpy_rr, q, ap, rr, st); }
+void launch_upd_xr(cudaStream_t s, const Geo &g, const SkewGeo &q, const double *pp, const double *ae,
                    const double *r0, double *xw, double *rr, double *rb0, double *rb1, const SolveState *st) {
-  launch_upd_xr_t<double>(s, q, indc, pp, ae, r0, xw, rr, rb0, rb1, st);
+  SL(k_upd_xr, g, q, pp, ae, r0, xw, rr, rb0, rb1, st);
 }
-void launch_upd_p(cudaStream_t s, const SkewGeo &q, const int *indc, const double *rr, const double *ap,
-                  double *pp, const SolveState *st) { launch_upd_p_t<double>(s, q, indc, rr, ap, pp, st); }
+void launch_upd_p(cudaStream_t s, const SkewGeo &q, const double *rr, const double *ap,
+                  double *pp, const SolveState *st) { FL(k_upd_p, q, rr, ap, pp, st); }
 void launch_x0(cudaStream_t s, const Geo &g, const SkewGeo &q, const int *indc, const double *xw, double *x0,
                const SolveState *st) { SL(k_x0, g, q, indc, xw, x0, st); }
 void launch_relres(cudaStream_t s, const Geo &g, const SkewGeo &q, const SkewSys &S, const double *b,
                    const double *x, double *rb0, double *rb1) { SL(k_relres, g, q, S, b, x, rb0, rb1); }
-void launch_dot2f(cudaStream_t s, const SkewGeo &q, const float *r0, const float *ap, double *rb,
-                  const SolveState *st) { SL(k_dot2f, q, r0, ap, rb, st); }
+void launch_dot2f(cudaStream_t s, const Geo &g, const SkewGeo &q, const float *r0, const float *ap, double *rb,
+                  const SolveState *st) { SL(k_dot2f, g, q, r0, ap, rb, st); }
 void launch_axpyf(cudaStream_t s, const SkewGeo &q, const float *ap, float *rr, const SolveState *st) {
-  SL(k_axpyf, q, ap, rr, st);
+  FL(k_axpyf, q, ap, rr, st);
 }
-void launch_dot5f(cudaStream_t s, const SkewGeo &q, const float *r0, const float *rr, const float *ae, double *rb,
-                  const SolveState *st) { SL(k_dot5f, q, r0, rr, ae, rb, st); }
+void launch_dot5f(cudaStream_t s, const Geo &g, const SkewGeo &q, const float *r0, const float *rr, const float *ae,
+                  double *rb, const SolveState *st) { SL(k_dot5f, g, q, r0, rr, ae, rb, st); }
 void launch_upd3f(cudaStream_t s, const SkewGeo &q, const float *ae, const float *ap, float *xw, float *rr,
-                  float *pp, const SolveState *st) { SL(k_upd3f, q, ae, ap, xw, rr, pp, st); }
+                  float *pp, const SolveState *st) { FL(k_upd3f, q, ae, ap, xw, rr, pp, st); }
 void launch_fin5(cudaStream_t s, const double *rb, long long nrows, SolveState *st, double epsa2, double epsr2,
                  double div2, int icgmax) {
   launch_pdl(k_fin5, dim3(1), dim3(1024), 0, s, 1, rb, nrows, st, epsa2, epsr2, div2, icgmax);
 }
 void launch_commit(cudaStream_t s, SolveState *st) { launch_pdl(k_commit, dim3(1), dim3(1), 0, s, 1, st); }
 void launch_sys_to_f(cudaStream_t s, const SkewGeo &q, const double *sys, float *sysf) {
-  const long long n = (long long)q.nb * q.W * q.T;
+  const long long n = skew_entries(q);
   launch_pdl(k_sys_to_f, dim3((unsigned)std::min<long long>((n + 255) / 256, 148LL * 16)), dim3(256), 0, s, 1, q, sys,
              sysf);
 }
-void launch_scale_to_f(cudaStream_t s, const SkewGeo &q, const int *indc, const double *r, double scale,
-                       float *rf) { SL(k_scale_to_f, q, indc, r, scale, rf); }
-void launch_add_f(cudaStream_t s, const SkewGeo &q, const int *indc, const float *d, double inv_scale,
-                  double *x) { SL(k_add_f, q, indc, d, inv_scale, x); }
+void launch_scale_to_f(cudaStream_t s, const SkewGeo &q, const double *r, double scale, float *rf) {
+  FL(k_scale_to_f, q, r, scale, rf);
+}
+void launch_add_f(cudaStream_t s, const SkewGeo &q, const float *d, double inv_scale, double *x) {
+  FL(k_add_f, q, d, inv_scale, x);
+}
+#undef FL
 #undef SL
 void launch_fin(cudaStream_t s, int mode, const double *rb0, const double *rb1, long long nrows,
                 SolveState *st, double *out, double epsa2, double epsr2, double div2, int icgmax) {
@@ -1816,7 +1896,7 @@ __global__ void kb_sys_to_f(const BatchMember *bm, const int *pre, int nm) {
   BATCH_BLOCK(BR_ELEM)
   if (!M.active) return;
   const long long e = (long long)lb_ * BATCH_ELEM + threadIdx.x;
-  if (e < (long long)M.q.nb * M.q.W * M.q.T) sys_to_f_elem(M.q, M.S.sys, M.Sf.sys, e);
+  if (e < skew_entries(M.q)) sys_to_f_elem(M.q, M.S.sys, M.Sf.sys, e);
 }
 template <int D>
 __global__ void kb_dcmp_f(const BatchMember *bm, const int *pre, int nm) {
@@ -1865,12 +1945,10 @@ __global__ void kb_gather(const BatchMember *bm, int nm, double *out) {
   o[4] = bm[m].dres[6]; o[5] = bm[m].dres[7];
 }
 // r = b - A x in FP64 and the slab partials of (b,b) and (r,r)
-__global__ void kb_residual(const BatchMember *bm, const int *pre, int nm, int part) {
+__global__ void kb_residual(const BatchMember *bm, const int *pre, int nm) {
   pdl_enter();
   BATCH_BLOCK(BR_SLAB)
-  if (part == 0) spmv_body<double>(M.g, M.q, M.S, M.vd[BD_X], M.vd[BD_Y2], M.st, lb_);
-  else if (part == 1) bmy_body(M.q, M.S.indc, M.vd[BD_B], M.vd[BD_Y2], M.st, lb_);
-  else dot_body<double>(M.q, M.S.indc, M.vd[BD_B], M.vd[BD_B], M.vd[BD_Y2], M.vd[BD_Y2], M.rb0, M.rb1, M.st, lb_);
+  resid_body(M.g, M.q, M.S, M.vd[BD_B], M.vd[BD_X], M.vd[BD_Y2], M.rb0, M.rb1, M.st, lb_);
 }
 // one block per member: the finaliser of its sums (tile partials after a
 // backward sweep with sums, slab-block partials otherwise)
@@ -1892,45 +1970,44 @@ __global__ void kb_commit(const BatchMember *bm, int nm) {
   const int m = blockIdx.x * blockDim.x + threadIdx.x;
   if (m < nm && bm[m].st->stop) bm[m].st->done = 1;
 }
-// the inner solve's start: BF = R/|r|, its vectors zeroed
-__global__ void kb_start_f(const BatchMember *bm, const int *pre, int nm) {
+// the inner solve's start: BF = R/|r|, D = 0
+__global__ void __launch_bounds__(256) kb_start_f(const BatchMember *bm, const int *pre, int nm) {
   pdl_enter();
-  BATCH_BLOCK(BR_SLAB)
+  BATCH_BLOCK(BR_FLAT)
   if (!M.active) return;
-  scale_to_f_body(M.q, M.S.indc, M.vd[BD_Y2], M.scale, M.vf[BF_B], lb_);
-  const long long slab = (long long)lb_ * ROWS_PER_BLOCK + (threadIdx.x >> 5);
-  if (slab < (long long)M.q.nb * M.q.W) {
-    const int zs[6] = {BF_X, BF_R0, BF_RR, BF_PV, BF_AP, BF_AE};
-    for (int t = threadIdx.x & 31; t < M.q.T; t += 32)
-      for (int c = 0; c < 6; ++c) M.vf[zs[c]][slab * M.q.T + t] = 0.0f;
-  }
+  scale_to_f_body(M.q, M.vd[BD_Y2], M.scale, M.vf[BF_B], lb_);
+  const unsigned BX_ = lb_;
+  float4 *x = reinterpret_cast<float4 *>(M.vf[BF_X]);
+  FLAT_LOOP_BEGIN(M.q, 4, 4)
+  EACH(4) x[e[u]] = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+  FLAT_LOOP_END
 }
 __global__ void kb_dot_r0f(const BatchMember *bm, const int *pre, int nm) {
   pdl_enter();
   BATCH_BLOCK(BR_SLAB)
-  dot_body<float>(M.q, M.S.indc, M.vf[BF_R0], M.vf[BF_R0], nullptr, nullptr, M.rb0, nullptr, M.st, lb_);
+  dot_body<float>(M.g, M.q, M.vf[BF_R0], M.vf[BF_R0], nullptr, nullptr, M.rb0, nullptr, M.st, lb_);
 }
-__global__ void kb_copy2_f(const BatchMember *bm, const int *pre, int nm) {
+__global__ void __launch_bounds__(256) kb_copy2_f(const BatchMember *bm, const int *pre, int nm) {
   pdl_enter();
-  BATCH_BLOCK(BR_SLAB)
-  copy2_body<float>(M.q, M.S.indc, M.vf[BF_R0], M.vf[BF_RR], M.vf[BF_PV], M.st, lb_);
+  BATCH_BLOCK(BR_FLAT)
+  copy2_body<float>(M.q, M.vf[BF_R0], M.vf[BF_RR], M.vf[BF_PV], M.st, lb_);
 }
-__global__ void kb_axpyf(const BatchMember *bm, const int *pre, int nm) {
+__global__ void __launch_bounds__(256) kb_axpyf(const BatchMember *bm, const int *pre, int nm) {
   pdl_enter();
-  BATCH_BLOCK(BR_SLAB)
+  BATCH_BLOCK(BR_FLAT)
   axpyf_body(M.q, M.vf[BF_AP], M.vf[BF_RR], M.st, lb_);
 }
-__global__ void kb_upd3f(const BatchMember *bm, const int *pre, int nm) {
+__global__ void __launch_bounds__(256) kb_upd3f(const BatchMember *bm, const int *pre, int nm) {
   pdl_enter();
-  BATCH_BLOCK(BR_SLAB)
+  BATCH_BLOCK(BR_FLAT)
   upd3f_body(M.q, M.vf[BF_AE], M.vf[BF_AP], M.vf[BF_X], M.vf[BF_RR], M.vf[BF_PV], M.st, lb_);
 }
 // XW += |r| D on the members whose inner solve ended within ICGMAX
-__global__ void kb_add_f(const BatchMember *bm, const int *pre, int nm) {
+__global__ void __launch_bounds__(256) kb_add_f(const BatchMember *bm, const int *pre, int nm) {
   pdl_enter();
-  BATCH_BLOCK(BR_SLAB)
+  BATCH_BLOCK(BR_FLAT)
   if (!M.active || M.st->iter < 0 || M.st->iter > M.icgmax) return;
-  add_f_body(M.q, M.S.indc, M.vf[BF_X], M.rn, M.vd[BD_X], lb_);
+  add_f_body(M.q, M.vf[BF_X], M.rn, M.vd[BD_X], lb_);
 }
 __global__ void kb_x0(const BatchMember *bm, const int *pre, int nm) {
   pdl_enter();
@@ -2034,8 +2111,7 @@ void launch_b_gather(cudaStream_t s, const BatchMember *bm, int nm, double *out)
   launch_pdl(kb_gather, bmem(nm), dim3(256), 0, s, 1, bm, nm, out);
 }
 void launch_b_residual(cudaStream_t s, const BatchMember *bm, const int *pre, int nm, long long nslab) {
-  for (int part = 0; part < 3; ++part)
-    launch_pdl(kb_residual, bgrid(nslab), dim3(ROW_THREADS), 0, s, 1, bm, pre, nm, part);
+  launch_pdl(kb_residual, bgrid(nslab), dim3(ROW_THREADS), 0, s, 1, bm, pre, nm);
 }
 void launch_b_fin(cudaStream_t s, int mode, const BatchMember *bm, int nm, bool tile_partials) {
   launch_pdl(kb_fin, dim3((unsigned)nm), dim3(1024), 0, s, 1, bm, nm, mode, tile_partials ? 1 : 0);
@@ -2046,14 +2122,14 @@ void launch_b_fin5(cudaStream_t s, const BatchMember *bm, int nm) {
 void launch_b_commit(cudaStream_t s, const BatchMember *bm, int nm) {
   launch_pdl(kb_commit, bmem(nm), dim3(256), 0, s, 1, bm, nm);
 }
-#define BSL(kern) launch_pdl(kern, bgrid(nslab), dim3(ROW_THREADS), 0, s, 1, bm, pre, nm)
-void launch_b_start_f(cudaStream_t s, const BatchMember *bm, const int *pre, int nm, long long nslab) { BSL(kb_start_f); }
-void launch_b_dot_r0f(cudaStream_t s, const BatchMember *bm, const int *pre, int nm, long long nslab) { BSL(kb_dot_r0f); }
-void launch_b_copy2_f(cudaStream_t s, const BatchMember *bm, const int *pre, int nm, long long nslab) { BSL(kb_copy2_f); }
-void launch_b_axpyf(cudaStream_t s, const BatchMember *bm, const int *pre, int nm, long long nslab) { BSL(kb_axpyf); }
-void launch_b_upd3f(cudaStream_t s, const BatchMember *bm, const int *pre, int nm, long long nslab) { BSL(kb_upd3f); }
-void launch_b_add_f(cudaStream_t s, const BatchMember *bm, const int *pre, int nm, long long nslab) { BSL(kb_add_f); }
-void launch_b_x0(cudaStream_t s, const BatchMember *bm, const int *pre, int nm, long long nslab) { BSL(kb_x0); }
+#define BSL(kern, n) launch_pdl(kern, bgrid(n), dim3(ROW_THREADS), 0, s, 1, bm, pre, nm)
+void launch_b_start_f(cudaStream_t s, const BatchMember *bm, const int *pre, int nm, long long nflat) { BSL(kb_start_f, nflat); }
+void launch_b_dot_r0f(cudaStream_t s, const BatchMember *bm, const int *pre, int nm, long long nslab) { BSL(kb_dot_r0f, nslab); }
+void launch_b_copy2_f(cudaStream_t s, const BatchMember *bm, const int *pre, int nm, long long nflat) { BSL(kb_copy2_f, nflat); }
+void launch_b_axpyf(cudaStream_t s, const BatchMember *bm, const int *pre, int nm, long long nflat) { BSL(kb_axpyf, nflat); }
+void launch_b_upd3f(cudaStream_t s, const BatchMember *bm, const int *pre, int nm, long long nflat) { BSL(kb_upd3f, nflat); }
+void launch_b_add_f(cudaStream_t s, const BatchMember *bm, const int *pre, int nm, long long nflat) { BSL(kb_add_f, nflat); }
+void launch_b_x0(cudaStream_t s, const BatchMember *bm, const int *pre, int nm, long long nslab) { BSL(kb_x0, nslab); }
 #undef BSL
 
 }  // namespace cadmas

@@ -42,14 +42,33 @@ template <typename V> struct SkewSysT {
 };
 using SkewSys = SkewSysT<double>;
 using SkewSysF = SkewSysT<float>;
+//
+// A tile's wavefront has W = (NK-2)+(TI-1)+(TJ-1) slabs, but its ramps (the
+// first and last TI+TJ-2 of them) are only partly used.  So the tiles
+// overlap: tile b starts at slab b*WS with WS = NK-2, and the entries that
+// its last slabs use are those that the first slabs of tile b+1 leave free
+// (column (ti,tj) of a slab w' < WS of tile b+1 belongs to tile b when
+// w' < ti+tj).  Every entry with a column inside the grid then holds exactly
+// one cell, and whole-array passes move no ramp: on 512 tiles of 16x16 x 126
+// 16.5 M entries instead of 20.4 M.  Where a tile has fewer layers than
+// ramp, WS = W and nothing overlaps.  Entries that hold no cell (columns
+// past the grid, the padding column, the free ends of the first and last
+// tile) are never written and stay as cadmas_create leaves them: 0, INDC -1.
 struct SkewGeo {
   int TI, TJ, TIp, T, W;  // layout tile TI x TJ columns (T = TIp*TJ slots), W slabs per tile
+  int WS;                 // slabs from one tile's start to the next's (0: W)
   int ntx, nb;            // layout tiles along x, tiles in total
   int split;  // layout tiles per preconditioner block along y (1 or 2)
   int occ;    // thread blocks of the sweeps per SM to leave shared memory for (0: one, at full depth)
   int ring;   // 1: the sweeps' bulk-copy form (the stall injection's subject), 0: by the rule of launch_sweep
 };
 
+__host__ __device__ inline int skew_stride(const SkewGeo &q) { return q.WS ? q.WS : q.W; }
+// slabs and entries of a skewed array
+__host__ __device__ inline long long skew_slabs(const SkewGeo &q) {
+  return (long long)q.nb * skew_stride(q) + (q.W - skew_stride(q));
+}
+__host__ __device__ inline long long skew_entries(const SkewGeo &q) { return skew_slabs(q) * q.T; }
 // SYS_T of column t
 __host__ __device__ inline long long sys_t(long long slab, int T, int t) { return slab * SYS_N * T + t; }
 // chunk c of column t
@@ -135,7 +154,7 @@ struct SweepLane {
   int wstride, dst, bytes, arr, dlo, dhi;
 };
 __host__ __device__ inline bool sweep_lane(const SkewGeo &q, int mode, int b, int c, SweepLane &l, int es) {
-  const long long slab0 = (long long)b * q.W;
+  const long long slab0 = (long long)b * skew_stride(q);
   l.dlo = 0; l.dhi = q.W - 1;
   const int sys_c = (mode == SWEEP_FWD) ? 1 : 0;  // copy index of the system block
   if (c == sys_c) {
@@ -185,7 +204,7 @@ __host__ __device__ inline bool sweep_lane(const SkewGeo &q, int mode, int b, in
   } else {
     return false;
   }
-  l.base = ((long long)nb_tile * q.W + dw) * q.T + toff;
+  l.base = ((long long)nb_tile * skew_stride(q) + dw) * q.T + toff;
   l.dlo = dw < 0 ? -dw : 0;                 // 0 <= w + dw
   l.dhi = dw > 0 ? q.W - 1 - dw : q.W - 1;  // w + dw <= W-1
   return true;
@@ -209,10 +228,12 @@ __host__ __device__ inline bool sweep_copy(const SkewGeo &q, int mode, int b, in
 // factorisation, slab blocks for the vector kernels, blocks of 256 layout
 // entries for the conversions), a block finding its member in the
 // prefix table and running the member's kernel body with its block index
-// inside the member.  BatchMember is a member's part of the solve.
+// inside the member.  Ranges: tiles, blocks of slab sums, blocks of 256
+// wavefront entries, blocks of FLAT_BLOCK entries of the arrays.  BatchMember is a member's part of the solve.
 enum BatchVecF { BF_B = 0, BF_X, BF_R0, BF_RR, BF_PV, BF_AP, BF_AE, BF_Y2, BF_N };
 enum BatchVecD { BD_B = 0, BD_X, BD_Y2, BD_N };
-enum BatchRange { BR_TILE = 0, BR_SLAB = 1, BR_ELEM = 2, BR_N = 3 };
+enum BatchRange { BR_TILE = 0, BR_SLAB = 1, BR_ELEM = 2, BR_FLAT = 3, BR_N = 4 };
+constexpr int FLAT_BLOCK = 4096;  // entries per block of the whole-array passes
 constexpr int BATCH_ELEM = 256;  // layout entries per block of the conversions
 struct BatchMember {
   Geo g;
@@ -318,12 +339,12 @@ void launch_b_residual(cudaStream_t s, const BatchMember *bm, const int *pre, in
 void launch_b_fin(cudaStream_t s, int mode, const BatchMember *bm, int nm, bool tile_partials);
 void launch_b_fin5(cudaStream_t s, const BatchMember *bm, int nm);
 void launch_b_commit(cudaStream_t s, const BatchMember *bm, int nm);
-void launch_b_start_f(cudaStream_t s, const BatchMember *bm, const int *pre, int nm, long long nslab);
+void launch_b_start_f(cudaStream_t s, const BatchMember *bm, const int *pre, int nm, long long nflat);
 void launch_b_dot_r0f(cudaStream_t s, const BatchMember *bm, const int *pre, int nm, long long nslab);
-void launch_b_copy2_f(cudaStream_t s, const BatchMember *bm, const int *pre, int nm, long long nslab);
-void launch_b_axpyf(cudaStream_t s, const BatchMember *bm, const int *pre, int nm, long long nslab);
-void launch_b_upd3f(cudaStream_t s, const BatchMember *bm, const int *pre, int nm, long long nslab);
-void launch_b_add_f(cudaStream_t s, const BatchMember *bm, const int *pre, int nm, long long nslab);
+void launch_b_copy2_f(cudaStream_t s, const BatchMember *bm, const int *pre, int nm, long long nflat);
+void launch_b_axpyf(cudaStream_t s, const BatchMember *bm, const int *pre, int nm, long long nflat);
+void launch_b_upd3f(cudaStream_t s, const BatchMember *bm, const int *pre, int nm, long long nflat);
+void launch_b_add_f(cudaStream_t s, const BatchMember *bm, const int *pre, int nm, long long nflat);
 void launch_b_x0(cudaStream_t s, const BatchMember *bm, const int *pre, int nm, long long nslab);
 // the FP32 backward sweep with the inner products after it summed on the
 // way, one partial per tile (rb + c*nb); false when not available for the
@@ -340,25 +361,17 @@ template <typename V>
 void launch_spmv_t(cudaStream_t s, const Geo &g, const SkewGeo &q, const SkewSysT<V> &S, const V *x, V *y,
                    const SolveState *st);
 template <typename V>
-void launch_dot_t(cudaStream_t s, const SkewGeo &q, const int *indc, const V *x0, const V *y0, const V *x1,
+void launch_dot_t(cudaStream_t s, const Geo &g, const SkewGeo &q, const V *x0, const V *y0, const V *x1,
                   const V *y1, double *rb0, double *rb1, const SolveState *st);
 template <typename V>
-void launch_copy2_t(cudaStream_t s, const SkewGeo &q, const int *indc, const V *r0, V *rr, V *pp,
-                    const SolveState *st);
-template <typename V>
-void launch_axpy_rr_t(cudaStream_t s, const SkewGeo &q, const int *indc, const V *ap, V *rr, const SolveState *st);
-template <typename V>
-void launch_upd_xr_t(cudaStream_t s, const SkewGeo &q, const int *indc, const V *pp, const V *ae, const V *r0,
-                     V *xw, V *rr, double *rb0, double *rb1, const SolveState *st);
-template <typename V>
-void launch_upd_p_t(cudaStream_t s, const SkewGeo &q, const int *indc, const V *rr, const V *ap, V *pp,
+void launch_copy2_t(cudaStream_t s, const SkewGeo &q, const V *r0, V *rr, V *pp,
                     const SolveState *st);
 // Regrouped FP32 inner iteration (k_poisson.cu): vectors zero where
 // INDC = -1, four entries per lane; rb5 holds 5 x nslab partials.
-void launch_dot2f(cudaStream_t s, const SkewGeo &q, const float *r0, const float *ap, double *rb,
+void launch_dot2f(cudaStream_t s, const Geo &g, const SkewGeo &q, const float *r0, const float *ap, double *rb,
                   const SolveState *st);
 void launch_axpyf(cudaStream_t s, const SkewGeo &q, const float *ap, float *rr, const SolveState *st);
-void launch_dot5f(cudaStream_t s, const SkewGeo &q, const float *r0, const float *rr, const float *ae, double *rb5,
+void launch_dot5f(cudaStream_t s, const Geo &g, const SkewGeo &q, const float *r0, const float *rr, const float *ae, double *rb5,
                   const SolveState *st);
 // One iteration's tail: launch_dot5f, launch_fin5 (scalars; a finished
 // solve sets SolveState::stop), launch_upd3f (runs while `done` is clear,
@@ -369,27 +382,22 @@ void launch_fin5(cudaStream_t s, const double *rb5, long long nrows, SolveState 
                  double div2, int icgmax);
 void launch_commit(cudaStream_t s, SolveState *st);
 void launch_sys_to_f(cudaStream_t s, const SkewGeo &q, const double *sys, float *sysf);
-void launch_scale_to_f(cudaStream_t s, const SkewGeo &q, const int *indc, const double *r, double scale,
-                       float *rf);
-void launch_add_f(cudaStream_t s, const SkewGeo &q, const int *indc, const float *d, double inv_scale, double *x);
+void launch_scale_to_f(cudaStream_t s, const SkewGeo &q, const double *r, double scale, float *rf);
+void launch_add_f(cudaStream_t s, const SkewGeo &q, const float *d, double inv_scale, double *x);
 // Thread block of the sweeps for a tile of T slab entries (T consumer
 // threads rounded up to whole warps, plus the producer warp).
 inline int sweep_threads(int T) { return ((T + 31) & ~31) + 32; }
 // Whether the sweeps can run this tile geometry (block size, shared memory).
 bool sweep_supported(const SkewGeo &q);
-void launch_spmv(cudaStream_t s, const Geo &g, const SkewGeo &q, const SkewSys &S, const double *x, double *y,
-                 const SolveState *st);
-void launch_bmy(cudaStream_t s, const SkewGeo &q, const int *indc, const double *b, double *y,
-                const SolveState *st);
-void launch_dot(cudaStream_t s, const SkewGeo &q, const int *indc, const double *x0, const double *y0,
-                const double *x1, const double *y1, double *rb0, double *rb1, const SolveState *st);
-void launch_copy2(cudaStream_t s, const SkewGeo &q, const int *indc, const double *r0, double *rr, double *pp,
-                  const SolveState *st);
-void launch_axpy_rr(cudaStream_t s, const SkewGeo &q, const int *indc, const double *ap, double *rr,
+// Y = B - A*X where INDC != -1, else 0; with rb0, rb1 also the slab
+// partials of (B,B) and (Y,Y)
+void launch_resid(cudaStream_t s, const Geo &g, const SkewGeo &q, const SkewSys &S, const double *b, const double *x,
+                  double *y, double *rb0, double *rb1, const SolveState *st);
+void launch_axpy_rr(cudaStream_t s, const SkewGeo &q, const double *ap, double *rr,
                     const SolveState *st);
-void launch_upd_xr(cudaStream_t s, const SkewGeo &q, const int *indc, const double *pp, const double *ae,
+void launch_upd_xr(cudaStream_t s, const Geo &g, const SkewGeo &q, const double *pp, const double *ae,
                    const double *r0, double *xw, double *rr, double *rb0, double *rb1, const SolveState *st);
-void launch_upd_p(cudaStream_t s, const SkewGeo &q, const int *indc, const double *rr, const double *ap,
+void launch_upd_p(cudaStream_t s, const SkewGeo &q, const double *rr, const double *ap,
                   double *pp, const SolveState *st);
 void launch_x0(cudaStream_t s, const Geo &g, const SkewGeo &q, const int *indc, const double *xw, double *x0,
                const SolveState *st);

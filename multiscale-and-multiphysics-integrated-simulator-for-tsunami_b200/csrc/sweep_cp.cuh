@@ -98,6 +98,7 @@ __device__ __forceinline__ void sweep_cp_body(const Geo &g, const SkewGeo &q, co
   constexpr int R = D + 1, RP = D + 4;                            // slots of the rings
   using V2 = typename SweepPair<V>::type;
   if (st->done) return;
+  const int WS = skew_stride(q);
   const int T = CT > 0 ? CT : q.T, TIp = CT > 0 ? CTIP : q.TIp, TI = q.TI, TJ = CT > 0 ? CT / (CTIP > 0 ? CTIP : 1) : q.TJ;
   const int tid = threadIdx.x, b = bx + q.ntx * by, nty = q.nb / q.ntx;
   const int XB = T + 4;                                           // entries of an exchange buffer
@@ -127,7 +128,7 @@ __device__ __forceinline__ void sweep_cp_body(const Geo &g, const SkewGeo &q, co
     if (AX)
       for (int r = tid; r < RP; r += 2) pb[r * PS + T] = V(0);
   }
-  const long long slab0 = (long long)b * q.W + (BWD ? nsteps - 1 : 0);
+  const long long slab0 = (long long)b * WS + (BWD ? nsteps - 1 : 0);
   constexpr long long DIR = BWD ? -1 : 1;
   const long long vstep = DIR * T, sstep = DIR * SYS_N * T;
   // next values to copy: chunks, the plain vectors, P and its halo columns
@@ -144,10 +145,10 @@ __device__ __forceinline__ void sweep_cp_body(const Geo &g, const SkewGeo &q, co
   const int shx = hr ? -1 : 1, shy = hu ? -1 : 1;  // own step minus the neighbour's
   const V *lx = vin, *ly = vin;                    // halo values for P slot 0
   if (AX) {  // own step u: the neighbour's cell of the same layer; slot v = u - shx
-    if (hl) lx = vin + ((long long)(b - 1) * q.W + TI) * T + (TI - 1) + TIp * tj;
-    if (hr) lx = vin + ((long long)(b + 1) * q.W - TI) * T + TIp * tj;
-    if (hd) ly = vin + ((long long)(b - q.ntx) * q.W + TJ) * T + ti + TIp * (TJ - 1);
-    if (hu) ly = vin + ((long long)(b + q.ntx) * q.W - TJ) * T + ti;
+    if (hl) lx = vin + ((long long)(b - 1) * WS + TI) * T + (TI - 1) + TIp * tj;
+    if (hr) lx = vin + ((long long)(b + 1) * WS - TI) * T + TIp * tj;
+    if (hd) ly = vin + ((long long)(b - q.ntx) * WS + TJ) * T + ti + TIp * (TJ - 1);
+    if (hu) ly = vin + ((long long)(b + q.ntx) * WS - TJ) * T + ti;
   }
   V *vp = BWD ? vout + slab0 * T + tq : S.sys + sys_t(slab0, T, tq);
   auto active = [&](int u) { return (unsigned)(u - slo) <= nact; };
