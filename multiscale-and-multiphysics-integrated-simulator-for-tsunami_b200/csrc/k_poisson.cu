@@ -1632,33 +1632,38 @@ static int sweep_depth(const SkewGeo &q, int mode, int es) {
 // and handles with the stall injection on (SkewGeo::ring), whose subject is
 // the ring's waits.
 //
-// Depth of the thread copies: the deepest that the shared memory allows,
-// since a step (0.14 to 0.35 us) is far shorter than the latency of a copy:
-// on 128 tiles of 8x16 columns x 96 layers, FP64, depths 4 and 8 measured
-// 34.8 and 28.8 us (fused forward) and 21.2 and 16.5 us (backward).  More
-// blocks per SM at less depth gain nothing (512 tiles of 16x16 x 128, FP64
-// fused forward: one block at depth 8 240 us, two at depth 4 251 us; FP32:
-// two at depth 8 137 us, four at depth 4 139 us), so only q.occ > 0 limits
-// a block's share.
+// Depth of the thread copies: a step (0.1 to 0.35 us) is far shorter than the
+// latency of a copy, so as deep as the shared memory allows, shared by two
+// blocks per SM where there are more tiles than SMs (by q.occ blocks if that
+// is set) as long as that leaves depth 6.  Measured, us per sweep: 128 tiles
+// of 8x16 x 96 layers, FP64, depths 4, 8, 12: fused forward 34.8, 28.8, 26.8;
+// backward depths 4, 7, 15: 21.2, 14.5, 14.5 (in a solve, where the
+// system comes from memory, 19.6 at 7).  512 tiles of 16x16 x 126 layers: FP64
+// fused, one block at depth 8 242, at 6 250, two at 4 255; FP32 fused, two at
+// depth 6 132, one 143; backward FP64 at depth 7, one block 139, two 141.
 static int sweep_cp_threads(int T) { return (T + 31) & ~31; }
+static bool sweep_cp_unrolled(const SkewGeo &q, int mode, int es) {
+  const bool ct = (q.T == 128 && (q.TIp == 8 || q.TIp == 16)) || (q.T == 256 && q.TIp == 16);
+  return sweep_cp_unroll(mode, ct ? q.T : 0, es);
+}
 static int sweep_cp_depth(const SkewGeo &q, int mode, int es) {
   if (q.split != 1 || q.TI < 2 || q.TJ < 2) return 0;
-  const int nt = sweep_cp_threads(q.T);
-  const size_t cap = 227 * 1024, share = (q.occ > 1 ? 226 * 1024 / (size_t)q.occ : cap);
-  int best = 0;
-  for (int d : {16, 8, 4, 2, 1}) {
-    if (d == 16 && nt > 128) continue;
-    if (d == 1 && nt <= 576) continue;
-    const size_t n = sweep_cp_bytes(mode, d, q.T, q.TI, q.TJ, es);
-    if (n <= cap) best = d;   // the shallowest that fits, if none fits the share
-    if (n <= share) return d;
-  }
-  return best;
+  const int nt = sweep_cp_threads(q.T), blocks = q.occ > 0 ? q.occ : (q.nb > 148 ? 2 : 1);
+  const bool unr = sweep_cp_unrolled(q, mode, es);
+  const int ax[] = {12, 8, 6, 4, 2, 1}, plain[] = {15, 9, 3, 1};
+  for (size_t share : {226 * 1024 / (size_t)blocks, (size_t)(227 * 1024)})
+    for (int i = 0; i < (mode == SWEEP_FWD_AX ? 6 : 4); ++i) {
+      const int d = mode == SWEEP_FWD_AX ? ax[i] : plain[i];
+      if ((d >= 12 && nt > 128) || (d == 1 && nt <= 576)) continue;
+      if (q.occ == 0 && blocks > 1 && share < 227 * 1024 && d < 6) continue;
+      if (sweep_cp_bytes(mode, d, unr, q.T, q.TI, q.TJ, es) <= share) return d;
+    }
+  return 0;
 }
 template <int D, int MODE, int MAXT, typename V, int MINB>
 static void sweep_cp_go(cudaStream_t s, const Geo &g, const SkewGeo &q, const SkewSysT<V> &S, const V *vin, V *vout,
                         SolveState *st, const V *vin2, double *rb) {
-  const size_t bytes = sweep_cp_bytes(MODE, D, q.T, q.TI, q.TJ, (int)sizeof(V));
+  const size_t bytes = sweep_cp_bytes(MODE, D, sweep_cp_unrolled(q, MODE, (int)sizeof(V)), q.T, q.TI, q.TJ, (int)sizeof(V));
   const dim3 grid((unsigned)q.ntx, (unsigned)(q.nb / q.ntx)), block((unsigned)sweep_cp_threads(q.T));
 #define SWEEP_GO(CT, CI)                                                                                        \
   {                                                                                                             \
@@ -1698,24 +1703,48 @@ static void launch_sweep(cudaStream_t s, const Geo &g, const SkewGeo &q, const S
     sweep_cp_go<D, MODE, MT, V, MB>(s, g, q, S, vin, vout, st, vin2, rb);      \
     return;                                                                    \
   }
-  if (d > 0) {
+  // two blocks' registers for FP32, whose rings leave room for two blocks
+  constexpr int MB = sizeof(V) == 4 ? 2 : 1;
+  if constexpr (MODE == SWEEP_FWD_AX) {
+    if (d > 0) {
+      if (nt <= 128) {
+        if (d == 12) CP_GO(12, 128, 1)
+        if (d == 8) CP_GO(8, 128, 1)
+        if (d == 6) CP_GO(6, 128, 1)
+        if (d == 4) CP_GO(4, 128, 1)
+        CP_GO(2, 128, 1)
+      } else if (nt <= 256) {
+        if (d == 8) CP_GO(8, 256, MB)
+        if (d == 6) CP_GO(6, 256, MB)
+        if (d == 4) CP_GO(4, 256, MB)
+        CP_GO(2, 256, MB)
+      } else if (nt <= 576) {
+        if (d == 8) CP_GO(8, 576, 1)
+        if (d == 6) CP_GO(6, 576, 1)
+        if (d == 4) CP_GO(4, 576, 1)
+        CP_GO(2, 576, 1)
+      } else {
+        if (d == 8) CP_GO(8, 1024, 1)
+        if (d == 6) CP_GO(6, 1024, 1)
+        if (d == 4) CP_GO(4, 1024, 1)
+        if (d == 2) CP_GO(2, 1024, 1)
+        CP_GO(1, 1024, 1)
+      }
+    }
+  } else if (d > 0) {
     if (nt <= 128) {
-      if (d == 16) CP_GO(16, 128, 1)
-      if (d == 8) CP_GO(8, 128, 1)
-      if (d == 4) CP_GO(4, 128, 1)
-      CP_GO(2, 128, 1)
+      if (d == 15) CP_GO(15, 128, 1)
+      if (d == 9) CP_GO(9, 128, 1)
+      CP_GO(3, 128, 1)
     } else if (nt <= 256) {
-      if (d == 8) CP_GO(8, 256, 1)
-      if (d == 4) CP_GO(4, 256, 1)
-      CP_GO(2, 256, 1)
+      if (d == 9) CP_GO(9, 256, 2)
+      CP_GO(3, 256, 2)
     } else if (nt <= 576) {
-      if (d == 8) CP_GO(8, 576, 1)
-      if (d == 4) CP_GO(4, 576, 1)
-      CP_GO(2, 576, 1)
+      if (d == 9) CP_GO(9, 576, 1)
+      CP_GO(3, 576, 1)
     } else {
-      if (d == 8) CP_GO(8, 1024, 1)
-      if (d == 4) CP_GO(4, 1024, 1)
-      if (d == 2) CP_GO(2, 1024, 1)
+      if (d == 9) CP_GO(9, 1024, 1)
+      if (d == 3) CP_GO(3, 1024, 1)
       CP_GO(1, 1024, 1)
     }
   }
@@ -2049,7 +2078,9 @@ bool b_sweeps_supported(const SkewGeo &q) {
 template <int MODE>
 static bool launch_b_sweep_t(cudaStream_t s, const BatchMember *bm, const int *pre, int nm, long long ntiles,
                              const SkewGeo &q, int vin, int vout, int vin2, int rb5) {
-  const int d = q.ring ? 0 : sweep_cp_depth(q, MODE, 4), nt = sweep_cp_threads(q.T);
+  SkewGeo qa = q;  // the depth by the tiles of all members
+  qa.nb = (int)std::min<long long>(ntiles, 1 << 30);
+  const int d = q.ring ? 0 : sweep_cp_depth(qa, MODE, 4), nt = sweep_cp_threads(q.T);
   if (d == 0) {
     const int dr = sweep_depth(q, MODE, 4);
     if (dr < 2) return false;
@@ -2059,7 +2090,7 @@ static bool launch_b_sweep_t(cudaStream_t s, const BatchMember *bm, const int *p
                vout, vin2, rb5, dr);
     return true;
   }
-  const size_t bytes = sweep_cp_bytes(MODE, d, q.T, q.TI, q.TJ, 4);
+  const size_t bytes = sweep_cp_bytes(MODE, d, sweep_cp_unrolled(q, MODE, 4), q.T, q.TI, q.TJ, 4);
   const dim3 block((unsigned)nt);
 #define BSWEEP(D, MT, MB, CT, CI)                                                                             \
   {                                                                                                           \
@@ -2067,28 +2098,34 @@ static bool launch_b_sweep_t(cudaStream_t s, const BatchMember *bm, const int *p
     launch_pdl(kb_sweep<D, MODE, MT, MB, CT, CI>, bgrid(ntiles), block, bytes, s, 1, bm, pre, nm, vin, vout, vin2, rb5); \
     return true;                                                                                              \
   }
+#define BSWEEP_128(D)                                            \
+  {                                                              \
+    if (q.T == 128 && q.TIp == 8) BSWEEP(D, 128, 1, 128, 8)      \
+    if (q.T == 128 && q.TIp == 16) BSWEEP(D, 128, 1, 128, 16)    \
+    BSWEEP(D, 128, 1, 0, 0)                                      \
+  }
 #define BSWEEP_D(D)                                              \
   {                                                              \
-    if (nt <= 128) {                                             \
-      if (q.T == 128 && q.TIp == 8) BSWEEP(D, 128, 1, 128, 8)    \
-      if (q.T == 128 && q.TIp == 16) BSWEEP(D, 128, 1, 128, 16)  \
-      BSWEEP(D, 128, 1, 0, 0)                                    \
-    }                                                            \
+    if (nt <= 128) BSWEEP_128(D)                                 \
     if (nt <= 256) {                                             \
-      if (q.T == 256 && q.TIp == 16) BSWEEP(D, 256, 1, 256, 16)  \
-      BSWEEP(D, 256, 1, 0, 0)                                    \
+      if (q.T == 256 && q.TIp == 16) BSWEEP(D, 256, 2, 256, 16)  \
+      BSWEEP(D, 256, 2, 0, 0)                                    \
     }                                                            \
     BSWEEP(D, 576, 1, 0, 0)                                      \
   }
-  if (d == 16) {
-    if (q.T == 128 && q.TIp == 8) BSWEEP(16, 128, 1, 128, 8)
-    if (q.T == 128 && q.TIp == 16) BSWEEP(16, 128, 1, 128, 16)
-    BSWEEP(16, 128, 1, 0, 0)
+  if constexpr (MODE == SWEEP_FWD_AX) {
+    if (d == 12) BSWEEP_128(12)
+    if (d == 8) BSWEEP_D(8)
+    if (d == 6) BSWEEP_D(6)
+    if (d == 4) BSWEEP_D(4)
+    BSWEEP_D(2)
+  } else {
+    if (d == 15) BSWEEP_128(15)
+    if (d == 9) BSWEEP_D(9)
+    BSWEEP_D(3)
   }
-  if (d == 8) BSWEEP_D(8)
-  if (d == 4) BSWEEP_D(4)
-  BSWEEP_D(2)
 #undef BSWEEP_D
+#undef BSWEEP_128
 #undef BSWEEP
 }
 bool launch_b_sweep(cudaStream_t s, int mode, const BatchMember *bm, const int *pre, int nm, long long ntiles,

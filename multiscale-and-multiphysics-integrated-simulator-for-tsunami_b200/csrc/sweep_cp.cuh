@@ -52,6 +52,10 @@ __device__ __forceinline__ void sweep_sums(const double *a, double *rb, int nb, 
 //   * The result of step s and DD of step s+1 are published as one pair.
 //   * One barrier per step; the recurrence of step s and the preparation of
 //     step s+1 are independent and scheduled into one another.
+//   * For the tile shapes that are compiled in (CT, CTIP) the loop is
+//     unrolled over the ring, so that slots, buffers and the copies' sources
+//     are constant offsets: a warp's instructions per step, each waiting
+//     for the one before, are what a small grid's step takes.
 // Entry T of the shared P and X arrays is a zero that stands for neighbours
 // outside.  The expressions and their order are those of the reference loops.
 __device__ __forceinline__ void cpa16(unsigned dst, const void *src) {
@@ -79,9 +83,20 @@ __host__ __device__ constexpr int sweep_cp_plain(int mode) {
 }
 // elements of one slot of P: T, the zero, the halo columns; a multiple of 16 bytes
 __host__ __device__ inline int sweep_cp_pslot(int T, int TI, int TJ) { return (T + 1 + 2 * (TI + TJ) + 3) & ~3; }
+// The compiled-in shapes (ct = T; 0: any shape) run the unrolled loop, but
+// for the fused FP64 sweep of 256 columns, whose slots are so large that
+// the longer ring costs it two steps of depth (512 tiles: 250 against 242 us).
+__host__ __device__ constexpr bool sweep_cp_unroll(int mode, int ct, int es) {
+  return ct > 0 && !(mode == SWEEP_FWD_AX && es == 8 && ct >= 256);
+}
+// slots of the ring for depth D: the unrolled fused sweep takes as many as
+// P's
+__host__ __device__ constexpr int sweep_cp_slots(int mode, int D, bool unrolled) {
+  return D + (mode == SWEEP_FWD_AX && unrolled ? 4 : 1);
+}
 // shared memory of a block
-__host__ __device__ inline size_t sweep_cp_bytes(int mode, int D, int T, int TI, int TJ, int es) {
-  size_t n = (size_t)(D + 1) * (sweep_cp_chunked(mode, es) + sweep_cp_plain(mode)) * T;
+__host__ __device__ inline size_t sweep_cp_bytes(int mode, int D, bool unrolled, int T, int TI, int TJ, int es) {
+  size_t n = (size_t)sweep_cp_slots(mode, D, unrolled) * (sweep_cp_chunked(mode, es) + sweep_cp_plain(mode)) * T;
   n += 2 * (size_t)(T + 4) * (mode >= SWEEP_BWD ? 1 : 2);
   if (mode == SWEEP_FWD_AX) n += (size_t)(D + 4) * sweep_cp_pslot(T, TI, TJ);
   return n * es;
@@ -95,7 +110,10 @@ __device__ __forceinline__ void sweep_cp_body(const Geo &g, const SkewGeo &q, co
   constexpr int ES = (int)sizeof(V), G = 16 / ES;                 // elements per chunk
   constexpr int C0 = sweep_cp_first(MODE, ES), NC = sweep_cp_chunked(MODE, ES) / G, NP = sweep_cp_plain(MODE);
   constexpr int E0 = SYS_AUI + C0 * G;                            // first coefficient
-  constexpr int R = D + 1, RP = D + 4;                            // slots of the rings
+  constexpr bool UNR = sweep_cp_unroll(MODE, CT, ES);
+  constexpr int R = sweep_cp_slots(MODE, D, UNR), RP = D + 4;     // slots of the rings
+  constexpr int U = UNR ? R : 1;                                  // steps per turn of the loop
+  static_assert(!UNR || (R % 2 == 0 && (!AX || R == RP)), "unrolled rings: even, and equal");
   using V2 = typename SweepPair<V>::type;
   if (st->done) return;
   const int WS = skew_stride(q);
@@ -143,6 +161,7 @@ __device__ __forceinline__ void sweep_cp_body(const Geo &g, const SkewGeo &q, co
   const int oxm = hl ? ehx : ((col && ti > 0) ? tq - 1 : T), oxp = hr ? ehx : ((col && ti < wi - 1) ? tq + 1 : T);
   const int oym = hd ? ehy : ((col && tj > 0) ? tq - TIp : T), oyp = hu ? ehy : ((col && tj < wj - 1) ? tq + TIp : T);
   const int shx = hr ? -1 : 1, shy = hu ? -1 : 1;  // own step minus the neighbour's
+  const bool hx = hl || hr, hy = hd || hu;
   const V *lx = vin, *ly = vin;                    // halo values for P slot 0
   if (AX) {  // own step u: the neighbour's cell of the same layer; slot v = u - shx
     if (hl) lx = vin + ((long long)(b - 1) * WS + TI) * T + (TI - 1) + TIp * tj;
@@ -155,28 +174,33 @@ __device__ __forceinline__ void sweep_cp_body(const Geo &g, const SkewGeo &q, co
   const unsigned ring0 = (unsigned)__cvta_generic_to_shared(ring) + (unsigned)(tq * 16),
                  plain0 = (unsigned)__cvta_generic_to_shared(ring + NC * G * T + tq);
   const unsigned pb0 = AX ? (unsigned)__cvta_generic_to_shared(pb) : 0u;
-  // chunks and plain vectors of step u into the slot at byte offset so
-  auto load = [&](int u, unsigned so) {
-    if (active(u)) {
+  // chunks and plain vectors of step u into the slot at byte offset so;
+  // sources r steps past the pointers
+  auto load = [&](int u, unsigned so, int r) {
+    if (!active(u)) return;
+    const V *c0 = lc + r * sstep;
 #pragma unroll
-      for (int c = 0; c < NC; ++c) cpa16(ring0 + so + (unsigned)(c * T * 16), lc + c * T * G);
-      if (!AX) cpa<ES>(plain0 + so, l0);
-      if (NDOT > 0) cpa<ES>(plain0 + so + (unsigned)(T * ES), l1);
-      if (NDOT == 5) cpa<ES>(plain0 + so + (unsigned)(2 * T * ES), l2);
-    }
-    lc += sstep;
-    if (!AX) l0 += (BWD ? sstep : vstep);
-    if (NDOT > 0) l1 += vstep;
-    if (NDOT == 5) l2 += vstep;
+    for (int c = 0; c < NC; ++c) cpa16(ring0 + so + (unsigned)(c * T * 16), c0 + c * T * G);
+    if (!AX) cpa<ES>(plain0 + so, l0 + r * (BWD ? sstep : vstep));
+    if (NDOT > 0) cpa<ES>(plain0 + so + (unsigned)(T * ES), l1 + r * vstep);
+    if (NDOT == 5) cpa<ES>(plain0 + so + (unsigned)(2 * T * ES), l2 + r * vstep);
   };
   // P of step v and the halo columns of slot v into the slot at byte offset po
-  auto loadp = [&](int v, unsigned po) {
-    if (active(v)) cpa<ES>(pb0 + po + (unsigned)(tq * ES), l0);
-    if ((hl || hr) && active(v + shx)) cpa<ES>(pb0 + po + (unsigned)(ehx * ES), lx);
-    if ((hd || hu) && active(v + shy)) cpa<ES>(pb0 + po + (unsigned)(ehy * ES), ly);
-    l0 += vstep;
-    lx += vstep;
-    ly += vstep;
+  auto loadp = [&](int v, unsigned po, int r) {
+    if (active(v)) cpa<ES>(pb0 + po + (unsigned)(tq * ES), l0 + r * vstep);
+    if (hx && active(v + shx)) cpa<ES>(pb0 + po + (unsigned)(ehx * ES), lx + r * vstep);
+    if (hy && active(v + shy)) cpa<ES>(pb0 + po + (unsigned)(ehy * ES), ly + r * vstep);
+  };
+  auto advance = [&](int n) {  // the sources of the chunks and plain vectors
+    lc += n * sstep;
+    if (!AX) l0 += n * (BWD ? sstep : vstep);
+    if (NDOT > 0) l1 += n * vstep;
+    if (NDOT == 5) l2 += n * vstep;
+  };
+  auto advancep = [&](int n) {
+    l0 += n * vstep;
+    lx += n * vstep;
+    ly += n * vstep;
   };
 
   V dd = V(0), y0 = V(0), c1 = V(0), c2 = V(0), c3 = V(0);  // prepared values of the step
@@ -247,15 +271,20 @@ __device__ __forceinline__ void sweep_cp_body(const Geo &g, const SkewGeo &q, co
   // P of slot s+3) and the barrier at its end shows that P to the others.
   const unsigned SB = (unsigned)(SS * ES), PSB = (unsigned)(PS * ES);
   if (AX) {
-    l0 -= vstep; lx -= vstep; ly -= vstep;
-    loadp(-1, 0u);
-    loadp(0, PSB);
-    loadp(1, 2 * PSB);
+    advancep(-1);
+    loadp(-1, 0u, 0);
+    loadp(0, PSB, 1);
+    loadp(1, 2 * PSB, 2);
+    advancep(3);
   }
 #pragma unroll 1
   for (int j = 0; j <= D; ++j) {
-    load(j, (unsigned)j * SB);
-    if (AX) loadp(j + 2, (unsigned)(j + 3) * PSB);
+    load(j, (unsigned)j * SB, 0);
+    advance(1);
+    if (AX) {
+      loadp(j + 2, (unsigned)(j + 3) * PSB, 0);
+      advancep(1);
+    }
     cpa_commit();
   }
   cpa_wait<D>();
@@ -269,13 +298,10 @@ __device__ __forceinline__ void sweep_cp_body(const Geo &g, const SkewGeo &q, co
     V2 z; z.x = V(0); z.y = dd;
     xd[XB + tid] = z;
   }
-  const V *cs = ring + SS, *const cend = ring + (size_t)R * SS;           // slot of step s+1
-  const V *pm = pb + PS, *pp = pb + 3 * PS, *const pend = pb + RP * PS;   // P slots s, s+2
-  unsigned wso = 0u, wpo = 0u;                                            // slots of the next group
-  int wr = 0, rd = XB;                                                    // exchange buffers
-  __syncthreads();
-#pragma unroll 1
-  for (int s = 0; s < nsteps; ++s) {
+  // iteration s, the r-th of a turn; cs: slot of step s+1; pm, pp: P slots
+  // s and s+2; wso, wpo: byte offsets of the next group's slots; wr, rd: the
+  // exchange buffers of steps s and s-1
+  auto iterate = [&](int s, int r, const V *cs, const V *pm, const V *pp, unsigned wso, unsigned wpo, int wr, int rd) {
     cpa_wait<D - 1>();
     V x1, x2, d1 = V(0), d2 = V(0), pxm = V(0), pym = V(0), pxp = V(0), pyp = V(0), p2 = V(0);
     if (BWD) {
@@ -287,8 +313,8 @@ __device__ __forceinline__ void sweep_cp_body(const Geo &g, const SkewGeo &q, co
     }
     if (AX) { pxm = pm[oxm]; pym = pm[oym]; pxp = pp[oxp]; pyp = pp[oyp]; p2 = pp[tq]; }
     const Vals f = fetch(cs);
-    load(s + 1 + D, wso);
-    if (AX) loadp(s + 3 + D, wpo);
+    load(s + 1 + D, wso, r);
+    if (AX) loadp(s + 3 + D, wpo, r);
     cpa_commit();
     if (NDOT > 0) sums(xk1, zk0, zk1);  // of step s-1
     const bool a = active(s), live = a && dd != V(0);
@@ -299,28 +325,71 @@ __device__ __forceinline__ void sweep_cp_body(const Geo &g, const SkewGeo &q, co
     prepare(s + 1, f, d1, d2, pxm, pym, pxp, pyp, p2);
     if (AX) { p0 = p1; p1 = p2; }
     if (BWD) {
-      if (tid < T) xb[wr + tid] = x;
-    } else if (tid < T) {
+      if (UNR || tid < T) xb[wr + tid] = x;
+    } else if (UNR || tid < T) {
       V2 z; z.x = x; z.y = dd;
       xd[wr + tid] = z;
     }
-    if (a) *vp = x;
-    vp += BWD ? vstep : sstep;
+    if (a) vp[r * (BWD ? vstep : sstep)] = x;
     xk1 = x;
-    cs += SS;
-    if (cs == cend) cs = ring;
-    wso += SB;
-    if (wso == R * SB) wso = 0u;
-    if (AX) {
-      pm += PS;
-      if (pm == pend) pm = pb;
-      pp += PS;
-      if (pp == pend) pp = pb;
-      wpo += PSB;
-      if (wpo == RP * PSB) wpo = 0u;
+  };
+  __syncthreads();
+  if constexpr (UNR) {
+    int s0 = 0;
+#pragma unroll 1
+    for (; s0 < nsteps; s0 += U) {
+#pragma unroll
+      for (int r = 0; r < U; ++r) {
+        if (s0 + r >= nsteps) break;
+        // group s goes where step s (chunks, D = R-1) or, with R = D+4,
+        // step s-3 lay; P slot s+3+D where slot s-1 lay
+        iterate(s0 + r, r, ring + ((r + 1) % R) * SS, pb + ((r + 1) % RP) * PS, pb + ((r + 3) % RP) * PS,
+                (unsigned)((r + 1 + D) % R) * SB, (unsigned)((r + 4 + D) % RP) * PSB, (r & 1) * XB, ((r + 1) & 1) * XB);
+        __syncthreads();
+      }
+      advance(U);
+      if (AX) advancep(U);
+      vp += U * (BWD ? vstep : sstep);
     }
-    const int xs = wr; wr = rd; rd = xs;
-    __syncthreads();
+  } else {
+    const V *cs = ring + SS, *const cend = ring + (size_t)R * SS;
+    const V *pm = pb + PS, *pp = pb + 3 * PS, *const pend = pb + RP * PS;
+    unsigned wso = 0u, wpo = 0u;
+    int wr = 0, rd = XB;
+    // the warp's steps, one before its first cell to one after its last
+    const int wfirst = __reduce_min_sync(0xffffffffu, slo) - 1;
+    const int wlast = __reduce_max_sync(0xffffffffu, col ? slo + (int)nact : -1) + 1;
+#pragma unroll 1
+    for (int s = 0; s < nsteps; ++s) {
+      if (CT > 0 || (s >= wfirst && s <= wlast)) {
+        iterate(s, 0, cs, pm, pp, wso, wpo, wr, rd);
+      } else {  // no column of the warp has a cell at step s or s+1: only the copies
+        cpa_wait<D - 1>();
+        load(s + 1 + D, wso, 0);
+        if (AX) {
+          loadp(s + 3 + D, wpo, 0);
+          p0 = p1; p1 = pp[tq];
+        }
+        cpa_commit();
+      }
+      advance(1);
+      vp += BWD ? vstep : sstep;
+      cs += SS;
+      if (cs == cend) cs = ring;
+      wso += SB;
+      if (wso == R * SB) wso = 0u;
+      if (AX) {
+        advancep(1);
+        pm += PS;
+        if (pm == pend) pm = pb;
+        pp += PS;
+        if (pp == pend) pp = pb;
+        wpo += PSB;
+        if (wpo == RP * PSB) wpo = 0u;
+      }
+      const int xs = wr; wr = rd; rd = xs;
+      __syncthreads();
+    }
   }
   cpa_wait<0>();
   if (NDOT > 0) {
