@@ -164,30 +164,45 @@ __device__ __forceinline__ void row_store(double s, double *rowbuf, long long ro
   if ((threadIdx.x & 31) == 0 && row < nrows) rowbuf[row] = s;
 }
 
-// Second stage: one block of 1024 threads sums the row partials.
-__device__ __forceinline__ double block_final(const double *rowbuf, long long nrows) {
-  __shared__ double w[32];
+// Second stage: one block of 1024 threads sums the row partials of N
+// buffers (together, so that one sum's latencies hide the others').
+template <int N>
+__device__ __forceinline__ void block_final_n(const double *const (&rowbuf)[N], long long nrows, double (&out)[N]) {
+  __shared__ double w[N][32];
   // thread t sums rows t, t+1024, t+2048, ... in that order; the loads of
   // eight of them are issued before their additions
-  double s = 0.0;
-  for (long long r0 = threadIdx.x; r0 < nrows; r0 += 8 * 1024) {
-    double v[8];
+  double s[N];
 #pragma unroll
-    for (int j = 0; j < 8; ++j) v[j] = (r0 + j * 1024 < nrows) ? rowbuf[r0 + j * 1024] : 0.0;
+  for (int c = 0; c < N; ++c) s[c] = 0.0;
+  constexpr int L = N > 2 ? 2 : 8;
+  for (long long r0 = threadIdx.x; r0 < nrows; r0 += L * 1024) {
+    double v[N][L];
 #pragma unroll
-    for (int j = 0; j < 8; ++j)
-      if (r0 + j * 1024 < nrows) s = s + v[j];
+    for (int c = 0; c < N; ++c)
+#pragma unroll
+      for (int j = 0; j < L; ++j) v[c][j] = (r0 + j * 1024 < nrows) ? rowbuf[c][r0 + j * 1024] : 0.0;
+#pragma unroll
+    for (int c = 0; c < N; ++c)
+#pragma unroll
+      for (int j = 0; j < L; ++j)
+        if (r0 + j * 1024 < nrows) s[c] = s[c] + v[c][j];
   }
-  s = warp_tree(s);
-  if ((threadIdx.x & 31) == 0) w[threadIdx.x >> 5] = s;
+#pragma unroll
+  for (int c = 0; c < N; ++c) s[c] = warp_tree(s[c]);
+  if ((threadIdx.x & 31) == 0)
+#pragma unroll
+    for (int c = 0; c < N; ++c) w[c][threadIdx.x >> 5] = s[c];
   __syncthreads();
-  double t = 0.0;
-  if (threadIdx.x < 32) {
-    t = w[threadIdx.x];
-    t = warp_tree(t);
-  }
+  if (threadIdx.x < 32)
+#pragma unroll
+    for (int c = 0; c < N; ++c) out[c] = warp_tree(w[c][threadIdx.x]);  // valid in thread 0
   __syncthreads();
-  return t;  // valid in thread 0
+}
+__device__ __forceinline__ double block_final(const double *rowbuf, long long nrows) {
+  const double *const b[1] = {rowbuf};
+  double t[1] = {0.0};
+  block_final_n<1>(b, nrows, t);
+  return t[0];  // valid in thread 0
 }
 
 // -------------------------------------------------------- solver scalars

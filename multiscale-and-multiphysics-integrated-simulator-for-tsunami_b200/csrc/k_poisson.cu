@@ -1292,10 +1292,11 @@ __global__ void __launch_bounds__(256) k_upd3f(SkewGeo q, const float *AE, const
 __device__ __forceinline__ void fin5_body(const double *rb, long long nrows, SolveState *st, double epsa2,
                                           double epsr2, double div2, int icgmax) {
   if (st->done) return;
-  const double rae = block_final(rb, nrows), aeae = block_final(rb + nrows, nrows),
-               rrrr = block_final(rb + 2 * nrows, nrows), r0rr = block_final(rb + 3 * nrows, nrows),
-               r0ae = block_final(rb + 4 * nrows, nrows);
+  const double *const b[5] = {rb, rb + nrows, rb + 2 * nrows, rb + 3 * nrows, rb + 4 * nrows};
+  double t[5] = {0.0, 0.0, 0.0, 0.0, 0.0};
+  block_final_n<5>(b, nrows, t);
   if (threadIdx.x != 0) return;
+  const double rae = t[0], aeae = t[1], rrrr = t[2], r0rr = t[3], r0ae = t[4];
   const double omega = rae / aeae;
   st->omega = omega;
   st->w1 = rae;
@@ -1422,8 +1423,16 @@ __device__ __forceinline__ void fin_body(int mode, const double *rb0, const doub
                                          int icgmax) {
   if (mode < FIN_ALPHA && mode != FIN_STORE && mode != FIN_RELRES && st->done) return;
   if (mode >= FIN_ALPHA && st->done) return;
-  double a = block_final(rb0, nrows);
-  double b = (rb1 ? block_final(rb1, nrows) : 0.0);
+  double a, b = 0.0;
+  if (rb1) {
+    const double *const bufs[2] = {rb0, rb1};
+    double t[2] = {0.0, 0.0};
+    block_final_n<2>(bufs, nrows, t);
+    a = t[0];
+    b = t[1];
+  } else {
+    a = block_final(rb0, nrows);
+  }
   if (threadIdx.x != 0) return;
   switch (mode) {
     case FIN_BNORM:

@@ -334,10 +334,12 @@ __device__ __forceinline__ void sweep_cp_body(const Geo &g, const SkewGeo &q, co
     xk1 = x;
   };
   __syncthreads();
-  if constexpr (UNR) {
-    int s0 = 0;
+  if (!__any_sync(0xffffffffu, col)) {  // a warp past the grid's edge (a ragged tile)
 #pragma unroll 1
-    for (; s0 < nsteps; s0 += U) {
+    for (int s = 0; s < nsteps; ++s) __syncthreads();
+  } else if constexpr (UNR) {
+#pragma unroll 1
+    for (int s0 = 0; s0 < nsteps; s0 += U) {
 #pragma unroll
       for (int r = 0; r < U; ++r) {
         if (s0 + r >= nsteps) break;
