@@ -1665,14 +1665,14 @@ static int sweep_cp_depth(const SkewGeo &q, int mode, int es) {
       const int d = mode == SWEEP_FWD_AX ? ax[i] : plain[i];
       if ((d >= 12 && nt > 128) || (d == 1 && nt <= 576)) continue;
       if (q.occ == 0 && blocks > 1 && share < 227 * 1024 && d < 6) continue;
-      if (sweep_cp_bytes(mode, d, unr, q.T, q.TI, q.TJ, es) <= share) return d;
+      if (sweep_cp_bytes(mode, d, unr, q.T, q.TIp, q.TI, q.TJ, es) <= share) return d;
     }
   return 0;
 }
 template <int D, int MODE, int MAXT, typename V, int MINB>
 static void sweep_cp_go(cudaStream_t s, const Geo &g, const SkewGeo &q, const SkewSysT<V> &S, const V *vin, V *vout,
                         SolveState *st, const V *vin2, double *rb) {
-  const size_t bytes = sweep_cp_bytes(MODE, D, sweep_cp_unrolled(q, MODE, (int)sizeof(V)), q.T, q.TI, q.TJ, (int)sizeof(V));
+  const size_t bytes = sweep_cp_bytes(MODE, D, sweep_cp_unrolled(q, MODE, (int)sizeof(V)), q.T, q.TIp, q.TI, q.TJ, (int)sizeof(V));
   const dim3 grid((unsigned)q.ntx, (unsigned)(q.nb / q.ntx)), block((unsigned)sweep_cp_threads(q.T));
 #define SWEEP_GO(CT, CI)                                                                                        \
   {                                                                                                             \
@@ -2099,7 +2099,7 @@ static bool launch_b_sweep_t(cudaStream_t s, const BatchMember *bm, const int *p
                vout, vin2, rb5, dr);
     return true;
   }
-  const size_t bytes = sweep_cp_bytes(MODE, d, sweep_cp_unrolled(q, MODE, 4), q.T, q.TI, q.TJ, 4);
+  const size_t bytes = sweep_cp_bytes(MODE, d, sweep_cp_unrolled(q, MODE, 4), q.T, q.TIp, q.TI, q.TJ, 4);
   const dim3 block((unsigned)nt);
 #define BSWEEP(D, MT, MB, CT, CI)                                                                             \
   {                                                                                                           \

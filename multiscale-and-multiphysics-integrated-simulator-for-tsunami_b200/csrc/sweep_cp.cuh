@@ -56,8 +56,7 @@ __device__ __forceinline__ void sweep_sums(const double *a, double *rb, int nb, 
 //     unrolled over the ring, so that slots, buffers and the copies' sources
 //     are constant offsets: a warp's instructions per step, each waiting
 //     for the one before, are what a small grid's step takes.
-// Entry T of the shared P and X arrays is a zero that stands for neighbours
-// outside.  The expressions and their order are those of the reference loops.
+// Zero entries of the shared P and X arrays stand for neighbours outside.  The expressions and their order are those of the reference loops.
 __device__ __forceinline__ void cpa16(unsigned dst, const void *src) {
   asm volatile("cp.async.cg.shared.global [%0], [%1], 16;\n" ::"r"(dst), "l"(src) : "memory");
 }
@@ -81,8 +80,39 @@ __host__ __device__ constexpr int sweep_cp_chunked(int mode, int es) {
 __host__ __device__ constexpr int sweep_cp_plain(int mode) {
   return mode == SWEEP_FWD_AX ? 0 : (mode == SWEEP_FWD ? 1 : 1 + (mode - SWEEP_BWD));
 }
-// elements of one slot of P: T, the zero, the halo columns; a multiple of 16 bytes
-__host__ __device__ inline int sweep_cp_pslot(int T, int TI, int TJ) { return (T + 1 + 2 * (TI + TJ) + 3) & ~3; }
+// One slot of P: the tile's T entries from `main` on, the halo rows and
+// columns, a zero.  Up to 256 columns each halo value lies in the bank that
+// its reader's own neighbour entry would have (the lower row before the
+// tile's entries, the upper one after them, left and right ones spread by
+// TIp), so that a warp's load has no conflicts; larger tiles, whose rings are
+// short of memory, pack them.
+struct SweepP {
+  int main, zero, left, right, xs, down, up, size;  // left + xs*tj, right + xs*tj, down + ti, up + ti
+};
+__host__ __device__ inline SweepP sweep_cp_pslot(int T, int TIp, int TI, int TJ) {
+  SweepP p;
+  if (T <= 256) {
+    p.main = (TIp + 31) & ~31;
+    p.down = p.main - TIp;
+    p.up = p.main + T;
+    p.zero = (p.up + TIp + 31) & ~31;
+    p.xs = TIp;
+    p.left = p.zero + 31;
+    p.right = p.zero + TIp;
+    p.size = p.zero + TIp * (TJ - 1) + (TIp > 31 ? TIp : 31) + 1;
+  } else {
+    p.main = 0;
+    p.zero = T;
+    p.xs = 1;
+    p.left = T + 1;
+    p.right = T + 1 + TJ;
+    p.down = T + 1 + 2 * TJ;
+    p.up = T + 1 + 2 * TJ + TI;
+    p.size = T + 1 + 2 * (TI + TJ);
+  }
+  p.size = (p.size + 3) & ~3;  // 16 bytes
+  return p;
+}
 // The compiled-in shapes (ct = T; 0: any shape) run the unrolled loop, but
 // for the fused FP64 sweep of 256 columns, whose slots are so large that
 // the longer ring costs it two steps of depth (512 tiles: 250 against 242 us).
@@ -95,10 +125,10 @@ __host__ __device__ constexpr int sweep_cp_slots(int mode, int D, bool unrolled)
   return D + (mode == SWEEP_FWD_AX && unrolled ? 4 : 1);
 }
 // shared memory of a block
-__host__ __device__ inline size_t sweep_cp_bytes(int mode, int D, bool unrolled, int T, int TI, int TJ, int es) {
+__host__ __device__ inline size_t sweep_cp_bytes(int mode, int D, bool unrolled, int T, int TIp, int TI, int TJ, int es) {
   size_t n = (size_t)sweep_cp_slots(mode, D, unrolled) * (sweep_cp_chunked(mode, es) + sweep_cp_plain(mode)) * T;
-  n += 2 * (size_t)(T + 4) * (mode >= SWEEP_BWD ? 1 : 2);
-  if (mode == SWEEP_FWD_AX) n += (size_t)(D + 4) * sweep_cp_pslot(T, TI, TJ);
+  n += 2 * (size_t)(T + 16) * (mode >= SWEEP_BWD ? 1 : 2);
+  if (mode == SWEEP_FWD_AX) n += (size_t)(D + 4) * sweep_cp_pslot(T, TIp, TI, TJ).size;
   return n * es;
 }
 
@@ -119,8 +149,9 @@ __device__ __forceinline__ void sweep_cp_body(const Geo &g, const SkewGeo &q, co
   const int WS = skew_stride(q);
   const int T = CT > 0 ? CT : q.T, TIp = CT > 0 ? CTIP : q.TIp, TI = q.TI, TJ = CT > 0 ? CT / (CTIP > 0 ? CTIP : 1) : q.TJ;
   const int tid = threadIdx.x, b = bx + q.ntx * by, nty = q.nb / q.ntx;
-  const int XB = T + 4;                                           // entries of an exchange buffer
-  const int SS = (NC * G + NP) * T, PS = AX ? sweep_cp_pslot(T, TI, TJ) : 0;
+  const int XB = T + 16;                                          // entries of an exchange buffer
+  const int SS = (NC * G + NP) * T, PS = AX ? sweep_cp_pslot(T, TIp, TI, TJ).size : 0;
+  const SweepP po = sweep_cp_pslot(T, TIp, TI, TJ);
   extern __shared__ __align__(16) double sm[];
   V *ring = reinterpret_cast<V *>(sm);                            // R slots: chunks, then plain vectors
   V *pb = ring + (size_t)R * SS;                                  // RP slots of P
@@ -134,7 +165,7 @@ __device__ __forceinline__ void sweep_cp_body(const Geo &g, const SkewGeo &q, co
   const int slo = col ? (BWD ? ri + rj : ti + tj) : (1 << 29);
   const unsigned nact = (unsigned)(g.NK - 3);
   const int tq = min(tid, T - 1);
-  const int o1 = (col && (BWD ? ri > 0 : ti > 0)) ? tq + (BWD ? 1 : -1) : T;
+  const int o1 = (col && (BWD ? ri > 0 : ti > 0)) ? tq + (BWD ? 1 : -1) : (BWD ? T : T + 15);
   const int o2 = (col && (BWD ? rj > 0 : tj > 0)) ? tq + (BWD ? TIp : -TIp) : T;
   if (tid < 2) {  // the zeros
     if (BWD) {
@@ -142,9 +173,10 @@ __device__ __forceinline__ void sweep_cp_body(const Geo &g, const SkewGeo &q, co
     } else {
       V2 z; z.x = V(0); z.y = V(0);
       xd[tid * XB + T] = z;
+      xd[tid * XB + T + 15] = z;  // the left column's: in the bank that its neighbours leave free
     }
     if (AX)
-      for (int r = tid; r < RP; r += 2) pb[r * PS + T] = V(0);
+      for (int r = tid; r < RP; r += 2) pb[r * PS + po.zero] = V(0);
   }
   const long long slab0 = (long long)b * WS + (BWD ? nsteps - 1 : 0);
   constexpr long long DIR = BWD ? -1 : 1;
@@ -157,9 +189,10 @@ __device__ __forceinline__ void sweep_cp_body(const Geo &g, const SkewGeo &q, co
   // lower) and after (right, upper)
   const bool hl = AX && col && ti == 0 && bx > 0, hr = AX && col && ti == wi - 1 && bx < q.ntx - 1;
   const bool hd = AX && col && tj == 0 && by > 0, hu = AX && col && tj == wj - 1 && by < nty - 1;
-  const int ehx = T + 1 + (hr ? TJ : 0) + min(tj, TJ - 1), ehy = T + 1 + 2 * TJ + (hu ? TI : 0) + min(ti, TI - 1);
-  const int oxm = hl ? ehx : ((col && ti > 0) ? tq - 1 : T), oxp = hr ? ehx : ((col && ti < wi - 1) ? tq + 1 : T);
-  const int oym = hd ? ehy : ((col && tj > 0) ? tq - TIp : T), oyp = hu ? ehy : ((col && tj < wj - 1) ? tq + TIp : T);
+  const int ehx = (hr ? po.right : po.left) + po.xs * min(tj, TJ - 1), ehy = (hu ? po.up : po.down) + min(ti, TI - 1);
+  const int tp = po.main + tq;
+  const int oxm = hl ? ehx : ((col && ti > 0) ? tp - 1 : po.zero), oxp = hr ? ehx : ((col && ti < wi - 1) ? tp + 1 : po.zero);
+  const int oym = hd ? ehy : ((col && tj > 0) ? tp - TIp : po.zero), oyp = hu ? ehy : ((col && tj < wj - 1) ? tp + TIp : po.zero);
   const int shx = hr ? -1 : 1, shy = hu ? -1 : 1;  // own step minus the neighbour's
   const bool hx = hl || hr, hy = hd || hu;
   const V *lx = vin, *ly = vin;                    // halo values for P slot 0
@@ -185,11 +218,11 @@ __device__ __forceinline__ void sweep_cp_body(const Geo &g, const SkewGeo &q, co
     if (NDOT > 0) cpa<ES>(plain0 + so + (unsigned)(T * ES), l1 + r * vstep);
     if (NDOT == 5) cpa<ES>(plain0 + so + (unsigned)(2 * T * ES), l2 + r * vstep);
   };
-  // P of step v and the halo columns of slot v into the slot at byte offset po
-  auto loadp = [&](int v, unsigned po, int r) {
-    if (active(v)) cpa<ES>(pb0 + po + (unsigned)(tq * ES), l0 + r * vstep);
-    if (hx && active(v + shx)) cpa<ES>(pb0 + po + (unsigned)(ehx * ES), lx + r * vstep);
-    if (hy && active(v + shy)) cpa<ES>(pb0 + po + (unsigned)(ehy * ES), ly + r * vstep);
+  // P of step v and the halo columns of slot v into the slot at byte offset so
+  auto loadp = [&](int v, unsigned so, int r) {
+    if (active(v)) cpa<ES>(pb0 + so + (unsigned)(tp * ES), l0 + r * vstep);
+    if (hx && active(v + shx)) cpa<ES>(pb0 + so + (unsigned)(ehx * ES), lx + r * vstep);
+    if (hy && active(v + shy)) cpa<ES>(pb0 + so + (unsigned)(ehy * ES), ly + r * vstep);
   };
   auto advance = [&](int n) {  // the sources of the chunks and plain vectors
     lc += n * sstep;
@@ -290,7 +323,7 @@ __device__ __forceinline__ void sweep_cp_body(const Geo &g, const SkewGeo &q, co
   cpa_wait<D>();
   __syncthreads();
   V pz = V(0);
-  if (AX) { p1 = pb[PS + tq]; pz = pb[2 * PS + tq]; }
+  if (AX) { p1 = pb[PS + tp]; pz = pb[2 * PS + tp]; }
   prepare(0, fetch(ring), V(0), V(0), AX ? pb[oxm] : V(0), AX ? pb[oym] : V(0), AX ? pb[2 * PS + oxp] : V(0),
           AX ? pb[2 * PS + oyp] : V(0), pz);
   p0 = p1; p1 = pz;
@@ -311,7 +344,7 @@ __device__ __forceinline__ void sweep_cp_body(const Geo &g, const SkewGeo &q, co
       const V2 n1 = xd[rd + o1], n2 = xd[rd + o2];
       x1 = n1.x; d1 = n1.y; x2 = n2.x; d2 = n2.y;
     }
-    if (AX) { pxm = pm[oxm]; pym = pm[oym]; pxp = pp[oxp]; pyp = pp[oyp]; p2 = pp[tq]; }
+    if (AX) { pxm = pm[oxm]; pym = pm[oym]; pxp = pp[oxp]; pyp = pp[oyp]; p2 = pp[tp]; }
     const Vals f = fetch(cs);
     load(s + 1 + D, wso, r);
     if (AX) loadp(s + 3 + D, wpo, r);
@@ -370,7 +403,7 @@ __device__ __forceinline__ void sweep_cp_body(const Geo &g, const SkewGeo &q, co
         load(s + 1 + D, wso, 0);
         if (AX) {
           loadp(s + 3 + D, wpo, 0);
-          p0 = p1; p1 = pp[tq];
+          p0 = p1; p1 = pp[tp];
         }
         cpa_commit();
       }
