@@ -25,9 +25,11 @@ struct Geo {
 __device__ __forceinline__ long long cid(const Geo &g, int i, int j, int k) {
   return (long long)(i - 1) + (long long)g.NI * ((long long)(j - 1) + (long long)g.NJ * (long long)(k - 1));
 }
-__device__ __forceinline__ double gx(const Geo &g, int m, int i) { return g.XX[(m - 1) + 6 * (i - 1)]; }
-__device__ __forceinline__ double gy(const Geo &g, int m, int j) { return g.YY[(m - 1) + 6 * (j - 1)]; }
-__device__ __forceinline__ double gz(const Geo &g, int m, int k) { return g.ZZ[(m - 1) + 6 * (k - 1)]; }
+// The metrics are constant: read-only loads, which stay valid across the
+// kernels' stores.
+__device__ __forceinline__ double gx(const Geo &g, int m, int i) { return __ldg(g.XX + (m - 1) + 6 * (i - 1)); }
+__device__ __forceinline__ double gy(const Geo &g, int m, int j) { return __ldg(g.YY + (m - 1) + 6 * (j - 1)); }
+__device__ __forceinline__ double gz(const Geo &g, int m, int k) { return __ldg(g.ZZ + (m - 1) + 6 * (k - 1)); }
 
 // MAX/MIN with the comparison the oracle uses (first operand on ties).
 __device__ __forceinline__ double dmax(double a, double b) { return (a < b) ? b : a; }
@@ -139,6 +141,64 @@ inline unsigned row_blocks(const Geo &g) {
 #define ROW_LOOP_END \
     }                \
   }
+
+// A "cell kernel" (no sum over the grid) gives every thread one cell: the
+// threads of a block take consecutive cells of an x-y plane, blockIdx.y the
+// plane.  No lane walks a row on its own, so a row costs one cell's latency
+// and not NI/32 of them, a small grid fills the chip (66x10x34 cells: 204
+// blocks instead of 43) and a ragged row leaves no lanes idle.
+constexpr int CELL_THREADS = 128;
+inline dim3 cell_grid(const Geo &g, int kper = 1) {
+  const int ny = (g.NK + kper - 1) / kper;
+  return dim3(((unsigned)g.NI * (unsigned)g.NJ + CELL_THREADS - 1) / CELL_THREADS, (unsigned)(ny < 65535 ? ny : 65535));
+}
+#define CELL_IJ(g)                                             \
+  const unsigned p_ = blockIdx.x * CELL_THREADS + threadIdx.x; \
+  if (p_ < (unsigned)(g).NI * (unsigned)(g).NJ) {              \
+    const int J = (int)(p_ / (unsigned)(g).NI) + 1;            \
+    const int I = (int)(p_ % (unsigned)(g).NI) + 1;
+#define CELL_LOOP_BEGIN(g) \
+  CELL_IJ(g)               \
+    for (int K = (int)blockIdx.y + 1; K <= (g).NK; K += (int)gridDim.y) {
+#define CELL_LOOP_END \
+    }                 \
+  }
+// A "scan kernel" acts on the few cells whose flag n_ satisfies `pred`:
+// a thread reads the flags of SCAN_K planes at once and visits its hits.
+// (The kernels that change the flags in place change a cell's flag only
+// from its own thread.)
+constexpr int SCAN_K = 4;
+#define SCAN_LOOP_BEGIN(g, NF_, pred)                                                             \
+  CELL_IJ(g)                                                                                      \
+    const long long plane_ = (long long)(g).NI * (g).NJ;                                          \
+    for (int K0_ = (int)blockIdx.y * SCAN_K + 1; K0_ <= (g).NK; K0_ += (int)gridDim.y * SCAN_K) { \
+      unsigned m_ = 0;                                                                            \
+      int v_[SCAN_K];                                                                             \
+      _Pragma("unroll") for (int u_ = 0; u_ < SCAN_K; ++u_)                                       \
+        v_[u_] = (NF_)[p_ + plane_ * (min(K0_ + u_, (g).NK) - 1)];                                \
+      _Pragma("unroll") for (int u_ = 0; u_ < SCAN_K; ++u_) {                                     \
+        const int n_ = v_[u_];                                                                    \
+        if (K0_ + u_ <= (g).NK && (pred)) m_ |= 1u << u_;                                         \
+      }                                                                                           \
+      for (; m_; m_ &= m_ - 1) {                                                                  \
+        const int K = K0_ + __ffs((int)m_) - 1;
+#define SCAN_LOOP_END \
+      }               \
+    }                 \
+  }
+// Loads that stay where they are written, so that those of a cell are all in
+// flight together (left to itself the compiler sinks each into the branch
+// that uses it).  Not for arrays that the kernel writes.
+__device__ __forceinline__ double ld_now(const double *p) {
+  double v;
+  asm volatile("ld.global.f64 %0, [%1];" : "=d"(v) : "l"(p));
+  return v;
+}
+__device__ __forceinline__ int ld_now(const int *p) {
+  int v;
+  asm volatile("ld.global.s32 %0, [%1];" : "=r"(v) : "l"(p));
+  return v;
+}
 
 // Programmatic dependent launch.  The solver's kernels are launched with
 // programmatic stream serialisation (launch_pdl), so a kernel may be

@@ -189,10 +189,10 @@ __device__ __noinline__ double bsuwt_z(const Geo &g, const int *NF, const double
   return (DR * VL + DL * VR) / (DR + DL);
 }
 
-__global__ void __launch_bounds__(ROW_THREADS, 4) k_bsuwt(Geo g, Fld f, Prm p) {
+__global__ void __launch_bounds__(CELL_THREADS) k_bsuwt(Geo g, Fld f, Prm p) {
   const int S0 = (p.ibsuw0 == 0);
   const int *NF = f.nf;
-  ROW_LOOP_BEGIN(g)
+  CELL_LOOP_BEGIN(g)
   const long long c = cid(g, I, J, K);
   const int NI = g.NI, NJ = g.NJ, NK = g.NK;
   // x faces K=2..NK-1, J=2..NJ-1, I=3..NI-1; y faces K=2..NK-1, J=3..NJ-1,
@@ -218,7 +218,7 @@ __global__ void __launch_bounds__(ROW_THREADS, 4) k_bsuwt(Geo g, Fld f, Prm p) {
       else if (NLz != 0 && NR != 0) f.ww[c] = bsuwt_z(g, NF, f.ww, S0, I, J, K, NLz, NR);
     }
   }
-  ROW_LOOP_END
+  CELL_LOOP_END
 }
 
 __device__ __forceinline__ bool surf_interior(const Geo &g, int I, int J, int K) {
@@ -226,10 +226,10 @@ __device__ __forceinline__ bool surf_interior(const Geo &g, int I, int J, int K)
 }
 
 // ----------------------------------------------------------- VF_BSUWT2
-__global__ void k_bsuwt2(Geo g, Fld f) {
+__global__ void __launch_bounds__(CELL_THREADS) k_bsuwt2(Geo g, Fld f) {
   const int *NF = f.nf;
   double *UU = f.uu, *VV = f.vv, *WW = f.ww;
-  ROW_LOOP_BEGIN(g)
+  SCAN_LOOP_BEGIN(g, f.nf, n_ >= 1 && n_ <= 6)
   const long long c = cid(g, I, J, K);
   const int NF0 = NF[c];
   if (NF0 >= 1 && NF0 <= 6 && surf_interior(g, I, J, K)) {
@@ -266,14 +266,14 @@ __global__ void k_bsuwt2(Geo g, Fld f) {
       A(WW, I, J, L1) = A(WW, I, J, L2);
     }
   }
-  ROW_LOOP_END
+  SCAN_LOOP_END
 }
 
 // ------------------------------------------------------------ VF_BSUWN
-__global__ void k_bsuwn(Geo g, Fld f) {
+__global__ void __launch_bounds__(CELL_THREADS) k_bsuwn(Geo g, Fld f) {
   double *UU = f.uu, *VV = f.vv, *WW = f.ww;
   const double *GGX = f.ggx, *GGY = f.ggy, *GGZ = f.ggz;
-  ROW_LOOP_BEGIN(g)
+  SCAN_LOOP_BEGIN(g, f.nf, n_ >= 1 && n_ <= 6)
   const long long c = cid(g, I, J, K);
   const int NF0 = f.nf[c];
   if (NF0 >= 1 && NF0 <= 6 && surf_interior(g, I, J, K)) {
@@ -288,7 +288,7 @@ __global__ void k_bsuwn(Geo g, Fld f) {
     else if (NF0 == 1) A(UU, I1, J, K) = (FXM - XX_(2, I) * (YY_(4, J) * (FYP - FYM) + ZZ_(4, K) * (FZP - FZM))) / A(GGX, I1, J, K);
     else if (NF0 == 2) UU[c] = (FXP + XX_(2, I) * (YY_(4, J) * (FYP - FYM) + ZZ_(4, K) * (FZP - FZM))) / GGX[c];
   }
-  ROW_LOOP_END
+  SCAN_LOOP_END
 }
 
 // ----------------------------------------------------------- VF_BSUWN3
@@ -298,11 +298,11 @@ __device__ __forceinline__ void lat(const Geo &g, const int *NF, long long a, lo
     if (NF[a] != -1 && NF[b] != -1) { is = 1; d = dv; v = vv; }
 }
 
-__global__ void __launch_bounds__(ROW_THREADS, 3) k_bsuwn3(Geo g, Fld f, Prm p) {
+__global__ void __launch_bounds__(CELL_THREADS) k_bsuwn3(Geo g, Fld f, Prm p) {
   const int S0 = (p.ibsuw0 == 0);
   const int *NF = f.nf;
   double *UU = f.uu, *VV = f.vv, *WW = f.ww;
-  ROW_LOOP_BEGIN(g)
+  SCAN_LOOP_BEGIN(g, f.nf, n_ >= 1 && n_ <= 6)
   const long long c = cid(g, I, J, K);
   const int NF0 = NF[c];
   if (NF0 >= 1 && NF0 <= 6 && surf_interior(g, I, J, K)) {
@@ -376,15 +376,15 @@ __global__ void __launch_bounds__(ROW_THREADS, 3) k_bsuwn3(Geo g, Fld f, Prm p) 
     double *arr = (NF0 >= 5) ? WW : (NF0 >= 3 ? VV : UU);
     arr[out] = val;
   }
-  ROW_LOOP_END
+  SCAN_LOOP_END
 }
 
 // ----------------------------------------------------------- VF_BSUWEM
 // NLIM of each cell = number of surface neighbours for which it is a
 // lateral (non-normal) neighbour (vf_bsuwem.f:55-78), as a gather.
-__global__ void k_bsuwem_count(Geo g, Fld f, int *NLIM) {
+__global__ void __launch_bounds__(CELL_THREADS) k_bsuwem_count(Geo g, Fld f, int *NLIM) {
   const int *NF = f.nf;
-  ROW_LOOP_BEGIN(g)
+  CELL_LOOP_BEGIN(g)
   const long long c = cid(g, I, J, K);
   int n = 0;
   if (I >= 2 && I <= g.NI - 1 && J >= 2 && J <= g.NJ - 1 && K >= 2 && K <= g.NK - 1) {
@@ -397,13 +397,13 @@ __global__ void k_bsuwem_count(Geo g, Fld f, int *NLIM) {
     s = A(NF, I, J, K + 1); if (s >= 1 && s <= 4) n++;
   }
   NLIM[c] = n;
-  ROW_LOOP_END
+  CELL_LOOP_END
 }
 
-__global__ void k_bsuwem_fix(Geo g, Fld f, const int *NLIM) {
+__global__ void __launch_bounds__(CELL_THREADS) k_bsuwem_fix(Geo g, Fld f, const int *NLIM) {
   const int *NF = f.nf;
   double *UU = f.uu, *VV = f.vv, *WW = f.ww;
-  ROW_LOOP_BEGIN(g)
+  SCAN_LOOP_BEGIN(g, f.nf, n_ == 8)
   const long long c = cid(g, I, J, K);
   if (surf_interior(g, I, J, K) && NLIM[c] >= 2 && NF[c] == 8) {
     if (A(NF, I - 1, J, K) == 8 && A(NLIM, I - 1, J, K) < 2)
@@ -419,15 +419,15 @@ __global__ void k_bsuwem_fix(Geo g, Fld f, const int *NLIM) {
     if (A(NF, I, J, K + 1) == 8 && A(NLIM, I, J, K + 1) < 2)
       if (A(NF, I, J, K - 1) != 8) A(WW, I, J, K + 1) = WW[c];
   }
-  ROW_LOOP_END
+  SCAN_LOOP_END
 }
 
 // ------------------------------------------------------------- VF_BSPP
-__global__ void k_bspp(Geo g, Fld f) {
+__global__ void __launch_bounds__(CELL_THREADS) k_bspp(Geo g, Fld f) {
   const double PPS = 0.0;
   double *PP = f.pp;
   const double *FF = f.ff;
-  ROW_LOOP_BEGIN(g)
+  SCAN_LOOP_BEGIN(g, f.nf, n_ >= 1 && n_ <= 8 && n_ != 7)
   const long long c = cid(g, I, J, K);
   if (surf_interior(g, I, J, K)) {
     const int n = f.nf[c];
@@ -440,7 +440,7 @@ __global__ void k_bspp(Geo g, Fld f) {
     else if (n == 1) { PSI = XX_(3, I) / (0.5 * XX_(2, I - 1) + FF[c] * XX_(2, I)); PP[c] = (1.0 - PSI) * A(PP, I - 1, J, K) + PSI * PPS; }
     else if (n == 2) { PSI = XX_(3, I + 1) / (0.5 * XX_(2, I + 1) + FF[c] * XX_(2, I)); PP[c] = (1.0 - PSI) * A(PP, I + 1, J, K) + PSI * PPS; }
   }
-  ROW_LOOP_END
+  SCAN_LOOP_END
 }
 
 // ---------------------------------------------------- boundary-list rules
@@ -622,9 +622,11 @@ __global__ void k_cdtcal_fin(const double *rb, long long nrows, double dt0, doub
 
 // ------------------------------------------------------------ launchers
 #define RL(kern, ...) (kern<<<row_blocks(g), ROW_THREADS, 0, s>>>(__VA_ARGS__), count_launch())
+#define CL(kern, ...) (kern<<<cell_grid(g), CELL_THREADS, 0, s>>>(__VA_ARGS__), count_launch())
+#define SCL(kern, ...) (kern<<<cell_grid(g, SCAN_K), CELL_THREADS, 0, s>>>(__VA_ARGS__), count_launch())
 #define BL(kern, ...) if (g.NB > 0) (kern<<<(g.NB + 255) / 256, 256, 0, s>>>(__VA_ARGS__), count_launch())
-void launch_bsuwt(cudaStream_t s, const Geo &g, const Fld &f, const Prm &p) { RL(k_bsuwt, g, f, p); }
-void launch_bsuwt2(cudaStream_t s, const Geo &g, const Fld &f) { RL(k_bsuwt2, g, f); }
+void launch_bsuwt(cudaStream_t s, const Geo &g, const Fld &f, const Prm &p) { CL(k_bsuwt, g, f, p); }
+void launch_bsuwt2(cudaStream_t s, const Geo &g, const Fld &f) { SCL(k_bsuwt2, g, f); }
 // Wave-source part of VF_BSUWN (vf_bsuwn.f:81-118): on the source's line,
 // the first surface cell of each column from the bottom (obstacle, fluid
 // and gas cells skipped) passes the source flow 2 XX(4,I) SRCUV (or
@@ -663,18 +665,18 @@ __global__ void k_bsuwn_src(Geo g, Fld f, Prm p) {
   }
 }
 
-void launch_bsuwn(cudaStream_t s, const Geo &g, const Fld &f) { RL(k_bsuwn, g, f); }
+void launch_bsuwn(cudaStream_t s, const Geo &g, const Fld &f) { SCL(k_bsuwn, g, f); }
 void launch_bsuwn_src(cudaStream_t s, const Geo &g, const Fld &f, const Prm &p) {
   const int n = (p.iws != 0 ? g.NJ : g.NI) - 2;
   k_bsuwn_src<<<(n + 127) / 128, 128, 0, s>>>(g, f, p);
   count_launch();
 }
-void launch_bsuwn3(cudaStream_t s, const Geo &g, const Fld &f, const Prm &p) { RL(k_bsuwn3, g, f, p); }
+void launch_bsuwn3(cudaStream_t s, const Geo &g, const Fld &f, const Prm &p) { SCL(k_bsuwn3, g, f, p); }
 void launch_bsuwem(cudaStream_t s, const Geo &g, const Fld &f, int *nlim) {
-  RL(k_bsuwem_count, g, f, nlim);
-  RL(k_bsuwem_fix, g, f, nlim);
+  CL(k_bsuwem_count, g, f, nlim);
+  SCL(k_bsuwem_fix, g, f, nlim);
 }
-void launch_bspp(cudaStream_t s, const Geo &g, const Fld &f) { RL(k_bspp, g, f); }
+void launch_bspp(cudaStream_t s, const Geo &g, const Fld &f) { SCL(k_bspp, g, f); }
 // VF_BWFFSF (vf_bwffsf.f:48-128): F of the column next to a fixed-water-
 // level side from the level wl = WVLVL + the table's level, per cell
 // height; obstacle cells keep theirs.  One thread per cell of the column.
@@ -708,6 +710,8 @@ void launch_cdtcal(cudaStream_t s, const Geo &g, const Fld &f, double *rb, doubl
   count_launch();
 }
 #undef RL
+#undef CL
+#undef SCL
 #undef BL
 
 }  // namespace cadmas

@@ -140,18 +140,18 @@ __device__ bool bwkelg_cell(const Geo &g, const Fld &f, const Prm &p, double akc
 
 // VF_BWKELG after VF_F1CAL (vf_a1main.f:1120): k and e in place on the
 // fluid cells (new NF) next to log-law or rough walls.
-__global__ void k_bwkelg(Geo g, Fld f, Prm p, KeConst kc, double *AK, double *AE, int *err) {
-  ROW_LOOP_BEGIN(g)
+__global__ void __launch_bounds__(CELL_THREADS) k_bwkelg(Geo g, Fld f, Prm p, KeConst kc, double *AK, double *AE, int *err) {
+  CELL_LOOP_BEGIN(g)
   const long long c = cid(g, I, J, K);
   if (kint(g, I, J, K) && f.nf[c] == 0) {
     double ak, ae;
     if (bwkelg_cell(g, f, p, kc.akcmu, c, I, J, K, ak, ae, err)) { AK[c] = ak; AE[c] = ae; }
   }
-  ROW_LOOP_END
+  CELL_LOOP_END
 }
 
-__global__ void k_kstep(Geo g, Fld f, Prm p, KeConst kc, KeArrays t, double *AKN, double *AEN, int *err) {
-  ROW_LOOP_BEGIN(g)
+__global__ void __launch_bounds__(CELL_THREADS) k_kstep(Geo g, Fld f, Prm p, KeConst kc, KeArrays t, double *AKN, double *AEN, int *err) {
+  CELL_LOOP_BEGIN(g)
   const long long c = cid(g, I, J, K);
   double akn = t.ak[c], aen = t.ae[c];
   if (kint(g, I, J, K) && f.nf[c] == 0) {
@@ -249,13 +249,13 @@ __global__ void k_kstep(Geo g, Fld f, Prm p, KeConst kc, KeArrays t, double *AKN
   }
   AKN[c] = akn;
   AEN[c] = aen;
-  ROW_LOOP_END
+  CELL_LOOP_END
 }
 
 // BS: VF_BSSS on k and e; NUT: then VF_CNUT0 and VF_CNU00 on the same cell.
 template <bool BS, bool NUT>
-__global__ void k_kbsss(Geo g, Fld f, KeConst kc, double *AK, double *AE, double *ANUT, double *ANU) {
-  ROW_LOOP_BEGIN(g)
+__global__ void __launch_bounds__(CELL_THREADS) k_kbsss(Geo g, Fld f, KeConst kc, double *AK, double *AE, double *ANUT, double *ANU) {
+  CELL_LOOP_BEGIN(g)
   if (kint(g, I, J, K)) {
     const long long c = cid(g, I, J, K);
     const int n = f.nf[c];
@@ -284,7 +284,7 @@ __global__ void k_kbsss(Geo g, Fld f, KeConst kc, double *AK, double *AE, double
       ANU[c] = (n != -1) ? kc.anu0 + nut : 0.0;
     }
   }
-  ROW_LOOP_END
+  CELL_LOOP_END
 }
 
 __global__ void k_bwke(Geo g, Fld f, KeArrays t, int *err) {
@@ -305,8 +305,8 @@ __global__ void k_bwke(Geo g, Fld f, KeArrays t, int *err) {
   else if (IBE != 1) atomicOr(err, ERR_PG);
 }
 
-__global__ void k_kinit(Geo g, Fld f, KeConst kc, double *AK, double *AE, double *ANUT, double *ANU) {
-  ROW_LOOP_BEGIN(g)
+__global__ void __launch_bounds__(CELL_THREADS) k_kinit(Geo g, Fld f, KeConst kc, double *AK, double *AE, double *ANUT, double *ANU) {
+  CELL_LOOP_BEGIN(g)
   const long long c = cid(g, I, J, K);
   double ak = 0.0, ae = 0.0, nut = 0.0, nu = 0.0;
   if (kint(g, I, J, K)) {
@@ -319,7 +319,7 @@ __global__ void k_kinit(Geo g, Fld f, KeConst kc, double *AK, double *AE, double
     }
   }
   AK[c] = ak; AE[c] = ae; ANUT[c] = nut; ANU[c] = nu;
-  ROW_LOOP_END
+  CELL_LOOP_END
 }
 
 #undef A
@@ -327,21 +327,21 @@ __global__ void k_kinit(Geo g, Fld f, KeConst kc, double *AK, double *AE, double
 #undef YY_
 #undef ZZ_
 
-#define RL(kern, ...) (kern<<<row_blocks(g), ROW_THREADS, 0, s>>>(__VA_ARGS__), count_launch())
+#define CL(kern, ...) (kern<<<cell_grid(g), CELL_THREADS, 0, s>>>(__VA_ARGS__), count_launch())
 void launch_bwkelg(cudaStream_t s, const Geo &g, const Fld &f, const Prm &p, const KeConst &kc, double *ak, double *ae,
                    int *err) {
-  k_bwkelg<<<row_blocks(g), ROW_THREADS, 0, s>>>(g, f, p, kc, ak, ae, err);
+  k_bwkelg<<<cell_grid(g), CELL_THREADS, 0, s>>>(g, f, p, kc, ak, ae, err);
   count_launch();
 }
 void launch_kstep(cudaStream_t s, const Geo &g, const Fld &f, const Prm &p, const KeConst &kc, const KeArrays &t,
                   double *akn, double *aen, int *err) {
-  RL(k_kstep, g, f, p, kc, t, akn, aen, err);
+  CL(k_kstep, g, f, p, kc, t, akn, aen, err);
 }
 void launch_kbsss(cudaStream_t s, const Geo &g, const Fld &f, const KeConst &kc, double *ak, double *ae, double *anut,
                   double *anu, bool bsss, bool nut) {
-  if (bsss && nut) RL((k_kbsss<true, true>), g, f, kc, ak, ae, anut, anu);
-  else if (bsss) RL((k_kbsss<true, false>), g, f, kc, ak, ae, anut, anu);
-  else if (nut) RL((k_kbsss<false, true>), g, f, kc, ak, ae, anut, anu);
+  if (bsss && nut) CL((k_kbsss<true, true>), g, f, kc, ak, ae, anut, anu);
+  else if (bsss) CL((k_kbsss<true, false>), g, f, kc, ak, ae, anut, anu);
+  else if (nut) CL((k_kbsss<false, true>), g, f, kc, ak, ae, anut, anu);
 }
 void launch_bwke(cudaStream_t s, const Geo &g, const Fld &f, const KeArrays &t, int *err) {
   if (g.NB <= 0) return;
@@ -350,7 +350,7 @@ void launch_bwke(cudaStream_t s, const Geo &g, const Fld &f, const KeArrays &t, 
 }
 void launch_kinit(cudaStream_t s, const Geo &g, const Fld &f, const KeConst &kc, double *ak, double *ae, double *anut,
                   double *anu) {
-  RL(k_kinit, g, f, kc, ak, ae, anut, anu);
+  CL(k_kinit, g, f, kc, ak, ae, anut, anu);
 }
 
 }  // namespace cadmas

@@ -9,9 +9,18 @@
 //              the values before the update, as in the reference
 //   k_bwuwn    VF_BWUWN boundary-list loop (vf_bwuwn.f:93-160)
 //
-// Roofline: HBM bound.  k_flux reads u,v,w,ANU,GLX..Z,GGX..Z,NF,INDX..Z,INDC
-// once (plus cached neighbours) and writes 9 flux arrays; k_predict reads
-// the 9 fluxes, u,v,w,p,GGV,GLV,CD0,GGX..Z,NF,INDX..Z and writes u,v,w.
+// Traffic: k_flux reads u,v,w,ANU,GLX..Z,GGX..Z,NF,INDX..Z,INDC once (plus
+// cached neighbours) and writes 9 flux arrays; k_predict reads the 9 fluxes,
+// u,v,w,p,GGV,GLV,CD0,GGX..Z,NF,INDX..Z and writes u,v,w: 2.2 and 2.0 GB on
+// 1026x130x130 cells, 340 and 310 us at the memory's rate.  Both are bound by
+// the latency of their loads.  One cell per thread, its flags loaded together
+// and then the values of a component (26 and 23) together: k_flux 1100 -> 980
+// us there, k_predict 916 -> 452 us; on 519x63x85 cells 334 -> 236 and 279 ->
+// 111 us.  More blocks per SM pay more than loads per thread: k_predict takes
+// 559 us with 88 registers, 488 with 78 and 452 with 64 (a few spilled),
+// k_flux 1022 with 128 and all its loads first, 995, 980 and 1107 with 128, 96
+// and 80 by component, and 1016 to 1047 with one component per block (its
+// double-precision arithmetic, some 300 operations a cell, is the next bound).
 #include "cadmas_dev.cuh"
 #include "kernels.h"
 
@@ -27,28 +36,58 @@ __device__ __forceinline__ double bnd_tan(const Fld &f, int IS, int nsFirst, dou
   return bc[IS - 1];
 }
 
-__global__ void __launch_bounds__(ROW_THREADS, 3) k_flux(Geo g, Fld f, Prm p, double *FLUU, double *FLUV, double *FLUW,
+__global__ void __launch_bounds__(CELL_THREADS, 5) k_flux(Geo g, Fld f, Prm p, double *FLUU, double *FLUV, double *FLUW,
                        double *FLVU, double *FLVV, double *FLVW, double *FLWU, double *FLWV,
                        double *FLWW) {
   const double SU = p.scmvp, SC = 1.0 - p.scmvp;
   const double *UU = f.uu, *VV = f.vv, *WW = f.ww, *ANU = f.anu;
   const int *NF = f.nf;
-  ROW_LOOP_BEGIN(g)
+  CELL_LOOP_BEGIN(g)
   const long long c = cid(g, I, J, K);
   const int NI = g.NI, NJ = g.NJ, NK = g.NK;
 #define A(a, i, j, k) a[cid(g, i, j, k)]
 #define XX_(m, i) gx(g, m, i)
 #define YY_(m, j) gy(g, m, j)
 #define ZZ_(m, k) gz(g, m, k)
+  if (I < 2 || J < 2 || K < 2) {
+    FLUU[c] = 0.0; FLUV[c] = 0.0; FLUW[c] = 0.0; FLVU[c] = 0.0; FLVV[c] = 0.0;
+    FLVW[c] = 0.0; FLWU[c] = 0.0; FLWV[c] = 0.0; FLWW[c] = 0.0;
+    continue;
+  }
+  // The flags first; then, component by component, all the values that its
+  // fluxes may use, in flight together.
+  const long long sj = NI, sk = (long long)NI * NJ;
+  const int n0 = ld_now(NF + c), nx = ld_now(NF + c - 1), ny = ld_now(NF + c - sj), nz = ld_now(NF + c - sk),
+            nxy = ld_now(NF + c - 1 - sj), nxz = ld_now(NF + c - 1 - sk), nyz = ld_now(NF + c - sj - sk);
+  const int ix0 = ld_now(f.indx + c), ixy = ld_now(f.indx + c - sj), ixz = ld_now(f.indx + c - sk),
+            iy0 = ld_now(f.indy + c), iyx = ld_now(f.indy + c - 1), iyz = ld_now(f.indy + c - sk),
+            iz0 = ld_now(f.indz + c), izx = ld_now(f.indz + c - 1), izy = ld_now(f.indz + c - sj);
+  const bool dd = K <= NK - 1 && J <= NJ - 1 && I <= NI - 1 && ld_now(f.indc + c) != -1;
+  const int ICxy = nxy * ny * nx * n0, ICxz = nxz * nz * nx * n0, ICyz = nyz * nz * ny * n0;
+  if (!dd && ICxy != 0 && ICxz != 0 && ICyz != 0) {
+    FLUU[c] = 0.0; FLUV[c] = 0.0; FLUW[c] = 0.0; FLVU[c] = 0.0; FLVV[c] = 0.0;
+    FLVW[c] = 0.0; FLWU[c] = 0.0; FLWV[c] = 0.0; FLWW[c] = 0.0;
+    continue;
+  }
+  const long long xp = I < NI ? c + 1 : c, yp = J < NJ ? c + sj : c, zp = K < NK ? c + sk : c;
+  {
+    const double u0 = ld_now(UU + c), ux = ld_now(UU + xp), uy = ld_now(UU + c - sj), uz = ld_now(UU + c - sk),
+                 v0 = ld_now(VV + c), vx = ld_now(VV + c - 1), w0 = ld_now(WW + c), wx = ld_now(WW + c - 1),
+                 lx0 = ld_now(f.glx + c), lxx = ld_now(f.glx + xp), ly0 = ld_now(f.gly + c),
+                 lyx = ld_now(f.gly + c - 1), lz0 = ld_now(f.glz + c), lzx = ld_now(f.glz + c - 1),
+                 gx0 = ld_now(f.ggx + c), gxx = ld_now(f.ggx + xp), gy0 = ld_now(f.ggy + c),
+                 gyx = ld_now(f.ggy + c - 1), gz0 = ld_now(f.ggz + c), gzx = ld_now(f.ggz + c - 1),
+                 an0 = ld_now(ANU + c), anx = ld_now(ANU + c - 1), any = ld_now(ANU + c - sj),
+                 anz = ld_now(ANU + c - sk), anxy = ld_now(ANU + c - 1 - sj), anxz = ld_now(ANU + c - 1 - sk);
   // ---------------- FLUU (Gx*u)*u, Gx*Nu*2du/dx   vf_vflxdu.f:71-91
   {
     double F = 0.0;
-    if (K >= 2 && K <= NK - 1 && J >= 2 && J <= NJ - 1 && I >= 2 && I <= NI - 1 && f.indc[c] != -1) {
-      double WIN = (A(f.glx, I, J, K) * A(UU, I, J, K) + A(f.glx, I + 1, J, K) * A(UU, I + 1, J, K)) * 0.5;
-      double FG = WIN * (A(UU, I, J, K) + A(UU, I + 1, J, K)) * 0.5;
-      F = F - SU * (dmax(WIN, 0.0) * A(UU, I, J, K) - dmax(-WIN, 0.0) * A(UU, I + 1, J, K)) - SC * FG;
-      F = F + (A(f.ggx, I, J, K) + A(f.ggx, I + 1, J, K)) * A(ANU, I, J, K) * XX_(4, I) *
-                  (A(UU, I + 1, J, K) - A(UU, I, J, K));
+    if (dd) {
+      double WIN = (lx0 * u0 + lxx * ux) * 0.5;
+      double FG = WIN * (u0 + ux) * 0.5;
+      F = F - SU * (dmax(WIN, 0.0) * u0 - dmax(-WIN, 0.0) * ux) - SC * FG;
+      F = F + (gx0 + gxx) * an0 * XX_(4, I) *
+                  (ux - u0);
     }
     FLUU[c] = F;
   }
@@ -56,20 +95,20 @@ __global__ void __launch_bounds__(ROW_THREADS, 3) k_flux(Geo g, Fld f, Prm p, do
   {
     double F = 0.0;
     if (K >= 2 && J >= 2 && I >= 3 && I <= NI - 1) {
-      int IC = A(NF, I - 1, J - 1, K) * A(NF, I, J - 1, K) * A(NF, I - 1, J, K) * A(NF, I, J, K);
-      int IT = A(f.indx, I, J, K), IB = A(f.indx, I, J - 1, K);
+      const int IC = ICxy;
+      const int IT = ix0, IB = ixy;
       if (IC != 0 || (IT != 0 && IB != 0)) {
       } else if (IT == 0 && IB == 0) {
-        double WIN = XX_(6, I) * (XX_(2, I - 1) * A(f.gly, I, J, K) * A(VV, I, J, K) +
-                                  XX_(2, I) * A(f.gly, I - 1, J, K) * A(VV, I - 1, J, K));
-        double FG = WIN * YY_(6, J) * (YY_(2, J - 1) * A(UU, I, J, K) + YY_(2, J) * A(UU, I, J - 1, K));
-        F = F - SU * (dmax(WIN, 0.0) * A(UU, I, J - 1, K) - dmax(-WIN, 0.0) * A(UU, I, J, K)) - SC * FG;
-        double GG = XX_(6, I) * (XX_(2, I - 1) * A(f.ggy, I, J, K) + XX_(2, I) * A(f.ggy, I - 1, J, K));
-        double ANR = YY_(6, J) * (YY_(2, J - 1) * A(ANU, I, J, K) + YY_(2, J) * A(ANU, I, J - 1, K));
-        double ANL = YY_(6, J) * (YY_(2, J - 1) * A(ANU, I - 1, J, K) + YY_(2, J) * A(ANU, I - 1, J - 1, K));
+        double WIN = XX_(6, I) * (XX_(2, I - 1) * ly0 * v0 +
+                                  XX_(2, I) * lyx * vx);
+        double FG = WIN * YY_(6, J) * (YY_(2, J - 1) * u0 + YY_(2, J) * uy);
+        F = F - SU * (dmax(WIN, 0.0) * uy - dmax(-WIN, 0.0) * u0) - SC * FG;
+        double GG = XX_(6, I) * (XX_(2, I - 1) * gy0 + XX_(2, I) * gyx);
+        double ANR = YY_(6, J) * (YY_(2, J - 1) * an0 + YY_(2, J) * any);
+        double ANL = YY_(6, J) * (YY_(2, J - 1) * anx + YY_(2, J) * anxy);
         double AN = XX_(6, I) * (XX_(2, I - 1) * ANR + XX_(2, I) * ANL);
-        double D1 = YY_(5, J) * (A(UU, I, J, K) - A(UU, I, J - 1, K));
-        double D2 = XX_(5, I) * (A(VV, I, J, K) - A(VV, I - 1, J, K));
+        double D1 = YY_(5, J) * (u0 - uy);
+        double D2 = XX_(5, I) * (v0 - vx);
         F = F + GG * AN * (D1 + D2);
       } else {
         double BR, BL;
@@ -109,20 +148,20 @@ __global__ void __launch_bounds__(ROW_THREADS, 3) k_flux(Geo g, Fld f, Prm p, do
   {
     double F = 0.0;
     if (K >= 2 && J >= 2 && J <= NJ - 1 && I >= 3 && I <= NI - 1) {
-      int IC = A(NF, I - 1, J, K - 1) * A(NF, I, J, K - 1) * A(NF, I - 1, J, K) * A(NF, I, J, K);
-      int IT = A(f.indx, I, J, K), IB = A(f.indx, I, J, K - 1);
+      const int IC = ICxz;
+      const int IT = ix0, IB = ixz;
       if (IC != 0 || (IT != 0 && IB != 0)) {
       } else if (IT == 0 && IB == 0) {
-        double WIN = XX_(6, I) * (XX_(2, I - 1) * A(f.glz, I, J, K) * A(WW, I, J, K) +
-                                  XX_(2, I) * A(f.glz, I - 1, J, K) * A(WW, I - 1, J, K));
-        double FG = WIN * ZZ_(6, K) * (ZZ_(2, K - 1) * A(UU, I, J, K) + ZZ_(2, K) * A(UU, I, J, K - 1));
-        F = F - SU * (dmax(WIN, 0.0) * A(UU, I, J, K - 1) - dmax(-WIN, 0.0) * A(UU, I, J, K)) - SC * FG;
-        double GG = XX_(6, I) * (XX_(2, I - 1) * A(f.ggz, I, J, K) + XX_(2, I) * A(f.ggz, I - 1, J, K));
-        double ANR = ZZ_(6, K) * (ZZ_(2, K - 1) * A(ANU, I, J, K) + ZZ_(2, K) * A(ANU, I, J, K - 1));
-        double ANL = ZZ_(6, K) * (ZZ_(2, K - 1) * A(ANU, I - 1, J, K) + ZZ_(2, K) * A(ANU, I - 1, J, K - 1));
+        double WIN = XX_(6, I) * (XX_(2, I - 1) * lz0 * w0 +
+                                  XX_(2, I) * lzx * wx);
+        double FG = WIN * ZZ_(6, K) * (ZZ_(2, K - 1) * u0 + ZZ_(2, K) * uz);
+        F = F - SU * (dmax(WIN, 0.0) * uz - dmax(-WIN, 0.0) * u0) - SC * FG;
+        double GG = XX_(6, I) * (XX_(2, I - 1) * gz0 + XX_(2, I) * gzx);
+        double ANR = ZZ_(6, K) * (ZZ_(2, K - 1) * an0 + ZZ_(2, K) * anz);
+        double ANL = ZZ_(6, K) * (ZZ_(2, K - 1) * anx + ZZ_(2, K) * anxz);
         double AN = XX_(6, I) * (XX_(2, I - 1) * ANR + XX_(2, I) * ANL);
-        double D1 = ZZ_(5, K) * (A(UU, I, J, K) - A(UU, I, J, K - 1));
-        double D2 = XX_(5, I) * (A(WW, I, J, K) - A(WW, I - 1, J, K));
+        double D1 = ZZ_(5, K) * (u0 - uz);
+        double D2 = XX_(5, I) * (w0 - wx);
         F = F + GG * AN * (D1 + D2);
       } else {
         double BR, BL;
@@ -158,15 +197,25 @@ __global__ void __launch_bounds__(ROW_THREADS, 3) k_flux(Geo g, Fld f, Prm p, do
     }
     FLUW[c] = F;
   }
+  }
+  {
+    const double v0 = ld_now(VV + c), vx = ld_now(VV + c - 1), vy = ld_now(VV + yp), vz = ld_now(VV + c - sk),
+                 u0 = ld_now(UU + c), uy = ld_now(UU + c - sj), w0 = ld_now(WW + c), wy = ld_now(WW + c - sj),
+                 ly0 = ld_now(f.gly + c), lyy = ld_now(f.gly + yp), lx0 = ld_now(f.glx + c),
+                 lxy = ld_now(f.glx + c - sj), lz0 = ld_now(f.glz + c), lzy = ld_now(f.glz + c - sj),
+                 gy0 = ld_now(f.ggy + c), gyy = ld_now(f.ggy + yp), gx0 = ld_now(f.ggx + c),
+                 gxy = ld_now(f.ggx + c - sj), gz0 = ld_now(f.ggz + c), gzy = ld_now(f.ggz + c - sj),
+                 an0 = ld_now(ANU + c), anx = ld_now(ANU + c - 1), any = ld_now(ANU + c - sj),
+                 anz = ld_now(ANU + c - sk), anxy = ld_now(ANU + c - 1 - sj), anyz = ld_now(ANU + c - sj - sk);
   // ---------------- FLVV (Gy*v)*v   vf_vflxdv.f:71-91
   {
     double F = 0.0;
-    if (K >= 2 && K <= NK - 1 && J >= 2 && J <= NJ - 1 && I >= 2 && I <= NI - 1 && f.indc[c] != -1) {
-      double WIN = (A(f.gly, I, J, K) * A(VV, I, J, K) + A(f.gly, I, J + 1, K) * A(VV, I, J + 1, K)) * 0.5;
-      double FG = WIN * (A(VV, I, J, K) + A(VV, I, J + 1, K)) * 0.5;
-      F = F - SU * (dmax(WIN, 0.0) * A(VV, I, J, K) - dmax(-WIN, 0.0) * A(VV, I, J + 1, K)) - SC * FG;
-      F = F + (A(f.ggy, I, J, K) + A(f.ggy, I, J + 1, K)) * A(ANU, I, J, K) * YY_(4, J) *
-                  (A(VV, I, J + 1, K) - A(VV, I, J, K));
+    if (dd) {
+      double WIN = (ly0 * v0 + lyy * vy) * 0.5;
+      double FG = WIN * (v0 + vy) * 0.5;
+      F = F - SU * (dmax(WIN, 0.0) * v0 - dmax(-WIN, 0.0) * vy) - SC * FG;
+      F = F + (gy0 + gyy) * an0 * YY_(4, J) *
+                  (vy - v0);
     }
     FLVV[c] = F;
   }
@@ -174,20 +223,20 @@ __global__ void __launch_bounds__(ROW_THREADS, 3) k_flux(Geo g, Fld f, Prm p, do
   {
     double F = 0.0;
     if (K >= 2 && J >= 3 && J <= NJ - 1 && I >= 2) {
-      int IC = A(NF, I - 1, J - 1, K) * A(NF, I - 1, J, K) * A(NF, I, J - 1, K) * A(NF, I, J, K);
-      int IT = A(f.indy, I, J, K), IB = A(f.indy, I - 1, J, K);
+      const int IC = ICxy;
+      const int IT = iy0, IB = iyx;
       if (IC != 0 || (IT != 0 && IB != 0)) {
       } else if (IT == 0 && IB == 0) {
-        double WIN = YY_(6, J) * (YY_(2, J - 1) * A(f.glx, I, J, K) * A(UU, I, J, K) +
-                                  YY_(2, J) * A(f.glx, I, J - 1, K) * A(UU, I, J - 1, K));
-        double FG = WIN * XX_(6, I) * (XX_(2, I - 1) * A(VV, I, J, K) + XX_(2, I) * A(VV, I - 1, J, K));
-        F = F - SU * (dmax(WIN, 0.0) * A(VV, I - 1, J, K) - dmax(-WIN, 0.0) * A(VV, I, J, K)) - SC * FG;
-        double GG = YY_(6, J) * (YY_(2, J - 1) * A(f.ggx, I, J, K) + YY_(2, J) * A(f.ggx, I, J - 1, K));
-        double ANR = XX_(6, I) * (XX_(2, I - 1) * A(ANU, I, J, K) + XX_(2, I) * A(ANU, I - 1, J, K));
-        double ANL = XX_(6, I) * (XX_(2, I - 1) * A(ANU, I, J - 1, K) + XX_(2, I) * A(ANU, I - 1, J - 1, K));
+        double WIN = YY_(6, J) * (YY_(2, J - 1) * lx0 * u0 +
+                                  YY_(2, J) * lxy * uy);
+        double FG = WIN * XX_(6, I) * (XX_(2, I - 1) * v0 + XX_(2, I) * vx);
+        F = F - SU * (dmax(WIN, 0.0) * vx - dmax(-WIN, 0.0) * v0) - SC * FG;
+        double GG = YY_(6, J) * (YY_(2, J - 1) * gx0 + YY_(2, J) * gxy);
+        double ANR = XX_(6, I) * (XX_(2, I - 1) * an0 + XX_(2, I) * anx);
+        double ANL = XX_(6, I) * (XX_(2, I - 1) * any + XX_(2, I) * anxy);
         double AN = YY_(6, J) * (YY_(2, J - 1) * ANR + YY_(2, J) * ANL);
-        double D1 = XX_(5, I) * (A(VV, I, J, K) - A(VV, I - 1, J, K));
-        double D2 = YY_(5, J) * (A(UU, I, J, K) - A(UU, I, J - 1, K));
+        double D1 = XX_(5, I) * (v0 - vx);
+        double D2 = YY_(5, J) * (u0 - uy);
         F = F + GG * AN * (D1 + D2);
       } else {
         double BR, BL;
@@ -227,20 +276,20 @@ __global__ void __launch_bounds__(ROW_THREADS, 3) k_flux(Geo g, Fld f, Prm p, do
   {
     double F = 0.0;
     if (K >= 2 && J >= 3 && J <= NJ - 1 && I >= 2 && I <= NI - 1) {
-      int IC = A(NF, I, J - 1, K - 1) * A(NF, I, J, K - 1) * A(NF, I, J - 1, K) * A(NF, I, J, K);
-      int IT = A(f.indy, I, J, K), IB = A(f.indy, I, J, K - 1);
+      const int IC = ICyz;
+      const int IT = iy0, IB = iyz;
       if (IC != 0 || (IT != 0 && IB != 0)) {
       } else if (IT == 0 && IB == 0) {
-        double WIN = YY_(6, J) * (YY_(2, J - 1) * A(f.glz, I, J, K) * A(WW, I, J, K) +
-                                  YY_(2, J) * A(f.glz, I, J - 1, K) * A(WW, I, J - 1, K));
-        double FG = WIN * ZZ_(6, K) * (ZZ_(2, K - 1) * A(VV, I, J, K) + ZZ_(2, K) * A(VV, I, J, K - 1));
-        F = F - SU * (dmax(WIN, 0.0) * A(VV, I, J, K - 1) - dmax(-WIN, 0.0) * A(VV, I, J, K)) - SC * FG;
-        double GG = YY_(6, J) * (YY_(2, J - 1) * A(f.ggz, I, J, K) + YY_(2, J) * A(f.ggz, I, J - 1, K));
-        double ANR = ZZ_(6, K) * (ZZ_(2, K - 1) * A(ANU, I, J, K) + ZZ_(2, K) * A(ANU, I, J, K - 1));
-        double ANL = ZZ_(6, K) * (ZZ_(2, K - 1) * A(ANU, I, J - 1, K) + ZZ_(2, K) * A(ANU, I, J - 1, K - 1));
+        double WIN = YY_(6, J) * (YY_(2, J - 1) * lz0 * w0 +
+                                  YY_(2, J) * lzy * wy);
+        double FG = WIN * ZZ_(6, K) * (ZZ_(2, K - 1) * v0 + ZZ_(2, K) * vz);
+        F = F - SU * (dmax(WIN, 0.0) * vz - dmax(-WIN, 0.0) * v0) - SC * FG;
+        double GG = YY_(6, J) * (YY_(2, J - 1) * gz0 + YY_(2, J) * gzy);
+        double ANR = ZZ_(6, K) * (ZZ_(2, K - 1) * an0 + ZZ_(2, K) * anz);
+        double ANL = ZZ_(6, K) * (ZZ_(2, K - 1) * any + ZZ_(2, K) * anyz);
         double AN = YY_(6, J) * (YY_(2, J - 1) * ANR + YY_(2, J) * ANL);
-        double D1 = ZZ_(5, K) * (A(VV, I, J, K) - A(VV, I, J, K - 1));
-        double D2 = YY_(5, J) * (A(WW, I, J, K) - A(WW, I, J - 1, K));
+        double D1 = ZZ_(5, K) * (v0 - vz);
+        double D2 = YY_(5, J) * (w0 - wy);
         F = F + GG * AN * (D1 + D2);
       } else {
         double BR, BL;
@@ -276,15 +325,25 @@ __global__ void __launch_bounds__(ROW_THREADS, 3) k_flux(Geo g, Fld f, Prm p, do
     }
     FLVW[c] = F;
   }
+  }
+  {
+    const double w0 = ld_now(WW + c), wx = ld_now(WW + c - 1), wy = ld_now(WW + c - sj), wz = ld_now(WW + zp),
+                 u0 = ld_now(UU + c), uz = ld_now(UU + c - sk), v0 = ld_now(VV + c), vz = ld_now(VV + c - sk),
+                 lz0 = ld_now(f.glz + c), lzz = ld_now(f.glz + zp), lx0 = ld_now(f.glx + c),
+                 lxz = ld_now(f.glx + c - sk), ly0 = ld_now(f.gly + c), lyz = ld_now(f.gly + c - sk),
+                 gz0 = ld_now(f.ggz + c), gzz = ld_now(f.ggz + zp), gx0 = ld_now(f.ggx + c),
+                 gxz = ld_now(f.ggx + c - sk), gy0 = ld_now(f.ggy + c), gyz = ld_now(f.ggy + c - sk),
+                 an0 = ld_now(ANU + c), anx = ld_now(ANU + c - 1), any = ld_now(ANU + c - sj),
+                 anz = ld_now(ANU + c - sk), anxz = ld_now(ANU + c - 1 - sk), anyz = ld_now(ANU + c - sj - sk);
   // ---------------- FLWW (Gz*w)*w   vf_vflxdw.f:62-82
   {
     double F = 0.0;
-    if (K >= 2 && K <= NK - 1 && J >= 2 && J <= NJ - 1 && I >= 2 && I <= NI - 1 && f.indc[c] != -1) {
-      double WIN = (A(f.glz, I, J, K) * A(WW, I, J, K) + A(f.glz, I, J, K + 1) * A(WW, I, J, K + 1)) * 0.5;
-      double FG = WIN * (A(WW, I, J, K) + A(WW, I, J, K + 1)) * 0.5;
-      F = F - SU * (dmax(WIN, 0.0) * A(WW, I, J, K) - dmax(-WIN, 0.0) * A(WW, I, J, K + 1)) - SC * FG;
-      F = F + (A(f.ggz, I, J, K) + A(f.ggz, I, J, K + 1)) * A(ANU, I, J, K) * ZZ_(4, K) *
-                  (A(WW, I, J, K + 1) - A(WW, I, J, K));
+    if (dd) {
+      double WIN = (lz0 * w0 + lzz * wz) * 0.5;
+      double FG = WIN * (w0 + wz) * 0.5;
+      F = F - SU * (dmax(WIN, 0.0) * w0 - dmax(-WIN, 0.0) * wz) - SC * FG;
+      F = F + (gz0 + gzz) * an0 * ZZ_(4, K) *
+                  (wz - w0);
     }
     FLWW[c] = F;
   }
@@ -292,20 +351,20 @@ __global__ void __launch_bounds__(ROW_THREADS, 3) k_flux(Geo g, Fld f, Prm p, do
   {
     double F = 0.0;
     if (K >= 3 && K <= NK - 1 && J >= 2 && J <= NJ - 1 && I >= 2) {
-      int IC = A(NF, I - 1, J, K - 1) * A(NF, I - 1, J, K) * A(NF, I, J, K - 1) * A(NF, I, J, K);
-      int IT = A(f.indz, I, J, K), IB = A(f.indz, I - 1, J, K);
+      const int IC = ICxz;
+      const int IT = iz0, IB = izx;
       if (IC != 0 || (IT != 0 && IB != 0)) {
       } else if (IT == 0 && IB == 0) {
-        double WIN = ZZ_(6, K) * (ZZ_(2, K - 1) * A(f.glx, I, J, K) * A(UU, I, J, K) +
-                                  ZZ_(2, K) * A(f.glx, I, J, K - 1) * A(UU, I, J, K - 1));
-        double FG = WIN * XX_(6, I) * (XX_(2, I - 1) * A(WW, I, J, K) + XX_(2, I) * A(WW, I - 1, J, K));
-        F = F - SU * (dmax(WIN, 0.0) * A(WW, I - 1, J, K) - dmax(-WIN, 0.0) * A(WW, I, J, K)) - SC * FG;
-        double GG = ZZ_(6, K) * (ZZ_(2, K - 1) * A(f.ggx, I, J, K) + ZZ_(2, K) * A(f.ggx, I, J, K - 1));
-        double ANR = XX_(6, I) * (XX_(2, I - 1) * A(ANU, I, J, K) + XX_(2, I) * A(ANU, I - 1, J, K));
-        double ANL = XX_(6, I) * (XX_(2, I - 1) * A(ANU, I, J, K - 1) + XX_(2, I) * A(ANU, I - 1, J, K - 1));
+        double WIN = ZZ_(6, K) * (ZZ_(2, K - 1) * lx0 * u0 +
+                                  ZZ_(2, K) * lxz * uz);
+        double FG = WIN * XX_(6, I) * (XX_(2, I - 1) * w0 + XX_(2, I) * wx);
+        F = F - SU * (dmax(WIN, 0.0) * wx - dmax(-WIN, 0.0) * w0) - SC * FG;
+        double GG = ZZ_(6, K) * (ZZ_(2, K - 1) * gx0 + ZZ_(2, K) * gxz);
+        double ANR = XX_(6, I) * (XX_(2, I - 1) * an0 + XX_(2, I) * anx);
+        double ANL = XX_(6, I) * (XX_(2, I - 1) * anz + XX_(2, I) * anxz);
         double AN = ZZ_(6, K) * (ZZ_(2, K - 1) * ANR + ZZ_(2, K) * ANL);
-        double D1 = XX_(5, I) * (A(WW, I, J, K) - A(WW, I - 1, J, K));
-        double D2 = ZZ_(5, K) * (A(UU, I, J, K) - A(UU, I, J, K - 1));
+        double D1 = XX_(5, I) * (w0 - wx);
+        double D2 = ZZ_(5, K) * (u0 - uz);
         F = F + GG * AN * (D1 + D2);
       } else {
         double BR, BL;
@@ -345,20 +404,20 @@ __global__ void __launch_bounds__(ROW_THREADS, 3) k_flux(Geo g, Fld f, Prm p, do
   {
     double F = 0.0;
     if (K >= 3 && K <= NK - 1 && J >= 2 && I >= 2 && I <= NI - 1) {
-      int IC = A(NF, I, J - 1, K - 1) * A(NF, I, J - 1, K) * A(NF, I, J, K - 1) * A(NF, I, J, K);
-      int IT = A(f.indz, I, J, K), IB = A(f.indz, I, J - 1, K);
+      const int IC = ICyz;
+      const int IT = iz0, IB = izy;
       if (IC != 0 || (IT != 0 && IB != 0)) {
       } else if (IT == 0 && IB == 0) {
-        double WIN = ZZ_(6, K) * (ZZ_(2, K - 1) * A(f.gly, I, J, K) * A(VV, I, J, K) +
-                                  ZZ_(2, K) * A(f.gly, I, J, K - 1) * A(VV, I, J, K - 1));
-        double FG = WIN * YY_(6, J) * (YY_(2, J - 1) * A(WW, I, J, K) + YY_(2, J) * A(WW, I, J - 1, K));
-        F = F - SU * (dmax(WIN, 0.0) * A(WW, I, J - 1, K) - dmax(-WIN, 0.0) * A(WW, I, J, K)) - SC * FG;
-        double GG = ZZ_(6, K) * (ZZ_(2, K - 1) * A(f.ggy, I, J, K) + ZZ_(2, K) * A(f.ggy, I, J, K - 1));
-        double ANR = YY_(6, J) * (YY_(2, J - 1) * A(ANU, I, J, K) + YY_(2, J) * A(ANU, I, J - 1, K));
-        double ANL = YY_(6, J) * (YY_(2, J - 1) * A(ANU, I, J, K - 1) + YY_(2, J) * A(ANU, I, J - 1, K - 1));
+        double WIN = ZZ_(6, K) * (ZZ_(2, K - 1) * ly0 * v0 +
+                                  ZZ_(2, K) * lyz * vz);
+        double FG = WIN * YY_(6, J) * (YY_(2, J - 1) * w0 + YY_(2, J) * wy);
+        F = F - SU * (dmax(WIN, 0.0) * wy - dmax(-WIN, 0.0) * w0) - SC * FG;
+        double GG = ZZ_(6, K) * (ZZ_(2, K - 1) * gy0 + ZZ_(2, K) * gyz);
+        double ANR = YY_(6, J) * (YY_(2, J - 1) * an0 + YY_(2, J) * any);
+        double ANL = YY_(6, J) * (YY_(2, J - 1) * anz + YY_(2, J) * anyz);
         double AN = ZZ_(6, K) * (ZZ_(2, K - 1) * ANR + ZZ_(2, K) * ANL);
-        double D1 = YY_(5, J) * (A(WW, I, J, K) - A(WW, I, J - 1, K));
-        double D2 = ZZ_(5, K) * (A(VV, I, J, K) - A(VV, I, J, K - 1));
+        double D1 = YY_(5, J) * (w0 - wy);
+        double D2 = ZZ_(5, K) * (v0 - vz);
         F = F + GG * AN * (D1 + D2);
       } else {
         double BR, BL;
@@ -394,11 +453,12 @@ __global__ void __launch_bounds__(ROW_THREADS, 3) k_flux(Geo g, Fld f, Prm p, do
     }
     FLWV[c] = F;
   }
+  }
 #undef A
 #undef XX_
 #undef YY_
 #undef ZZ_
-  ROW_LOOP_END
+  CELL_LOOP_END
 }
 
 // ----------------------------------------------------- sources + update
@@ -412,7 +472,7 @@ __device__ __forceinline__ double sponge_dmax(const Prm &p, double X, double Y, 
   return DMAX;
 }
 
-__global__ void __launch_bounds__(ROW_THREADS, 3) k_predict(Geo g, Fld f, Prm p, const double *FLUU, const double *FLUV,
+__global__ void __launch_bounds__(CELL_THREADS, 8) k_predict(Geo g, Fld f, Prm p, const double *FLUU, const double *FLUV,
                           const double *FLUW, const double *FLVU, const double *FLVV,
                           const double *FLVW, const double *FLWU, const double *FLWV,
                           const double *FLWW, double *UN, double *VN, double *WN) {
@@ -420,48 +480,65 @@ __global__ void __launch_bounds__(ROW_THREADS, 3) k_predict(Geo g, Fld f, Prm p,
                *CD0 = f.cd0;
   const int *NF = f.nf;
   const double RI = 1.0 / p.rho0, DT = p.dtnow, VM = p.vvmax;
-  ROW_LOOP_BEGIN(g)
+  CELL_LOOP_BEGIN(g)
   const long long c = cid(g, I, J, K);
   const int NI = g.NI, NJ = g.NJ, NK = g.NK;
 #define A(a, i, j, k) a[cid(g, i, j, k)]
-#define XX_(m, i) gx(g, m, i)
-#define YY_(m, j) gy(g, m, j)
-#define ZZ_(m, k) gz(g, m, k)
+// (plain loads of the metrics: 452 us, read-only ones 10 % more)
+#define XX_(m, i) g.XX[(m) - 1 + 6 * ((i) - 1)]
+#define YY_(m, j) g.YY[(m) - 1 + 6 * ((j) - 1)]
+#define ZZ_(m, k) g.ZZ[(m) - 1 + 6 * ((k) - 1)]
+  const long long sj = NI, sk = (long long)NI * NJ;
+  const double u0 = ld_now(UU + c), v0 = ld_now(VV + c), w0 = ld_now(WW + c);
+  const bool inner = K >= 2 && K <= NK - 1 && J >= 2 && J <= NJ - 1 && I >= 2 && I <= NI - 1;
+  if (!inner) { UN[c] = u0; VN[c] = v0; WN[c] = w0; continue; }
+  const int n0 = ld_now(NF + c), nx = ld_now(NF + c - 1), ny = ld_now(NF + c - sj), nz = ld_now(NF + c - sk),
+            ix = ld_now(f.indx + c), iy = ld_now(f.indy + c), iz = ld_now(f.indz + c);
+  const bool dox = I >= 3 && ix == 0 && nx * n0 == 0, doy = J >= 3 && iy == 0 && ny * n0 == 0,
+             doz = K >= 3 && iz == 0 && nz * n0 == 0;
+  if (!dox && !doy && !doz) { UN[c] = u0; VN[c] = v0; WN[c] = w0; continue; }
+  const double gv0 = ld_now(GGV + c), cd0 = ld_now(CD0 + c), gl0 = ld_now(GLV + c), p0 = ld_now(PP + c);
   // ------------------------------------------------ x velocity
   {
-    double U = UU[c];
-    if (K >= 2 && K <= NK - 1 && J >= 2 && J <= NJ - 1 && I >= 3 && I <= NI - 1 &&
-        f.indx[c] == 0 && A(NF, I - 1, J, K) * A(NF, I, J, K) == 0) {
+    double U = u0;
+    if (dox) {
+      const long long m = c - 1;
+      const double gv1 = ld_now(GGV + m), cd1 = ld_now(CD0 + m), gl1 = ld_now(GLV + m), p1 = ld_now(PP + m);
+      const double a0 = v0, a1 = ld_now(VV + c + sj), a2 = ld_now(VV + m), a3 = ld_now(VV + m + sj);
+      const double b0 = w0, b1 = ld_now(WW + c + sk), b2 = ld_now(WW + m), b3 = ld_now(WW + m + sk);
+      const double gg = ld_now(f.ggx + c);
+      const double f0 = ld_now(FLUU + c), f1 = ld_now(FLUU + m), f2 = ld_now(FLUV + c), f3 = ld_now(FLUV + c + sj),
+                   f4 = ld_now(FLUW + c), f5 = ld_now(FLUW + c + sk);
       const int I1 = I - 1;
       // VF_VGENE vf_vgene.f:94-110
-      double GVg = XX_(6, I) * (XX_(2, I) * GGV[c] + XX_(2, I1) * A(GGV, I1, J, K));
-      double CD = XX_(6, I) * (XX_(2, I) * CD0[c] + XX_(2, I1) * A(CD0, I1, J, K));
+      double GVg = XX_(6, I) * (XX_(2, I) * gv0 + XX_(2, I1) * gv1);
+      double CD = XX_(6, I) * (XX_(2, I) * cd0 + XX_(2, I1) * cd1);
       double Q = 0.0;
-      Q = Q + GVg * RI * XX_(5, I) * (A(PP, I1, J, K) - PP[c]);
-      double Uc = UU[c];
-      double V = XX_(6, I) * (XX_(2, I1) * (A(VV, I, J, K) + A(VV, I, J + 1, K)) +
-                              XX_(2, I) * (A(VV, I1, J, K) + A(VV, I1, J + 1, K))) * 0.5;
-      double W = XX_(6, I) * (XX_(2, I1) * (A(WW, I, J, K) + A(WW, I, J, K + 1)) +
-                              XX_(2, I) * (A(WW, I1, J, K) + A(WW, I1, J, K + 1))) * 0.5;
+      Q = Q + GVg * RI * XX_(5, I) * (p1 - p0);
+      double Uc = u0;
+      double V = XX_(6, I) * (XX_(2, I1) * (a0 + a1) +
+                              XX_(2, I) * (a2 + a3)) * 0.5;
+      double W = XX_(6, I) * (XX_(2, I1) * (b0 + b1) +
+                              XX_(2, I) * (b2 + b3)) * 0.5;
       double UVW = sqrt(Uc * Uc + V * V + W * W);
-      Q = Q - 0.5 * CD * XX_(5, I) * (1.0 - f.ggx[c]) * Uc * UVW;
+      Q = Q - 0.5 * CD * XX_(5, I) * (1.0 - gg) * Uc * UVW;
       // wave source of an x line (vf_vgene.f:149-152)
       if (p.iws != 0 && (p.iws == I || p.iws + 1 == I)) {
         const double QS = 2.0 * XX_(4, p.iws) * f.srcuv[(J - 1) + (long long)NJ * (K - 1)];
-        Q = Q + UU[c] * QS * XX_(2, p.iws) * XX_(5, I) * 0.5;
+        Q = Q + u0 * QS * XX_(2, p.iws) * XX_(5, I) * 0.5;
       }
       // VF_VEULER vf_veuler.f:119-128
-      double GV = XX_(6, I) * (XX_(2, I) * GLV[c] + XX_(2, I - 1) * A(GLV, I - 1, J, K));
-      double GV0 = XX_(6, I) * (XX_(2, I) * GLV[c] + XX_(2, I - 1) * A(GLV, I - 1, J, K));
-      double DU = (XX_(5, I) * (FLUU[c] - A(FLUU, I - 1, J, K)) + YY_(4, J) * (A(FLUV, I, J + 1, K) - FLUV[c]) +
-                   ZZ_(4, K) * (A(FLUW, I, J, K + 1) - FLUW[c]) + Q);
+      double GV = XX_(6, I) * (XX_(2, I) * gl0 + XX_(2, I - 1) * gl1);
+      double GV0 = XX_(6, I) * (XX_(2, I) * gl0 + XX_(2, I - 1) * gl1);
+      double DU = (XX_(5, I) * (f0 - f1) + YY_(4, J) * (f3 - f2) +
+                   ZZ_(4, K) * (f5 - f4) + Q);
       U = (GV * U + DT * DU) / GV0;
       if (U > VM) U = VM;
       if (U < -VM) U = -VM;
       if (p.ipa != 0) {
         double X = XX_(1, I), Y = (YY_(1, J) + YY_(1, J + 1)) * 0.5;
         double DMAX = sponge_dmax(p, X, Y, false);
-        double G = XX_(6, I) * (XX_(2, I) * GGV[c] + XX_(2, I - 1) * A(GGV, I - 1, J, K));
+        double G = XX_(6, I) * (XX_(2, I) * gv0 + XX_(2, I - 1) * gv1);
         double D = GV0 / (GV0 + DT * G * DMAX);
         U = U * D;
       }
@@ -470,37 +547,43 @@ __global__ void __launch_bounds__(ROW_THREADS, 3) k_predict(Geo g, Fld f, Prm p,
   }
   // ------------------------------------------------ y velocity
   {
-    double V = VV[c];
-    if (K >= 2 && K <= NK - 1 && J >= 3 && J <= NJ - 1 && I >= 2 && I <= NI - 1 &&
-        f.indy[c] == 0 && A(NF, I, J - 1, K) * A(NF, I, J, K) == 0) {
+    double V = v0;
+    if (doy) {
+      const long long m = c - sj;
+      const double gv1 = ld_now(GGV + m), cd1 = ld_now(CD0 + m), gl1 = ld_now(GLV + m), p1 = ld_now(PP + m);
+      const double a0 = u0, a1 = ld_now(UU + c + 1), a2 = ld_now(UU + m), a3 = ld_now(UU + m + 1);
+      const double b0 = w0, b1 = ld_now(WW + c + sk), b2 = ld_now(WW + m), b3 = ld_now(WW + m + sk);
+      const double gg = ld_now(f.ggy + c);
+      const double f0 = ld_now(FLVU + c), f1 = ld_now(FLVU + c + 1), f2 = ld_now(FLVV + c), f3 = ld_now(FLVV + m),
+                   f4 = ld_now(FLVW + c), f5 = ld_now(FLVW + c + sk);
       const int J1 = J - 1;
-      double GVg = YY_(6, J) * (YY_(2, J) * GGV[c] + YY_(2, J1) * A(GGV, I, J1, K));
-      double CD = YY_(6, J) * (YY_(2, J) * CD0[c] + YY_(2, J1) * A(CD0, I, J1, K));
+      double GVg = YY_(6, J) * (YY_(2, J) * gv0 + YY_(2, J1) * gv1);
+      double CD = YY_(6, J) * (YY_(2, J) * cd0 + YY_(2, J1) * cd1);
       double Q = 0.0;
-      Q = Q + GVg * RI * YY_(5, J) * (A(PP, I, J1, K) - PP[c]);
-      double U = YY_(6, J) * (YY_(2, J1) * (A(UU, I, J, K) + A(UU, I + 1, J, K)) +
-                              YY_(2, J) * (A(UU, I, J1, K) + A(UU, I + 1, J1, K))) * 0.5;
-      double Vc = VV[c];
-      double W = YY_(6, J) * (YY_(2, J1) * (A(WW, I, J, K) + A(WW, I, J, K + 1)) +
-                              YY_(2, J) * (A(WW, I, J1, K) + A(WW, I, J1, K + 1))) * 0.5;
+      Q = Q + GVg * RI * YY_(5, J) * (p1 - p0);
+      double U = YY_(6, J) * (YY_(2, J1) * (a0 + a1) +
+                              YY_(2, J) * (a2 + a3)) * 0.5;
+      double Vc = v0;
+      double W = YY_(6, J) * (YY_(2, J1) * (b0 + b1) +
+                              YY_(2, J) * (b2 + b3)) * 0.5;
       double UVW = sqrt(U * U + Vc * Vc + W * W);
-      Q = Q - 0.5 * CD * YY_(5, J) * (1.0 - f.ggy[c]) * Vc * UVW;
+      Q = Q - 0.5 * CD * YY_(5, J) * (1.0 - gg) * Vc * UVW;
       // wave source of a y line (vf_vgene.f:225-228)
       if (p.jws != 0 && (p.jws == J || p.jws + 1 == J)) {
         const double QS = 2.0 * YY_(4, p.jws) * f.srcuv[(I - 1) + (long long)NI * (K - 1)];
-        Q = Q + VV[c] * QS * YY_(2, p.jws) * YY_(5, J) * 0.5;
+        Q = Q + v0 * QS * YY_(2, p.jws) * YY_(5, J) * 0.5;
       }
-      double GV = YY_(6, J) * (YY_(2, J) * GLV[c] + YY_(2, J - 1) * A(GLV, I, J - 1, K));
-      double GV0 = YY_(6, J) * (YY_(2, J) * GLV[c] + YY_(2, J - 1) * A(GLV, I, J - 1, K));
-      double DV = (XX_(4, I) * (A(FLVU, I + 1, J, K) - FLVU[c]) + YY_(5, J) * (FLVV[c] - A(FLVV, I, J - 1, K)) +
-                   ZZ_(4, K) * (A(FLVW, I, J, K + 1) - FLVW[c]) + Q);
+      double GV = YY_(6, J) * (YY_(2, J) * gl0 + YY_(2, J - 1) * gl1);
+      double GV0 = YY_(6, J) * (YY_(2, J) * gl0 + YY_(2, J - 1) * gl1);
+      double DV = (XX_(4, I) * (f1 - f0) + YY_(5, J) * (f2 - f3) +
+                   ZZ_(4, K) * (f5 - f4) + Q);
       V = (GV * V + DT * DV) / GV0;
       if (V > VM) V = VM;
       if (V < -VM) V = -VM;
       if (p.ipa != 0) {
         double X = (XX_(1, I) + XX_(1, I + 1)) * 0.5, Y = YY_(1, J);
         double DMAX = sponge_dmax(p, X, Y, false);
-        double G = YY_(6, J) * (YY_(2, J) * GGV[c] + YY_(2, J - 1) * A(GGV, I, J - 1, K));
+        double G = YY_(6, J) * (YY_(2, J) * gv0 + YY_(2, J - 1) * gv1);
         double D = GV0 / (GV0 + DT * G * DMAX);
         V = V * D;
       }
@@ -509,48 +592,54 @@ __global__ void __launch_bounds__(ROW_THREADS, 3) k_predict(Geo g, Fld f, Prm p,
   }
   // ------------------------------------------------ z velocity
   {
-    double W = WW[c];
-    if (K >= 3 && K <= NK - 1 && J >= 2 && J <= NJ - 1 && I >= 2 && I <= NI - 1 &&
-        f.indz[c] == 0 && A(NF, I, J, K - 1) * A(NF, I, J, K) == 0) {
+    double W = w0;
+    if (doz) {
+      const long long m = c - sk;
+      const double gv1 = ld_now(GGV + m), cd1 = ld_now(CD0 + m), gl1 = ld_now(GLV + m), p1 = ld_now(PP + m);
+      const double a0 = u0, a1 = ld_now(UU + c + 1), a2 = ld_now(UU + m), a3 = ld_now(UU + m + 1);
+      const double b0 = v0, b1 = ld_now(VV + c + sj), b2 = ld_now(VV + m), b3 = ld_now(VV + m + sj);
+      const double gg = ld_now(f.ggz + c);
+      const double f0 = ld_now(FLWU + c), f1 = ld_now(FLWU + c + 1), f2 = ld_now(FLWV + c), f3 = ld_now(FLWV + c + sj),
+                   f4 = ld_now(FLWW + c), f5 = ld_now(FLWW + m);
       const int K1 = K - 1;
-      double GVg = ZZ_(6, K) * (ZZ_(2, K) * GGV[c] + ZZ_(2, K1) * A(GGV, I, J, K1));
-      double CD = ZZ_(6, K) * (ZZ_(2, K) * CD0[c] + ZZ_(2, K1) * A(CD0, I, J, K1));
+      double GVg = ZZ_(6, K) * (ZZ_(2, K) * gv0 + ZZ_(2, K1) * gv1);
+      double CD = ZZ_(6, K) * (ZZ_(2, K) * cd0 + ZZ_(2, K1) * cd1);
       double Q = 0.0;
-      Q = Q + GVg * RI * ZZ_(5, K) * (A(PP, I, J, K1) - PP[c]);
-      double U = ZZ_(6, K) * (ZZ_(2, K1) * (A(UU, I, J, K) + A(UU, I + 1, J, K)) +
-                              ZZ_(2, K) * (A(UU, I, J, K1) + A(UU, I + 1, J, K1))) * 0.5;
-      double V = ZZ_(6, K) * (ZZ_(2, K1) * (A(VV, I, J, K) + A(VV, I, J + 1, K)) +
-                              ZZ_(2, K) * (A(VV, I, J, K1) + A(VV, I, J + 1, K1))) * 0.5;
-      double Wc = WW[c];
+      Q = Q + GVg * RI * ZZ_(5, K) * (p1 - p0);
+      double U = ZZ_(6, K) * (ZZ_(2, K1) * (a0 + a1) +
+                              ZZ_(2, K) * (a2 + a3)) * 0.5;
+      double V = ZZ_(6, K) * (ZZ_(2, K1) * (b0 + b1) +
+                              ZZ_(2, K) * (b2 + b3)) * 0.5;
+      double Wc = w0;
       double UVW = sqrt(U * U + V * V + Wc * Wc);
-      Q = Q - 0.5 * CD * ZZ_(5, K) * (1.0 - f.ggz[c]) * Wc * UVW;
+      Q = Q - 0.5 * CD * ZZ_(5, K) * (1.0 - gg) * Wc * UVW;
       Q = Q - GVg * p.grz0;
       // wave source (vf_vgene.f:304-315)
       if (p.iws == I) {
         const double Q1 = 2.0 * XX_(4, I) * f.srcuv[(J - 1) + (long long)NJ * (K - 2)];
         const double Q2 = 2.0 * XX_(4, I) * f.srcuv[(J - 1) + (long long)NJ * (K - 1)];
         Q = Q + ZZ_(5, K) * (Q2 - Q1) * p.anu0 / 3.0;
-        Q = Q + WW[c] * (Q1 + Q2) * 0.5;
+        Q = Q + w0 * (Q1 + Q2) * 0.5;
       }
       if (p.jws == J) {
         const double Q1 = 2.0 * YY_(4, J) * f.srcuv[(I - 1) + (long long)NI * (K - 2)];
         const double Q2 = 2.0 * YY_(4, J) * f.srcuv[(I - 1) + (long long)NI * (K - 1)];
         Q = Q + ZZ_(5, K) * (Q2 - Q1) * p.anu0 / 3.0;
-        Q = Q + WW[c] * (Q1 + Q2) * 0.5;
+        Q = Q + w0 * (Q1 + Q2) * 0.5;
       }
       double DR = 0.0;
       Q = Q - GVg * p.grz0 * DR / p.rho0;
-      double GV = ZZ_(6, K) * (ZZ_(2, K) * GLV[c] + ZZ_(2, K - 1) * A(GLV, I, J, K - 1));
-      double GV0 = ZZ_(6, K) * (ZZ_(2, K) * GLV[c] + ZZ_(2, K - 1) * A(GLV, I, J, K - 1));
-      double DW = (XX_(4, I) * (A(FLWU, I + 1, J, K) - FLWU[c]) + YY_(4, J) * (A(FLWV, I, J + 1, K) - FLWV[c]) +
-                   ZZ_(5, K) * (FLWW[c] - A(FLWW, I, J, K - 1)) + Q);
+      double GV = ZZ_(6, K) * (ZZ_(2, K) * gl0 + ZZ_(2, K - 1) * gl1);
+      double GV0 = ZZ_(6, K) * (ZZ_(2, K) * gl0 + ZZ_(2, K - 1) * gl1);
+      double DW = (XX_(4, I) * (f1 - f0) + YY_(4, J) * (f3 - f2) +
+                   ZZ_(5, K) * (f4 - f5) + Q);
       W = (GV * W + DT * DW) / GV0;
       if (W > VM) W = VM;
       if (W < -VM) W = -VM;
       if (p.ipa != 0) {
         double X = (XX_(1, I) + XX_(1, I + 1)) * 0.5, Y = (YY_(1, J) + YY_(1, J + 1)) * 0.5;
         double DMAX = sponge_dmax(p, X, Y, true);
-        double G = ZZ_(6, K) * (ZZ_(2, K) * GGV[c] + ZZ_(2, K - 1) * A(GGV, I, J, K - 1));
+        double G = ZZ_(6, K) * (ZZ_(2, K) * gv0 + ZZ_(2, K - 1) * gv1);
         double D = GV0 / (GV0 + DT * G * DMAX);
         W = W * D;
       }
@@ -561,7 +650,7 @@ __global__ void __launch_bounds__(ROW_THREADS, 3) k_predict(Geo g, Fld f, Prm p,
 #undef XX_
 #undef YY_
 #undef ZZ_
-  ROW_LOOP_END
+  CELL_LOOP_END
 }
 
 // ------------------------------------------------------------ VF_BWUWN
@@ -893,13 +982,13 @@ void launch_open(cudaStream_t s, const Geo &g, const Fld &f, const OpenDev &o, c
   count_launch();
 }
 void launch_flux(cudaStream_t s, const Geo &g, const Fld &f, const Prm &p, double *const *fl) {
-  k_flux<<<row_blocks(g), ROW_THREADS, 0, s>>>(g, f, p, fl[0], fl[1], fl[2], fl[3], fl[4], fl[5],
+  k_flux<<<cell_grid(g), CELL_THREADS, 0, s>>>(g, f, p, fl[0], fl[1], fl[2], fl[3], fl[4], fl[5],
                                                 fl[6], fl[7], fl[8]);
   count_launch();
 }
 void launch_predict(cudaStream_t s, const Geo &g, const Fld &f, const Prm &p,
                     double *const *fl, double *un, double *vn, double *wn) {
-  k_predict<<<row_blocks(g), ROW_THREADS, 0, s>>>(g, f, p, fl[0], fl[1], fl[2], fl[3], fl[4],
+  k_predict<<<cell_grid(g), CELL_THREADS, 0, s>>>(g, f, p, fl[0], fl[1], fl[2], fl[3], fl[4],
                                                    fl[5], fl[6], fl[7], fl[8], un, vn, wn);
   count_launch();
 }

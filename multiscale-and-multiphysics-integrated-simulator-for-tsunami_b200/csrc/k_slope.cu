@@ -295,9 +295,9 @@ __device__ __forceinline__ void slope_side(const Fld &f, int NF0, double FF0, lo
   }
 }
 
-__global__ void k_fslope(Geo g, Fld f, Prm p, int *IST, double *SX, double *SY, double *SZ, double *SA, int *err) {
+__global__ void __launch_bounds__(CELL_THREADS) k_fslope(Geo g, Fld f, Prm p, int *IST, double *SX, double *SY, double *SZ, double *SA, int *err) {
   const double ZERO = 1.0e-20;
-  ROW_LOOP_BEGIN(g)
+  CELL_LOOP_BEGIN(g)
   const long long c = cid(g, I, J, K);
   int ist = 0;
   double s1 = 0.0, s2 = 0.0, s3 = 0.0, sa = 0.0;
@@ -358,7 +358,7 @@ __global__ void k_fslope(Geo g, Fld f, Prm p, int *IST, double *SX, double *SY, 
     }
   }
   IST[c] = ist; SX[c] = s1; SY[c] = s2; SZ[c] = s3; SA[c] = sa;
-  ROW_LOOP_END
+  CELL_LOOP_END
 }
 
 // ------------------------------------------------------------ k_fconvs
@@ -398,12 +398,12 @@ __device__ __forceinline__ double slope_flux(const Geo &g, const Fld &f, const i
   return dmin(FVX, VG);
 }
 
-__global__ void k_fconvs(Geo g, Fld f, Prm p, const int *IST, const double *SX, const double *SY, const double *SZ,
+__global__ void __launch_bounds__(CELL_THREADS) k_fconvs(Geo g, Fld f, Prm p, const int *IST, const double *SX, const double *SY, const double *SZ,
                          const double *SA, double *FLFU, double *FLFV, double *FLFW) {
   const double DT = p.dtnow, FL = p.flower;
   const int *NF = f.nf;
   const double *FF = f.ff, *GGV = f.ggv;
-  ROW_LOOP_BEGIN(g)
+  CELL_LOOP_BEGIN(g)
   const long long c = cid(g, I, J, K);
   const int NI = g.NI, NJ = g.NJ, NK = g.NK;
   double fu = 0.0, fv = 0.0, fw = 0.0;
@@ -471,7 +471,7 @@ __global__ void k_fconvs(Geo g, Fld f, Prm p, const int *IST, const double *SX, 
     fw = 0.0 - (double)LSN * fl;
   }
   FLFU[c] = fu; FLFV[c] = fv; FLFW[c] = fw;
-  ROW_LOOP_END
+  CELL_LOOP_END
 }
 
 #undef A
@@ -481,9 +481,9 @@ __global__ void k_fconvs(Geo g, Fld f, Prm p, const int *IST, const double *SX, 
 
 void launch_fconvs(cudaStream_t s, const Geo &g, const Fld &f, const Prm &p, int *ist, double *sx, double *sy,
                    double *sz, double *sa, double *flfu, double *flfv, double *flfw, int *err) {
-  k_fslope<<<row_blocks(g), ROW_THREADS, 0, s>>>(g, f, p, ist, sx, sy, sz, sa, err);
+  k_fslope<<<cell_grid(g), CELL_THREADS, 0, s>>>(g, f, p, ist, sx, sy, sz, sa, err);
   count_launch();
-  k_fconvs<<<row_blocks(g), ROW_THREADS, 0, s>>>(g, f, p, ist, sx, sy, sz, sa, flfu, flfv, flfw);
+  k_fconvs<<<cell_grid(g), CELL_THREADS, 0, s>>>(g, f, p, ist, sx, sy, sz, sa, flfu, flfv, flfw);
   count_launch();
 }
 

@@ -21,6 +21,12 @@
 //   k_cindc        VF_CINDC  (vf_cindc.f:35-53), also counts NUMS
 //   k_bsppfl       VF_BSPPFL (vf_bsppfl.f:40-67) into a second buffer
 //
+// Bound by the latency of their loads, so a cell's are issued together and
+// the passes that act on few cells scan several flags at once (cell and scan
+// kernels of cadmas_dev.cuh): on 519x63x85 cells k_fconv 122 -> 63 us,
+// k_fnf_init 54 -> 22, k_bsuwn3 46 -> 11, k_fmod1_target 68 -> 26; the VOF
+// stage 282 -> 180 us and the flags 471 -> 368 us.
+//
 // The surface list INDS of the reference is not kept: every loop over it
 // is a pass over the grid that acts on cells with NF in 1..6 (or 7).  The
 // loops are free of ordering effects because FNFPRV gives each surface
@@ -40,63 +46,49 @@ namespace cadmas {
 #define ZZ_(m, k) gz(g, m, k)
 
 // ------------------------------------------------------------ VF_FCONV
-__global__ void k_fconv(Geo g, Fld f, Prm p, double *FLFU, double *FLFV, double *FLFW) {
+__global__ void __launch_bounds__(CELL_THREADS) k_fconv(Geo g, Fld f, Prm p, double *FLFU, double *FLFV, double *FLFW) {
   const double DT = p.dtnow, FL = p.flower;
   const int *NF = f.nf;
   const double *FF = f.ff, *GGV = f.ggv;
-  ROW_LOOP_BEGIN(g)
+  CELL_LOOP_BEGIN(g)
   const long long c = cid(g, I, J, K);
   const int NI = g.NI, NJ = g.NJ, NK = g.NK;
   double fu = 0.0, fv = 0.0, fw = 0.0;
-  if (K >= 2 && K <= NK - 1 && J >= 2 && J <= NJ - 1 && I >= 2 && f.indx[c] != -1) {
-    double C = DT * f.ggx[c] * f.uu[c];
-    int LSN, LA, LD, LDM;
-    if (C >= 0.0) { LSN = 1; LA = I; LD = I - 1; LDM = I - 2; } else { LSN = -1; LA = I - 1; LD = I; LDM = I + 1; }
-    int N = A(NF, LD, J, K);
-    int ndm = (N != -1) ? A(NF, LDM, J, K) : -1;
-    double fdm = (N != -1 && ndm != -1) ? A(FF, LDM, J, K) : 0.0;
-    double vd = (N != -1) ? XX_(2, LD) * A(GGV, LD, J, K) : 0.0;
-    double bcf = (N == -1) ? f.bcf[f.indx[c] - 1] : 0.0;
-    int na = A(NF, LA, J, K);
-    double fl = fconv_face(C, N, (N != -1) ? A(FF, LD, J, K) : 0.0, ndm, fdm, vd, XX_(2, LD), bcf, na,
-                           (na != -1) ? A(FF, LA, J, K) : 0.0, 3, 4, 5, 6, FL);
-    fu = 0.0 - (double)LSN * fl;
-  }
-  if (K >= 2 && K <= NK - 1 && J >= 2 && I >= 2 && I <= NI - 1 && f.indy[c] != -1) {
-    double C = DT * f.ggy[c] * f.vv[c];
-    int LSN, LA, LD, LDM;
-    if (C >= 0.0) { LSN = 1; LA = J; LD = J - 1; LDM = J - 2; } else { LSN = -1; LA = J - 1; LD = J; LDM = J + 1; }
-    int N = A(NF, I, LD, K);
-    int ndm = (N != -1) ? A(NF, I, LDM, K) : -1;
-    double fdm = (N != -1 && ndm != -1) ? A(FF, I, LDM, K) : 0.0;
-    double vd = (N != -1) ? YY_(2, LD) * A(GGV, I, LD, K) : 0.0;
-    double bcf = (N == -1) ? f.bcf[f.indy[c] - 1] : 0.0;
-    int na = A(NF, I, LA, K);
-    double fl = fconv_face(C, N, (N != -1) ? A(FF, I, LD, K) : 0.0, ndm, fdm, vd, YY_(2, LD), bcf, na,
-                           (na != -1) ? A(FF, I, LA, K) : 0.0, 1, 2, 5, 6, FL);
-    fv = 0.0 - (double)LSN * fl;
-  }
-  if (K >= 2 && J >= 2 && J <= NJ - 1 && I >= 2 && I <= NI - 1 && f.indz[c] != -1) {
-    double C = DT * f.ggz[c] * f.ww[c];
-    int LSN, LA, LD, LDM;
-    if (C >= 0.0) { LSN = 1; LA = K; LD = K - 1; LDM = K - 2; } else { LSN = -1; LA = K - 1; LD = K; LDM = K + 1; }
-    int N = A(NF, I, J, LD);
-    int ndm = (N != -1) ? A(NF, I, J, LDM) : -1;
-    double fdm = (N != -1 && ndm != -1) ? A(FF, I, J, LDM) : 0.0;
-    double vd = (N != -1) ? ZZ_(2, LD) * A(GGV, I, J, LD) : 0.0;
-    double bcf = (N == -1) ? f.bcf[f.indz[c] - 1] : 0.0;
-    int na = A(NF, I, J, LA);
-    double fl = fconv_face(C, N, (N != -1) ? A(FF, I, J, LD) : 0.0, ndm, fdm, vd, ZZ_(2, LD), bcf, na,
-                           (na != -1) ? A(FF, I, J, LA) : 0.0, 1, 2, 3, 4, FL);
-    fw = 0.0 - (double)LSN * fl;
+  if (K >= 2 && J >= 2 && I >= 2) {
+    const bool dox = K <= NK - 1 && J <= NJ - 1, doy = K <= NK - 1 && I <= NI - 1, doz = J <= NJ - 1 && I <= NI - 1;
+    // All that the three faces may use, in flight together (cells that a
+    // face does not use may lie outside of the grid: any address serves).
+    const long long sj = NI, sk = (long long)NI * NJ, last = g.N - 1;
+    const int ix = ld_now(f.indx + c), iy = ld_now(f.indy + c), iz = ld_now(f.indz + c);
+    const double cx = DT * ld_now(f.ggx + c) * ld_now(f.uu + c), cy = DT * ld_now(f.ggy + c) * ld_now(f.vv + c),
+                 cz = DT * ld_now(f.ggz + c) * ld_now(f.ww + c);
+    const int n0 = ld_now(NF + c);
+    const double f0 = ld_now(FF + c), g0 = ld_now(GGV + c);
+    // the cell across the face (a), the one behind it (b), the next on this side (d)
+    const auto face = [&](bool doit, double C, int ind, long long st, double wa, double w0, int d1, int d2, int d3, int d4) {
+      const long long ca = c - st, cb = max(c - 2 * st, 0LL), cd = min(c + st, last);
+      const int na = ld_now(NF + ca), nb = ld_now(NF + cb), nd = ld_now(NF + cd);
+      const double fa = ld_now(FF + ca), fb = ld_now(FF + cb), fd = ld_now(FF + cd), ga = ld_now(GGV + ca);
+      if (!doit || ind == -1) return 0.0;
+      const bool fwd = C >= 0.0;  // the donor is a, else this cell
+      const int N = fwd ? na : n0, ndm = (N != -1) ? (fwd ? nb : nd) : -1, nac = fwd ? n0 : na;
+      const double fdm = (N != -1 && ndm != -1) ? (fwd ? fb : fd) : 0.0, wd = fwd ? wa : w0;
+      const double vd = (N != -1) ? wd * (fwd ? ga : g0) : 0.0, bcf = (N == -1) ? f.bcf[ind - 1] : 0.0;
+      const double fl = fconv_face(C, N, (N != -1) ? (fwd ? fa : f0) : 0.0, ndm, fdm, vd, wd, bcf, nac,
+                                   (nac != -1) ? (fwd ? f0 : fa) : 0.0, d1, d2, d3, d4, FL);
+      return 0.0 - (double)(fwd ? 1 : -1) * fl;
+    };
+    fu = face(dox, cx, ix, 1, XX_(2, I - 1), XX_(2, I), 3, 4, 5, 6);
+    fv = face(doy, cy, iy, sj, YY_(2, J - 1), YY_(2, J), 1, 2, 5, 6);
+    fw = face(doz, cz, iz, sk, ZZ_(2, K - 1), ZZ_(2, K), 1, 2, 3, 4);
   }
   FLFU[c] = fu; FLFV[c] = fv; FLFW[c] = fw;
-  ROW_LOOP_END
+  CELL_LOOP_END
 }
 
 // ----------------------------------------------------------- VF_FEULER
-__global__ void k_feuler(Geo g, Fld f, Prm p, const double *FLFU, const double *FLFV, const double *FLFW) {
-  ROW_LOOP_BEGIN(g)
+__global__ void __launch_bounds__(CELL_THREADS) k_feuler(Geo g, Fld f, Prm p, const double *FLFU, const double *FLFV, const double *FLFW) {
+  CELL_LOOP_BEGIN(g)
   if (I >= 2 && I <= g.NI - 1 && J >= 2 && J <= g.NJ - 1 && K >= 2 && K <= g.NK - 1) {
     const long long c = cid(g, I, J, K);
     if (f.nf[c] != -1) {
@@ -122,7 +114,7 @@ __global__ void k_feuler(Geo g, Fld f, Prm p, const double *FLFU, const double *
       f.ff[c] = (G0 * f.ff[c] + DF) / G;
     }
   }
-  ROW_LOOP_END
+  CELL_LOOP_END
 }
 
 // ------------------------------------------------------------ VF_FMOD1
@@ -144,12 +136,12 @@ __device__ __forceinline__ bool is_surf(int n) { return n >= 1 && n <= 6; }
 // Offset (-K): the cell below; it points up at us if it is NF=5 (fluid
 // below it, so we are its E) or NF=6 (we are its F).
 struct NbSel { int di, dj, dk, nE, nF; };
-__constant__ NbSel c_nb[6] = {
+__device__ constexpr NbSel c_nb[6] = {
     {0, 0, -1, 5, 6}, {0, -1, 0, 3, 4}, {-1, 0, 0, 1, 2},
     {1, 0, 0, 2, 1},  {0, 1, 0, 4, 3},  {0, 0, 1, 6, 5}};
 
-__global__ void k_fmod1_count(Geo g, Fld f, int *NLIM) {
-  ROW_LOOP_BEGIN(g)
+__global__ void __launch_bounds__(CELL_THREADS) k_fmod1_count(Geo g, Fld f, int *NLIM) {
+  CELL_LOOP_BEGIN(g)
   const long long c = cid(g, I, J, K);
   int n = 0;
   if (I >= 2 && I <= g.NI - 1 && J >= 2 && J <= g.NJ - 1 && K >= 2 && K <= g.NK - 1) {
@@ -160,16 +152,16 @@ __global__ void k_fmod1_count(Geo g, Fld f, int *NLIM) {
     }
   }
   NLIM[c] = n;
-  ROW_LOOP_END
+  CELL_LOOP_END
 }
 
 __device__ __forceinline__ double cellvol(const Geo &g, const double *GGV, int I, int J, int K) {
   return gx(g, 2, I) * gy(g, 2, J) * gz(g, 2, K) * GGV[cid(g, I, J, K)];
 }
 
-__global__ void k_fmod1_redist(Geo g, Fld f, const int *NLIM) {
+__global__ void __launch_bounds__(CELL_THREADS) k_fmod1_redist(Geo g, Fld f, const int *NLIM) {
   double *FF = f.ff;
-  ROW_LOOP_BEGIN(g)
+  SCAN_LOOP_BEGIN(g, f.nf, n_ >= 1 && n_ <= 6)
   const long long s = cid(g, I, J, K);
   int N = f.nf[s];
   if (is_surf(N) && I >= 2 && I <= g.NI - 1 && J >= 2 && J <= g.NJ - 1 && K >= 2 && K <= g.NK - 1) {
@@ -189,22 +181,29 @@ __global__ void k_fmod1_redist(Geo g, Fld f, const int *NLIM) {
       else FF[s] = FF[s] + SS / VS;
     }
   }
-  ROW_LOOP_END
+  SCAN_LOOP_END
 }
 
 // Loop 400 for E/F cells (non-surface), gathering from surface neighbours.
-__global__ void k_fmod1_target(Geo g, Fld f) {
+__global__ void __launch_bounds__(CELL_THREADS) k_fmod1_target(Geo g, Fld f) {
   double *FF = f.ff;
-  ROW_LOOP_BEGIN(g)
+  CELL_LOOP_BEGIN(g)
   const long long c = cid(g, I, J, K);
   if (!is_surf(f.nf[c]) && I >= 2 && I <= g.NI - 1 && J >= 2 && J <= g.NJ - 1 && K >= 2 && K <= g.NK - 1) {
+    int nb[6];
+    bool any = false;
+#pragma unroll
+    for (int q = 0; q < 6; ++q) nb[q] = ld_now(&A(f.nf, I + c_nb[q].di, J + c_nb[q].dj, K + c_nb[q].dk));
+#pragma unroll
+    for (int q = 0; q < 6; ++q) any = any || is_surf(nb[q]);
+    if (!any) continue;  // away from the surface
     double v = FF[c];
     bool touched = false;
 #pragma unroll
     for (int q = 0; q < 6; ++q) {
       const int Is = I + c_nb[q].di, Js = J + c_nb[q].dj, Ks = K + c_nb[q].dk;
       const long long s = cid(g, Is, Js, Ks);
-      const int n = f.nf[s];
+      const int n = nb[q];
       if (n == c_nb[q].nE) {            // we are the E cell of s
         double fs = FF[s];
         if (fs > 1.0) {
@@ -223,11 +222,11 @@ __global__ void k_fmod1_target(Geo g, Fld f) {
     }
     if (touched) FF[c] = v;
   }
-  ROW_LOOP_END
+  CELL_LOOP_END
 }
 
-__global__ void k_fmod1_clamp(Geo g, Fld f) {
-  ROW_LOOP_BEGIN(g)
+__global__ void __launch_bounds__(CELL_THREADS) k_fmod1_clamp(Geo g, Fld f) {
+  SCAN_LOOP_BEGIN(g, f.nf, n_ >= 1 && n_ <= 6)
   const long long s = cid(g, I, J, K);
   if (is_surf(f.nf[s]) && I >= 2 && I <= g.NI - 1 && J >= 2 && J <= g.NJ - 1 && K >= 2 && K <= g.NK - 1) {
     double v = f.ff[s];
@@ -235,7 +234,7 @@ __global__ void k_fmod1_clamp(Geo g, Fld f) {
     else if (v < 0.0) v = 0.0;
     f.ff[s] = v;
   }
-  ROW_LOOP_END
+  SCAN_LOOP_END
 }
 
 // ----------------------------------------------------------- VF_FCUT01
@@ -262,24 +261,23 @@ __global__ void k_fcut(Geo g, Fld f, Prm p, double *rb_sum, double *rb_cut) {
 // ----------------------------------------------------------- VF_FNFINI
 // Phase 1+2: non-obstacle cells to fluid, then gas where F < FLOWER and no
 // neighbour face carries F > FUPPER (vf_fnfini.f:39-103).
-__global__ void k_fnf_init(Geo g, Fld f, Prm p) {
+__global__ void __launch_bounds__(CELL_THREADS) k_fnf_init(Geo g, Fld f, Prm p) {
   const double FU = p.fupper;
   const double *FF = f.ff;
-  ROW_LOOP_BEGIN(g)
+  CELL_LOOP_BEGIN(g)
   const long long c = cid(g, I, J, K);
   if (K >= 2 && K <= g.NK - 1) {
+    const double F = ld_now(FF + c);
     int n = f.nf[c];
     if (n != -1) {
       n = 0;
-      if (I >= 2 && I <= g.NI - 1 && J >= 2 && J <= g.NJ - 1 && FF[c] < p.flower) {
+      if (I >= 2 && I <= g.NI - 1 && J >= 2 && J <= g.NJ - 1 && F < p.flower) {
         int IX1 = f.indx[c], IX2 = A(f.indx, I + 1, J, K), IY1 = f.indy[c], IY2 = A(f.indy, I, J + 1, K);
         int IZ1 = f.indz[c], IZ2 = A(f.indz, I, J, K + 1);
-        double FX1 = IX1 >= 1 ? f.bcf[IX1 - 1] : A(FF, I - 1, J, K);
-        double FX2 = IX2 >= 1 ? f.bcf[IX2 - 1] : A(FF, I + 1, J, K);
-        double FY1 = IY1 >= 1 ? f.bcf[IY1 - 1] : A(FF, I, J - 1, K);
-        double FY2 = IY2 >= 1 ? f.bcf[IY2 - 1] : A(FF, I, J + 1, K);
-        double FZ1 = IZ1 >= 1 ? f.bcf[IZ1 - 1] : A(FF, I, J, K - 1);
-        double FZ2 = IZ2 >= 1 ? f.bcf[IZ2 - 1] : A(FF, I, J, K + 1);
+        // a face with IND >= 1 does not count, whatever its boundary value
+        const double FX1 = ld_now(&A(FF, I - 1, J, K)), FX2 = ld_now(&A(FF, I + 1, J, K));
+        const double FY1 = ld_now(&A(FF, I, J - 1, K)), FY2 = ld_now(&A(FF, I, J + 1, K));
+        const double FZ1 = ld_now(&A(FF, I, J, K - 1)), FZ2 = ld_now(&A(FF, I, J, K + 1));
         if (!(FZ1 > FU && IZ1 == 0) && !(FY1 > FU && IY1 == 0) && !(FY2 > FU && IY2 == 0) &&
             !(FX1 > FU && IX1 == 0) && !(FX2 > FU && IX2 == 0) && !(FZ2 > FU && IZ2 == 0))
           n = 8;
@@ -287,45 +285,61 @@ __global__ void k_fnf_init(Geo g, Fld f, Prm p) {
       f.nf[c] = n;
     }
   }
-  ROW_LOOP_END
+  CELL_LOOP_END
 }
 
 __device__ __forceinline__ bool interior3(const Geo &g, int I, int J, int K) {
   return I >= 2 && I <= g.NI - 1 && J >= 2 && J <= g.NJ - 1 && K >= 2 && K <= g.NK - 1;
 }
 
-// loop 1100: cells next to gas become surface (7)
-__global__ void k_fnf_mark7(Geo g, int *NF, const int *done) {
+// loop 1100: cells next to gas become surface (7).  A thread takes SCAN_K
+// cells of a column: their flags and those above and below them at once,
+// then the lateral ones of all that may change.
+__global__ void __launch_bounds__(CELL_THREADS) k_fnf_mark7(Geo g, int *NF, const int *done) {
   if (*done) return;
-  ROW_LOOP_BEGIN(g)
-  const long long c = cid(g, I, J, K);
-  if (interior3(g, I, J, K)) {
-    int n = NF[c];
-    if (n != -1 && n != 8) {
-      if (A(NF, I, J, K + 1) == 8 || A(NF, I, J + 1, K) == 8 || A(NF, I, J - 1, K) == 8 ||
-          A(NF, I + 1, J, K) == 8 || A(NF, I - 1, J, K) == 8 || A(NF, I, J, K - 1) == 8)
-        NF[c] = 7;
+  CELL_IJ(g)
+    if (I < 2 || I > g.NI - 1 || J < 2 || J > g.NJ - 1) return;
+    const long long sj = g.NI, sk = (long long)g.NI * g.NJ;
+    for (int K0 = (int)blockIdx.y * SCAN_K + 1; K0 <= g.NK; K0 += (int)gridDim.y * SCAN_K) {
+      int v[SCAN_K + 2];
+      bool any = false;
+#pragma unroll
+      for (int u = 0; u < SCAN_K + 2; ++u) v[u] = NF[p_ + sk * (min(max(K0 + u - 1, 1), g.NK) - 1)];
+#pragma unroll
+      for (int u = 1; u <= SCAN_K; ++u) any = any || (v[u] != -1 && v[u] != 8);
+      if (!any) continue;
+      bool gas[SCAN_K];
+#pragma unroll
+      for (int u = 0; u < SCAN_K; ++u) {
+        const int *q = NF + p_ + sk * (min(K0 + u, g.NK) - 1);
+        const int a = q[-1], b = q[1], c = q[-sj], d = q[sj];
+        gas[u] = (a == 8) | (b == 8) | (c == 8) | (d == 8) | (v[u] == 8) | (v[u + 2] == 8);
+      }
+#pragma unroll
+      for (int u = 0; u < SCAN_K; ++u) {
+        const int K = K0 + u;
+        if (K >= 2 && K <= g.NK - 1 && v[u + 1] != -1 && v[u + 1] != 8 && gas[u]) NF[p_ + sk * (K - 1)] = 7;
+      }
     }
   }
-  ROW_LOOP_END
 }
 // loop 1200: surface cells without a fluid neighbour become gas
-__global__ void k_fnf_to8(Geo g, int *NF, const int *done) {
+__global__ void __launch_bounds__(CELL_THREADS) k_fnf_to8(Geo g, int *NF, const int *done) {
   if (*done) return;
-  ROW_LOOP_BEGIN(g)
+  SCAN_LOOP_BEGIN(g, NF, n_ == 7)
   const long long c = cid(g, I, J, K);
   if (interior3(g, I, J, K) && NF[c] == 7) {
     if (A(NF, I, J, K + 1) != 0 && A(NF, I, J + 1, K) != 0 && A(NF, I, J - 1, K) != 0 &&
         A(NF, I + 1, J, K) != 0 && A(NF, I - 1, J, K) != 0 && A(NF, I, J, K - 1) != 0)
       NF[c] = 8;
   }
-  ROW_LOOP_END
+  SCAN_LOOP_END
 }
 // loop 1300: surface cells not between fluid and gas along any axis -> -7
-__global__ void k_fnf_markm7(Geo g, int *NF, int *nch, const int *done) {
+__global__ void __launch_bounds__(CELL_THREADS) k_fnf_markm7(Geo g, int *NF, int *nch, const int *done) {
   if (*done) return;
   int cnt = 0;
-  ROW_LOOP_BEGIN(g)
+  SCAN_LOOP_BEGIN(g, NF, n_ == 7)
   const long long c = cid(g, I, J, K);
   if (interior3(g, I, J, K) && NF[c] == 7) {
     if (A(NF, I, J, K - 1) != 0 || A(NF, I, J, K + 1) != 8)
@@ -335,7 +349,7 @@ __global__ void k_fnf_markm7(Geo g, int *NF, int *nch, const int *done) {
             if (A(NF, I, J + 1, K) != 0 || A(NF, I, J - 1, K) != 8)
               if (A(NF, I, J, K + 1) != 0 || A(NF, I, J, K - 1) != 8) { NF[c] = -7; cnt++; }
   }
-  ROW_LOOP_END
+  SCAN_LOOP_END
   if (cnt) atomicAdd(nch, cnt);
 }
 // loop exit test: NCH = 0 ends the iteration; the counter is cleared for
@@ -349,12 +363,12 @@ __global__ void k_fnf_check(int *nch, int *done, int *iter, int cap, int *err) {
   else if (*iter >= cap) { *done = 1; atomicOr(err, ERR_CAP); }
 }
 // loop 1400: -7 -> gas
-__global__ void k_fnf_m7to8(Geo g, int *NF, const int *done) {
+__global__ void __launch_bounds__(CELL_THREADS) k_fnf_m7to8(Geo g, int *NF, const int *done) {
   if (*done) return;
-  ROW_LOOP_BEGIN(g)
+  SCAN_LOOP_BEGIN(g, NF, n_ == -7)
   const long long c = cid(g, I, J, K);
   if (NF[c] == -7) NF[c] = 8;
-  ROW_LOOP_END
+  SCAN_LOOP_END
 }
 
 // ----------------------------------------------------------- VF_FBUBUP
@@ -382,10 +396,10 @@ __global__ void k_fbubup(Geo g, Fld f, Prm p, const unsigned char *active) {
 // ----------------------------------------------------------- VF_FNFPRV
 __device__ __forceinline__ double bcf_or(const Fld &f, int ind, double v) { return ind >= 1 ? f.bcf[ind - 1] : v; }
 
-__global__ void __launch_bounds__(ROW_THREADS, 3) k_fnfprv(Geo g, Fld f, int *err) {
+__global__ void __launch_bounds__(CELL_THREADS) k_fnfprv(Geo g, Fld f, int *err) {
   const double *FF = f.ff;
   int *NF = f.nf;
-  ROW_LOOP_BEGIN(g)
+  SCAN_LOOP_BEGIN(g, f.nf, n_ == 7)
   const long long c = cid(g, I, J, K);
   if (interior3(g, I, J, K) && NF[c] == 7) {
     double FM = -1.0, FS;
@@ -447,26 +461,34 @@ __global__ void __launch_bounds__(ROW_THREADS, 3) k_fnfprv(Geo g, Fld f, int *er
     NF[c] = res;
     if (res == 7) atomicOr(err, ERR_PG);
   }
-  ROW_LOOP_END
+  SCAN_LOOP_END
 }
 
 // ------------------------------------------------------------ VF_CINDC
-__global__ void k_cindc(Geo g, Fld f, int *nums) {
+__global__ void __launch_bounds__(CELL_THREADS) k_cindc(Geo g, Fld f, int *nums) {
   int cnt = 0;
-  ROW_LOOP_BEGIN(g)
-  if (interior3(g, I, J, K)) {
-    const long long c = cid(g, I, J, K);
-    int n = f.nf[c];
-    f.indc[c] = (n == 8 || n == -1) ? -1 : 0;
-    if (n >= 1 && n <= 7) cnt++;
+  CELL_IJ(g)
+    const long long sk = (long long)g.NI * g.NJ;
+    if (I >= 2 && I <= g.NI - 1 && J >= 2 && J <= g.NJ - 1)
+      for (int K0 = (int)blockIdx.y * SCAN_K + 1; K0 <= g.NK; K0 += (int)gridDim.y * SCAN_K) {
+        int v[SCAN_K];
+#pragma unroll
+        for (int u = 0; u < SCAN_K; ++u) v[u] = f.nf[p_ + sk * (min(K0 + u, g.NK) - 1)];
+#pragma unroll
+        for (int u = 0; u < SCAN_K; ++u) {
+          const int K = K0 + u, n = v[u];
+          if (K < 2 || K > g.NK - 1) continue;
+          f.indc[p_ + sk * (K - 1)] = (n == 8 || n == -1) ? -1 : 0;
+          if (n >= 1 && n <= 7) cnt++;
+        }
+      }
   }
-  ROW_LOOP_END
   if (cnt) atomicAdd(nums, cnt);
 }
 
 // ----------------------------------------------------------- VF_BSPPFL
-__global__ void k_bsppfl(Geo g, Fld f, const double *PP0, double *PPN) {
-  ROW_LOOP_BEGIN(g)
+__global__ void __launch_bounds__(CELL_THREADS) k_bsppfl(Geo g, Fld f, const double *PP0, double *PPN) {
+  CELL_LOOP_BEGIN(g)
   const long long c = cid(g, I, J, K);
   double v = PP0[c];
   if (interior3(g, I, J, K) && f.nf[c] == 0 && f.nf0[c] == 8) {
@@ -480,7 +502,7 @@ __global__ void k_bsppfl(Geo g, Fld f, const double *PP0, double *PPN) {
     v = (SUMF < 1.0e-20) ? 0.0 : SUMP / SUMF;
   }
   PPN[c] = v;
-  ROW_LOOP_END
+  CELL_LOOP_END
 }
 
 #undef A
@@ -490,32 +512,36 @@ __global__ void k_bsppfl(Geo g, Fld f, const double *PP0, double *PPN) {
 
 // ------------------------------------------------------------ launchers
 #define RL(kern, ...) (kern<<<row_blocks(g), ROW_THREADS, 0, s>>>(__VA_ARGS__), count_launch())
-void launch_fconv(cudaStream_t s, const Geo &g, const Fld &f, const Prm &p, double *a, double *b, double *c) { RL(k_fconv, g, f, p, a, b, c); }
-void launch_feuler(cudaStream_t s, const Geo &g, const Fld &f, const Prm &p, const double *a, const double *b, const double *c) { RL(k_feuler, g, f, p, a, b, c); }
+#define CL(kern, ...) (kern<<<cell_grid(g), CELL_THREADS, 0, s>>>(__VA_ARGS__), count_launch())
+#define SCL(kern, ...) (kern<<<cell_grid(g, SCAN_K), CELL_THREADS, 0, s>>>(__VA_ARGS__), count_launch())
+void launch_fconv(cudaStream_t s, const Geo &g, const Fld &f, const Prm &p, double *a, double *b, double *c) { CL(k_fconv, g, f, p, a, b, c); }
+void launch_feuler(cudaStream_t s, const Geo &g, const Fld &f, const Prm &p, const double *a, const double *b, const double *c) { CL(k_feuler, g, f, p, a, b, c); }
 void launch_fmod1(cudaStream_t s, const Geo &g, const Fld &f, int *nlim) {
-  RL(k_fmod1_count, g, f, nlim);
-  RL(k_fmod1_redist, g, f, nlim);
-  RL(k_fmod1_target, g, f);
-  RL(k_fmod1_clamp, g, f);
+  CL(k_fmod1_count, g, f, nlim);
+  SCL(k_fmod1_redist, g, f, nlim);
+  CL(k_fmod1_target, g, f);
+  SCL(k_fmod1_clamp, g, f);
 }
 void launch_fcut(cudaStream_t s, const Geo &g, const Fld &f, const Prm &p, double *rbs, double *rbc) { RL(k_fcut, g, f, p, rbs, rbc); }
-void launch_fnf_init(cudaStream_t s, const Geo &g, const Fld &f, const Prm &p) { RL(k_fnf_init, g, f, p); }
+void launch_fnf_init(cudaStream_t s, const Geo &g, const Fld &f, const Prm &p) { CL(k_fnf_init, g, f, p); }
 void launch_fnf_sweep(cudaStream_t s, const Geo &g, int *nf, int *nch, int *done, int *iter, int cap, int *err) {
-  RL(k_fnf_mark7, g, nf, done);
-  RL(k_fnf_to8, g, nf, done);
-  RL(k_fnf_markm7, g, nf, nch, done);
+  SCL(k_fnf_mark7, g, nf, done);
+  SCL(k_fnf_to8, g, nf, done);
+  SCL(k_fnf_markm7, g, nf, nch, done);
   k_fnf_check<<<1, 1, 0, s>>>(nch, done, iter, cap, err);
   count_launch();
-  RL(k_fnf_m7to8, g, nf, done);
+  SCL(k_fnf_m7to8, g, nf, done);
 }
 void launch_fbubup(cudaStream_t s, const Geo &g, const Fld &f, const Prm &p, const unsigned char *active) {
   int n = (g.NI - 2) * (g.NJ - 2);
   k_fbubup<<<(n + 255) / 256, 256, 0, s>>>(g, f, p, active);
   count_launch();
 }
-void launch_fnfprv(cudaStream_t s, const Geo &g, const Fld &f, int *err) { RL(k_fnfprv, g, f, err); }
-void launch_cindc(cudaStream_t s, const Geo &g, const Fld &f, int *nums) { RL(k_cindc, g, f, nums); }
-void launch_bsppfl(cudaStream_t s, const Geo &g, const Fld &f, const double *pp0, double *ppn) { RL(k_bsppfl, g, f, pp0, ppn); }
+void launch_fnfprv(cudaStream_t s, const Geo &g, const Fld &f, int *err) { SCL(k_fnfprv, g, f, err); }
+void launch_cindc(cudaStream_t s, const Geo &g, const Fld &f, int *nums) { SCL(k_cindc, g, f, nums); }
+void launch_bsppfl(cudaStream_t s, const Geo &g, const Fld &f, const double *pp0, double *ppn) { CL(k_bsppfl, g, f, pp0, ppn); }
 #undef RL
+#undef CL
+#undef SCL
 
 }  // namespace cadmas

@@ -60,14 +60,14 @@ __global__ void k_ws_features(Geo g, Fld f, const double *BB, const double *scal
   x4[4 * i + 0] = v0; x4[4 * i + 1] = v1; x4[4 * i + 2] = v2; x4[4 * i + 3] = v3;
 }
 
-__global__ void k_ws_output(Geo g, const int *INDC, const float *y, const double *scal, double *PT, int X, int Y) {
-  ROW_LOOP_BEGIN(g)
+__global__ void __launch_bounds__(CELL_THREADS) k_ws_output(Geo g, const int *INDC, const float *y, const double *scal, double *PT, int X, int Y) {
+  CELL_LOOP_BEGIN(g)
   const long long c = cid(g, I, J, K);
   double v = 0.0;
   if (ws_inner(g, I, J, K) && INDC[c] != -1)
     v = scal[0] * scal[3] * (double)y[(long long)(I - 1) + (long long)X * ((long long)(J - 1) + (long long)Y * (K - 1))];
   PT[c] = v;
-  ROW_LOOP_END
+  CELL_LOOP_END
 }
 
 __global__ void k_ws_resid(Geo g, SysPtr a, const int *INDC, const double *PT, double *r0, double *r1) {
@@ -120,7 +120,7 @@ void launch_warm_guess(cudaStream_t s, const Geo &g, const Fld &f, const SysPtr 
   k_ws_features<<<(unsigned)((V + 255) / 256), 256, 0, s>>>(g, f, a.bb, scal, unet_input(net), X, Y, Z);
   count_launch(3);
   unet_run_forward(net);
-  k_ws_output<<<row_blocks(g), ROW_THREADS, 0, s>>>(g, f.indc, unet_output(net), scal, PT, X, Y);
+  k_ws_output<<<cell_grid(g), CELL_THREADS, 0, s>>>(g, f.indc, unet_output(net), scal, PT, X, Y);
   k_ws_resid<<<row_blocks(g), ROW_THREADS, 0, s>>>(g, a, f.indc, PT, rows0, rows1);
   k_ws_decide<<<1, 1024, 0, s>>>(rows0, rows1, nrows, unet_error(net), scal, cnt);
   k_ws_clear<<<296, 256, 0, s>>>(g.N, cnt, PT);
