@@ -192,12 +192,16 @@ struct Piece {
 };
 
 bool upload_setup(cadmas_unet *n) {
-  if (n->pin) return true;
-  if (cudaMallocHost((void **)&n->pin, UP_T * 2 * UP_CHUNK) != cudaSuccess) { n->pin = nullptr; return false; }
+  if (!n->pin && cudaMallocHost((void **)&n->pin, UP_T * 2 * UP_CHUNK) != cudaSuccess) n->pin = nullptr;
+  bool ok = n->pin != nullptr;
   for (auto &t : n->pin_ev)
     for (cudaEvent_t &e : t)
-      if (!e && cudaEventCreateWithFlags(&e, cudaEventDisableTiming) != cudaSuccess) return false;
-  return true;
+      if (ok && !e && cudaEventCreateWithFlags(&e, cudaEventDisableTiming) != cudaSuccess) {
+        e = nullptr;
+        ok = false;
+      }
+  if (!ok) cudaGetLastError();  // the caller copies without them
+  return ok;
 }
 
 // Host arrays to the device on the upload stream; n->s waits for them.
@@ -222,8 +226,12 @@ int upload(cadmas_unet *n, std::initializer_list<Piece> pieces) {
       chunks.push_back({(char *)p.dst + o, (const char *)p.src + o, std::min(UP_CHUNK, p.bytes - o)});
   }
   cudaGetLastError();  // cudaPointerGetAttributes may leave an error for plain memory
+  if (!chunks.empty() && !upload_setup(n)) {  // no pinned memory to be had: as the small arrays
+    for (const Piece &c : chunks)
+      if (cudaMemcpyAsync(c.dst, c.src, c.bytes, cudaMemcpyHostToDevice, n->sc) != cudaSuccess) return CADMAS_ECUDA;
+    chunks.clear();
+  }
   if (!chunks.empty()) {
-    if (!upload_setup(n)) return CADMAS_ENOMEM;
     std::atomic<size_t> next{0};
     std::atomic<bool> bad{false};
     auto work = [&](int t) {
