@@ -2,10 +2,10 @@
 //
 //   k_vpcoef            VF_VPCOEF (vf_vpcoef.f:117-437)
 //   k_dcmp  (tile)      VF_MZDCMP (vf_mzdcmp.f:53-67)
-//   k_fwd   (tile)      VF_MZFRWD (vf_mzfrwd.f:37-48), optionally fused with
-//                       the SpMV VF_MZAX (vf_mzax.f:42-56) of its input
-//   k_bwd   (tile)      VF_MZBKWD (vf_mzbkwd.f:37-47)
-//   row kernels         the vector updates and VF_MZIP dot products of
+//   k_sweep_cp, k_sweep VF_MZFRWD (vf_mzfrwd.f:37-48), optionally fused with
+//    (tile)             the SpMV VF_MZAX (vf_mzax.f:42-56) of its input, and
+//                       VF_MZBKWD (vf_mzbkwd.f:37-47)
+//   slab, flat kernels  the vector updates and VF_MZIP dot products of
 //                       VF_M1BCGS (vf_m1bcgs.f:76-266)
 //   k_vmodif            VF_VMODIF (vf_vmodif.f:58-215)
 //
@@ -471,7 +471,8 @@ __global__ void k_dcmp(Geo g, SkewGeo q, V U, SkewSysT<V> S, int *pivot_bad) {
 // count); the T consumer threads wait on the mbarrier of the step they
 // need and then work purely from shared memory.  One block barrier per
 // step orders the exchange of the sweep values between neighbouring
-// columns and frees the slot of step s-2 for the producer.
+// columns and frees the slot of step s-2 for the producer.  launch_sweep says
+// which sweeps run in this form.
 __device__ __forceinline__ unsigned smem_u32(const void *p) { return (unsigned)__cvta_generic_to_shared(p); }
 __device__ __forceinline__ void mbar_init(unsigned bar, unsigned count) {
   asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;\n" ::"r"(bar), "r"(count) : "memory");
