@@ -66,7 +66,7 @@ STAGE_BYTES = {
 # the 256x32x96 flume with 16x16 and 8x16 blocks (the same sweep variants
 # as the bench's 512x32x96, one block per SM), so the traffic per launch
 # scales with the cells.
-NCU_TRAFFIC_PER_CELL = {(16, 16): {"fwd": 97.4, "bwd": 52.6}, (8, 16): {"fwd": 91.0, "bwd": 50.3}}
+NCU_TRAFFIC_PER_CELL = {(16, 16): {"fwd": 72.6, "bwd": 40.2}, (8, 16): {"fwd": 72.3, "bwd": 40.1}}
 
 
 def _load_pkg():
@@ -474,13 +474,11 @@ def roofline_of(stages, cells, peak, peak_kind, bytes_table, traffic_per_cell=No
 # DRAM bytes (dram__bytes_read.sum + dram__bytes_write.sum) per interior
 # cell of one launch of the dominant sweeps on the beach (1024x128x128,
 # 16x16 tiles), from an ncu capture of a 1024x80x128 beach: the same
-# layers, tile shape and sweep variants (320 tiles, two blocks per SM for
-# the backward and FP32 sweeps), so the traffic per launch scales with the
-# cells.  FP32 backward: the mean of the sweeps after AP (33.6) and after
-# AE (38.8); the four-blocks-per-SM instances that now run them on both
-# beaches issue the same bulk copies per step.
-NCU_TRAFFIC_BEACH = {"fwd": 99.8, "bwd": 57.9}
-NCU_TRAFFIC_BEACH_F32 = {"fwd": 49.9, "bwd": 36.2}
+# layers, tile shape and sweep variants (320 tiles), so the traffic per
+# launch scales with the cells.  FP32 backward: the mean of the sweeps after
+# AP (28.9) and after AE (33.6).
+NCU_TRAFFIC_BEACH = {"fwd": 85.4, "bwd": 49.4}
+NCU_TRAFFIC_BEACH_F32 = {"fwd": 42.3, "bwd": 31.3}
 
 
 def field_errors(a, b, case):

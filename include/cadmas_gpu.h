@@ -158,16 +158,11 @@ typedef struct cadmas_params {
      2 s.                                                                 */
   double wait_limit_s;
   /* Thread blocks of the MILU sweeps per SM (no counterpart in the
-     reference): 1 = one block per SM with the deepest bulk-copy ring; 2 =
-     two blocks per SM (registers capped, shallower ring), so that the
-     wavefronts of two tiles interleave on each SM; it needs blocks of at
-     most 256 columns and applies where the ring fits.  0 = the default:
-     two blocks for the backward sweeps and the FP32 sweeps when the grid
-     has at least two preconditioner blocks per SM, one otherwise; four
-     for the FP32 backward sweeps (the mixed solver's) of 16x16 blocks
-     (ring depth 4, at most 56 registers) when it has more than two per
-     SM.  4 = four blocks for those sweeps at any size, the default for
-     the others.  The results do not depend on it.                        */
+     reference): 1, 2 or 4 = the blocks to leave shared memory for (a
+     sweep's copy ring is as deep as its share allows); 0 = the default:
+     two where the grid has more preconditioner blocks than the GPU has
+     SMs and the ring keeps a depth of six steps, one otherwise.  The
+     results do not depend on it.                                         */
   int    sweep_occupancy;
   /* Inner products of the mixed solver's FP32 iteration (solver 1; no
      counterpart in the reference): 0 = summed by the backward MILU sweeps
