@@ -70,16 +70,6 @@ __device__ __forceinline__ bool cta_wait(uint64_t *bar, uint32_t parity) {
 }
 
 // ------------------------------------------------------------- k_conv
-constexpr int CONV_M = 128;
-// Tiling of one convolution: tiles of bx x by voxels, nxt x nyt of them per
-// layer; P = bx + 2 voxels per padded row; MT row blocks of 128; PL rows
-// of a staged layer (the last row block reads 2 P + 2 rows past its own);
-// NST stages (3: all layers resident, 2: the third reuses the first's).
-struct ConvPlan {
-  int bx, by, nxt, nyt, P, PL, MT, NST;
-  uint32_t a_bytes, b_bytes;  // of one stage
-  size_t smem;
-};
 constexpr int CONV_T = 256;  // threads: eight warps share the copies and the epilogue's row blocks
 __global__ void __launch_bounds__(CONV_T) k_conv(Vol g, const bf16 *__restrict__ X, int Cin,
                                               const bf16 *__restrict__ W, const float *__restrict__ bias,
@@ -741,45 +731,6 @@ __global__ void k_fill_bf16(long long n, bf16 *a) {
 // ------------------------------------------------------------ launchers
 static inline unsigned nb(long long n, int t) { return (unsigned)((n + t - 1) / t); }
 
-// The CTAs that share an SM must find their TMEM columns free (512 per
-// SM): a CTA with more columns asks for more shared memory.
-static size_t smem_floor(size_t b, uint32_t cols) {
-  const size_t f = cols <= 128 ? 56 * 1024 : (cols <= 256 ? 80 * 1024 : 120 * 1024);
-  return b < f ? f : b;
-}
-// Tile of a convolution: rows of at most 126 voxels; as many rows as make
-// the least work per voxel, counting the MMAs' rows (128 per row block) and
-// half as much for each staged voxel, within the shared memory of two CTAs
-// per SM where that can be (else of one) and 256 TMEM columns (one row block
-// may use more).  Three stages where they fit.
-static ConvPlan conv_plan(const Vol &g, int Cin, int Cout) {
-  ConvPlan best{};
-  double cost = 0.0;
-  const int nxt0 = (g.X + 125) / 126;
-  for (size_t cap : {(size_t)112 * 1024, (size_t)225 * 1024}) {
-    for (int nxt = nxt0; nxt <= nxt0 + 3; ++nxt)
-      for (int nst = 3; nst >= 2; --nst) {
-        const int bx = (g.X + nxt - 1) / nxt, P = bx + 2;
-        for (int by = 1; by <= g.Y && by <= 128; ++by) {
-          ConvPlan p{};
-          p.bx = bx; p.by = by; p.nxt = nxt; p.nyt = (g.Y + by - 1) / by; p.P = P; p.NST = nst;
-          p.MT = (by * P + CONV_M - 1) / CONV_M;
-          if (p.MT > 1 && p.MT * Cout > 256) break;
-          p.PL = (p.MT * CONV_M + 2 * P + 2 + 7) & ~7;
-          p.PL += 4;  // the two 8-channel rows of a voxel in different banks
-          p.a_bytes = (uint32_t)(Cin / 8 * p.PL * 16);
-          p.b_bytes = (uint32_t)(9 * Cin * Cout * 2);
-          const size_t need = (size_t)nst * (p.a_bytes + p.b_bytes) + 64;
-          if (need > cap) break;
-          p.smem = smem_floor(need, umma::tmem_cols(p.MT * Cout));
-          const double c = (double)nxt * p.nyt * (p.MT * 128.0 + 0.5 * (by + 2) * P + 128.0) * (nst == 2 ? 1.15 : 1.0);
-          if (best.MT == 0 || c < cost) { best = p; cost = c; }
-        }
-      }
-    if (best.MT > 0) break;
-  }
-  return best;
-}
 static size_t wgrad_smem_bytes(int Cout, int WG_ST) {
   return smem_floor((size_t)WG_ST * (128 + Cout) * WG_K * 2 + 64, umma::tmem_cols(Cout));
 }
@@ -796,10 +747,9 @@ bool unet_kernels_configure() {
   return ok;
 }
 
-void launch_conv(cudaStream_t s, int X, int Y, int Z, int B, const void *x, int Cin, const void *w, const float *bias,
-                 int Cout, int mode, const void *mask, void *y, int *err) {
+void launch_conv(cudaStream_t s, const ConvPlan &p, int X, int Y, int Z, int B, const void *x, int Cin, const void *w,
+                 const float *bias, int Cout, int mode, const void *mask, void *y, int *err) {
   const Vol g{X, Y, Z, B};
-  const ConvPlan p = conv_plan(g, Cin, Cout);
   k_conv<<<(unsigned)((long long)p.nxt * p.nyt * Z * B), CONV_T, p.smem, s>>>(
       g, (const bf16 *)x, Cin, (const bf16 *)w, bias, Cout, mode, (const bf16 *)mask, y, err, p);
   count_launch();

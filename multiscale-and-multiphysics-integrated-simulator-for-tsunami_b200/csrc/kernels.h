@@ -3,6 +3,7 @@
 #include <cuda_runtime.h>
 #include <atomic>
 #include "cadmas_dev.cuh"
+#include "conv_plan.h"
 #include "wavetheory.cuh"
 
 namespace cadmas {
@@ -416,8 +417,8 @@ void launch_fconv(cudaStream_t s, const Geo &g, const Fld &f, const Prm &p, doub
 enum { CONV_BF16 = 0, CONV_RELU_BF16 = 1, CONV_MASK_BF16 = 2, CONV_F32 = 3 };
 bool unet_kernels_configure();
 long long wgrad_slices(long long V);
-void launch_conv(cudaStream_t s, int X, int Y, int Z, int B, const void *x, int Cin, const void *w, const float *bias,
-                 int Cout, int mode, const void *mask, void *y, int *err);
+void launch_conv(cudaStream_t s, const ConvPlan &p, int X, int Y, int Z, int B, const void *x, int Cin, const void *w,
+                 const float *bias, int Cout, int mode, const void *mask, void *y, int *err);
 void launch_wgrad(cudaStream_t s, int X, int Y, int Z, int B, const void *x, int Cin, const void *dy, int Cout,
                   float *part, float *dw, int *err);
 void launch_bias_grad(cudaStream_t s, long long V, const void *dy, int C, float *part, float *db);

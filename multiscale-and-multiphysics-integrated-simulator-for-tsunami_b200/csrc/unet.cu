@@ -72,6 +72,7 @@ struct cadmas_unet {
   float *p = nullptr, *g = nullptr, *m = nullptr, *v = nullptr;
   long long step = 0;
   void *wf[NL] = {}, *wt[NL] = {};
+  ConvPlan pf[NL] = {}, pt[NL] = {};  // tilings of layer l's convolution and of its input gradient
   // activations (BF16) and their gradients
   void *xin = nullptr, *a[NL] = {}, *p1 = nullptr, *p2 = nullptr, *u2 = nullptr, *u1 = nullptr;
   void *d[NL] = {}, *du2 = nullptr, *du1 = nullptr, *dp1 = nullptr, *dp2 = nullptr;
@@ -98,11 +99,22 @@ void dims(const cadmas_unet *n, int res, int &X, int &Y, int &Z) {
   Z = n->Z >> res;
 }
 
-void conv(cadmas_unet *n, int res, const void *x, int cin, const void *w, const float *b, int cout, int mode,
-          const void *mask, void *y) {
+// convolution of layer l with ReLU
+void conv(cadmas_unet *n, int l, const void *x) {
+  const Layer &L = TAB.L[l];
   int X, Y, Z;
-  dims(n, res, X, Y, Z);
-  launch_conv(n->s, X, Y, Z, n->B, x, cin, w, b, cout, mode, mask, y, n->err);
+  dims(n, L.res, X, Y, Z);
+  launch_conv(n->s, n->pf[l], X, Y, Z, n->B, x, L.cin, n->wf[l], n->p + L.b, L.cout, CONV_RELU_BF16, nullptr, n->a[l],
+              n->err);
+}
+// its input gradient, times the ReLU derivative of the layer below where
+// `mask` gives that layer's activations
+void conv_t(cadmas_unet *n, int l, const void *mask, void *dx) {
+  const Layer &L = TAB.L[l];
+  int X, Y, Z;
+  dims(n, L.res, X, Y, Z);
+  launch_conv(n->s, n->pt[l], X, Y, Z, n->B, n->d[l], L.cout, n->wt[l], nullptr, L.cin, mask ? CONV_MASK_BF16 : CONV_BF16,
+              mask, dx, n->err);
 }
 
 void cast_weights(cadmas_unet *n) {
@@ -120,22 +132,21 @@ int check(cadmas_unet *n) {
 
 // forward of the batch in n->x4 (FP32, 4 channels) to n->y
 void forward(cadmas_unet *n) {
-  const auto &L = TAB.L;
   launch_pack_in(n->s, n->V[0], n->x4, n->xin);
-  conv(n, 0, n->xin, 16, n->wf[0], n->p + L[0].b, 16, CONV_RELU_BF16, nullptr, n->a[0]);
-  conv(n, 0, n->a[0], 16, n->wf[1], n->p + L[1].b, 16, CONV_RELU_BF16, nullptr, n->a[1]);
+  conv(n, 0, n->xin);
+  conv(n, 1, n->a[0]);
   launch_pool(n->s, n->X / 2, n->Y / 2, n->Z / 2, n->B, n->a[1], 16, n->p1);
-  conv(n, 1, n->p1, 16, n->wf[2], n->p + L[2].b, 32, CONV_RELU_BF16, nullptr, n->a[2]);
-  conv(n, 1, n->a[2], 32, n->wf[3], n->p + L[3].b, 32, CONV_RELU_BF16, nullptr, n->a[3]);
+  conv(n, 2, n->p1);
+  conv(n, 3, n->a[2]);
   launch_pool(n->s, n->X / 4, n->Y / 4, n->Z / 4, n->B, n->a[3], 32, n->p2);
-  conv(n, 2, n->p2, 32, n->wf[4], n->p + L[4].b, 64, CONV_RELU_BF16, nullptr, n->a[4]);
-  conv(n, 2, n->a[4], 64, n->wf[5], n->p + L[5].b, 64, CONV_RELU_BF16, nullptr, n->a[5]);
+  conv(n, 4, n->p2);
+  conv(n, 5, n->a[4]);
   launch_upcat(n->s, n->X / 2, n->Y / 2, n->Z / 2, n->B, n->a[5], 64, n->a[3], 32, n->u2);
-  conv(n, 1, n->u2, 96, n->wf[6], n->p + L[6].b, 32, CONV_RELU_BF16, nullptr, n->a[6]);
-  conv(n, 1, n->a[6], 32, n->wf[7], n->p + L[7].b, 32, CONV_RELU_BF16, nullptr, n->a[7]);
+  conv(n, 6, n->u2);
+  conv(n, 7, n->a[6]);
   launch_upcat(n->s, n->X, n->Y, n->Z, n->B, n->a[7], 32, n->a[1], 16, n->u1);
-  conv(n, 0, n->u1, 48, n->wf[8], n->p + L[8].b, 16, CONV_RELU_BF16, nullptr, n->a[8]);
-  conv(n, 0, n->a[8], 16, n->wf[9], n->p + L[9].b, 16, CONV_RELU_BF16, nullptr, n->a[9]);
+  conv(n, 8, n->u1);
+  conv(n, 9, n->a[8]);
   launch_head(n->s, n->V[0], n->a[9], 16, n->p + TAB.head_w, n->p + TAB.head_b, n->y);
 }
 
@@ -155,33 +166,33 @@ void backward(cadmas_unet *n) {
   launch_bias_reduce(n->s, n->bpart, nbh, 17, n->g + TAB.head_w);
   // c52, c51
   layer_grads(n, 9, n->a[8], n->d[9]);
-  conv(n, 0, n->d[9], 16, n->wt[9], nullptr, 16, CONV_MASK_BF16, n->a[8], n->d[8]);
+  conv_t(n, 9, n->a[8], n->d[8]);
   layer_grads(n, 8, n->u1, n->d[8]);
-  conv(n, 0, n->d[8], 16, n->wt[8], nullptr, 48, CONV_MASK_BF16, n->u1, n->du1);
+  conv_t(n, 8, n->u1, n->du1);
   // split: d of c42's output (coarse, 32) and of skip1 (16)
   launch_upcat_bwd(n->s, n->X, n->Y, n->Z, n->B, n->du1, 32, 16, n->d[7], n->d[1]);
   // c42, c41
   layer_grads(n, 7, n->a[6], n->d[7]);
-  conv(n, 1, n->d[7], 32, n->wt[7], nullptr, 32, CONV_MASK_BF16, n->a[6], n->d[6]);
+  conv_t(n, 7, n->a[6], n->d[6]);
   layer_grads(n, 6, n->u2, n->d[6]);
-  conv(n, 1, n->d[6], 32, n->wt[6], nullptr, 96, CONV_MASK_BF16, n->u2, n->du2);
+  conv_t(n, 6, n->u2, n->du2);
   launch_upcat_bwd(n->s, n->X / 2, n->Y / 2, n->Z / 2, n->B, n->du2, 64, 32, n->d[5], n->d[3]);
   // c32, c31
   layer_grads(n, 5, n->a[4], n->d[5]);
-  conv(n, 2, n->d[5], 64, n->wt[5], nullptr, 64, CONV_MASK_BF16, n->a[4], n->d[4]);
+  conv_t(n, 5, n->a[4], n->d[4]);
   layer_grads(n, 4, n->p2, n->d[4]);
-  conv(n, 2, n->d[4], 64, n->wt[4], nullptr, 32, CONV_BF16, nullptr, n->dp2);
+  conv_t(n, 4, nullptr, n->dp2);
   // skip2 gets the pooled path too, then the ReLU of c22
   launch_pool_bwd(n->s, n->X / 4, n->Y / 4, n->Z / 4, n->B, n->dp2, 32, n->d[3], n->a[3]);
   // c22, c21
   layer_grads(n, 3, n->a[2], n->d[3]);
-  conv(n, 1, n->d[3], 32, n->wt[3], nullptr, 32, CONV_MASK_BF16, n->a[2], n->d[2]);
+  conv_t(n, 3, n->a[2], n->d[2]);
   layer_grads(n, 2, n->p1, n->d[2]);
-  conv(n, 1, n->d[2], 32, n->wt[2], nullptr, 16, CONV_BF16, nullptr, n->dp1);
+  conv_t(n, 2, nullptr, n->dp1);
   launch_pool_bwd(n->s, n->X / 2, n->Y / 2, n->Z / 2, n->B, n->dp1, 16, n->d[1], n->a[1]);
   // c12, c11
   layer_grads(n, 1, n->a[0], n->d[1]);
-  conv(n, 0, n->d[1], 16, n->wt[1], nullptr, 16, CONV_MASK_BF16, n->a[0], n->d[0]);
+  conv_t(n, 1, n->a[0], n->d[0]);
   layer_grads(n, 0, n->xin, n->d[0]);
 }
 
@@ -329,6 +340,15 @@ int unet_new(int nx, int ny, int nz, int batch, cudaStream_t stream, cadmas_unet
   if (!unet_kernels_configure()) return CADMAS_ECUDA;
   cadmas_unet *n = new cadmas_unet();
   n->X = nx; n->Y = ny; n->Z = nz; n->B = batch;
+  for (int l = 0; l < NL; ++l) {
+    const Layer &L = TAB.L[l];
+    n->pf[l] = conv_plan(nx >> L.res, ny >> L.res, L.cin, L.cout);
+    if (l > 0) n->pt[l] = conv_plan(nx >> L.res, ny >> L.res, L.cout, L.cin);
+    if (n->pf[l].MT == 0 || (l > 0 && n->pt[l].MT == 0)) {
+      delete n;
+      return CADMAS_EUNSUPPORTED;
+    }
+  }
   for (int r = 0; r < 3; ++r) n->V[r] = (long long)(nx >> r) * (ny >> r) * (nz >> r) * batch;
   int rc = CADMAS_OK;
   if (stream) {
