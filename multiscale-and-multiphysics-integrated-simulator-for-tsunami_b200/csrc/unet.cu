@@ -215,7 +215,12 @@ bool upload_setup(cadmas_unet *n) {
   return ok;
 }
 
-// Host arrays to the device on the upload stream; n->s waits for them.
+// Whether the launches since the last look went through: looked at before
+// anything that may clear the runtime's last error.
+int launched() { return cudaGetLastError() == cudaSuccess ? CADMAS_OK : CADMAS_ECUDA; }
+
+// Host arrays to the device on the upload stream; n->s waits for them.  It
+// may clear the runtime's last error.
 // Small or pinned arrays go straight; pageable ones in chunks through the
 // pinned buffers.  Returns when the arrays have been read or the copies of
 // the pinned ones are queued (every entry point synchronises before it
@@ -227,16 +232,19 @@ int upload(cadmas_unet *n, std::initializer_list<Piece> pieces) {
   size_t total = 0;
   for (const Piece &p : pieces) total += p.bytes;
   for (const Piece &p : pieces) {
-    cudaPointerAttributes at{};
-    if (total < UP_MIN ||
-        (cudaPointerGetAttributes(&at, p.src) == cudaSuccess && at.type != cudaMemoryTypeUnregistered)) {
+    bool straight = total < UP_MIN;
+    if (!straight) {
+      cudaPointerAttributes at{};
+      if (cudaPointerGetAttributes(&at, p.src) == cudaSuccess) straight = at.type != cudaMemoryTypeUnregistered;
+      else cudaGetLastError();  // plain memory, to older drivers
+    }
+    if (straight) {
       if (cudaMemcpyAsync(p.dst, p.src, p.bytes, cudaMemcpyHostToDevice, n->sc) != cudaSuccess) return CADMAS_ECUDA;
       continue;
     }
     for (size_t o = 0; o < p.bytes; o += UP_CHUNK)
       chunks.push_back({(char *)p.dst + o, (const char *)p.src + o, std::min(UP_CHUNK, p.bytes - o)});
   }
-  cudaGetLastError();  // cudaPointerGetAttributes may leave an error for plain memory
   if (!chunks.empty() && !upload_setup(n)) {  // no pinned memory to be had: as the small arrays
     for (const Piece &c : chunks)
       if (cudaMemcpyAsync(c.dst, c.src, c.bytes, cudaMemcpyHostToDevice, n->sc) != cudaSuccess) return CADMAS_ECUDA;
@@ -462,7 +470,9 @@ int cadmas_unet_grad(cadmas_unet *n, const float *x, const float *t, const float
   if (rc) return rc;
   forward(n);
   double cnt_inv = 0.0, l = 0.0;
-  if ((rc = upload(n, {{n->t, t, V * sizeof(float)}, {n->mk, m, V * sizeof(float)}})) || (rc = mask_inv(n, cnt_inv)))
+  if ((rc = launched()) ||
+      (rc = upload(n, {{n->t, t, V * sizeof(float)}, {n->mk, m, V * sizeof(float)}})) ||
+      (rc = mask_inv(n, cnt_inv)))
     return rc;
   const float inv = (float)cnt_inv;
   launch_mse(n->s, V, n->y, n->t, n->mk, inv, n->dy, n->lpart);
@@ -484,7 +494,8 @@ int cadmas_unet_train_sys(cadmas_unet *n, const float *x, const float *t, const 
   if (rc) return rc;
   forward(n);
   double inv = 0.0, l[2];
-  if ((rc = upload(n, {{n->mk, m, V * sizeof(float)}, {n->t, t, V * sizeof(float)}, {n->a7, a7, V * 7 * sizeof(float)}})) ||
+  if ((rc = launched()) ||
+      (rc = upload(n, {{n->mk, m, V * sizeof(float)}, {n->t, t, V * sizeof(float)}, {n->a7, a7, V * 7 * sizeof(float)}})) ||
       (rc = mask_inv(n, inv)))
     return rc;
   // mean-square error of y against t, weighted by w_mse in the gradient;
