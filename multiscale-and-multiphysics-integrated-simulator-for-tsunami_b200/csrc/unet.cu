@@ -130,6 +130,16 @@ int check(cadmas_unet *n) {
   return e ? CADMAS_ETIMEOUT : CADMAS_OK;
 }
 
+// The end of an entry point: after an error, waits for what is still queued,
+// so that nothing reads or writes the caller's arrays any more.
+int leave(cadmas_unet *n, int rc) {
+  if (rc) {
+    cudaStreamSynchronize(n->sc);
+    cudaStreamSynchronize(n->s);
+  }
+  return rc;
+}
+
 // forward of the batch in n->x4 (FP32, 4 channels) to n->y
 void forward(cadmas_unet *n) {
   launch_pack_in(n->s, n->V[0], n->x4, n->xin);
@@ -223,8 +233,8 @@ int launched() { return cudaGetLastError() == cudaSuccess ? CADMAS_OK : CADMAS_E
 // may clear the runtime's last error.
 // Small or pinned arrays go straight; pageable ones in chunks through the
 // pinned buffers.  Returns when the arrays have been read or the copies of
-// the pinned ones are queued (every entry point synchronises before it
-// returns to their owner).
+// the pinned ones are queued (the entry points wait for them before they
+// return to the arrays' owner: check(), and leave() after an error).
 int upload(cadmas_unet *n, std::initializer_list<Piece> pieces) {
   int dev = 0;
   if (cudaGetDevice(&dev) != cudaSuccess) return CADMAS_ECUDA;
@@ -417,10 +427,7 @@ int unet_error_host(cadmas_unet *n) { return check(n); }
 
 }  // namespace cadmas
 
-extern "C" {
-
-int cadmas_unet_set_params(cadmas_unet *n, const float *p) {
-  if (!n || !p) return CADMAS_EINVAL;
+static int set_params(cadmas_unet *n, const float *p) {
   if (cudaMemcpyAsync(n->p, p, TAB.n * sizeof(float), cudaMemcpyHostToDevice, n->s) != cudaSuccess)
     return CADMAS_ECUDA;
   cudaMemsetAsync(n->m, 0, TAB.n * sizeof(float), n->s);
@@ -430,15 +437,13 @@ int cadmas_unet_set_params(cadmas_unet *n, const float *p) {
   return check(n);
 }
 
-int cadmas_unet_get_params(cadmas_unet *n, float *p) {
-  if (!n || !p) return CADMAS_EINVAL;
+static int get_params(cadmas_unet *n, float *p) {
   if (cudaMemcpyAsync(p, n->p, TAB.n * sizeof(float), cudaMemcpyDeviceToHost, n->s) != cudaSuccess)
     return CADMAS_ECUDA;
   return check(n);
 }
 
-int cadmas_unet_forward(cadmas_unet *n, const float *x, float *y) {
-  if (!n || !x || !y) return CADMAS_EINVAL;
+static int forward_host(cadmas_unet *n, const float *x, float *y) {
   int rc = upload(n, {{n->x4, x, n->V[0] * 4 * sizeof(float)}});
   if (rc) return rc;
   forward(n);
@@ -447,8 +452,7 @@ int cadmas_unet_forward(cadmas_unet *n, const float *x, float *y) {
   return check(n);
 }
 
-int cadmas_unet_time_forward(cadmas_unet *n, int reps, float *ms) {
-  if (!n || reps < 1 || !ms) return CADMAS_EINVAL;
+static int time_forward(cadmas_unet *n, int reps, float *ms) {
   cudaEvent_t e0, e1;
   if (cudaEventCreate(&e0) != cudaSuccess || cudaEventCreate(&e1) != cudaSuccess) return CADMAS_ECUDA;
   cudaEventRecord(e0, n->s);
@@ -463,8 +467,7 @@ int cadmas_unet_time_forward(cadmas_unet *n, int reps, float *ms) {
   return rc;
 }
 
-int cadmas_unet_grad(cadmas_unet *n, const float *x, const float *t, const float *m, float *loss, float *grad) {
-  if (!n || !x || !t || !m || !loss) return CADMAS_EINVAL;
+static int grad_host(cadmas_unet *n, const float *x, const float *t, const float *m, float *loss, float *grad) {
   const long long V = n->V[0];
   int rc = upload(n, {{n->x4, x, V * 4 * sizeof(float)}});
   if (rc) return rc;
@@ -484,9 +487,8 @@ int cadmas_unet_grad(cadmas_unet *n, const float *x, const float *t, const float
   return check(n);
 }
 
-int cadmas_unet_train_sys(cadmas_unet *n, const float *x, const float *t, const float *m, const float *a7, float c,
-                          float w_mse, float w_res, float lr, int update, float *loss, float *grad) {
-  if (!n || !x || !t || !m || !a7 || !loss || !(c > 0.0f)) return CADMAS_EINVAL;
+static int train_sys(cadmas_unet *n, const float *x, const float *t, const float *m, const float *a7, float c,
+                     float w_mse, float w_res, float lr, int update, float *loss, float *grad) {
   const long long V = n->V[0];
   if (!n->a7 && (dmalloc(&n->a7, (size_t)V * 7) || dmalloc(&n->r, (size_t)V))) return CADMAS_ENOMEM;
   // the forward runs while the targets, masks and systems come
@@ -519,8 +521,8 @@ int cadmas_unet_train_sys(cadmas_unet *n, const float *x, const float *t, const 
   return check(n);
 }
 
-int cadmas_unet_train_step(cadmas_unet *n, const float *x, const float *t, const float *m, float lr, float *loss) {
-  int rc = cadmas_unet_grad(n, x, t, m, loss, nullptr);
+static int train_step(cadmas_unet *n, const float *x, const float *t, const float *m, float lr, float *loss) {
+  int rc = grad_host(n, x, t, m, loss, nullptr);
   if (rc) return rc;
   n->step += 1;
   const float b1 = 0.9f, b2 = 0.999f;
@@ -528,6 +530,36 @@ int cadmas_unet_train_step(cadmas_unet *n, const float *x, const float *t, const
   launch_adam(n->s, (long long)TAB.n, n->p, n->g, n->m, n->v, lr, b1, b2, 1.0e-8f, c1, c2);
   cast_weights(n);
   return check(n);
+}
+
+extern "C" {
+
+int cadmas_unet_set_params(cadmas_unet *n, const float *p) {
+  return n && p ? leave(n, set_params(n, p)) : CADMAS_EINVAL;
+}
+
+int cadmas_unet_get_params(cadmas_unet *n, float *p) { return n && p ? leave(n, get_params(n, p)) : CADMAS_EINVAL; }
+
+int cadmas_unet_forward(cadmas_unet *n, const float *x, float *y) {
+  return n && x && y ? leave(n, forward_host(n, x, y)) : CADMAS_EINVAL;
+}
+
+int cadmas_unet_time_forward(cadmas_unet *n, int reps, float *ms) {
+  return n && reps >= 1 && ms ? leave(n, time_forward(n, reps, ms)) : CADMAS_EINVAL;
+}
+
+int cadmas_unet_grad(cadmas_unet *n, const float *x, const float *t, const float *m, float *loss, float *grad) {
+  return n && x && t && m && loss ? leave(n, grad_host(n, x, t, m, loss, grad)) : CADMAS_EINVAL;
+}
+
+int cadmas_unet_train_sys(cadmas_unet *n, const float *x, const float *t, const float *m, const float *a7, float c,
+                          float w_mse, float w_res, float lr, int update, float *loss, float *grad) {
+  if (!n || !x || !t || !m || !a7 || !loss || !(c > 0.0f)) return CADMAS_EINVAL;
+  return leave(n, train_sys(n, x, t, m, a7, c, w_mse, w_res, lr, update, loss, grad));
+}
+
+int cadmas_unet_train_step(cadmas_unet *n, const float *x, const float *t, const float *m, float lr, float *loss) {
+  return n && x && t && m && loss ? leave(n, train_step(n, x, t, m, lr, loss)) : CADMAS_EINVAL;
 }
 
 }  // extern "C"

@@ -31,3 +31,7 @@ def run(exe, mode):
 
 def test_failed_launches_are_reported(exe):
     run(exe, "launch")
+
+
+def test_nothing_is_queued_after_a_call(exe):
+    run(exe, "runtime")
