@@ -131,7 +131,7 @@ struct cadmas_handle {
   double *xw = nullptr, *y2 = nullptr, *r0 = nullptr, *rr = nullptr, *pv = nullptr,
          *ap = nullptr, *ae = nullptr;
   double *rb0 = nullptr, *rb1 = nullptr, *dres = nullptr;
-  double *rb5 = nullptr;  // 5 x nslab sum partials of the regrouped FP32 iteration (solver 1)
+  double *rb5 = nullptr;  // 5 x sum_partials of the regrouped FP32 iteration (solver 1)
   // skewed-layout copies of the system for the MILU kernels, and the
   // forward-sweep result
   SkewGeo q;
@@ -1127,7 +1127,7 @@ int cadmas_create(const cadmas_dims *d, const cadmas_params *p, cadmas_handle **
   h->q.WS = (TI - 1) + (TJl - 1) <= d->numk - 2 ? d->numk - 2 : h->q.W;
   h->nsl = (size_t)skew_entries(h->q);
   h->nslab = (long long)h->q.nb * h->q.W;
-  h->nrb = (h->nslab + ROWS_PER_BLOCK - 1) / ROWS_PER_BLOCK;
+  h->nrb = slab_partials(h->q);
   {
     const size_t nsl = h->nsl;
     AL(h->S.sys, (size_t)SYS_N * nsl);
@@ -1142,7 +1142,7 @@ int cadmas_create(const cadmas_dims *d, const cadmas_params *p, cadmas_handle **
       AL(h->Sf.sys, (size_t)SYS_N * nsl);
       AL(h->bf, nsl); AL(h->xf, nsl); AL(h->r0f, nsl); AL(h->rrf, nsl); AL(h->pvf, nsl);
       AL(h->apf, nsl); AL(h->aef, nsl); AL(h->y2f, nsl);
-      AL(h->rb5, 5 * (size_t)h->nrb);
+      AL(h->rb5, 5 * (size_t)sum_partials(h->q));
     } else if (p->solver != 0) {
       rc = rc ? rc : CADMAS_EINVAL;
     }

@@ -1852,9 +1852,7 @@ bool launch_bwd_f_dot5(cudaStream_t s, const Geo &g, const SkewGeo &q, const Ske
                        const float *rr, float *x, double *rb, SolveState *st) {
   return launch_bwd_dots<SWEEP_BWD5>(s, g, q, S, r0, rr, x, rb, st);
 }
-static inline unsigned slab_blocks(const SkewGeo &q) {
-  return (unsigned)(((long long)q.nb * q.W + ROWS_PER_BLOCK - 1) / ROWS_PER_BLOCK);
-}
+static inline unsigned slab_blocks(const SkewGeo &q) { return (unsigned)slab_partials(q); }
 #define SL(kern, ...) launch_pdl(kern, dim3(slab_blocks(q)), dim3(ROW_THREADS), 0, s, 1, __VA_ARGS__)
 static inline unsigned flat_blocks(const SkewGeo &q) { return (unsigned)((skew_entries(q) + FLAT_BLOCK - 1) / FLAT_BLOCK); }
 #define FL(kern, ...) launch_pdl(kern, dim3(flat_blocks(q)), dim3(256), 0, s, 1, __VA_ARGS__)

@@ -70,6 +70,11 @@ __host__ __device__ inline long long skew_slabs(const SkewGeo &q) {
   return (long long)q.nb * skew_stride(q) + (q.W - skew_stride(q));
 }
 __host__ __device__ inline long long skew_entries(const SkewGeo &q) { return skew_slabs(q) * q.T; }
+// Partials of a sum over the grid: a slab sum leaves one per block of
+// ROWS_PER_BLOCK wavefront slabs, a backward sweep with sums one per tile,
+// which is more where a tile has fewer slabs than that.
+inline long long slab_partials(const SkewGeo &q) { return ((long long)q.nb * q.W + ROWS_PER_BLOCK - 1) / ROWS_PER_BLOCK; }
+inline long long sum_partials(const SkewGeo &q) { return slab_partials(q) > q.nb ? slab_partials(q) : q.nb; }
 // SYS_T of column t
 __host__ __device__ inline long long sys_t(long long slab, int T, int t) { return slab * SYS_N * T + t; }
 // chunk c of column t
