@@ -1119,6 +1119,7 @@ int cadmas_create(const cadmas_dims *d, const cadmas_params *p, cadmas_handle **
   h->q.ntx = (d->numi - 2 + TI - 1) / TI;
   h->q.nb = h->q.ntx * ((d->numj - 2 + TJl - 1) / TJl);
   h->q.occ = (p->sweep_occupancy == 1 || p->sweep_occupancy == 2 || p->sweep_occupancy == 4) ? p->sweep_occupancy : 0;
+  h->q.nsm = sm_count();
   if (!sweep_supported(h->q)) {
     g_last_error = "preconditioner block too large for the MILU sweeps; set precond_ti/precond_tj";
     rc = CADMAS_EUNSUPPORTED;

@@ -1673,35 +1673,6 @@ static int sweep_depth(const SkewGeo &q, int mode, int es) {
 // bulk-copy ring (k_sweep) serves clusters (split 2), tiles one column wide
 // and handles with the stall injection on (SkewGeo::ring), whose subject is
 // the ring's waits.
-//
-// Depth of the thread copies: a step (0.1 to 0.35 us) is far shorter than the
-// latency of a copy, so as deep as the shared memory allows, shared by two
-// blocks per SM where there are more tiles than SMs (by q.occ blocks if that
-// is set) as long as that leaves depth 6.  Measured, us per sweep: 128 tiles
-// of 8x16 x 96 layers, FP64, depths 4, 8, 12: fused forward 34.8, 28.8, 26.8;
-// backward depths 4, 7, 15: 21.2, 14.5, 14.5 (in a solve, where the
-// system comes from memory, 19.6 at 7).  512 tiles of 16x16 x 126 layers: FP64
-// fused, one block at depth 8 242, at 6 250, two at 4 255; FP32 fused, two at
-// depth 6 132, one 143; backward FP64 at depth 7, one block 139, two 141.
-static int sweep_cp_threads(int T) { return (T + 31) & ~31; }
-static bool sweep_cp_unrolled(const SkewGeo &q, int mode, int es) {
-  const bool ct = (q.T == 128 && (q.TIp == 8 || q.TIp == 16)) || (q.T == 256 && q.TIp == 16);
-  return sweep_cp_unroll(mode, ct ? q.T : 0, es);
-}
-static int sweep_cp_depth(const SkewGeo &q, int mode, int es) {
-  if (q.split != 1 || q.TI < 2 || q.TJ < 2) return 0;
-  const int nt = sweep_cp_threads(q.T), blocks = q.occ > 0 ? q.occ : (q.nb > 148 ? 2 : 1);
-  const bool unr = sweep_cp_unrolled(q, mode, es);
-  const int ax[] = {12, 8, 6, 4, 2, 1}, plain[] = {15, 9, 3, 1};
-  for (size_t share : {226 * 1024 / (size_t)blocks, (size_t)(227 * 1024)})
-    for (int i = 0; i < (mode == SWEEP_FWD_AX ? 6 : 4); ++i) {
-      const int d = mode == SWEEP_FWD_AX ? ax[i] : plain[i];
-      if ((d >= 12 && nt > 128) || (d == 1 && nt <= 576)) continue;
-      if (q.occ == 0 && blocks > 1 && share < 227 * 1024 && d < 6) continue;
-      if (sweep_cp_bytes(mode, d, unr, q.T, q.TIp, q.TI, q.TJ, es) <= share) return d;
-    }
-  return 0;
-}
 template <int D, int MODE, int MAXT, typename V, int MINB>
 static void sweep_cp_go(cudaStream_t s, const Geo &g, const SkewGeo &q, const SkewSysT<V> &S, const V *vin, V *vout,
                         SolveState *st, const V *vin2, double *rb) {

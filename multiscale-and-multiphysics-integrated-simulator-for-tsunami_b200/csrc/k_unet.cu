@@ -766,7 +766,7 @@ void launch_wgrad(cudaStream_t s, int X, int Y, int Z, int B, const void *x, int
   dim3 grid((27 * Cin + 127) / 128, ns);
   // Where the CTAs leave the SMs half empty, eight stages (one CTA per SM)
   // hide the copies' latency; else three stages and up to four CTAs do.
-  if ((long long)grid.x * grid.y <= 2 * 148)
+  if ((long long)grid.x * grid.y <= 2 * sm_count())
     k_wgrad<8><<<grid, 128, wgrad_smem_bytes(Cout, 8), s>>>(g, (const bf16 *)x, Cin, (const bf16 *)dy, Cout, WGRAD_SLICE,
                                                             part, err);
   else

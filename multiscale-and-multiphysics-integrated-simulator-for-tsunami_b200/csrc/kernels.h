@@ -16,6 +16,13 @@ inline void count_launch(long long n = 1) { g_kernel_launches.fetch_add(n, std::
 // stepped from several host threads at once never take it away from one
 // another's launches.
 void raise_dynamic_smem(const void *kern, size_t bytes);
+// SMs of the current device (148, a B200's, where the runtime does not say).
+inline int sm_count() {
+  int dev = 0, n = 0;
+  if (cudaGetDevice(&dev) != cudaSuccess || cudaDeviceGetAttribute(&n, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess)
+    return 148;
+  return n > 0 ? n : 148;
+}
 // Record the failing CUDA call and its message as the text cadmas_strerror
 // gives for CADMAS_ECUDA on this host thread.
 void set_cuda_error(const char *call, cudaError_t e);
@@ -60,6 +67,7 @@ struct SkewGeo {
   int WS;                 // slabs from one tile's start to the next's (0: W)
   int ntx, nb;            // layout tiles along x, tiles in total
   int split;  // layout tiles per preconditioner block along y (1 or 2)
+  int nsm;    // the device's SMs
   int occ;    // thread blocks of the sweeps per SM to leave shared memory for (0: one, at full depth)
   int ring;   // 1: the sweeps' bulk-copy form (the stall injection's subject), 0: by the rule of launch_sweep
 };
