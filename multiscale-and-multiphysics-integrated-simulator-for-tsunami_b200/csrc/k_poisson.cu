@@ -597,15 +597,16 @@ __device__ __forceinline__ void cluster_barrier() {
 // INDC = -1 and a positive (or NaN) DD elsewhere, and a zero or negative
 // pivot ends the solve before any sweep runs.
 //
-// Only the recurrence sits between two block barriers: the neighbours'
+// Between two block barriers lie the recurrence of step s (the neighbours'
 // results of step s-1 are read, combined in five dependent operations and
-// published.  Everything that does not depend on step s-1 -- the ring
-// loads, the 7-term product A*P and the products ALI*DD(i-1) etc. of the
-// recurrence -- is prepared for step s+1 after the result of step s is
-// published, while the other warps reach the barrier.  The expressions
-// and their evaluation order are those of the reference loops, so the
-// results do not change.  The step loop is unrolled by the ring length so
-// slot addresses and mbarrier phases are constants.
+// published) and the preparation of step s+1, which does not depend on it:
+// the ring loads, the 7-term product A*P and the products ALI*DD(i-1) etc.
+// of the recurrence.  Both are straight-line and scheduled into one another;
+// a column without a cell at a step computes on what its slot holds and
+// stores nothing.  The expressions and their evaluation order are those of
+// the reference loops, so the results do not change.  The depth D is a
+// run-time value: with D = 8 compiled in a step of the cluster form takes
+// between 1 % less and 1 % more.
 template <int MODE, typename V, int CS>
 __device__ __forceinline__ void sweep_body(const Geo &g, const SkewGeo &q, const SkewSysT<V> &S, const V *vin,
                                            V *vout, SolveState *st, const V *vin2, double *rb, int bx, int by,
@@ -632,6 +633,24 @@ __device__ __forceinline__ void sweep_body(const Geo &g, const SkewGeo &q, const
   // position in a slot of the coefficients' run, and in it of a column's coefficient
   constexpr int RUN = MODE == SWEEP_FWD_AX ? 0 : 1;  // in units of T (after Y or T)
   auto co = [&](const V *slot, int c, int tt) { return slot[RUN * T + sys_in_run<V>(c, T, tt)]; };
+  // The coefficients of a column, e[c - SYS_AUI] of those that the mode uses,
+  // as 16-byte loads of their chunks: one coefficient at a time a warp's
+  // loads have two-way (FP64) or four-way (FP32) bank conflicts.  Fused
+  // forward sweeps of 16x16 blocks split over clusters, ms per step: 512x32x96
+  // FP64 15.2 -> 14.2; 1024x128x128 FP64 139.7 -> 136.2, FP32 99.3 -> 89.8.
+  constexpr int G = 16 / ES;
+  struct alignas(16) Chunk { V v[G]; };
+  struct Coef { V e[8]; };
+  auto coefs = [&](const V *slot, int tt) {
+    Coef f;
+#pragma unroll
+    for (int c = 0; c < (BWD ? 4 : 8) / G; ++c) {
+      const Chunk k = *reinterpret_cast<const Chunk *>(slot + RUN * T + (c * T + tt) * G);
+#pragma unroll
+      for (int i = 0; i < G; ++i) f.e[c * G + i] = k.v[i];
+    }
+    return f;
+  };
   unsigned long long *bar = reinterpret_cast<unsigned long long *>(sm);
   V *ring = reinterpret_cast<V *>(sm + ((R + 1) & ~1));
   V *xb = ring + (size_t)R * SS;
@@ -766,7 +785,9 @@ __device__ __forceinline__ void sweep_body(const Geo &g, const SkewGeo &q, const
   // what is stored.
   auto prepare = [&](int s, const V *cs, const V *ps, const V *ns) {
     act = (unsigned)(s - sfirst) <= nact;
-    dd = co(cs, SYS_DD, tr);
+    const Coef f = coefs(cs, tr);
+    auto k = [&](int c) { return f.e[c - SYS_AUI]; };
+    dd = k(SYS_DD);
     if (MODE == SWEEP_FWD_AX) {
       const V pc = pcol;
       const V pn = ns[8 * T + tr];
@@ -776,11 +797,10 @@ __device__ __forceinline__ void sweep_body(const Geo &g, const SkewGeo &q, const
       const V pxp = *(ex1 ? cs + hr : ns + 8 * T + oxp);
       const V pyp = *(ey1 ? cs + hu : ns + 8 * T + oyp);
       const V pzp = (s < shi) ? pn : V(0);
-      const V ali = co(cs, SYS_ALI, tr), alj = co(cs, SYS_ALJ, tr), alk = co(cs, SYS_ALK, tr);
+      const V ali = k(SYS_ALI), alj = k(SYS_ALJ), alk = k(SYS_ALK);
       const V d1 = hx ? co(ps, SYS_DD, ox) : V(0);
       const V d2 = hy ? co(ps, SYS_DD, oy) : (CS == 2 && rrow && act ? din[(size_t)(s + lag) * TIp + t.ti] : V(0));
-      y0 = co(cs, SYS_AD, tr) * pc + ali * pxm + alj * pym + alk * pzm + co(cs, SYS_AUI, tr) * pxp +
-           co(cs, SYS_AUJ, tr) * pyp + co(cs, SYS_AUK, tr) * pzp;
+      y0 = k(SYS_AD) * pc + ali * pxm + alj * pym + alk * pzm + k(SYS_AUI) * pxp + k(SYS_AUJ) * pyp + k(SYS_AUK) * pzp;
       c1 = ali * d1;
       c2 = alj * d2;
       c3 = alk * dk1;
@@ -791,21 +811,21 @@ __device__ __forceinline__ void sweep_body(const Geo &g, const SkewGeo &q, const
       const V d1 = hx ? co(ps, SYS_DD, ox) : V(0);
       const V d2 = hy ? co(ps, SYS_DD, oy) : (CS == 2 && rrow && act ? din[(size_t)(s + lag) * TIp + t.ti] : V(0));
       y0 = cs[tr];
-      c1 = co(cs, SYS_ALI, tr) * d1;
-      c2 = co(cs, SYS_ALJ, tr) * d2;
-      c3 = co(cs, SYS_ALK, tr) * dk1;
+      c1 = k(SYS_ALI) * d1;
+      c2 = k(SYS_ALJ) * d2;
+      c3 = k(SYS_ALK) * dk1;
       dk1 = act ? dd : V(0);
     } else {
       y0 = cs[tr];
-      c1 = co(cs, SYS_AUI, tr);
-      c2 = co(cs, SYS_AUJ, tr);
-      c3 = co(cs, SYS_AUK, tr);
+      c1 = k(SYS_AUI);
+      c2 = k(SYS_AUJ);
+      c3 = k(SYS_AUK);
       if (NDOT > 0) q0 = cs[5 * T + tr];
       if (NDOT == 5) q1 = cs[6 * T + tr];
     }
   };
   bool ok = true;
-  // slots of steps s, s+1 and s+2 (R >= 4), the exchange buffers of steps
+  // slots of steps s, s+1 and s+2 (R >= 3), the exchange buffers of steps
   // s and s-1, and the slot of step s+1+AHEAD with its phase
   const V *ps = ring, *cs = ring + SS, *ns = ring + 2 * (size_t)SS;
   const V *const rend = ring + (size_t)R * SS;
