@@ -2059,7 +2059,7 @@ static void solve_mixed_batch(cadmas_batch *b, const std::vector<int> &idx, std:
   pre[BR_ELEM * (nm + 1) + nm] = (int)nelem;
   pre[BR_FLAT * (nm + 1) + nm] = (int)nflat;
   SkewGeo qref = hs[0]->q;
-  for (int j = 0; j < nm; ++j) qref.ring |= hs[j]->q.ring;
+  for (int j = 0; j < nm; ++j) qref.ring |= hs[j]->q.ring | (int)sweep_one_wide(hs[j]->q);
   const BatchMember *bm = b->d_m;
   const int *dp = b->d_pre;
   auto upload = [&]() -> bool {

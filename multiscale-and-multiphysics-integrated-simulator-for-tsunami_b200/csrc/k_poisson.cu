@@ -1691,8 +1691,11 @@ static int sweep_depth(const SkewGeo &q, int mode, int es) {
 }
 // ---- dispatch.  The sweeps run in the thread-copy form (k_sweep_cp); the
 // bulk-copy ring (k_sweep) serves clusters (split 2), tiles one column wide
-// and handles with the stall injection on (SkewGeo::ring), whose subject is
-// the ring's waits.
+// with neighbours (sweep_one_wide) and handles with the stall injection on
+// (SkewGeo::ring), whose subject is the ring's waits.
+static int sweep_form_depth(const SkewGeo &q, int mode, int es) {  // 0: the ring
+  return q.ring || sweep_one_wide(q) ? 0 : sweep_cp_depth(q, mode, es);
+}
 template <int D, int MODE, int MAXT, typename V, int MINB>
 static void sweep_cp_go(cudaStream_t s, const Geo &g, const SkewGeo &q, const SkewSysT<V> &S, const V *vin, V *vout,
                         SolveState *st, const V *vin2, double *rb) {
@@ -1730,7 +1733,7 @@ static void sweep_ring_go(cudaStream_t s, const Geo &g, const SkewGeo &q, const 
 template <int MODE, typename V>
 static void launch_sweep(cudaStream_t s, const Geo &g, const SkewGeo &q, const SkewSysT<V> &S, const V *vin,
                          V *vout, SolveState *st, const V *vin2 = nullptr, double *rb = nullptr) {
-  const int d = q.ring ? 0 : sweep_cp_depth(q, MODE, (int)sizeof(V)), nt = sweep_cp_threads(q.T);
+  const int d = sweep_form_depth(q, MODE, (int)sizeof(V)), nt = sweep_cp_threads(q.T);
 #define CP_GO(D, MT, MB)                                                       \
   {                                                                            \
     sweep_cp_go<D, MODE, MT, V, MB>(s, g, q, S, vin, vout, st, vin2, rb);      \
@@ -1800,7 +1803,7 @@ template <typename V>
 static void launch_fwd_t(cudaStream_t s, const Geo &g, const SkewGeo &q, const SkewSysT<V> &S, const V *y,
                          const V *spmv_x, SolveState *st, V *ybuf) {
   const int es = (int)sizeof(V);
-  if (spmv_x && (q.ring || sweep_cp_depth(q, SWEEP_FWD_AX, es) == 0) && sweep_depth(q, SWEEP_FWD_AX, es) == 0) {
+  if (spmv_x && sweep_form_depth(q, SWEEP_FWD_AX, es) == 0 && sweep_depth(q, SWEEP_FWD_AX, es) == 0) {
     // Ring of the fused sweep too large for this tile: SpMV first.
     launch_spmv_t<V>(s, g, q, S, spmv_x, ybuf, st);
     y = ybuf;
@@ -1974,7 +1977,7 @@ __global__ void __launch_bounds__(MAXT, MINB) kb_sweep(const BatchMember *bm, co
                                           vout >= 0 ? M.vf[vout] : nullptr, M.st, vin2 >= 0 ? M.vf[vin2] : nullptr,
                                           rb5 ? M.rb5 : M.rb0, (int)(lb_ % M.q.ntx), (int)(lb_ / M.q.ntx));
 }
-// the bulk-copy ring: tiles one column wide, or a member with the stall on
+// the bulk-copy ring: a member's tiles are one column wide with neighbours, or its stall is on
 template <int MODE>
 __global__ void __launch_bounds__(512, 1) kb_sweep_ring(const BatchMember *bm, const int *pre, int nm, int vin,
                                                         int vout, int vin2, int rb5, int D) {

@@ -83,6 +83,10 @@ __host__ __device__ inline long long skew_entries(const SkewGeo &q) { return ske
 // which is more where a tile has fewer slabs than that.
 inline long long slab_partials(const SkewGeo &q) { return ((long long)q.nb * q.W + ROWS_PER_BLOCK - 1) / ROWS_PER_BLOCK; }
 inline long long sum_partials(const SkewGeo &q) { return slab_partials(q) > q.nb ? slab_partials(q) : q.nb; }
+// Whether tiles one column wide have neighbours on both sides along that
+// direction, which the thread copies of P (sweep_cp.cuh) cannot serve.  A vertical slice
+// (one row of columns, one tile along y) is not such a grid.
+inline bool sweep_one_wide(const SkewGeo &q) { return (q.TI < 2 && q.ntx > 1) || (q.TJ < 2 && q.nb > q.ntx); }
 // SYS_T of column t
 __host__ __device__ inline long long sys_t(long long slab, int T, int t) { return slab * SYS_N * T + t; }
 // chunk c of column t

@@ -46,9 +46,9 @@ __device__ __forceinline__ void sweep_sums(const double *a, double *rb, int nb, 
 //     visit a cell one step later.  A column on the tile's edge also copies
 //     its neighbour's P from the neighbouring tile, into the slot in which
 //     that neighbour's P would lie if it were a column of this tile.  (At most
-//     one along x and one along y: tiles have at least two columns each way,
-//     and only the last tile of a row, which has no right neighbour, may be
-//     one wide.)
+//     one along x and one along y: tiles have at least two columns each way
+//     unless one tile covers that direction, and only the last tile of a row,
+//     which has no right neighbour, may be one wide.)
 //   * The result of step s and DD of step s+1 are published as one pair.
 //   * One barrier per step; the recurrence of step s and the preparation of
 //     step s+1 are independent and scheduled into one another.
@@ -147,7 +147,7 @@ inline bool sweep_cp_unrolled(const SkewGeo &q, int mode, int es) {
   return sweep_cp_unroll(mode, ct ? q.T : 0, es);
 }
 inline int sweep_cp_depth(const SkewGeo &q, int mode, int es) {
-  if (q.split != 1 || q.TI < 2 || q.TJ < 2) return 0;
+  if (q.split != 1) return 0;
   const int nt = sweep_cp_threads(q.T), blocks = q.occ > 0 ? q.occ : (q.nb > q.nsm ? 2 : 1);
   const bool unr = sweep_cp_unrolled(q, mode, es);
   const int ax[] = {12, 8, 6, 4, 2, 1}, plain[] = {15, 9, 3, 1};

@@ -1,10 +1,11 @@
 // Host check of the sweeps' copy depth (sweep_cp_depth): the rule for two
 // blocks per SM counts the device's SMs, and every depth that the rule gives
-// fits the shared memory it leaves.  Prints the number of failures.
+// fits the shared memory it leaves; and which tiles run the thread copies.  Prints the number of failures.
 #include "cadmas_dev.cuh"
 #include "kernels.h"
 #include "sweep_cp.cuh"
 #include <cstdio>
+#include <vector>
 using namespace cadmas;
 
 static SkewGeo tiles(int TI, int TJ, int ntx, int nty, int nsm, int occ = 0) {
@@ -42,6 +43,25 @@ int main() {
             const SkewGeo q = tiles(t[0], t[1], n, n, 148, occ);
             if (sweep_cp_depth(q, mode, es) > 0) check(bytes(q, mode, es) <= 227 * 1024, "shared memory", q.T, mode);
           }
+  // one row of columns runs the thread copies, tiles one column wide beside
+  // others the ring; the slots of P hold every value of a row once
+  check(!sweep_one_wide(tiles(400, 1, 1, 1, 148)) && !sweep_one_wide(tiles(16, 1, 30, 1, 148)), "slice", 0, 0);
+  check(sweep_one_wide(tiles(16, 1, 1, 2, 148)) && sweep_one_wide(tiles(1, 16, 2, 1, 148)), "one wide", 0, 0);
+  check(!sweep_one_wide(tiles(2, 2, 9, 9, 148)), "two wide", 0, 0);
+  for (int TI : {3, 4, 16, 29, 31, 32, 33, 64, 255, 256, 257, 400, 800}) {
+    const SkewGeo q = tiles(TI, 1, 1, 1, 148);
+    for (int es : {4, 8})
+      for (int mode : {SWEEP_FWD, SWEEP_FWD_AX, SWEEP_BWD}) check(sweep_cp_depth(q, mode, es) > 0, "slice's depth", TI, mode);
+    const SweepP p = sweep_cp_pslot(q.T, q.TIp, TI, 1);
+    std::vector<char> s(p.size, 0);
+    auto put = [&](int e) {
+      check(e >= 0 && e < p.size && !s[e], "slice's P slot", TI, e);
+      if (e >= 0 && e < p.size) s[e] = 1;
+    };
+    for (int t = 0; t < q.T; ++t) put(p.main + t);
+    for (int i = 0; i < TI; ++i) { put(p.down + i); put(p.up + i); }
+    put(p.left); put(p.right); put(p.zero);
+  }
   printf("%lld checks, %lld failures\n", checks, fails);
   return fails != 0;
 }
