@@ -719,14 +719,6 @@ __global__ void k_pack_in(long long V, const float *x4, bf16 *x16) {
   }
   st8(x16 + i * 8, o);
 }
-__global__ void k_f32_to_bf16(long long n, const float *a, bf16 *b) {
-  const long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-  if (i < n) b[i] = __float2bfloat16(a[i]);
-}
-__global__ void k_fill_bf16(long long n, bf16 *a) {
-  const long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-  if (i < n) a[i] = __float2bfloat16(0.0f);
-}
 
 // ------------------------------------------------------------ launchers
 static inline unsigned nb(long long n, int t) { return (unsigned)((n + t - 1) / t); }
@@ -850,14 +842,6 @@ void launch_pack_in(cudaStream_t s, long long V, const float *x4, void *x16) {
 }
 void launch_bias_reduce(cudaStream_t s, const float *part, int n, int C, float *out) {
   k_bias_reduce<<<1, 256, 0, s>>>(part, n, C, out);
-  count_launch();
-}
-void launch_f32_to_bf16(cudaStream_t s, long long n, const float *a, void *b) {
-  k_f32_to_bf16<<<nb(n, 256), 256, 0, s>>>(n, a, (bf16 *)b);
-  count_launch();
-}
-void launch_fill_bf16(cudaStream_t s, long long n, void *a) {
-  k_fill_bf16<<<nb(n, 256), 256, 0, s>>>(n, (bf16 *)a);
   count_launch();
 }
 

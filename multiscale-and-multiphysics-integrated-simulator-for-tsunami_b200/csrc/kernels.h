@@ -454,8 +454,6 @@ void launch_head_bwd(cudaStream_t s, long long V, const float *dy, const void *a
 void launch_adam(cudaStream_t s, long long n, float *p, const float *g, float *m, float *v, float lr, float b1,
                  float b2, float eps, float c1, float c2);
 void launch_wcast(cudaStream_t s, const float *w, int Cin, int Cout, void *wf, void *wt);
-void launch_f32_to_bf16(cudaStream_t s, long long n, const float *a, void *b);
-void launch_fill_bf16(cudaStream_t s, long long n, void *a);
 void launch_pack_in(cudaStream_t s, long long V, const float *x4, void *x16);
 void launch_res_fwd(cudaStream_t s, int X, int Y, int Z, int B, const float *y, const float *a7, const float *x4,
                     const float *m, float c, float *r, float *lpart);
