@@ -1120,6 +1120,7 @@ int cadmas_create(const cadmas_dims *d, const cadmas_params *p, cadmas_handle **
   h->q.nb = h->q.ntx * ((d->numj - 2 + TJl - 1) / TJl);
   h->q.occ = (p->sweep_occupancy == 1 || p->sweep_occupancy == 2 || p->sweep_occupancy == 4) ? p->sweep_occupancy : 0;
   h->q.nsm = sm_count();
+  h->q.one = sweep_one_wide(h->q);
   if (!sweep_supported(h->q)) {
     g_last_error = "preconditioner block too large for the MILU sweeps; set precond_ti/precond_tj";
     rc = CADMAS_EUNSUPPORTED;
@@ -2059,7 +2060,7 @@ static void solve_mixed_batch(cadmas_batch *b, const std::vector<int> &idx, std:
   pre[BR_ELEM * (nm + 1) + nm] = (int)nelem;
   pre[BR_FLAT * (nm + 1) + nm] = (int)nflat;
   SkewGeo qref = hs[0]->q;
-  for (int j = 0; j < nm; ++j) qref.ring |= hs[j]->q.ring | (int)sweep_one_wide(hs[j]->q);
+  for (int j = 0; j < nm; ++j) { qref.ring |= hs[j]->q.ring; qref.one |= hs[j]->q.one; }
   const BatchMember *bm = b->d_m;
   const int *dp = b->d_pre;
   auto upload = [&]() -> bool {

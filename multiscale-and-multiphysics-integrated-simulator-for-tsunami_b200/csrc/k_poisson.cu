@@ -1693,21 +1693,21 @@ static int sweep_depth(const SkewGeo &q, int mode, int es) {
   return 0;
 }
 // ---- dispatch.  The sweeps run in the thread-copy form (k_sweep_cp); the
-// bulk-copy ring (k_sweep) serves clusters (split 2), tiles one column wide
-// with neighbours (sweep_one_wide) and handles with the stall injection on
-// (SkewGeo::ring), whose subject is the ring's waits.
+// bulk-copy ring (k_sweep) serves clusters (split 2), tiles too large for the
+// other and handles with the stall injection on (SkewGeo::ring), whose
+// subject is the ring's waits.
 static int sweep_form_depth(const SkewGeo &q, int mode, int es) {  // 0: the ring
-  return q.ring || sweep_one_wide(q) ? 0 : sweep_cp_depth(q, mode, es);
+  return q.ring ? 0 : sweep_cp_depth(q, mode, es);
 }
-template <int D, int MODE, int MAXT, typename V, int MINB>
+template <int D, int MODE, int MAXT, typename V, int MINB, bool ONE = false>
 static void sweep_cp_go(cudaStream_t s, const Geo &g, const SkewGeo &q, const SkewSysT<V> &S, const V *vin, V *vout,
                         SolveState *st, const V *vin2, double *rb) {
   const size_t bytes = sweep_cp_bytes(MODE, D, sweep_cp_unrolled(q, MODE, (int)sizeof(V)), q.T, q.TIp, q.TI, q.TJ, (int)sizeof(V));
   const dim3 grid((unsigned)q.ntx, (unsigned)(q.nb / q.ntx)), block((unsigned)sweep_cp_threads(q.T));
 #define SWEEP_GO(CT, CI)                                                                                        \
   {                                                                                                             \
-    set_smem(k_sweep_cp<D, MODE, MAXT, V, MINB, CT, CI>, bytes);                                                \
-    launch_pdl(k_sweep_cp<D, MODE, MAXT, V, MINB, CT, CI>, grid, block, bytes, s, 1, g, q, S, vin, vout, st, vin2, rb); \
+    set_smem(k_sweep_cp<D, MODE, MAXT, V, MINB, CT, CI, ONE>, bytes);                                           \
+    launch_pdl(k_sweep_cp<D, MODE, MAXT, V, MINB, CT, CI, ONE>, grid, block, bytes, s, 1, g, q, S, vin, vout, st, vin2, rb); \
     return;                                                                                                     \
   }
   if constexpr (MAXT == 128) {
@@ -1745,6 +1745,23 @@ static void launch_sweep(cudaStream_t s, const Geo &g, const SkewGeo &q, const S
   // two blocks' registers for FP32, whose rings leave room for two blocks
   constexpr int MB = sizeof(V) == 4 ? 2 : 1;
   if constexpr (MODE == SWEEP_FWD_AX) {
+#define CP_ONE(D, MT)                                                          \
+  {                                                                            \
+    sweep_cp_go<D, MODE, MT, V, 1, true>(s, g, q, S, vin, vout, st, vin2, rb); \
+    return;                                                                    \
+  }
+    if (d > 0 && q.one) {
+      if (nt <= 576) {
+        if (d == 8) CP_ONE(8, 576)
+        if (d == 4) CP_ONE(4, 576)
+        CP_ONE(2, 576)
+      }
+      if (d == 8) CP_ONE(8, 1024)
+      if (d == 4) CP_ONE(4, 1024)
+      if (d == 2) CP_ONE(2, 1024)
+      CP_ONE(1, 1024)
+    }
+#undef CP_ONE
     if (d > 0) {
       if (nt <= 128) {
         if (d == 12) CP_GO(12, 128, 1)
@@ -1971,16 +1988,17 @@ __global__ void kb_dcmp_f(const BatchMember *bm, const int *pre, int nm) {
   if (!M.active) return;
   dcmp_body<D, float>(M.g, M.q, (float)M.U, M.Sf, M.pivot_bad, (int)(lb_ % M.q.ntx), (int)(lb_ / M.q.ntx));
 }
-template <int D, int MODE, int MAXT, int MINB, int CT, int CTIP>
+template <int D, int MODE, int MAXT, int MINB, int CT, int CTIP, bool ONE = false>
 __global__ void __launch_bounds__(MAXT, MINB) kb_sweep(const BatchMember *bm, const int *pre, int nm, int vin,
                                                        int vout, int vin2, int rb5) {
   pdl_enter();
   BATCH_BLOCK(BR_TILE)
-  sweep_cp_body<D, MODE, float, CT, CTIP>(M.g, M.q, M.Sf, vin >= 0 ? M.vf[vin] : nullptr,
-                                          vout >= 0 ? M.vf[vout] : nullptr, M.st, vin2 >= 0 ? M.vf[vin2] : nullptr,
-                                          rb5 ? M.rb5 : M.rb0, (int)(lb_ % M.q.ntx), (int)(lb_ / M.q.ntx));
+  sweep_cp_body<D, MODE, float, CT, CTIP, ONE>(M.g, M.q, M.Sf, vin >= 0 ? M.vf[vin] : nullptr,
+                                               vout >= 0 ? M.vf[vout] : nullptr, M.st,
+                                               vin2 >= 0 ? M.vf[vin2] : nullptr, rb5 ? M.rb5 : M.rb0,
+                                               (int)(lb_ % M.q.ntx), (int)(lb_ / M.q.ntx));
 }
-// the bulk-copy ring: a member's tiles are one column wide with neighbours, or its stall is on
+// the bulk-copy ring: a member's stall is on
 template <int MODE>
 __global__ void __launch_bounds__(512, 1) kb_sweep_ring(const BatchMember *bm, const int *pre, int nm, int vin,
                                                         int vout, int vin2, int rb5, int D) {
@@ -2129,12 +2147,13 @@ static bool launch_b_sweep_t(cudaStream_t s, const BatchMember *bm, const int *p
   }
   const size_t bytes = sweep_cp_bytes(MODE, d, sweep_cp_unrolled(q, MODE, 4), q.T, q.TIp, q.TI, q.TJ, 4);
   const dim3 block((unsigned)nt);
-#define BSWEEP(D, MT, MB, CT, CI)                                                                             \
+#define BSWEEP_F(D, MT, MB, CT, CI, ONE)                                                                      \
   {                                                                                                           \
-    set_smem(kb_sweep<D, MODE, MT, MB, CT, CI>, bytes);                                                       \
-    launch_pdl(kb_sweep<D, MODE, MT, MB, CT, CI>, bgrid(ntiles), block, bytes, s, 1, bm, pre, nm, vin, vout, vin2, rb5); \
+    set_smem(kb_sweep<D, MODE, MT, MB, CT, CI, ONE>, bytes);                                                  \
+    launch_pdl(kb_sweep<D, MODE, MT, MB, CT, CI, ONE>, bgrid(ntiles), block, bytes, s, 1, bm, pre, nm, vin, vout, vin2, rb5); \
     return true;                                                                                              \
   }
+#define BSWEEP(D, MT, MB, CT, CI) BSWEEP_F(D, MT, MB, CT, CI, false)
 #define BSWEEP_128(D)                                            \
   {                                                              \
     if (q.T == 128 && q.TIp == 8) BSWEEP(D, 128, 1, 128, 8)      \
@@ -2151,6 +2170,11 @@ static bool launch_b_sweep_t(cudaStream_t s, const BatchMember *bm, const int *p
     BSWEEP(D, 576, 1, 0, 0)                                      \
   }
   if constexpr (MODE == SWEEP_FWD_AX) {
+    if (q.one) {
+      if (d == 8) BSWEEP_F(8, 576, 1, 0, 0, true)
+      if (d == 4) BSWEEP_F(4, 576, 1, 0, 0, true)
+      BSWEEP_F(2, 576, 1, 0, 0, true)
+    }
     if (d == 12) BSWEEP_128(12)
     if (d == 8) BSWEEP_D(8)
     if (d == 6) BSWEEP_D(6)
@@ -2164,6 +2188,7 @@ static bool launch_b_sweep_t(cudaStream_t s, const BatchMember *bm, const int *p
 #undef BSWEEP_D
 #undef BSWEEP_128
 #undef BSWEEP
+#undef BSWEEP_F
 }
 bool launch_b_sweep(cudaStream_t s, int mode, const BatchMember *bm, const int *pre, int nm, long long ntiles,
                     const SkewGeo &q, int vin, int vout, int vin2, bool rb5) {

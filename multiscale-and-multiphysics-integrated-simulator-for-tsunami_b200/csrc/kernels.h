@@ -69,6 +69,7 @@ struct SkewGeo {
   int split;  // layout tiles per preconditioner block along y (1 or 2)
   int nsm;    // the device's SMs
   int occ;    // thread blocks of the sweeps per SM to leave shared memory for (0: one, at full depth)
+  int one;    // 1: tiles one column wide with neighbours on both sides (sweep_one_wide; of a batch, a member's)
   int ring;   // 1: the sweeps' bulk-copy form (the stall injection's subject), 0: by the rule of launch_sweep
 };
 
@@ -84,8 +85,8 @@ __host__ __device__ inline long long skew_entries(const SkewGeo &q) { return ske
 inline long long slab_partials(const SkewGeo &q) { return ((long long)q.nb * q.W + ROWS_PER_BLOCK - 1) / ROWS_PER_BLOCK; }
 inline long long sum_partials(const SkewGeo &q) { return slab_partials(q) > q.nb ? slab_partials(q) : q.nb; }
 // Whether tiles one column wide have neighbours on both sides along that
-// direction, which the thread copies of P (sweep_cp.cuh) cannot serve.  A vertical slice
-// (one row of columns, one tile along y) is not such a grid.
+// direction (SkewGeo::one).  A vertical slice, one row of columns and one tile
+// along y, is not such a grid.
 inline bool sweep_one_wide(const SkewGeo &q) { return (q.TI < 2 && q.ntx > 1) || (q.TJ < 2 && q.nb > q.ntx); }
 // SYS_T of column t
 __host__ __device__ inline long long sys_t(long long slab, int T, int t) { return slab * SYS_N * T + t; }

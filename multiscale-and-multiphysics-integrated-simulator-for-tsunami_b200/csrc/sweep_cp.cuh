@@ -45,10 +45,11 @@ __device__ __forceinline__ void sweep_sums(const double *a, double *rb, int nb, 
 //     of the coefficients', because the neighbours to the right and above
 //     visit a cell one step later.  A column on the tile's edge also copies
 //     its neighbour's P from the neighbouring tile, into the slot in which
-//     that neighbour's P would lie if it were a column of this tile.  (At most
-//     one along x and one along y: tiles have at least two columns each way
-//     unless one tile covers that direction, and only the last tile of a row,
-//     which has no right neighbour, may be one wide.)
+//     that neighbour's P would lie if it were a column of this tile.  At most
+//     one along x and one along y: tiles have at least two columns each way,
+//     or one tile covers that direction, and only the last tile of a row,
+//     which has no right neighbour, may be one wide.  ONE is the form for
+//     tiles one column wide with neighbours on both sides (SkewGeo::one).
 //   * The result of step s and DD of step s+1 are published as one pair.
 //   * One barrier per step; the recurrence of step s and the preparation of
 //     step s+1 are independent and scheduled into one another.
@@ -148,20 +149,21 @@ inline bool sweep_cp_unrolled(const SkewGeo &q, int mode, int es) {
 }
 inline int sweep_cp_depth(const SkewGeo &q, int mode, int es) {
   if (q.split != 1) return 0;
+  const bool one = mode == SWEEP_FWD_AX && q.one;  // built for depths 8, 4, 2 and 1
   const int nt = sweep_cp_threads(q.T), blocks = q.occ > 0 ? q.occ : (q.nb > q.nsm ? 2 : 1);
   const bool unr = sweep_cp_unrolled(q, mode, es);
   const int ax[] = {12, 8, 6, 4, 2, 1}, plain[] = {15, 9, 3, 1};
   for (size_t share : {226 * 1024 / (size_t)blocks, (size_t)(227 * 1024)})
     for (int i = 0; i < (mode == SWEEP_FWD_AX ? 6 : 4); ++i) {
       const int d = mode == SWEEP_FWD_AX ? ax[i] : plain[i];
-      if ((d >= 12 && nt > 128) || (d == 1 && nt <= 576)) continue;
+      if ((d >= 12 && nt > 128) || (d == 1 && nt <= 576) || (one && (d == 12 || d == 6))) continue;
       if (q.occ == 0 && blocks > 1 && share < 227 * 1024 && d < 6) continue;
       if (sweep_cp_bytes(mode, d, unr, q.T, q.TIp, q.TI, q.TJ, es) <= share) return d;
     }
   return 0;
 }
 
-template <int D, int MODE, typename V, int CT, int CTIP>
+template <int D, int MODE, typename V, int CT, int CTIP, bool ONE = false>
 __device__ __forceinline__ void sweep_cp_body(const Geo &g, const SkewGeo &q, const SkewSysT<V> &S, const V *vin,
                                               V *vout, SolveState *st, const V *vin2, double *rb, int bx, int by) {
   constexpr bool BWD = MODE >= SWEEP_BWD, AX = MODE == SWEEP_FWD_AX;
@@ -218,18 +220,23 @@ __device__ __forceinline__ void sweep_cp_body(const Geo &g, const SkewGeo &q, co
   // lower) and after (right, upper)
   const bool hl = AX && col && ti == 0 && bx > 0, hr = AX && col && ti == wi - 1 && bx < q.ntx - 1;
   const bool hd = AX && col && tj == 0 && by > 0, hu = AX && col && tj == wj - 1 && by < nty - 1;
-  const int ehx = (hr ? po.right : po.left) + po.xs * min(tj, TJ - 1), ehy = (hu ? po.up : po.down) + min(ti, TI - 1);
+  const int el = po.left + po.xs * min(tj, TJ - 1), er = po.right + po.xs * min(tj, TJ - 1);
+  const int ed = po.down + min(ti, TI - 1), eu = po.up + min(ti, TI - 1);
+  const int ehx = hr ? er : el, ehy = hu ? eu : ed;
   const int tp = po.main + tq;
-  const int oxm = hl ? ehx : ((col && ti > 0) ? tp - 1 : po.zero), oxp = hr ? ehx : ((col && ti < wi - 1) ? tp + 1 : po.zero);
-  const int oym = hd ? ehy : ((col && tj > 0) ? tp - TIp : po.zero), oyp = hu ? ehy : ((col && tj < wj - 1) ? tp + TIp : po.zero);
+  const int oxm = hl ? el : ((col && ti > 0) ? tp - 1 : po.zero), oxp = hr ? er : ((col && ti < wi - 1) ? tp + 1 : po.zero);
+  const int oym = hd ? ed : ((col && tj > 0) ? tp - TIp : po.zero), oyp = hu ? eu : ((col && tj < wj - 1) ? tp + TIp : po.zero);
   const int shx = hr ? -1 : 1, shy = hu ? -1 : 1;  // own step minus the neighbour's
   const bool hx = hl || hr, hy = hd || hu;
   const V *lx = vin, *ly = vin;                    // halo values for P slot 0
+  const V *lr = vin, *lu = vin;                    // ONE: the right and upper ones (lx, ly the left and lower)
+  const long long hrofs = AX ? ((long long)(b + 1) * WS - TI) * T + TIp * tj : 0,
+                  huofs = AX ? ((long long)(b + q.ntx) * WS - TJ) * T + ti : 0;
   if (AX) {  // own step u: the neighbour's cell of the same layer; slot v = u - shx
     if (hl) lx = vin + ((long long)(b - 1) * WS + TI) * T + (TI - 1) + TIp * tj;
-    if (hr) lx = vin + ((long long)(b + 1) * WS - TI) * T + TIp * tj;
+    if (hr) (ONE ? lr : lx) = vin + hrofs;
     if (hd) ly = vin + ((long long)(b - q.ntx) * WS + TJ) * T + ti + TIp * (TJ - 1);
-    if (hu) ly = vin + ((long long)(b + q.ntx) * WS - TJ) * T + ti;
+    if (hu) (ONE ? lu : ly) = vin + huofs;
   }
   V *vp = BWD ? vout + slab0 * T + tq : S.sys + sys_t(slab0, T, tq);
   auto active = [&](int u) { return (unsigned)(u - slo) <= nact; };
@@ -250,6 +257,13 @@ __device__ __forceinline__ void sweep_cp_body(const Geo &g, const SkewGeo &q, co
   // P of step v and the halo columns of slot v into the slot at byte offset so
   auto loadp = [&](int v, unsigned so, int r) {
     if (active(v)) cpa<ES>(pb0 + so + (unsigned)(tp * ES), l0 + r * vstep);
+    if constexpr (ONE) {
+      if (hl && active(v + 1)) cpa<ES>(pb0 + so + (unsigned)(el * ES), lx + r * vstep);
+      if (hr && active(v - 1)) cpa<ES>(pb0 + so + (unsigned)(er * ES), lr + r * vstep);
+      if (hd && active(v + 1)) cpa<ES>(pb0 + so + (unsigned)(ed * ES), ly + r * vstep);
+      if (hu && active(v - 1)) cpa<ES>(pb0 + so + (unsigned)(eu * ES), lu + r * vstep);
+      return;
+    }
     if (hx && active(v + shx)) cpa<ES>(pb0 + so + (unsigned)(ehx * ES), lx + r * vstep);
     if (hy && active(v + shy)) cpa<ES>(pb0 + so + (unsigned)(ehy * ES), ly + r * vstep);
   };
@@ -263,6 +277,10 @@ __device__ __forceinline__ void sweep_cp_body(const Geo &g, const SkewGeo &q, co
     l0 += n * vstep;
     lx += n * vstep;
     ly += n * vstep;
+    if (ONE) {
+      lr += n * vstep;
+      lu += n * vstep;
+    }
   };
 
   V dd = V(0), y0 = V(0), c1 = V(0), c2 = V(0), c3 = V(0);  // prepared values of the step
@@ -462,11 +480,11 @@ __device__ __forceinline__ void sweep_cp_body(const Geo &g, const SkewGeo &q, co
     sweep_sums<NDOT>(a, rb, q.nb, b);
   }
 }
-template <int D, int MODE, int MAXT, typename V, int MINB, int CT, int CTIP>
+template <int D, int MODE, int MAXT, typename V, int MINB, int CT, int CTIP, bool ONE = false>
 __global__ void __launch_bounds__(MAXT, MINB)
     k_sweep_cp(Geo g, SkewGeo q, SkewSysT<V> S, const V *vin, V *vout, SolveState *st, const V *vin2, double *rb) {
   pdl_enter();
-  sweep_cp_body<D, MODE, V, CT, CTIP>(g, q, S, vin, vout, st, vin2, rb, (int)blockIdx.x, (int)blockIdx.y);
+  sweep_cp_body<D, MODE, V, CT, CTIP, ONE>(g, q, S, vin, vout, st, vin2, rb, (int)blockIdx.x, (int)blockIdx.y);
 }
 
 }  // namespace cadmas

@@ -12,6 +12,7 @@ static SkewGeo tiles(int TI, int TJ, int ntx, int nty, int nsm, int occ = 0) {
   SkewGeo q{};
   q.TI = TI; q.TJ = TJ; q.TIp = (TI + 3) & ~3; q.T = q.TIp * TJ; q.W = 126 + (TI - 1) + (TJ - 1);
   q.ntx = ntx; q.nb = ntx * nty; q.split = 1; q.nsm = nsm; q.occ = occ;
+  q.one = sweep_one_wide(q);
   return q;
 }
 static size_t bytes(const SkewGeo &q, int mode, int es) {
@@ -43,25 +44,36 @@ int main() {
             const SkewGeo q = tiles(t[0], t[1], n, n, 148, occ);
             if (sweep_cp_depth(q, mode, es) > 0) check(bytes(q, mode, es) <= 227 * 1024, "shared memory", q.T, mode);
           }
-  // one row of columns runs the thread copies, tiles one column wide beside
-  // others the ring; the slots of P hold every value of a row once
+  // tiles one column wide beside others are told from slices and from the rest
   check(!sweep_one_wide(tiles(400, 1, 1, 1, 148)) && !sweep_one_wide(tiles(16, 1, 30, 1, 148)), "slice", 0, 0);
   check(sweep_one_wide(tiles(16, 1, 1, 2, 148)) && sweep_one_wide(tiles(1, 16, 2, 1, 148)), "one wide", 0, 0);
   check(!sweep_one_wide(tiles(2, 2, 9, 9, 148)), "two wide", 0, 0);
-  for (int TI : {3, 4, 16, 29, 31, 32, 33, 64, 255, 256, 257, 400, 800}) {
-    const SkewGeo q = tiles(TI, 1, 1, 1, 148);
-    for (int es : {4, 8})
-      for (int mode : {SWEEP_FWD, SWEEP_FWD_AX, SWEEP_BWD}) check(sweep_cp_depth(q, mode, es) > 0, "slice's depth", TI, mode);
-    const SweepP p = sweep_cp_pslot(q.T, q.TIp, TI, 1);
-    std::vector<char> s(p.size, 0);
-    auto put = [&](int e) {
-      check(e >= 0 && e < p.size && !s[e], "slice's P slot", TI, e);
-      if (e >= 0 && e < p.size) s[e] = 1;
-    };
-    for (int t = 0; t < q.T; ++t) put(p.main + t);
-    for (int i = 0; i < TI; ++i) { put(p.down + i); put(p.up + i); }
-    put(p.left); put(p.right); put(p.zero);
-  }
+  // tiles one column wide along either direction, slices and others: a depth
+  // for every mode, among those that are built; every value has its own entry
+  // in a slot of P
+  for (int n : {1, 2, 3, 4, 16, 29, 31, 32, 33, 64, 200, 255, 256, 257, 400, 800})
+    for (int along = 0; along < 2; ++along)
+      for (int nb : {1, 3}) {
+        const int TI = along ? 1 : n, TJ = along ? n : 1;
+        const SkewGeo q = tiles(TI, TJ, along ? nb : 1, along ? 1 : nb, 148);
+        if (q.T > 800) continue;
+        for (int es : {4, 8})
+          for (int mode : {SWEEP_FWD, SWEEP_FWD_AX, SWEEP_BWD}) {
+            const int d = sweep_cp_depth(q, mode, es);
+            check(d > 0, "depth of a one-wide tile", q.T, mode);
+            if (mode == SWEEP_FWD_AX && q.one) check(d == 8 || d == 4 || d == 2 || (d == 1 && q.T > 576), "built", q.T, d);
+          }
+        const SweepP p = sweep_cp_pslot(q.T, q.TIp, TI, TJ);
+        std::vector<char> s(p.size, 0);
+        auto put = [&](int e) {
+          check(e >= 0 && e < p.size && !s[e], "P slot of a one-wide tile", q.T, e);
+          if (e >= 0 && e < p.size) s[e] = 1;
+        };
+        for (int t = 0; t < q.T; ++t) put(p.main + t);
+        for (int i = 0; i < TI; ++i) { put(p.down + i); put(p.up + i); }
+        for (int j = 0; j < TJ; ++j) { put(p.left + p.xs * j); put(p.right + p.xs * j); }
+        put(p.zero);
+      }
   printf("%lld checks, %lld failures\n", checks, fails);
   return fails != 0;
 }
