@@ -1751,15 +1751,9 @@ static void launch_sweep(cudaStream_t s, const Geo &g, const SkewGeo &q, const S
     return;                                                                    \
   }
     if (d > 0 && q.one) {
-      if (nt <= 576) {
-        if (d == 8) CP_ONE(8, 576)
-        if (d == 4) CP_ONE(4, 576)
-        CP_ONE(2, 576)
-      }
-      if (d == 8) CP_ONE(8, 1024)
-      if (d == 4) CP_ONE(4, 1024)
-      if (d == 2) CP_ONE(2, 1024)
-      CP_ONE(1, 1024)
+      if (d == 8) CP_ONE(8, 576)
+      if (d == 4) CP_ONE(4, 576)
+      CP_ONE(2, 576)
     }
 #undef CP_ONE
     if (d > 0) {
@@ -1779,7 +1773,7 @@ static void launch_sweep(cudaStream_t s, const Geo &g, const SkewGeo &q, const S
         if (d == 6) CP_GO(6, 576, 1)
         if (d == 4) CP_GO(4, 576, 1)
         CP_GO(2, 576, 1)
-      } else {
+      } else if constexpr (sizeof(V) == 4) {  // (FP64: never, sweep_cp_depth)
         if (d == 8) CP_GO(8, 1024, 1)
         if (d == 6) CP_GO(6, 1024, 1)
         if (d == 4) CP_GO(4, 1024, 1)
@@ -1823,8 +1817,9 @@ template <typename V>
 static void launch_fwd_t(cudaStream_t s, const Geo &g, const SkewGeo &q, const SkewSysT<V> &S, const V *y,
                          const V *spmv_x, SolveState *st, V *ybuf) {
   const int es = (int)sizeof(V);
-  if (spmv_x && sweep_form_depth(q, SWEEP_FWD_AX, es) == 0 && sweep_depth(q, SWEEP_FWD_AX, es) == 0) {
-    // Ring of the fused sweep too large for this tile: SpMV first.
+  const bool ring = q.ring || q.split == 2;
+  if (spmv_x && (ring ? sweep_depth(q, SWEEP_FWD_AX, es) : sweep_cp_depth(q, SWEEP_FWD_AX, es)) == 0) {
+    // No fused sweep for this tile: SpMV first.
     launch_spmv_t<V>(s, g, q, S, spmv_x, ybuf, st);
     y = ybuf;
     spmv_x = nullptr;

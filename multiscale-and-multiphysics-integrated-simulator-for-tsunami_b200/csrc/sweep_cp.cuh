@@ -142,6 +142,12 @@ __host__ __device__ inline size_t sweep_cp_bytes(int mode, int D, bool unrolled,
 // system comes from memory, 19.6 at 7).  512 tiles of 16x16 x 126 layers: FP64
 // fused, one block at depth 8 242, at 6 250, two at 4 255; FP32 fused, two at
 // depth 6 132, one 143; backward FP64 at depth 7, one block 139, two 141.
+// Tiles of more than 576 columns have 64 registers a thread and room for two
+// steps (FP64) in the fused sweep: A P on its own before the plain sweep takes
+// less, except in FP32 with few edge columns (0: no fused sweep).  Forward
+// stage, ms a step, fused and apart: FP64 32x20 18.5, 15.4; 32x25 26.9, 18.3;
+// 128x6 38.0, 20.6; 400x2 47.5, 21.6; 24x24 12.6, 14.9 (576 columns); FP32
+// 32x20 16.5, 18.7; 32x25 20.2, 21.5; 100x6 18.2, 16.3; 400x2 41.0, 24.3.
 inline int sweep_cp_threads(int T) { return (T + 31) & ~31; }
 inline bool sweep_cp_unrolled(const SkewGeo &q, int mode, int es) {
   const bool ct = (q.T == 128 && (q.TIp == 8 || q.TIp == 16)) || (q.T == 256 && q.TIp == 16);
@@ -149,8 +155,9 @@ inline bool sweep_cp_unrolled(const SkewGeo &q, int mode, int es) {
 }
 inline int sweep_cp_depth(const SkewGeo &q, int mode, int es) {
   if (q.split != 1) return 0;
-  const bool one = mode == SWEEP_FWD_AX && q.one;  // built for depths 8, 4, 2 and 1
+  const bool one = mode == SWEEP_FWD_AX && q.one;  // built for depths 8, 4 and 2
   const int nt = sweep_cp_threads(q.T), blocks = q.occ > 0 ? q.occ : (q.nb > q.nsm ? 2 : 1);
+  if (mode == SWEEP_FWD_AX && nt > 576 && (es == 8 || q.TI < 16 || q.TJ < 16)) return 0;
   const bool unr = sweep_cp_unrolled(q, mode, es);
   const int ax[] = {12, 8, 6, 4, 2, 1}, plain[] = {15, 9, 3, 1};
   for (size_t share : {226 * 1024 / (size_t)blocks, (size_t)(227 * 1024)})

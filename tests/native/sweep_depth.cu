@@ -60,8 +60,8 @@ int main() {
         for (int es : {4, 8})
           for (int mode : {SWEEP_FWD, SWEEP_FWD_AX, SWEEP_BWD}) {
             const int d = sweep_cp_depth(q, mode, es);
-            check(d > 0, "depth of a one-wide tile", q.T, mode);
-            if (mode == SWEEP_FWD_AX && q.one) check(d == 8 || d == 4 || d == 2 || (d == 1 && q.T > 576), "built", q.T, d);
+            check((d > 0) == (mode != SWEEP_FWD_AX || q.T <= 576), "depth of a one-wide tile", q.T, mode);
+            if (mode == SWEEP_FWD_AX && q.one && d > 0) check(d == 8 || d == 4 || d == 2, "built", q.T, d);
           }
         const SweepP p = sweep_cp_pslot(q.T, q.TIp, TI, TJ);
         std::vector<char> s(p.size, 0);
@@ -74,6 +74,11 @@ int main() {
         for (int j = 0; j < TJ; ++j) { put(p.left + p.xs * j); put(p.right + p.xs * j); }
         put(p.zero);
       }
+  // more than 576 columns: no fused FP64 sweep, an FP32 one for square tiles
+  check(sweep_cp_depth(tiles(24, 24, 4, 4, 148), SWEEP_FWD_AX, 8) == 2, "576 columns", 0, 0);
+  check(sweep_cp_depth(tiles(32, 20, 4, 4, 148), SWEEP_FWD_AX, 8) == 0, "640 columns, FP64", 0, 0);
+  check(sweep_cp_depth(tiles(32, 20, 4, 4, 148), SWEEP_FWD_AX, 4) == 8, "640 columns, FP32", 0, 0);
+  check(sweep_cp_depth(tiles(128, 5, 4, 4, 148), SWEEP_FWD_AX, 4) == 0, "640 flat columns, FP32", 0, 0);
   printf("%lld checks, %lld failures\n", checks, fails);
   return fails != 0;
 }
