@@ -1131,6 +1131,12 @@ __global__ void __launch_bounds__(256) k_copy2(SkewGeo q, const V *R0, V *RR, V 
   copy2_body<V>(q, R0, RR, PP, st, blockIdx.x);
 }
 
+// Whether a value's bits change.  The FP64 updates store only those: what is
+// not computed (air, obstacles) stays 0.  Updates of a step on 1024x128x128
+// cells, 16x16 blocks: 1 % water 19.9 -> 14.7 ms, the solitary beach 38.9 ->
+// 31.8 ms.
+__device__ __forceinline__ bool changed(double a, double b) { return __double_as_longlong(a) != __double_as_longlong(b); }
+
 // RR = RR - ALPHA*AP (vf_m1bcgs.f:181-189)
 __global__ void __launch_bounds__(256) k_axpy_rr(SkewGeo q, const double *AP, double *RR, const SolveState *st) {
   pdl_enter();
@@ -1143,9 +1149,8 @@ __global__ void __launch_bounds__(256) k_axpy_rr(SkewGeo q, const double *AP, do
   double2 r[4], a[4];
   EACH(4) { r[u] = rr[e[u]]; a[u] = ap[e[u]]; }
   EACH(4) {
-    r[u].x = r[u].x - alpha * a[u].x;
-    r[u].y = r[u].y - alpha * a[u].y;
-    rr[e[u]] = r[u];
+    const double2 n = make_double2(r[u].x - alpha * a[u].x, r[u].y - alpha * a[u].y);
+    if (changed(n.x, r[u].x) || changed(n.y, r[u].y)) rr[e[u]] = n;
   }
   FLAT_LOOP_END
 }
@@ -1167,11 +1172,14 @@ __global__ void k_upd_xr(Geo g, SkewGeo q, const double *PP, const double *AE, c
 #pragma unroll
     for (int u = 0; u < 4; ++u) xw[u] = pp[u] = rr[u] = ae[u] = r0[u] = 0.0;
     EACH(4) { xw[u] = XW[e + 32 * u]; pp[u] = PP[e + 32 * u]; rr[u] = RR[e + 32 * u]; ae[u] = AE[e + 32 * u]; r0[u] = R0[e + 32 * u]; }
-    EACH(4) XW[e + 32 * u] = xw[u] + (alpha * pp[u] + omega * rr[u]);
+    EACH(4) {
+      const double x = xw[u] + (alpha * pp[u] + omega * rr[u]);
+      if (changed(x, xw[u])) XW[e + 32 * u] = x;
+    }
 #pragma unroll
     for (int u = 0; u < 4; ++u) {
       const double r = in[u] ? rr[u] - omega * ae[u] : 0.0;
-      if (in[u]) RR[e + 32 * u] = r;
+      if (in[u] && changed(r, rr[u])) RR[e + 32 * u] = r;
       s0 = s0 + r * r;
       s1 = s1 + r0[u] * r;
     }
@@ -1194,9 +1202,8 @@ __global__ void __launch_bounds__(256) k_upd_p(SkewGeo q, const double *RR, cons
   double2 r[4], a[4], p[4];
   EACH(4) { r[u] = rr[e[u]]; a[u] = ap[e[u]]; p[u] = pp[e[u]]; }
   EACH(4) {
-    p[u].x = r[u].x + beta * (p[u].x - omega * a[u].x);
-    p[u].y = r[u].y + beta * (p[u].y - omega * a[u].y);
-    pp[e[u]] = p[u];
+    const double2 n = make_double2(r[u].x + beta * (p[u].x - omega * a[u].x), r[u].y + beta * (p[u].y - omega * a[u].y));
+    if (changed(n.x, p[u].x) || changed(n.y, p[u].y)) pp[e[u]] = n;
   }
   FLAT_LOOP_END
 }
