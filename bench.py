@@ -62,11 +62,10 @@ STAGE_BYTES = {
 
 
 # DRAM bytes (dram__bytes_read.sum + dram__bytes_write.sum) per interior
-# cell of one launch of each stage's dominant kernel, from ncu captures of
-# the 256x32x96 flume with 16x16 and 8x16 blocks (the same sweep variants
-# as the bench's 512x32x96, one block per SM), so the traffic per launch
-# scales with the cells.
-NCU_TRAFFIC_PER_CELL = {(16, 16): {"fwd": 72.6, "bwd": 40.2}, (8, 16): {"fwd": 72.3, "bwd": 40.1}}
+# cell of one launch of each stage's dominant kernel, from an ncu capture of
+# the 512x32x96 flume itself with 16x16 and 8x16 blocks.  What a launch
+# writes (8 B per cell) mostly stays in L2 past its end.
+NCU_TRAFFIC_PER_CELL = {(16, 16): {"fwd": 79.7, "bwd": 40.6}, (8, 16): {"fwd": 79.3, "bwd": 40.5}}
 
 
 def _load_pkg():
